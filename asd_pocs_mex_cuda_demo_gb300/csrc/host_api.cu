@@ -507,30 +507,28 @@ static int tv_host(const T *img, T *out, int nx, int ny, int nz, double alpha,
   if (!img || !out) return set_error(ASDPOCS_ERR_ARG, "null pointer");
   if (int e = check_tv_dims(nx, ny, nz)) return e;
   const size_t N = (size_t)nx * ny * nz;
-  const size_t tiles = (size_t)((nx + 31) / 32) * ((ny + 7) / 8) * nz;
   const size_t oI = 0, oO = align256(N * sizeof(T)), oA = oO + align256(N * sizeof(T)),
                oB = oA + align256(N * sizeof(T)), oS = oB + align256(N * sizeof(T)),
-               oP = oS + 256, oC = oP + align256(tiles * sizeof(double) * 3),
-               tot = oC + 256;
+               oP = oS + 256, tot = oP + align256(tv_partials_bytes());
   Workspace *w;
   if (int e = ws_acquire(w, tot)) return e;
   std::lock_guard<std::mutex> lk(w->mu);
   char *b = (char *)w->buf;
-  ASD_CUDA(cudaMemsetAsync(b + oC, 0, 256, w->st));
   ASD_CUDA(cudaMemcpyAsync(b + oI, img, N * sizeof(T), cudaMemcpyHostToDevice, w->st));
   if (old)
     ASD_CUDA(cudaMemcpyAsync(b + oO, old, N * sizeof(T), cudaMemcpyHostToDevice, w->st));
   cudaError_t e;
-  if (sizeof(T) == 8)
+  // the old image's buffer is also the third work image
+  if constexpr (sizeof(T) == 8)
     e = tv_minimize_f64((double *)(b + oI), old ? (const double *)(b + oO) : nullptr,
-                        (double *)(b + oA), (double *)(b + oB), (double *)(b + oS),
-                        (double *)(b + oP), (unsigned *)(b + oC), nx, ny, nz, alpha,
-                        n, pos, w->st);
+                        (double *)(b + oA), (double *)(b + oB), (double *)(b + oO),
+                        (double *)(b + oS), (double *)(b + oP), nx, ny, nz, alpha, n, pos,
+                        w->st, true);
   else
     e = tv_minimize_f32((float *)(b + oI), old ? (const float *)(b + oO) : nullptr,
-                        (float *)(b + oA), (float *)(b + oB), (double *)(b + oS),
-                        (double *)(b + oP), (unsigned *)(b + oC), nx, ny, nz, alpha,
-                        n, pos, w->st);
+                        (float *)(b + oA), (float *)(b + oB), (float *)(b + oO),
+                        (double *)(b + oS), (double *)(b + oP), nx, ny, nz, alpha, n, pos,
+                        w->st, true);
   ASD_CUDA(e);
   ASD_CUDA(cudaMemcpyAsync(out, b + oI, N * sizeof(T), cudaMemcpyDeviceToHost, w->st));
   ASD_CUDA(cudaStreamSynchronize(w->st));
@@ -566,20 +564,16 @@ int asdpocs_tv_device(float *img_d, const float *img_old_d, int nx, int ny,
   if (!img_d) return set_error(ASDPOCS_ERR_ARG, "null pointer");
   if (int e = check_tv_dims(nx, ny, nz)) return e;
   const size_t N = (size_t)nx * ny * nz;
-  const size_t tiles = (size_t)((nx + 31) / 32) * ((ny + 7) / 8) * nz;
-  const size_t oA = 0, oB = align256(N * 4), oS = oB + align256(N * 4),
-               oP = oS + 256, oC = oP + align256(tiles * sizeof(double) * 3),
-               tot = oC + 256;
+  const size_t oA = 0, oB = align256(N * 4), oD = oB + align256(N * 4), oS = oD + align256(N * 4),
+               oP = oS + 256, tot = oP + align256(tv_partials_bytes());
   Workspace *w;
   if (int e = ws_acquire(w, tot)) return e;
   std::lock_guard<std::mutex> lk(w->mu);
   char *b = (char *)w->buf;
   cudaStream_t st = (cudaStream_t)stream;
-  ASD_CUDA(cudaMemsetAsync(b + oC, 0, 256, st));
   ASD_CUDA(tv_minimize_f32(img_d, img_old_d, (float *)(b + oA), (float *)(b + oB),
-                           (double *)(b + oS), (double *)(b + oP),
-                           (unsigned *)(b + oC), nx, ny, nz, alpha, nTVIter, pos,
-                           st));
+                           (float *)(b + oD), (double *)(b + oS), (double *)(b + oP), nx, ny,
+                           nz, alpha, nTVIter, pos, st, true));
   // the workspace is reused by the next call: finish before releasing it
   ASD_CUDA(cudaStreamSynchronize(st));
   return 0;

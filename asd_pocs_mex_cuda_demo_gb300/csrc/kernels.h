@@ -59,15 +59,21 @@ cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
                             const int *zmap = nullptr);
 
 // ---- TV and scalars (kernels_tv.cu) ----
-// FP64 / FP32 TV minimisation on device buffers (reference semantics).
-cudaError_t tv_minimize_f64(double *img, const double *img_old, double *work_a,
-                            double *work_b, double *scal, double *partials,
-                            unsigned *counter, int nx, int ny, int nz,
-                            double alpha, int n_iter, int pos, cudaStream_t st);
-cudaError_t tv_minimize_f32(float *img, const float *img_old, float *work_a,
-                            float *work_b, double *scal, double *partials,
-                            unsigned *counter, int nx, int ny, int nz,
-                            double alpha, int n_iter, int pos, cudaStream_t st);
+// FP64 / FP32 TV minimisation on device buffers (reference semantics), in
+// place on img.  work_a, work_b, work_c: three images of scratch; work_c may
+// be img_old itself (which is read before work_c is written) or null, and
+// then only work_a is used, at two kernels a step.  scal: 1 double, partials:
+// tv_partials_bytes().  pdl: programmatic dependent launches (not for streams
+// that a caller may be capturing).
+size_t tv_partials_bytes();
+cudaError_t tv_minimize_f64(double *img, const double *img_old, double *work_a, double *work_b,
+                            double *work_c, double *scal, double *partials, int nx, int ny,
+                            int nz, double alpha, int n_iter, int pos, cudaStream_t st,
+                            bool pdl);
+cudaError_t tv_minimize_f32(float *img, const float *img_old, float *work_a, float *work_b,
+                            float *work_c, double *scal, double *partials, int nx, int ny,
+                            int nz, double alpha, int n_iter, int pos, cudaStream_t st,
+                            bool pdl);
 
 // Per-iteration ASD-POCS steps for a batch (ASD_POCS_cuda.m:137-170).
 cudaError_t launch_iter_begin(const Inst *insts, int batch, cudaStream_t st);

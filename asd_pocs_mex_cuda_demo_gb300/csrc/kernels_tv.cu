@@ -13,6 +13,7 @@
 // registers and the slices staged in shared memory (k_tv_walk3d).  The
 // end-of-sweep kernel provides ||v|| of the first step; the last step also
 // applies the positivity constraint and the alpha/beta step control.
+#include <algorithm>
 #include <type_traits>
 #include "kernels.h"
 #include "reduce.cuh"
@@ -23,13 +24,6 @@ namespace {
 
 constexpr int kThreads = kTileThreads;
 
-// num / sqrt(den): exact operations in FP64 (the mex-level entry points);
-// the hardware reciprocal square root in FP32 (the device-resident path,
-// within a few ulp of the FP64 stencil's value).
-__device__ __forceinline__ double tv_q(double num, double den) {
-  return num / sqrt(den);
-}
-
 template <class T>
 __device__ __forceinline__ T tv_eps();
 template <>
@@ -39,26 +33,6 @@ __device__ __forceinline__ double tv_eps<double>() {
 template <>
 __device__ __forceinline__ float tv_eps<float>() {
   return 1e-8f;
-}
-
-template <class T>
-__device__ __forceinline__ T sqr(T v) {
-  return v * v;
-}
-
-// imgTVGradMin.cpp:84-97; u(dx, dy, dz) reads the image at an offset from
-// the voxel (zero outside the image).  x = row index r (fastest).
-template <class T, class U>
-__device__ __forceinline__ T tv_grad2(const U &u) {
-  const T eps = tv_eps<T>();
-  const T c0 = u(0, 0, 0);
-  const T xm = u(-1, 0, 0), ym = u(0, -1, 0);
-  const T xp = u(1, 0, 0), yp = u(0, 1, 0);
-  const T xpym = u(1, -1, 0), xmyp = u(-1, 1, 0);
-  const T g1 = tv_q((c0 - xm) + (c0 - ym), eps + sqr(c0 - xm) + sqr(c0 - ym));
-  const T g2 = tv_q(-(xp - c0), eps + sqr(xp - c0) + sqr(xp - xpym));
-  const T g3 = tv_q(-(yp - c0), eps + sqr(yp - c0) + sqr(yp - xmyp));
-  return g1 + g2 + g3;
 }
 
 // FP32 form of the 2-D stencil with every rounding explicit, so that a
@@ -100,27 +74,6 @@ __device__ __forceinline__ float tv_grad2f(const U &u) {
   return tv2_combine(here.g1, right.q, below.t);
 }
 
-// imgTVGradMin3D.cpp:114-140 (image index x + y*Nx + z*Nx*Ny).
-template <class T, class U>
-__device__ __forceinline__ T tv_grad3(const U &u) {
-  const T eps = tv_eps<T>();
-  const T c0 = u(0, 0, 0);
-  const T xm = u(-1, 0, 0), ym = u(0, -1, 0), zm = u(0, 0, -1);
-  const T xp = u(1, 0, 0), yp = u(0, 1, 0), zp = u(0, 0, 1);
-  const T xm_zp = u(-1, 0, 1), ym_zp = u(0, -1, 1);
-  const T xm_yp = u(-1, 1, 0), yp_zm = u(0, 1, -1);
-  const T xp_ym = u(1, -1, 0), xp_zm = u(1, 0, -1);
-  const T g1 = tv_q(T(6) * c0 - T(2) * (xm + ym + zm),
-                    eps + sqr(c0 - xm) + sqr(c0 - ym) + sqr(c0 - zm));
-  const T g2 = tv_q(T(2) * c0 - T(2) * zp,
-                    eps + sqr(zp - xm_zp) + sqr(zp - ym_zp) + sqr(zp - c0));
-  const T g3 = tv_q(T(2) * c0 - T(2) * yp,
-                    eps + sqr(yp - xm_yp) + sqr(yp - c0) + sqr(yp - yp_zm));
-  const T g4 = tv_q(T(2) * c0 - T(2) * xp,
-                    eps + sqr(xp - c0) + sqr(xp - xp_ym) + sqr(xp - xp_zm));
-  return g1 + g2 + g3 + g4;
-}
-
 // FP32 form of the 3-D stencil with every rounding explicit.  At a voxel
 // with differences dx, dy, dz to its -x, -y, -z neighbours,
 //   r = 1/sqrt(eps + dx^2 + dy^2 + dz^2),
@@ -159,143 +112,355 @@ __device__ __forceinline__ float tv_grad3f(const U &u) {
   return __fmul_rn(2.f, tv3_u(tv3_inslice(c, xm, ym, zm, xp, yp, r, rx, ry), c, zp, rz));
 }
 
-template <class T, class U>
-__device__ __forceinline__ T tv_grad(const U &u, bool is3d) {
-  if (is3d) {
-    if constexpr (std::is_same<T, float>::value)
-      return tv_grad3f(u);
-    else
-      return tv_grad3<T>(u);
-  }
-  if constexpr (std::is_same<T, float>::value)
-    return tv_grad2f(u);
+template <bool k3D, class U>
+__device__ __forceinline__ float tv_grad_f(const U &u) {
+  if constexpr (k3D)
+    return tv_grad3f(u);
   else
-    return tv_grad2<T>(u);
+    return tv_grad2f(u);
 }
 
-// Global-memory accessor with zero padding (standalone entry points).
+// ------------------------------------- standalone TV (the TV entry points)
+// One kernel per TV step on plain buffers, FP64 (the mex functions) or FP32
+// (the device entry points).  A step needs ||v|| of its image before it can
+// update, so a step's kernel updates with the stencil that the kernel before
+// it left in memory and then evaluates the stencil of the updated image, for
+// the next step:
+//   m' = m - coef u(m)  (tile and halo),  u(m') and its block sums of squares,
+// with u = v in 2-D and v / 2 in 3-D (all four 3-D terms carry a factor 2,
+// which cancels in alpha d v / ||v||).  Storing u costs 2 accesses per voxel
+// and step and saves evaluating the stencil twice: the FP64 rate bounds the
+// mex functions, and one stencil there is one reciprocal square root and
+// about 20 other operations (the denominators of the reference's later terms
+// are its neighbours' first ones).  Blocks walk items of a 32 x 16 tile (and
+// a slab of slices in 3-D), the updated slices and the reciprocal roots of
+// the tile and its halo in shared memory, one barrier per slice.  Block sums
+// are added in block order by the blocks of the next kernel, so there is no
+// reduction pass and a run gives the same bits as any other.
+// Measured per step (ncu): 128^3 FP64 848 us as a norm and an update kernel
+// that each evaluated the stencil with a square root and a division per term.
+constexpr int kTvX = 32, kTvY = 16, kTvT = kTvX * kTvY;  // tile and threads
+constexpr int kTvBlocks = 2048;                          // most blocks of a step
+constexpr int kTvHalo = 2 * (kTvX + 2) + 2 * kTvY;       // halo cells of a slice
+constexpr int kTvRx = kTvX + kTvY + 1;                   // roots beside the tile
+static_assert(kTvHalo <= kTvT && kTvRx <= kTvT, "a thread takes at most one of each");
+
 template <class T>
-struct GlobalAt {
-  const T *p;
-  int nx, ny, nz, x, y, z;
-  __device__ __forceinline__ T operator()(int dx, int dy, int dz) const {
-    const int xx = x + dx, yy = y + dy, zz = z + dz;
-    if (xx < 0 || yy < 0 || zz < 0 || xx >= nx || yy >= ny || zz >= nz) return T(0);
-    return p[((long long)zz * ny + yy) * nx + xx];
+__device__ __forceinline__ T tv_recip_root(T den);
+template <>
+__device__ __forceinline__ float tv_recip_root(float den) {
+  return tv_rsqrt(den);
+}
+template <>
+__device__ __forceinline__ double tv_recip_root(double den) {
+  return rsqrt(den);
+}
+
+// Sums of np block partials (K arrays of stride kTvBlocks) by the block's
+// first four warps in a fixed order; valid in thread 0 after the call (every
+// thread must call it).
+template <int K>
+__device__ __forceinline__ void tv_sum_partials(const double *p, int np, double (&tot)[K]) {
+  __shared__ double sh[K][4];
+  const int t = threadIdx.x;
+  if (t < 128) {
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      double a = 0.0;
+      for (int i = t; i < np; i += 128) a += p[k * kTvBlocks + i];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if ((t & 31) == 0) sh[k][t >> 5] = a;
+    }
   }
+  __syncthreads();
+  if (t == 0)
+#pragma unroll
+    for (int k = 0; k < K; k++) tot[k] = (sh[k][0] + sh[k][1]) + (sh[k][2] + sh[k][3]);
+}
+
+// The step size alpha d / ||u|| from the partials of the kernel before:
+// u's squares first, then (step 0) the squared distance to the old image,
+// whose root d stays in scal[0] for the later steps.
+__device__ __forceinline__ double tv_step_size(const double *pin, int np, int step, double alpha,
+                                               double *scal) {
+  __shared__ double s_coef;
+  if (step == 0) {
+    double tot[2];
+    tv_sum_partials<2>(pin, np, tot);
+    if (threadIdx.x == 0) {
+      const double d = sqrt(tot[1]);
+      if (blockIdx.x == 0) scal[0] = d;
+      s_coef = alpha * d * rsqrt(tot[0]);
+    }
+  } else {
+    double tot[1];
+    tv_sum_partials<1>(pin, np, tot);
+    if (threadIdx.x == 0) s_coef = alpha * scal[0] * rsqrt(tot[0]);
+  }
+  __syncthreads();
+  return s_coef;
+}
+
+struct TvGrid {
+  int nx, ny, nz, tx, ty, slab, items;  // tiles per row and column, slices per item
 };
 
-// --------------------------------------------------- standalone TV kernels
-// scal[0] = d, scal[1] = ||v||, scal[2] = alpha*d/||v|| (+ FP32 copy at 3).
-__device__ __forceinline__ bool sum_all(float v, double *partials,
-                                        unsigned *counter, double &tot) {
-  const float vv[1] = {v};
-  double t[1];
-  const bool last = grid_sum<kThreads, 1>(vv, partials, counter, inst_block(),
-                                          inst_blocks(), t);
-  tot = t[0];
-  return last;
-}
-__device__ __forceinline__ bool sum_all(double v, double *partials,
-                                        unsigned *counter, double &tot) {
-  return grid_sum_d<kThreads>(v, partials, counter, inst_blocks(), tot);
-}
-
-template <class T>
-__global__ void __launch_bounds__(kThreads)
-    k_tv_dist(const T *__restrict__ img, const T *__restrict__ old, int nx,
-              int ny, int nz, double *scal, double *partials,
-              unsigned *counter) {
-  int ix, iy, iz;
-  T v = T(0);
-  if (tile_voxel(nx, ny, nz, ix, iy, iz)) {
-    const long long i = ((long long)iz * ny + iy) * nx + ix;
-    const T d = ASD_IN(i, (long long)nx * ny * nz) ? img[i] - (old ? old[i] : T(0)) : T(0);
-    v = d * d;
-  }
-  double tot;
-  if (sum_all(v, partials, counter, tot))
-    if (threadIdx.x == 0) scal[0] = sqrt(tot);
-}
-
-template <class T>
-__global__ void __launch_bounds__(kThreads)
-    k_tv_norm(const T *__restrict__ src, int nx, int ny, int nz, double alpha,
-              double *scal, double *partials, unsigned *counter) {
-  int ix, iy, iz;
-  T v = T(0);
-  if (tile_voxel(nx, ny, nz, ix, iy, iz)) {
-    const T g = tv_grad<T>(GlobalAt<T>{src, nx, ny, nz, ix, iy, iz}, nz >= 2);
-    v = g * g;
-  }
-  double tot;
-  if (sum_all(v, partials, counter, tot))
-    if (threadIdx.x == 0) {
-      scal[1] = sqrt(tot);
-      scal[2] = alpha * scal[0] / scal[1];
-      *(float *)(scal + 3) = (float)scal[2];  // for the FP32 update pass
+// kFirst: the stencil of the image itself (no update) and the squared
+// distance to `uin`, the old image (null: zeros).
+template <class T, bool k3D, bool kFirst>
+__global__ void __launch_bounds__(kTvT, sizeof(T) == 8 ? 2 : 3)
+    k_tv_step(const T *__restrict__ m, const T *__restrict__ uin, T *__restrict__ mout,
+              T *__restrict__ uout, TvGrid g, int step, double alpha, double *scal,
+              const double *__restrict__ pin, int np, double *__restrict__ pout) {
+  __shared__ T P[k3D ? 3 : 1][kTvY + 2][kTvX + 2];  // updated slices
+  __shared__ T R[k3D ? 2 : 1][kTvY + 1][kTvX + 1];  // their reciprocal roots
+  __shared__ double red[2][kTvT / 32];
+  pdl_enter();
+  const int t = threadIdx.x, lx = t & 31, ly = t >> 5;
+  // this thread's halo cell and root beside the tile (rows and columns of P)
+  const int hy = t < 34 ? 0 : t < 68 ? kTvY + 1 : 1 + (t - 68) % kTvY;
+  const int hx = t < 34 ? t : t < 68 ? t - 34 : t < 68 + kTvY ? 0 : kTvX + 1;
+  const bool halo = t < kTvHalo, rext = t < kTvRx;
+  const int ey = t <= kTvY ? 1 + t : 1 + kTvY, ex = t <= kTvY ? 1 + kTvX : t - kTvY;
+  const long long plane = (long long)g.nx * g.ny;
+  const long long nvox = plane * g.nz;
+  T coef = T(0);
+  double sum[2] = {0.0, 0.0};  // u^2, distance^2 (FP32: lane 0 of each warp)
+  bool sized = kFirst;
+  for (int item = blockIdx.x; item < g.items; item += gridDim.x) {
+    const int tile = item % (g.tx * g.ty), z0 = item / (g.tx * g.ty) * g.slab;
+    const int z1 = min(g.nz, z0 + g.slab);
+    const int x0 = tile % g.tx * kTvX, y0 = tile / g.tx * kTvY;
+    const int cx = x0 + lx, cy = y0 + ly, gx = x0 - 1 + hx, gy = y0 - 1 + hy;
+    const bool cin = cx < g.nx && cy < g.ny;
+    const bool hin = halo && gx >= 0 && gx < g.nx && gy >= 0 && gy < g.ny;
+    const long long co = (long long)cy * g.nx + cx, ho = (long long)gy * g.nx + gx;
+    T cm, cu, hm, hu;  // the slice in flight: tile cell and halo cell of m and u
+    auto fetch = [&](int z) {
+      const bool in = z >= 0 && z < g.nz;
+      const long long zo = (long long)z * plane;
+      const bool a = in && cin && ASD_IN(zo + co, nvox), b = in && hin && ASD_IN(zo + ho, nvox);
+      cm = a ? m[zo + co] : T(0);
+      hm = b ? m[zo + ho] : T(0);
+      if (kFirst) {
+        cu = a && uin ? uin[zo + co] : T(0);  // the old image
+        hu = T(0);
+      } else {
+        cu = a ? uin[zo + co] : T(0);
+        hu = b ? uin[zo + ho] : T(0);
+      }
+    };
+    // the fetched slice's updated values (cells outside the image are zeros:
+    // so is their u) into P[q]; returns the tile cell's
+    auto place = [&](int q) {
+      const T c = kFirst || !cin ? cm : cm - coef * cu;
+      const T h = kFirst || !hin ? hm : hm - coef * hu;
+      P[q][ly + 1][lx + 1] = c;
+      if (halo) P[q][hy][hx] = h;
+      return c;
+    };
+    // reciprocal root of cell (y, x) of P[q], over the slice P[q0] (3-D);
+    // s: the sum of its three differences
+    auto root = [&](int q, int q0, int y, int x, T &s) {
+      const T c = P[q][y][x];
+      const T dx = c - P[q][y][x - 1], dy = c - P[q][y - 1][x];
+      T den = tv_eps<T>() + dx * dx + dy * dy;
+      s = dx + dy;
+      if (k3D) {
+        const T dz = c - P[q0][y][x];
+        den += dz * dz;
+        s += dz;
+      }
+      return tv_recip_root(den);
+    };
+    auto roots = [&](int r, int q, int q0, T &s) {
+      const T own = root(q, q0, ly + 1, lx + 1, s);
+      R[r][ly][lx] = own;
+      if (rext) {
+        T dummy;
+        R[r][ey - 1][ex - 1] = root(q, q0, ey, ex, dummy);
+      }
+      return own;
+    };
+    float accf[2] = {0.f, 0.f};
+    auto add = [&](int k, T v) {
+      if (sizeof(T) == 8)
+        sum[k] += (double)v;
+      else
+        accf[k] += (float)v;
+    };
+    // u of the tile cell in P[q], R[r] and what the slice above it adds
+    auto emit = [&](long long zo, int q, int r, T s, T own, T above) {
+      const T c = P[q][ly + 1][lx + 1];
+      T u = s * own;
+      u += (c - P[q][ly + 2][lx + 1]) * R[r][ly + 1][lx];
+      u += (c - P[q][ly + 1][lx + 2]) * R[r][ly][lx + 1];
+      u += above;
+      if (!cin || !ASD_IN(zo + co, nvox)) return;
+      uout[zo + co] = u;
+      if (!kFirst) mout[zo + co] = c;
+      add(0, u * u);
+    };
+    auto distance = [&]() {
+      if (kFirst && cin) {
+        const T d = cm - cu;
+        add(1, d * d);
+      }
+    };
+    fetch(k3D ? z0 - 1 : 0);
+    if (!sized) coef = (T)tv_step_size(pin, np, step, alpha, scal);  // has a barrier
+    sized = true;
+    if (item != (int)blockIdx.x) __syncthreads();  // P and R are reused
+    if (!k3D) {
+      distance();
+      place(0);
+      __syncthreads();
+      T s;
+      const T own = roots(0, 0, 0, s);
+      __syncthreads();
+      emit(0, 0, 0, s, own, T(0));
+    } else {
+      place((z0 + 2) % 3);  // slice z in P[z % 3], its roots in R[z & 1]
+      fetch(z0);
+      distance();
+      T c = place(z0 % 3);
+      fetch(z0 + 1);
+      __syncthreads();
+      T s, own = roots(z0 & 1, z0 % 3, (z0 + 2) % 3, s);
+      int q = z0 % 3;
+      for (int z = z0; z < z1; z++) {
+        const int q1 = q == 2 ? 0 : q + 1;
+        if (z + 1 < z1) distance();  // slice z + 1 is in flight
+        const T n = place(q1);
+        if (z + 1 < z1) fetch(z + 2);
+        __syncthreads();
+        T s1;
+        const T own1 = roots((z + 1) & 1, q1, q, s1);
+        emit((long long)z * plane, q, z & 1, s, own, (c - n) * own1);
+        c = n;
+        s = s1;
+        own = own1;
+        q = q1;
+      }
     }
-}
-
-// img -= alpha*d*v/norm   (imgTVGradMin.cpp:104-107)
-template <class T>
-__global__ void __launch_bounds__(kThreads)
-    k_tv_update(const T *__restrict__ src, T *__restrict__ dst, int nx, int ny,
-                int nz, double alpha, const double *scal, int clamp) {
-  int ix, iy, iz;
-  if (!tile_voxel(nx, ny, nz, ix, iy, iz)) return;
-  const T g = tv_grad<T>(GlobalAt<T>{src, nx, ny, nz, ix, iy, iz}, nz >= 2);
-  const long long i = ((long long)iz * ny + iy) * nx + ix;
-  if (!ASD_IN(i, (long long)nx * ny * nz)) return;
-  T r;
-  if (sizeof(T) == 8) {
-    r = (T)((double)src[i] - alpha * scal[0] * (double)g / scal[1]);
-  } else {
-    const float coef = *(const float *)(scal + 3);
-    r = src[i] - coef * g;
+    if (sizeof(T) == 4) {  // an item's FP32 sums join the FP64 ones per warp
+#pragma unroll
+      for (int k = 0; k < (kFirst ? 2 : 1); k++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) accf[k] += __shfl_xor_sync(0xffffffffu, accf[k], o);
+        if (lx == 0) sum[k] += (double)accf[k];
+      }
+    }
   }
-  if (clamp && r < T(0)) r = T(0);
-  dst[i] = r;
+#pragma unroll
+  for (int k = 0; k < (kFirst ? 2 : 1); k++) {
+    if (sizeof(T) == 8)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+    if (lx == 0) red[k][ly] = sum[k];
+  }
+  __syncthreads();
+  if (t < kTvT / 32) {
+#pragma unroll
+    for (int k = 0; k < (kFirst ? 2 : 1); k++) {
+      double a = red[k][t];
+#pragma unroll
+      for (int o = kTvT / 64; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffu, a, o);
+      if (t == 0) pout[k * kTvBlocks + blockIdx.x] = a;
+    }
+  }
 }
 
+// The last step's update: img = m - coef u(m), positivity where asked
+// (imgTVGradMin.cpp:104-116).  m may be img.
 template <class T>
-__global__ void k_copy_clamp(const T *__restrict__ src, T *__restrict__ dst,
-                             long long n, int clamp) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    T v = src[i];
+__global__ void __launch_bounds__(kTvT)
+    k_tv_last(const T *m, const T *__restrict__ u, T *img, long long n, int step, double alpha,
+              double *scal, const double *__restrict__ pin, int np, int clamp) {
+  pdl_enter();
+  const T coef = (T)tv_step_size(pin, np, step, alpha, scal);
+  for (long long i = blockIdx.x * (long long)kTvT + threadIdx.x; i < n;
+       i += (long long)gridDim.x * kTvT) {
+    if (!ASD_IN(i, n)) continue;
+    T v = m[i] - coef * u[i];
     if (clamp && v < T(0)) v = T(0);
-    dst[i] = v;
+    img[i] = v;
   }
 }
 
+// Slices per item and blocks of a 3-D step: the slab whose rounds of items
+// over the resident blocks cost least (an item costs its slices and about
+// two more for the slices it shares with its neighbours).
 template <class T>
-cudaError_t tv_minimize(T *img, const T *old, T *wa, T *wb, double *scal,
-                        double *partials, unsigned *counter, int nx, int ny,
-                        int nz, double alpha, int n_iter, int pos,
-                        cudaStream_t st) {
-  const dim3 grid = tile_grid(nx, ny, nz, 1);
-  if ((long long)grid.x * grid.y > kMaxPartials || tile_rows(ny, nz) > kMaxGridRows)
-    return cudaErrorInvalidValue;
-  k_tv_dist<T><<<grid, kThreads, 0, st>>>(img, old, nx, ny, nz, scal, partials,
-                                          counter);
-  const T *src = img;
-  T *bufs[2] = {wa, wb};
-  for (int it = 0; it < n_iter; it++) {
-    T *dst = (it == n_iter - 1) ? img : bufs[it & 1];
-    if (dst == src) dst = bufs[(it + 1) & 1];
-    k_tv_norm<T><<<grid, kThreads, 0, st>>>(src, nx, ny, nz, alpha, scal,
-                                            partials, counter);
-    const int clamp_now = (it == n_iter - 1) && pos == 1;
-    k_tv_update<T><<<grid, kThreads, 0, st>>>(src, dst, nx, ny, nz, alpha,
-                                              scal, clamp_now);
-    src = dst;
+TvGrid tv_grid(int nx, int ny, int nz, int &blocks) {
+  TvGrid g{nx, ny, nz, (nx + kTvX - 1) / kTvX, (ny + kTvY - 1) / kTvY, 1, 0};
+  const long long tiles = (long long)g.tx * g.ty;
+  const long long resident = 152LL * (sizeof(T) == 8 ? 2 : 3);
+  long long best = 0, count = tiles;
+  if (nz > 1)
+    for (int s = 4; s <= 64; s *= 2) {
+      const long long n = tiles * ((nz + s - 1) / s);
+      const long long cost = ((n + resident - 1) / resident) * (std::min(s, nz) + 2);
+      if (best == 0 || cost < best) {
+        best = cost;
+        g.slab = s;
+        count = n;
+      }
+    }
+  g.items = (int)count;
+  blocks = (int)std::min<long long>(count, nz > 1 ? resident : kTvBlocks);
+  return g;
+}
+
+// wc null: two kernels per step (the stencil, then the update in place),
+// which need wa only.
+template <class T, bool k3D>
+cudaError_t tv_minimize_dim(T *img, const T *old, T *wa, T *wb, T *wc, double *scal,
+                            double *partials, int nx, int ny, int nz, double alpha, int n_iter,
+                            int pos, cudaStream_t st) {
+  int blocks = 0;
+  const TvGrid g = tv_grid<T>(nx, ny, nz, blocks);
+  const long long n = (long long)nx * ny * nz;
+  const dim3 grid(blocks), last((unsigned)std::min<long long>((n + kTvT - 1) / kTvT, 152 * 8));
+  double *p[2] = {partials, partials + 2 * kTvBlocks};
+  cudaError_t e = launch_iter(k_tv_step<T, k3D, true>, grid, dim3(kTvT), st, (const T *)img, old,
+                              (T *)nullptr, wa, g, 0, alpha, scal, (const double *)nullptr, 0,
+                              p[0]);
+  const T *m = img, *u = wa;
+  for (int s = 0; s < n_iter - 1 && e == cudaSuccess; s++) {
+    if (wc) {
+      T *mn = (s & 1) ? img : wb, *un = (s & 1) ? wa : wc;
+      e = launch_iter(k_tv_step<T, k3D, false>, grid, dim3(kTvT), st, m, u, mn, un, g, s, alpha,
+                      scal, (const double *)p[s & 1], blocks, p[1 - (s & 1)]);
+      m = mn;
+      u = un;
+    } else {
+      e = launch_iter(k_tv_last<T>, last, dim3(kTvT), st, m, u, img, n, s, alpha, scal,
+                      (const double *)p[s & 1], blocks, 0);
+      if (e == cudaSuccess)
+        e = launch_iter(k_tv_step<T, k3D, true>, grid, dim3(kTvT), st, (const T *)img,
+                        (const T *)nullptr, (T *)nullptr, wa, g, 0, alpha, scal,
+                        (const double *)nullptr, 0, p[1 - (s & 1)]);
+    }
   }
-  if (n_iter > 0 && src != img) {
-    const long long n = (long long)nx * ny * nz;
-    k_copy_clamp<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src, img, n, 0);
-  }
-  return cudaGetLastError();
+  if (e == cudaSuccess)
+    e = launch_iter(k_tv_last<T>, last, dim3(kTvT), st, m, u, img, n, n_iter - 1, alpha, scal,
+                    (const double *)p[(n_iter - 1) & 1], blocks, (int)(pos == 1));
+  return e;
+}
+
+template <class T>
+cudaError_t tv_minimize(T *img, const T *old, T *wa, T *wb, T *wc, double *scal,
+                        double *partials, int nx, int ny, int nz, double alpha, int n_iter,
+                        int pos, cudaStream_t st, bool pdl) {
+  if (n_iter <= 0) return cudaSuccess;
+  const PdlScope scope(pdl);
+  if (nz > 1)
+    return tv_minimize_dim<T, true>(img, old, wa, wb, wc, scal, partials, nx, ny, nz, alpha,
+                                    n_iter, pos, st);
+  return tv_minimize_dim<T, false>(img, old, wa, wb, wc, scal, partials, nx, ny, nz, alpha,
+                                   n_iter, pos, st);
 }
 
 // ------------------------------------------- batched ASD-POCS: tiled steps
@@ -416,7 +581,7 @@ __global__ void __launch_bounds__(kThreads)
       }
       if (tv) {
         const float gr =
-            tv_grad<float>(TileAt<1, k3D>{t, tx + 1, ty + 1, k3D ? 1 : 0}, k3D);
+            tv_grad_f<k3D>(TileAt<1, k3D>{t, tx + 1, ty + 1, k3D ? 1 : 0});
         v[3] += gr * gr;
       }
     }
@@ -1251,21 +1416,19 @@ cudaError_t launch_gather_done(const Inst *insts, int n, int *out,
   return cudaGetLastError();
 }
 
-cudaError_t tv_minimize_f64(double *img, const double *img_old, double *wa,
-                            double *wb, double *scal, double *partials,
-                            unsigned *counter, int nx, int ny, int nz,
-                            double alpha, int n_iter, int pos,
-                            cudaStream_t st) {
-  return tv_minimize<double>(img, img_old, wa, wb, scal, partials, counter, nx,
-                             ny, nz, alpha, n_iter, pos, st);
+size_t tv_partials_bytes() { return (size_t)4 * kTvBlocks * sizeof(double); }
+
+cudaError_t tv_minimize_f64(double *img, const double *img_old, double *wa, double *wb,
+                            double *wc, double *scal, double *partials, int nx, int ny, int nz,
+                            double alpha, int n_iter, int pos, cudaStream_t st, bool pdl) {
+  return tv_minimize<double>(img, img_old, wa, wb, wc, scal, partials, nx, ny, nz, alpha,
+                             n_iter, pos, st, pdl);
 }
-cudaError_t tv_minimize_f32(float *img, const float *img_old, float *wa,
-                            float *wb, double *scal, double *partials,
-                            unsigned *counter, int nx, int ny, int nz,
-                            double alpha, int n_iter, int pos,
-                            cudaStream_t st) {
-  return tv_minimize<float>(img, img_old, wa, wb, scal, partials, counter, nx,
-                            ny, nz, alpha, n_iter, pos, st);
+cudaError_t tv_minimize_f32(float *img, const float *img_old, float *wa, float *wb, float *wc,
+                            double *scal, double *partials, int nx, int ny, int nz, double alpha,
+                            int n_iter, int pos, cudaStream_t st, bool pdl) {
+  return tv_minimize<float>(img, img_old, wa, wb, wc, scal, partials, nx, ny, nz, alpha, n_iter,
+                            pos, st, pdl);
 }
 
 cudaError_t launch_iter_begin(const Inst *, int, cudaStream_t) {

@@ -6,8 +6,7 @@
 // enforced by a serving layer), a real-time loop where an allocation could
 // stall on a device-wide synchronisation, or a plugin host that forbids its
 // extensions from allocating.  For them this entry point keeps its scratch
-// (two work images, the reduction partials, the ticket counter and the step
-// scalars) in one file-scope __device__ array of fixed size, which every GPU
+// (the work images, the reduction partials and the step scalars) in one file-scope __device__ array of fixed size, which every GPU
 // that loads the library holds until the process exits.  The caller still
 // passes the image (in/out) and the reference image.
 //
@@ -27,12 +26,9 @@ namespace {
 
 constexpr size_t kMaxVoxels = size_t(1) << 20;
 constexpr size_t kMaxTiles = size_t(1) << 16;
-constexpr size_t kImgBytes = kMaxVoxels * sizeof(float);  // 4 MiB
-constexpr size_t kOffA = 0;
-constexpr size_t kOffB = kImgBytes;
-constexpr size_t kOffScal = 2 * kImgBytes;        // 256 B of step scalars
-constexpr size_t kOffCounter = kOffScal + 256;    // ticket, must start at 0
-constexpr size_t kOffPartials = kOffCounter + 256;
+constexpr size_t kWorkBytes = 2 * kMaxVoxels * sizeof(float);  // 8 MiB of work images
+constexpr size_t kOffScal = kWorkBytes;        // 256 B of step scalars
+constexpr size_t kOffPartials = kOffScal + 512;
 constexpr size_t kScratchBytes = kOffPartials + kMaxTiles * sizeof(double);
 
 static __device__ __align__(256) unsigned char g_tv_scratch[kScratchBytes];
@@ -90,12 +86,13 @@ extern "C" int asdpocs_tv_device_noalloc(float *img_d, const float *img_old_d,
   char *b = nullptr;
   if (int e = scratch_address(&b)) return e;
   cudaStream_t st = (cudaStream_t)stream;
-  // the ticket keeps the previous call's contents: clear it
-  ASD_CUDA(cudaMemsetAsync(b + kOffCounter, 0, 256, st));
-  ASD_CUDA(tv_minimize_f32(img_d, img_old_d, (float *)(b + kOffA),
-                           (float *)(b + kOffB), (double *)(b + kOffScal),
-                           (double *)(b + kOffPartials),
-                           (unsigned *)(b + kOffCounter), nx, ny, nz, alpha,
-                           nTVIter, pos, st));
+  // three work images where the array holds them, else one and two kernels a
+  // step (see tv_minimize_f32)
+  const size_t img_b = (N * sizeof(float) + 255) / 256 * 256;
+  const bool three = 3 * img_b <= kWorkBytes;
+  ASD_CUDA(tv_minimize_f32(img_d, img_old_d, (float *)b, three ? (float *)(b + img_b) : nullptr,
+                           three ? (float *)(b + 2 * img_b) : nullptr,
+                           (double *)(b + kOffScal), (double *)(b + kOffPartials), nx, ny, nz,
+                           alpha, nTVIter, pos, st, false));
   return 0;
 }

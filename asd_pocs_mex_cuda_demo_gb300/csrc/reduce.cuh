@@ -108,49 +108,3 @@ __device__ __forceinline__ bool grid_sum(const float (&v)[K], double *partials,
 }
 
 }  // namespace asd
-
-namespace asd {
-
-// FP64 variant for the FP64 entry points (the mex-level TV): every level of
-// the reduction in FP64, same deterministic last-block scheme.
-template <int NT>
-__device__ __forceinline__ bool grid_sum_d(double v, double *partials,
-                                           unsigned *counter, int nblocks,
-                                           double &tot) {
-  __shared__ double sh[NT / 32];
-  __shared__ bool last;
-  __shared__ double bc;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (lane == 0) sh[warp] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int w = 0; w < NT / 32; w++) s += sh[w];
-    partials[inst_block()] = s;
-    __threadfence();
-    last = atomicAdd(counter, 1u) == (unsigned)nblocks - 1;
-  }
-  __syncthreads();
-  if (!last) return false;
-  __threadfence();
-  double a = 0.0;
-  for (int b = threadIdx.x; b < nblocks; b += NT) a += ((volatile double *)partials)[b];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  __syncthreads();
-  if (lane == 0) sh[warp] = a;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int w = 0; w < NT / 32; w++) s += sh[w];
-    bc = s;
-    *counter = 0u;
-  }
-  __syncthreads();
-  tot = bc;
-  return true;
-}
-
-}  // namespace asd

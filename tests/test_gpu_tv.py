@@ -66,3 +66,43 @@ def test_tv_fp32_device_vs_oracle(gpu, oracle_mod, shape):
         img32, old32 = img32[:, :, 0], old32[:, :, 0]
     ref = oracle_mod.tv(img32, 0.2, 10, 1, old32)
     assert rel_l2(t.cpu().numpy(), ref.ravel(order="F")) < 1e-5
+
+
+@pytest.mark.parametrize("steps", [1, 2, 5])
+@pytest.mark.parametrize("shape", [(32, 16, 1), (33, 17, 1), (1, 40, 1), (31, 15, 1), (700, 9, 1),
+                                   (32, 16, 2), (33, 17, 5), (7, 3, 67), (65, 48, 12)])
+def test_tv_steps_at_tile_edges(gpu, oracle_mod, shape, steps):
+    """Images that end at, before and after a tile of 32 x 16 and a slab of
+    slices, in FP64 and FP32, with and without an old image."""
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    nx, ny, nz = shape
+    rng = np.random.default_rng(nx * 31 + ny + nz)
+    dims = shape if nz > 1 else shape[:2]
+    img, old = rng.random(dims), rng.random(dims)
+    fn = pkg.imgTVGradMin3D if nz > 1 else pkg.imgTVGradMin
+    assert rel_l2(fn(img, 0.1, steps, 1, old), oracle_mod.tv(img, 0.1, steps, 1, old)) < 1e-12
+    assert rel_l2(fn(img, 0.1, steps, 0), oracle_mod.tv(img, 0.1, steps, 0)) < 1e-12
+    t, o = (torch.tensor(a.ravel(order="F"), dtype=torch.float32, device=gpu) for a in (img, old))
+    f64 = [a.cpu().numpy().astype(np.float64).reshape(dims, order="F") for a in (t, o)]
+    check(load().asdpocs_tv_device(t.data_ptr(), o.data_ptr(), nx, ny, nz, 0.1, steps, 1,
+                                   torch.cuda.current_stream().cuda_stream))
+    ref = oracle_mod.tv(f64[0], 0.1, steps, 1, f64[1])
+    assert rel_l2(t.cpu().numpy(), ref.ravel(order="F")) < 1e-5
+
+
+def test_tv_noalloc_large_image(gpu):
+    """An image too large for three work images in the fixed scratch."""
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    a = torch.rand(1000 * 1001, device=gpu)
+    b, old = a.clone(), torch.rand(1000 * 1001, device=gpu)
+    s = torch.cuda.current_stream().cuda_stream
+    check(load().asdpocs_tv_device(a.data_ptr(), old.data_ptr(), 1000, 1001, 1, 0.1, 4, 1, s))
+    check(load().asdpocs_tv_device_noalloc(b.data_ptr(), old.data_ptr(), 1000, 1001, 1, 0.1, 4, 1,
+                                           s))
+    assert rel_l2(b.cpu().numpy(), a.cpu().numpy()) < 1e-5
