@@ -154,8 +154,7 @@ struct Scalars {
   // ASD-POCS step control (ASD_POCS_cuda.m:137-170), FP64 on the device
   double alpha, beta;
   double alpha_red, beta_red, r_max, epsilon, stopRelChg;
-  double dd2_acc;   // running ||P - Ax||^2 over the current sweep
-  double dd2;       // dd2 of the last complete sweep (out.dataTolerance)
+  double dd2;       // ||P - Ax||^2 (Inst::ddr summed) of the last complete sweep (out.dataTolerance)
   double dp;        // ||m - m_pre|| of the last sweep
   double d_tv;      // ||m - m_k1|| at TV entry (imgTVGradMin.cpp:57-60)
   double tv_coef;   // alpha*d/||v|| of the current TV step
@@ -167,7 +166,7 @@ struct Scalars {
   int iterations;   // out.IterationNum
   int maxIter, ng;
   int has_ref;      // I0 present
-  int cor_finite;   // current view: every residual finite (set by Ax)
+  int cor_bad;      // 1 + the last view with a residual that is not finite
 };
 
 struct Inst {
@@ -204,6 +203,9 @@ struct Inst {
   double *rmse;              // [maxIter]
   double *partials;          // reduction partials [blocks * kMaxReduceK]
   unsigned *counter;         // reduction ticket
+  double *ddr;               // [na*nb] the sweep's squared residuals of a ray
+                             //   (added up by its views, taken and cleared
+                             //   at the end of the sweep); follows counter
   Scalars *s;
 };
 
@@ -320,6 +322,6 @@ __device__ __forceinline__ OwnBlock own_block(dim3 own) {
               : -1;
   return b;
 }
-constexpr int kMaxReduceK = 4;          // values reduced together (partials sizing)
+constexpr int kMaxReduceK = 5;          // values reduced together (partials sizing)
 
 }  // namespace asd

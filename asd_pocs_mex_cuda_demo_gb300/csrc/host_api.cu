@@ -768,11 +768,12 @@ InstLayout layout_instance(const asdpocs_geometry &g, int max_iter,
   o.tvb = off; off += per_img;
   o.tvc = off; off += per_img;
   o.rmse = off; off += st ? align256((size_t)(max_iter + 1) * 8) : 0;
-  // block partials of the projector and tile kernels; the 2-D walks keep four
-  // values per strip and band
-  const size_t nparts = std::max(nblk * kMaxReduceK, (size_t)tv_partials_for(d) * 4);
+  // block partials of the tile kernels; the 2-D walks keep as many values
+  // per strip and band
+  const size_t nparts = std::max(nblk, (size_t)tv_partials_for(d)) * kMaxReduceK;
   o.part = off; off += st ? align256(nparts * 8) : 0;
   o.cnt = off; off += st ? 256 : 0;
+  o.ddr = off; off += st ? align256(M * 8) : 0;
   o.scal = off; off += st ? align256(sizeof(Scalars)) : 0;
   o.cor = off; off += geo ? align256(cor_floats * 4) : 0;
   o.m_il = off; off += geo ? align256(il_floats * 4) : 0;
@@ -799,6 +800,7 @@ void bind_state(Inst &I, char *b, const InstLayout &o) {
   I.rmse = (double *)(b + o.rmse);
   I.partials = (double *)(b + o.part);
   I.counter = (unsigned *)(b + o.cnt);
+  I.ddr = (double *)(b + o.ddr);
   I.s = (Scalars *)(b + o.scal);
 }
 
@@ -869,7 +871,9 @@ cudaError_t reset_instance(const Inst &I, const Scalars &s, cudaStream_t st) {
     e = cudaMemcpyAsync(I.m_pre, I.m_k1, bytes, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(I.m_res, I.m_k1, bytes, cudaMemcpyDeviceToDevice, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(I.counter, 0, 256, st);
+  // the ticket and, right after it, the squared residuals
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(I.counter, 0, 256 + (size_t)I.d.na * I.d.nb * 8, st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(I.s, &s, sizeof s, cudaMemcpyHostToDevice, st);
   return e;

@@ -11,7 +11,7 @@ namespace asd {
 // block's size.
 struct InstLayout {
   size_t P, m, m_pre, m_res, m_k1, I0, tvb, tvc, cor, m_il, ydet, zdet, trig,
-      rmse, part, cnt, scal, tabA, tabC, vflags, bytes;
+      rmse, part, cnt, ddr, scal, tabA, tabC, vflags, bytes;
   int p_fmt;  // sinogram storage (ASDPOCS_STORE_*)
 };
 

@@ -10,7 +10,6 @@
 #include <type_traits>
 #include "kernels.h"
 #include "projector.cuh"
-#include "reduce.cuh"
 
 namespace asd {
 
@@ -38,21 +37,18 @@ int atx_blocks(const Dims &d) {
 }
 
 // ------------------------------------------------------------------- Ax
-// A ray's columns are dealt to kAxCols warps: lane l of warp part p takes
-// columns l + 32 p, l + 32 p + 32 kAxCols, ...  The parts' lane partials are
-// added in part order (through shared memory), then the lanes by the xor
-// butterfly.  Every forward kernel sums a ray this way, so a ray's total
-// does not depend on the kernel that computed it.  One warp per ray
-// measured fastest for batches and cone beam (two: 14 % slower for a batch
-// of 64 and 27 % for 256^3, 7 % faster for one 512^2 instance).
-constexpr int kAxCols = 1;
-constexpr int kAxBlock = kAxWarps * kAxCols * 32;  // threads per block
+// One warp per ray: lane l takes columns l, l + 32, ..., and the lanes'
+// partial sums are added by the xor butterfly.  Every forward kernel sums a
+// ray this way, so a ray's total does not depend on the kernel that computed
+// it.  (Two warps per ray: 14 % slower for a batch of 64 and 27 % for 256^3.)
+constexpr int kAxBlock = kAxWarps * 32;  // threads per block
 
 // This lane's partial sums of ray r over its columns (no cross-lane sum).
 template <class Loader>
 __device__ __forceinline__ void ax_lane_partial(const ViewGeo &G, const Dims &D,
-                                                long long r, int first, Loader ld,
-                                                float &ys, float &ss) {
+                                                long long r, Loader ld, float &ys,
+                                                float &ss) {
+  const int lane = threadIdx.x & 31;
   const int ia = (int)(r % D.na), ib = (int)(r / D.na);
   const float zd = G.z_det[ib];
   const RayMarch R = ray_setup(G, D, G.y_det[ia], zd);
@@ -62,54 +58,25 @@ __device__ __forceinline__ void ax_lane_partial(const ViewGeo &G, const Dims &D,
   // three pieces per column already keep loads in flight; two measured 6 %
   // slower at 256^3)
   if (D.nz == 1 && zd == 0.0f)
-    ray_columns_planar_fast<2>(R, first, 32 * kAxCols, ld, ys, ss);
+    ray_columns_planar_fast<2>(R, lane, 32, ld, ys, ss);
   else
-    ray_columns_fast<1>(R, first, 32 * kAxCols, ld, ys, ss);
-}
-
-// The block's ray totals: each warp stores its lane partials of the K values
-// in sp[part][ray][k][lane]; after the barrier the part-0 warps add the parts
-// in order and sum their lanes.  Every thread of the block must call it.
-template <int K>
-__device__ __forceinline__ void ax_combine(float (&sp)[kAxCols][kAxWarps][K][32],
-                                           float (&v)[K], int part, int rw,
-                                           int lane) {
-  if constexpr (kAxCols == 1) {
-#pragma unroll
-    for (int k = 0; k < K; k++) v[k] = warp_sum(v[k]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < K; k++) sp[part][rw][k][lane] = v[k];
-    __syncthreads();
-    if (part == 0) {
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        float t = sp[0][rw][k][lane];
-#pragma unroll
-        for (int p = 1; p < kAxCols; p++) t += sp[p][rw][k][lane];
-        v[k] = warp_sum(t);
-      }
-    }
-  }
+    ray_columns_fast<1>(R, lane, 32, ld, ys, ss);
 }
 
 __global__ void __launch_bounds__(kAxBlock)
     k_ax(const float *__restrict__ x, float *__restrict__ y,
          float *__restrict__ sr, ViewGeo G, Dims D) {
-  __shared__ float sp[kAxCols][kAxWarps][2][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int rw = warp % kAxWarps, part = warp / kAxWarps;
-  const long long r = (long long)blockIdx.x * kAxWarps + rw;
-  const bool in = r < (long long)D.na * D.nb;
-  float v[2] = {0.f, 0.f};
-  if (in)
-    ax_lane_partial(G, D, r, lane + 32 * part,
-                    [&](unsigned i) { return ASD_IN(i, nvox(D)) ? __ldg(x + i) : 0.f; },
-                    v[0], v[1]);
-  ax_combine<2>(sp, v, part, rw, lane);
-  if (in && part == 0 && lane == 0 && ASD_IN(r, nray(D))) {
-    y[r] = v[0] * G.scale;
-    sr[r] = v[1] * G.scale;
+  const long long r = (long long)blockIdx.x * kAxWarps + warp;
+  if (r >= nray(D)) return;  // the whole warp
+  float ys, ss;
+  ax_lane_partial(G, D, r, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? __ldg(x + i) : 0.f; },
+                  ys, ss);
+  ys = warp_sum(ys);
+  ss = warp_sum(ss);
+  if (lane == 0) {
+    y[r] = ys * G.scale;
+    sr[r] = ss * G.scale;
   }
 }
 
@@ -424,14 +391,52 @@ __global__ void __launch_bounds__(128)
 
 // ASD_POCS_cuda.m:117-123: [proj,sumR]=Ax(m); sumR(sumR==0)=1;
 // cor0=P(:,ii)-proj; dd2+=||cor0||^2; cor=cor0./sumR.
-// Also records whether every residual is finite (Scalars::cor_finite), and
-// for 3D geometry writes the view's per-ray slopes ray_tab_c for the
-// backward step that follows (Inst::tabc_mode: a shared table's writer does
-// so even after its own iterations have ended).
+// A ray's squared residual joins its own sum (Inst::ddr), which the end of
+// the sweep adds up, and a residual that is not finite marks its view
+// (Scalars::cor_bad), so a forward step has no block or grid reduction: its
+// warps never wait for each other.  The sinogram value and the running sum
+// are loaded before the march, whose latency covers theirs.  With a ticketed
+// grid reduction per view instead, ten iterations of one 512^2 / 60-view
+// slice took 13.0 ms (11.1 now), four of a batch of 64 23.9 ms (22.2) and 60
+// views of a 256^3 volume 69.8 ms (64.4).
+struct RayOut {
+  float p;    // sinogram value
+  double dd;  // Inst::ddr
+};
+__device__ __forceinline__ RayOut ray_out_load(const Inst &I, int view, long long r,
+                                               long long nr) {
+  const long long pi = (long long)view * nr + r;
+  RayOut o;
+  o.p = ASD_IN(pi, nr * I.nv) ? sino_at(I, pi) : 0.f;
+  o.dd = ASD_IN(r, nr) ? I.ddr[r] : 0.0;
+  return o;
+}
+__device__ __forceinline__ void ray_out_store(const Inst &I, int view, long long r,
+                                              long long nr, const RayOut &o, float yv,
+                                              float srv) {
+  const float c0 = o.p - yv;
+  const float cr = c0 / (srv == 0.f ? 1.f : srv);
+  if (!ASD_IN(r, nr)) return;
+  I.cor[r * I.cor_stride] = cr;
+  I.ddr[r] = o.dd + (double)(c0 * c0);
+  if (!isfinite(cr)) I.s->cor_bad = view + 1;
+}
+
+// The view's ray slopes for the backward step that follows (3-D), rays r0 to
+// r0 + kAxWarps - 1 of the block, by the first lanes of its first warp.
+__device__ __forceinline__ void ray_slopes(const Inst &I, const ViewGeo &G, const Dims &D,
+                                           int view, long long r0, long long nr) {
+  const long long r = r0 + threadIdx.x;
+  if (threadIdx.x >= kAxWarps || r >= nr || !ASD_IN(r, nr)) return;
+  const int ia = (int)(r % D.na), ib = (int)(r / D.na);
+  I.tabC[r] = ray_tab_c(I.tabA[(long long)view * D.na + ia], G.z_det[ib]);
+}
+
+// For 3D geometry also writes the view's ray slopes (Inst::tabc_mode: a
+// shared table's writer does so even after its own iterations have ended).
 template <bool k3D>
 __global__ void __launch_bounds__(kAxBlock)
     k_sart_ax(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap) {
-  __shared__ float sp[kAxCols][kAxWarps][2][32];
   pdl_enter();
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
   if (view >= I.nv) return;
@@ -439,46 +444,24 @@ __global__ void __launch_bounds__(kAxBlock)
   const bool tabc = k3D && (I.tabc_mode == kTabcShared || (!done && I.tabc_mode == kTabcOwn));
   if (done && !tabc) return;
   const Dims D = I.d;
-  const long long nr = (long long)D.na * D.nb;
-  const OwnBlock ob = own_block(dim3((unsigned)((nr + kAxWarps - 1) / kAxWarps), 1));
-  if (ob.bid < 0) return;
+  const long long nr = nray(D), r0 = (long long)blockIdx.x * kAxWarps;
   const ViewGeo G = view_of(I, view);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int rw = warp % kAxWarps, part = warp / kAxWarps;
-  const long long r = (long long)blockIdx.x * kAxWarps + rw;
-  if (tabc && part == 0 && lane == 0 && r < nr && ASD_IN(r, nr)) {
-    const int ia = (int)(r % D.na), ib = (int)(r / D.na);
-    I.tabC[r] = ray_tab_c(I.tabA[(long long)view * D.na + ia], G.z_det[ib]);
-  }
-  if (done) return;  // the whole instance: no reduction
-  float v[2] = {0.f, 0.f};
-  if (r < nr) {
-    const float *m = I.m;
-    ax_lane_partial(G, D, r, lane + 32 * part,
-                    [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; }, v[0], v[1]);
-  }
-  ax_combine<2>(sp, v, part, rw, lane);
-  float pt[2] = {0.f, 0.f};  // dd2, non-finite residuals
-  if (r < nr && part == 0 && lane == 0) {
-    const float yv = v[0] * G.scale, srv = v[1] * G.scale;
-    const long long pi = (long long)view * nr + r;
-    const float c0 = (ASD_IN(pi, nr * I.nv) ? sino_at(I, pi) : 0.f) - yv;
-    const float cr = c0 / (srv == 0.f ? 1.f : srv);
-    if (ASD_IN(r, nr)) I.cor[r * I.cor_stride] = cr;
-    pt[0] = c0 * c0;
-    pt[1] = isfinite(cr) ? 0.f : 1.f;
-  }
-  double tot[2];
-  if (grid_sum<kAxBlock, 2>(pt, I.partials, I.counter, ob.bid, ob.nblocks, tot)) {
-    if (threadIdx.x == 0) {
-      I.s->dd2_acc += tot[0];
-      I.s->cor_finite = tot[1] == 0.0;
-    }
-  }
+  if (tabc) ray_slopes(I, G, D, view, r0, nr);
+  const int lane = threadIdx.x & 31;
+  const long long r = r0 + (threadIdx.x >> 5);
+  if (done || r >= nr) return;  // the whole warp
+  RayOut o{0.f, 0.0};
+  if (lane == 0) o = ray_out_load(I, view, r, nr);
+  const float *m = I.m;
+  float ys, ss;
+  ax_lane_partial(G, D, r, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; }, ys, ss);
+  ys = warp_sum(ys);
+  ss = warp_sum(ss);
+  if (lane == 0) ray_out_store(I, view, r, nr, o, ys * G.scale, ss * G.scale);
 }
 
 // k_sart_ax with the exact projection (siddon_warp_rays): a warp per 32 rays,
-// lane j ray j's residual, normalisation and partial sums.
+// lane j ray j's residual and normalisation.
 template <bool k3D>
 __global__ void __launch_bounds__(kAxBlock)
     k_sart_ax_exact(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap) {
@@ -489,9 +472,7 @@ __global__ void __launch_bounds__(kAxBlock)
   const bool tabc = k3D && (I.tabc_mode == kTabcShared || (!done && I.tabc_mode == kTabcOwn));
   if (done && !tabc) return;
   const Dims D = I.d;
-  const long long nr = (long long)D.na * D.nb;
-  const OwnBlock ob = own_block(dim3((unsigned)((nr + kSidRays - 1) / kSidRays), 1));
-  if (ob.bid < 0) return;
+  const long long nr = nray(D);
   const ViewGeo G = view_of(I, view);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long r0 = ((long long)blockIdx.x * kAxWarps + warp) * 32, r = r0 + lane;
@@ -499,30 +480,13 @@ __global__ void __launch_bounds__(kAxBlock)
     const int ia = (int)(r % D.na), ib = (int)(r / D.na);
     I.tabC[r] = ray_tab_c(I.tabA[(long long)view * D.na + ia], G.z_det[ib]);
   }
-  if (done) return;  // the whole instance: no reduction
+  if (done || r0 >= nr) return;  // the whole warp
   float yv = 0.f, sv = 0.f;
-  if (r0 < nr) {  // warp-uniform
-    const float *m = I.m;
-    siddon_warp_rays(G, D, r0, nr, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; },
-                     yv, sv);
-  }
-  float pt[2] = {0.f, 0.f};  // dd2, non-finite residuals
-  if (r < nr) {
-    const float yy = yv * G.scale, srv = sv * G.scale;
-    const long long pi = (long long)view * nr + r;
-    const float c0 = (ASD_IN(pi, nr * I.nv) ? sino_at(I, pi) : 0.f) - yy;
-    const float cr = c0 / (srv == 0.f ? 1.f : srv);
-    if (ASD_IN(r, nr)) I.cor[r * I.cor_stride] = cr;
-    pt[0] = c0 * c0;
-    pt[1] = isfinite(cr) ? 0.f : 1.f;
-  }
-  double tot[2];
-  if (grid_sum<kAxBlock, 2>(pt, I.partials, I.counter, ob.bid, ob.nblocks, tot)) {
-    if (threadIdx.x == 0) {
-      I.s->dd2_acc += tot[0];
-      I.s->cor_finite = tot[1] == 0.0;
-    }
-  }
+  const float *m = I.m;
+  siddon_warp_rays(G, D, r0, nr, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; },
+                   yv, sv);
+  if (r < nr)
+    ray_out_store(I, view, r, nr, ray_out_load(I, view, r, nr), yv * G.scale, sv * G.scale);
 }
 
 // Planar chord for a window whose rays share dominant axis AX (1: x, 2: y;
@@ -736,7 +700,7 @@ __global__ void __launch_bounds__(kAtxThreads, 4)
   const ViewGeo G = view_of(I, view);
   const float4 *tabA = I.tabA + (long long)view * D.na;
   const int vf = I.vflags[view];
-  const bool narrow = !(vf & kViewAxisParallel) && I.s->cor_finite &&
+  const bool narrow = !(vf & kViewAxisParallel) && I.s->cor_bad != view + 1 &&
                       (!kPlanar || G.z_det[0] == 0.0f);
   if (kPlanar && narrow && I.chtab)
     sart_atx_tiles_tab(I, G, D, I.chtab + (size_t)view * chord_view_words(D, I.chK), I.chK);
@@ -913,7 +877,7 @@ __global__ void __launch_bounds__(kAtxThreads, 4)
   if (!zcol_thread(D, seg, ix, iy, z0, z1)) return;
   const ViewGeo G = view_of(I, view);
   const float4 *tabA = I.tabA + (long long)view * D.na;
-  const bool narrow = !(I.vflags[view] & kViewAxisParallel) && I.s->cor_finite;
+  const bool narrow = !(I.vflags[view] & kViewAxisParallel) && I.s->cor_bad != view + 1;
   const float beta = I.s->beta_f;
   float *m = I.m;
   const float *__restrict__ cor = I.cor;
@@ -1328,7 +1292,7 @@ __global__ void __launch_bounds__(kAtxThreads, kPlanar ? 4 : 5)
     s_beta[threadIdx.x] = Ib.s->beta_f;
     if (live) {
       atomicOr(&s_active, 1u << threadIdx.x);
-      if (!Ib.s->cor_finite) atomicAnd(&s_finite, 0);
+      if (Ib.s->cor_bad == view + 1) atomicAnd(&s_finite, 0);
     }
   }
   __syncthreads();
@@ -1363,9 +1327,9 @@ __global__ void __launch_bounds__(kAtxThreads, kPlanar ? 4 : 5)
 // instances.  The column march (cells and weights) is evaluated once per ray
 // and each piece reads the group's voxel values with kShareGroup / 4 float4 loads
 // from the interleaved images; every instance accumulates its pieces in the
-// order of k_sart_ax and sums lanes with the same butterfly, and its block
-// partials, reduction order and epilogue are those of k_sart_ax, so its
-// projection, residual, dd2 and flags are bit-identical to it.
+// order of k_sart_ax and sums lanes with the same butterfly, and its
+// epilogue is that of k_sart_ax, so its projection, residual, squares and
+// flags are bit-identical to it.
 // ---------------------------------------------------------------------------
 // columns per round of loads in the shared forward step: two for fan beams
 // (measured 6 % faster than one); one for cone beams, whose three pieces per
@@ -1392,11 +1356,6 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
   pdl_enter();
   // this block: kQ of the group's quads (4 instances each), from q0
   constexpr int kS = 4 * kQ;
-  __shared__ unsigned s_active;
-  __shared__ float sp[kAxCols][kAxWarps][kS + 1][32];
-  __shared__ float s_part[2][kAxWarps][kS];
-  __shared__ int s_last[kS];
-  __shared__ int s_nlast;
   const int q0 = (int)(blockIdx.z % (kQuads / kQ)) * kQ;
   const int gz = (int)(blockIdx.z / (kQuads / kQ));                  // the group
   const int g0 = gtab ? gtab[gz].x : gz * kShareGroup;
@@ -1406,35 +1365,26 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
   const Inst &I0 = insts[g0];
   if (view >= I0.nv) return;
   const Dims D = I0.d;
-  const long long nr = (long long)D.na * D.nb;
-  const OwnBlock ob = own_block(dim3((unsigned)((nr + kAxWarps - 1) / kAxWarps), 1));
-  if (ob.bid < 0) return;
-  if (threadIdx.x == 0) {
-    s_active = 0u;
-    s_nlast = 0;
-  }
-  __syncthreads();
-  if (threadIdx.x < gn &&
-      ((volatile int *)&insts[gi + threadIdx.x].s->done)[0] == 0)
-    atomicOr(&s_active, 1u << threadIdx.x);
-  __syncthreads();
-  const unsigned active = s_active;
+  const long long nr = nray(D), r0 = (long long)blockIdx.x * kAxWarps;
+  const int lane = threadIdx.x & 31;
+  const long long r = r0 + (threadIdx.x >> 5);
   const ViewGeo G = view_of(I0, view);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int rw = warp % kAxWarps, part = warp / kAxWarps;
-  const long long r = (long long)blockIdx.x * kAxWarps + rw;
   // cone beam: the plan's one ray-slope table, refreshed by group 0 every
   // view whether or not its instances still run
-  if (k3D && blockIdx.z == 0 && part == 0 && lane == 0 && r < nr && ASD_IN(r, nr)) {
-    const int ia = (int)(r % D.na), ib = (int)(r / D.na);
-    I0.tabC[r] = ray_tab_c(I0.tabA[(long long)view * D.na + ia], G.z_det[ib]);
-  }
+  if (k3D && blockIdx.z == 0) ray_slopes(I0, G, D, view, r0, nr);
+  if (r >= nr) return;  // the whole warp
+  // lane b: instance gi + b
+  const Inst &Ib = insts[gi + min(lane, gn - 1)];
+  const bool live = lane < gn && ((volatile int *)&Ib.s->done)[0] == 0;
+  const unsigned active = __ballot_sync(0xffffffffu, live);
   if (!active) return;
+  RayOut o{0.f, 0.0};
+  if (live) o = ray_out_load(Ib, view, r, nr);
   float v[kS + 1];  // the instances' sums, then the weights' sum
 #pragma unroll
   for (int b = 0; b <= kS; b++) v[b] = 0.f;
   const float4 *__restrict__ mg = (const float4 *)I0.m_il;
-  if (r < nr) {
+  {
     const int ia = (int)(r % D.na), ib = (int)(r / D.na);
     const float zd = G.z_det[ib];
     const RayMarch R = ray_setup(G, D, G.y_det[ia], zd);
@@ -1443,13 +1393,13 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
     // (predicated) loads, then the accumulation in column and piece order
     auto march = [&](auto pieces) {
       constexpr int kP = decltype(pieces)::value;
-      for (int iu0 = lane + 32 * part; iu0 < R.nu; iu0 += 32 * kAxCols * kU) {
+      for (int iu0 = lane; iu0 < R.nu; iu0 += 32 * kU) {
         unsigned id[kU][kP];
         float w[kU][kP];
         bool f[kU][kP];
 #pragma unroll
         for (int u = 0; u < kU; u++) {
-          const int iu = iu0 + u * 32 * kAxCols;
+          const int iu = iu0 + u * 32;
           if constexpr (kP == 2)
             column_pieces_planar(R, iu, id[u], w[u], f[u]);
           else
@@ -1490,58 +1440,13 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
     else if constexpr (k3D)
       march(std::integral_constant<int, 3>());
   }
-  ax_combine<kS + 1>(sp, v, part, rw, lane);
-  // part-0 lane b: the epilogue of k_sart_ax for instance gi + b
+#pragma unroll
+  for (int b = 0; b <= kS; b++) v[b] = warp_sum(v[b]);
   float yb = 0.f;
 #pragma unroll
   for (int b = 0; b < kS; b++)
     if (lane == b) yb = v[b];
-  float p0 = 0.f, p1 = 0.f;
-  if (part == 0 && lane < gn && ((active >> lane) & 1u) && r < nr) {
-    const Inst &Ib = insts[gi + lane];
-    const float yv = yb * G.scale, srv = v[kS] * G.scale;
-    const long long pi = (long long)view * nr + r;
-    const float c0 = (ASD_IN(pi, nr * Ib.nv) ? sino_at(Ib, pi) : 0.f) - yv;
-    const float cr = c0 / (srv == 0.f ? 1.f : srv);
-    if (ASD_IN(r, nr)) Ib.cor[r * Ib.cor_stride] = cr;
-    p0 = c0 * c0;
-    p1 = isfinite(cr) ? 0.f : 1.f;
-  }
-  if (part == 0 && lane < kS) {
-    s_part[0][rw][lane] = p0;
-    s_part[1][rw][lane] = p1;
-  }
-  __syncthreads();
-  // per instance: the block total of k_sart_ax's block_sum_f (lane 0 of the
-  // part-0 warps 0..3 the only nonzero values; combined as
-  // (w0 + w2) + (w1 + w3)), its partial, its ticket
-  static_assert(kAxWarps == 4, "block totals below follow block_sum_f for 4 warps");
-  if (threadIdx.x < gn && ((active >> threadIdx.x) & 1u)) {
-    const int b = threadIdx.x;
-    const Inst &Ib = insts[gi + b];
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const float t = (s_part[k][0][b] + s_part[k][2][b]) + (s_part[k][1][b] + s_part[k][3][b]);
-      Ib.partials[(long long)ob.bid * 2 + k] = (double)t;
-    }
-    __threadfence();
-    if (atomicAdd(Ib.counter, 1u) == (unsigned)ob.nblocks - 1)
-      s_last[atomicAdd(&s_nlast, 1)] = b;
-  }
-  __syncthreads();
-  const int nlast = s_nlast;
-  if (nlast == 0) return;
-  __threadfence();
-  for (int i = 0; i < nlast; i++) {
-    const Inst &Ib = insts[gi + s_last[i]];
-    double tot[2];
-    // the final sum of k_sart_ax's reduction (its kAxBlock threads' order)
-    grid_sum_final<kAxBlock, 2>(Ib.partials, Ib.counter, ob.nblocks, tot);
-    if (threadIdx.x == 0) {
-      Ib.s->dd2_acc += tot[0];
-      Ib.s->cor_finite = tot[1] == 0.0;
-    }
-  }
+  if (live) ray_out_store(Ib, view, r, nr, o, yb * G.scale, v[kS] * G.scale);
 }
 
 // Rounds an FP32 sinogram to FP16 / BF16 storage (round to nearest, ties to
@@ -1790,11 +1695,6 @@ cudaError_t launch_view_tables(const Inst *insts, int batch, const Dims &d,
 ASD_CHECKED_READER(checked_take_proj)
 #endif
 
-int reduce_blocks_for(const Dims &d) {
-  const long long nr = (long long)d.na * d.nb;
-  const long long ax = (nr + kAxWarps - 1) / kAxWarps;
-  const long long at = atx_blocks(d);
-  return (int)(ax > at ? ax : at);
-}
+int reduce_blocks_for(const Dims &d) { return atx_blocks(d); }
 
 }  // namespace asd

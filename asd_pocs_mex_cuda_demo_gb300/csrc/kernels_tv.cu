@@ -59,21 +59,6 @@ __device__ __forceinline__ Tv2Terms tv2_terms(float dx, float dy) {
   const float r = tv_rsqrt(__fmaf_rn(dy, dy, __fmaf_rn(dx, dx, eps)));
   return Tv2Terms{__fmul_rn(__fadd_rn(dx, dy), r), __fmul_rn(dx, r), __fmul_rn(dy, r)};
 }
-__device__ __forceinline__ float tv2_combine(float g1, float q_right, float t_below) {
-  return __fsub_rn(__fsub_rn(g1, q_right), t_below);
-}
-template <class U>
-__device__ __forceinline__ float tv_grad2f(const U &u) {
-  const float c0 = u(0, 0, 0);
-  const float xm = u(-1, 0, 0), ym = u(0, -1, 0);
-  const float xp = u(1, 0, 0), yp = u(0, 1, 0);
-  const float xpym = u(1, -1, 0), xmyp = u(-1, 1, 0);
-  const Tv2Terms here = tv2_terms(__fsub_rn(c0, xm), __fsub_rn(c0, ym));
-  const Tv2Terms right = tv2_terms(__fsub_rn(xp, c0), __fsub_rn(xp, xpym));
-  const Tv2Terms below = tv2_terms(__fsub_rn(yp, xmyp), __fsub_rn(yp, c0));
-  return tv2_combine(here.g1, right.q, below.t);
-}
-
 // FP32 form of the 3-D stencil with every rounding explicit.  At a voxel
 // with differences dx, dy, dz to its -x, -y, -z neighbours,
 //   r = 1/sqrt(eps + dx^2 + dy^2 + dz^2),
@@ -110,14 +95,6 @@ __device__ __forceinline__ float tv_grad3f(const U &u) {
   const float ry = tv3_r(__fsub_rn(yp, u(-1, 1, 0)), __fsub_rn(yp, c), __fsub_rn(yp, u(0, 1, -1)));
   const float rz = tv3_r(__fsub_rn(zp, u(-1, 0, 1)), __fsub_rn(zp, u(0, -1, 1)), __fsub_rn(zp, c));
   return __fmul_rn(2.f, tv3_u(tv3_inslice(c, xm, ym, zm, xp, yp, r, rx, ry), c, zp, rz));
-}
-
-template <bool k3D, class U>
-__device__ __forceinline__ float tv_grad_f(const U &u) {
-  if constexpr (k3D)
-    return tv_grad3f(u);
-  else
-    return tv_grad2f(u);
 }
 
 // ------------------------------------- standalone TV (the TV entry points)
@@ -526,11 +503,11 @@ __device__ __forceinline__ void finish_scalars(Scalars *s, double dg2) {
 
 // The sweep's scalars from the totals of (m - m_pre)^2, (m - m_k1)^2,
 // (m - I0)^2 and v(m)^2 (ASD_POCS_cuda.m:137-149, imgTVGradMin.cpp:57-60).
-__device__ __forceinline__ void sweep_scalars(const Inst &I, const double (&tot)[4]) {
+__device__ __forceinline__ void sweep_scalars(const Inst &I, const double (&tot)[4],
+                                              double dd2) {
   Scalars *s = I.s;
   const double N = (double)I.d.nx * I.d.ny * I.d.nz;
-  s->dd2 = s->dd2_acc;
-  s->dd2_acc = 0.0;
+  s->dd2 = dd2;
   s->dp = sqrt(tot[0]);
   if (s->has_ref) I.rmse[s->k - 1] = sqrt(tot[2] / N);
   s->iterations = s->k;
@@ -543,13 +520,28 @@ __device__ __forceinline__ void sweep_scalars(const Inst &I, const double (&tot)
   }
 }
 
+// Part `u` of `n` of the sweep's squared residuals (Inst::ddr), summed by a
+// warp in a fixed order and cleared for the next sweep.
+__device__ __forceinline__ double take_residuals(const Inst &I, int u, int n) {
+  const long long nr = (long long)I.d.na * I.d.nb, per = (nr + n - 1) / n;
+  const long long end = min(nr, (u + 1) * per);
+  double a = 0.0;
+  for (long long r = u * per + (threadIdx.x & 31); r < end; r += 32) {
+    if (!ASD_IN(r, nr)) continue;
+    a += I.ddr[r];
+    I.ddr[r] = 0.0;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
+}
+
 // After the SART sweep (ASD_POCS_cuda.m:137-149): dd, m_res, RMSE, dp and the
 // stop test; d = ||m - m_k1|| (imgTVGradMin.cpp:57-60) and ||v|| of the first
 // TV step, giving its step size alpha*d/||v||.
-template <bool k3D>
 __global__ void __launch_bounds__(kThreads)
     k_after_sweep(const Inst *__restrict__ insts, const int *__restrict__ zmap) {
-  __shared__ Tile<1, k3D> t;
+  __shared__ Tile<1, true> t;
   pdl_enter();
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
   if (inst_done(I)) return;
@@ -581,15 +573,21 @@ __global__ void __launch_bounds__(kThreads)
       }
       if (tv) {
         const float gr =
-            tv_grad_f<k3D>(TileAt<1, k3D>{t, tx + 1, ty + 1, k3D ? 1 : 0});
+            tv_grad3f(TileAt<1, true>{t, tx + 1, ty + 1, 1});
         v[3] += gr * gr;
       }
     }
     __syncthreads();  // the tile is reused by the next group member
   }
-  double tot[4];
+  double *const ddp = I.partials + 4ll * ob.nblocks;  // after grid_sum's partials
+  if (threadIdx.x < 32) {
+    const double dd = take_residuals(I, ob.bid, ob.nblocks);
+    if (threadIdx.x == 0) ddp[ob.bid] = dd;  // published by grid_sum's fence
+  }
+  double tot[4], dd2[1];
   if (grid_sum<kThreads, 4>(v, I.partials, I.counter, ob.bid, ob.nblocks, tot)) {
-    if (threadIdx.x == 0) sweep_scalars(I, tot);
+    grid_sum_final<kThreads, 1>(ddp, I.counter, ob.nblocks, dd2);
+    if (threadIdx.x == 0) sweep_scalars(I, tot, dd2[0]);
   }
 }
 
@@ -880,7 +878,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 8)
 }
 
 // End of the SART sweep for 2-D instances as column walks (the work of
-// k_after_sweep<false>): the same strips, bands and ring as k_tv_walk2d,
+// k_after_sweep): the same strips, bands and ring as k_tv_walk2d,
 // streaming m, m_pre, m_k1 and the reference image I0 through four rings.
 // Each output voxel copies m to m_res and adds (m - m_pre)^2, (m - m_k1)^2,
 // (m - I0)^2 and v(m)^2 (tv2_terms, the TV step's own stencil) to its
@@ -989,6 +987,12 @@ __global__ void __launch_bounds__(kWalkWarps * 32)
   const int y0 = b0 * kBandRows, y1 = min(D.ny, (b0 + bands) * kBandRows);
   const int xa = strip * kWalkOut - 2 + 2 * lane;
   const bool tv = I.s->ng > 0;
+  // the squared residuals: a part per strip and band, as the other partials
+  const int P = S * NB;
+  for (int b = b0; b < min(NB, b0 + bands); b++) {
+    const double dd = take_residuals(I, b * S + strip, P);
+    if (lane == 0) I.partials[4ll * P + b * S + strip] = dd;
+  }
   if ((D.nx & 1) == 0)
     sweep_walk<true>(I, y0, y1, xa, strip, S, tv, ring[threadIdx.x >> 5]);
   else
@@ -1001,8 +1005,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32)
   ticket = __shfl_sync(0xffffffffu, ticket, 0);
   if (ticket != (unsigned)walks - 1) return;
   __threadfence();
-  const int P = S * NB;
-  double tot[4];
+  double tot[4], dd2 = 0.0;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     double a = 0.0;
@@ -1011,9 +1014,12 @@ __global__ void __launch_bounds__(kWalkWarps * 32)
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     tot[k] = a;
   }
+  for (int p = lane; p < P; p += 32) dd2 += ((volatile const double *)I.partials)[4ll * P + p];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dd2 += __shfl_xor_sync(0xffffffffu, dd2, o);
   if (lane == 0) {
     *I.counter = 0u;
-    sweep_scalars(I, tot);
+    sweep_scalars(I, tot, dd2);
   }
 }
 
@@ -1439,7 +1445,7 @@ cudaError_t launch_after_sweep(const Inst *insts, int batch, const Dims &d,
                                cudaStream_t st, const int *zmap) {
   const dim3 grid = group_grid(d.nx, d.ny, d.nz, batch);
   if (d.nz > 1) {
-    return launch_iter(k_after_sweep<true>, grid, dim3(kThreads), st, insts, zmap);
+    return launch_iter(k_after_sweep, grid, dim3(kThreads), st, insts, zmap);
   } else {
     // one band per walk up to a wave of walks (24 resident warps per SM at
     // 80 registers), then longer walks
