@@ -1393,17 +1393,25 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
     // (predicated) loads, then the accumulation in column and piece order
     auto march = [&](auto pieces) {
       constexpr int kP = decltype(pieces)::value;
-      for (int iu0 = lane; iu0 < R.nu; iu0 += 32 * kU) {
+      for (int iu0 = lane; iu0 - lane < R.nu; iu0 += 32 * kU) {
         unsigned id[kU][kP];
         float w[kU][kP];
         bool f[kU][kP];
+        if constexpr (kP == 2) {
 #pragma unroll
-        for (int u = 0; u < kU; u++) {
-          const int iu = iu0 + u * 32;
-          if constexpr (kP == 2)
-            column_pieces_planar(R, iu, id[u], w[u], f[u]);
-          else
-            column_pieces3(R, iu, id[u], w[u], f[u]);
+          for (int u = 0; u < kU; u++)
+            column_pieces_planar(R, iu0 + u * 32, id[u], w[u], f[u]);
+        } else {
+          Column3 c[kU];
+          bool some = false;
+#pragma unroll
+          for (int u = 0; u < kU; u++) {
+            c[u] = column_cells3(R, iu0 + u * 32);
+            some = some || ((c[u].vlo || c[u].vhi) && (c[u].zlo || c[u].zhi));
+          }
+          if (!any_lane(some)) continue;
+#pragma unroll
+          for (int u = 0; u < kU; u++) column_pieces3(R, iu0 + u * 32, c[u], id[u], w[u], f[u]);
         }
         float4 x[kU][kP][kQ];
 #pragma unroll
