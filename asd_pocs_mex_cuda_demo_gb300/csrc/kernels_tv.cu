@@ -109,18 +109,27 @@ __device__ __forceinline__ float tv_grad3f(const U &u) {
 // and step and saves evaluating the stencil twice: the FP64 rate bounds the
 // mex functions, and one stencil there is one reciprocal square root and
 // about 20 other operations (the denominators of the reference's later terms
-// are its neighbours' first ones).  Blocks walk items of a 32 x 16 tile (and
-// a slab of slices in 3-D), the updated slices and the reciprocal roots of
+// are its neighbours' first ones).  Blocks walk items of a 32 x 32 tile and a
+// slab of slices (2-D: a 32 x 16 tile), the updated slices and the reciprocal roots of
 // the tile and its halo in shared memory, one barrier per slice.  Block sums
 // are added in block order by the blocks of the next kernel, so there is no
 // reduction pass and a run gives the same bits as any other.
-// Measured per step (ncu): 128^3 FP64 848 us as a norm and an update kernel
-// that each evaluated the stencil with a square root and a division per term.
-constexpr int kTvX = 32, kTvY = 16, kTvT = kTvX * kTvY;  // tile and threads
-constexpr int kTvBlocks = 2048;                          // most blocks of a step
-constexpr int kTvHalo = 2 * (kTvX + 2) + 2 * kTvY;       // halo cells of a slice
-constexpr int kTvRx = kTvX + kTvY + 1;                   // roots beside the tile
-static_assert(kTvHalo <= kTvT && kTvRx <= kTvT, "a thread takes at most one of each");
+// Measured per step (ncu), against a norm and an update kernel that each
+// evaluated the stencil from global memory with a square root and a division
+// per term: 256^3 FP32 64 us (459 us; 40 us at HBM rate), 128^3 FP64 108 us
+// (848 us; bound by the FP64 units, 85 % busy).
+constexpr int kTvX = 32, kTvT = 256;  // tile width, threads (a warp per kRows rows)
+constexpr int kTvBlocks = 2048;       // most blocks of a step
+// rows of a thread: four in 3-D (the halo and the barriers cost a quarter of
+// what they do at one; the rows above and below come from registers), two in
+// 2-D, where a 256^2 image would not fill the SMs with taller tiles
+template <bool k3D>
+constexpr int kTvRows = k3D ? 4 : 2;
+template <bool k3D>
+constexpr int kTvY = kTvT / kTvX * kTvRows<k3D>;
+// resident blocks per SM: as many as the registers hold without spills
+template <class T, bool k3D>
+constexpr int kTvResident = (sizeof(T) == 8 ? 2 : 4) + (k3D ? 0 : 1);
 
 template <class T>
 __device__ __forceinline__ T tv_recip_root(T den);
@@ -186,20 +195,26 @@ struct TvGrid {
 // kFirst: the stencil of the image itself (no update) and the squared
 // distance to `uin`, the old image (null: zeros).
 template <class T, bool k3D, bool kFirst>
-__global__ void __launch_bounds__(kTvT, sizeof(T) == 8 ? 2 : 3)
+__global__ void __launch_bounds__(kTvT, (kTvResident<T, k3D>))
     k_tv_step(const T *__restrict__ m, const T *__restrict__ uin, T *__restrict__ mout,
               T *__restrict__ uout, TvGrid g, int step, double alpha, double *scal,
               const double *__restrict__ pin, int np, double *__restrict__ pout) {
-  __shared__ T P[k3D ? 3 : 1][kTvY + 2][kTvX + 2];  // updated slices
-  __shared__ T R[k3D ? 2 : 1][kTvY + 1][kTvX + 1];  // their reciprocal roots
+  constexpr int kR = kTvRows<k3D>, kY = kTvY<k3D>;
+  constexpr int kHalo = 2 * (kTvX + 2) + 2 * kY;  // halo cells of a slice
+  constexpr int kRx = kTvX + kY + 1;              // roots beside the tile
+  constexpr int kRx0 = kTvT - (kRx + 31) / 32 * 32;  // taken by the last warps
+  static_assert(kHalo <= kTvT && kRx0 >= 0, "a thread takes at most one of each");
+  __shared__ T P[k3D ? 3 : 1][kY + 2][kTvX + 2];  // updated slices
+  __shared__ T R[k3D ? 2 : 1][kY + 1][kTvX + 1];  // their reciprocal roots
   __shared__ double red[2][kTvT / 32];
   pdl_enter();
-  const int t = threadIdx.x, lx = t & 31, ly = t >> 5;
+  const int t = threadIdx.x, lx = t & 31, wy = t >> 5, ly = wy * kR;
   // this thread's halo cell and root beside the tile (rows and columns of P)
-  const int hy = t < 34 ? 0 : t < 68 ? kTvY + 1 : 1 + (t - 68) % kTvY;
-  const int hx = t < 34 ? t : t < 68 ? t - 34 : t < 68 + kTvY ? 0 : kTvX + 1;
-  const bool halo = t < kTvHalo, rext = t < kTvRx;
-  const int ey = t <= kTvY ? 1 + t : 1 + kTvY, ex = t <= kTvY ? 1 + kTvX : t - kTvY;
+  const int hy = t < 34 ? 0 : t < 68 ? kY + 1 : 1 + (t - 68) % kY;
+  const int hx = t < 34 ? t : t < 68 ? t - 34 : t < 68 + kY ? 0 : kTvX + 1;
+  const int e = t - kRx0;
+  const bool halo = t < kHalo, rext = e >= 0 && e < kRx;
+  const int ey = e <= kY ? 1 + e : 1 + kY, ex = e <= kY ? 1 + kTvX : e - kY;
   const long long plane = (long long)g.nx * g.ny;
   const long long nvox = plane * g.nz;
   T coef = T(0);
@@ -208,57 +223,69 @@ __global__ void __launch_bounds__(kTvT, sizeof(T) == 8 ? 2 : 3)
   for (int item = blockIdx.x; item < g.items; item += gridDim.x) {
     const int tile = item % (g.tx * g.ty), z0 = item / (g.tx * g.ty) * g.slab;
     const int z1 = min(g.nz, z0 + g.slab);
-    const int x0 = tile % g.tx * kTvX, y0 = tile / g.tx * kTvY;
+    const int x0 = tile % g.tx * kTvX, y0 = tile / g.tx * kY;
     const int cx = x0 + lx, cy = y0 + ly, gx = x0 - 1 + hx, gy = y0 - 1 + hy;
-    const bool cin = cx < g.nx && cy < g.ny;
     const bool hin = halo && gx >= 0 && gx < g.nx && gy >= 0 && gy < g.ny;
-    const long long co = (long long)cy * g.nx + cx, ho = (long long)gy * g.nx + gx;
-    T cm, cu, hm, hu;  // the slice in flight: tile cell and halo cell of m and u
+    const int rows = cx < g.nx ? min(max(g.ny - cy, 0), kR) : 0;  // in the image
+    // the thread's first cell and its halo cell in the slice to fetch
+    long long co = (long long)cy * g.nx + cx, ho = (long long)gy * g.nx + gx;
+    long long wo = co;  // the first cell in the slice to write
+    if (k3D) {
+      co += (z0 - 1) * plane;
+      ho += (z0 - 1) * plane;
+      wo += z0 * plane;
+    }
+    T cm[kR], cu[kR], hm, hu;  // the slice in flight: m and u of both
     auto fetch = [&](int z) {
-      const bool in = z >= 0 && z < g.nz;
-      const long long zo = (long long)z * plane;
-      const bool a = in && cin && ASD_IN(zo + co, nvox), b = in && hin && ASD_IN(zo + ho, nvox);
-      cm = a ? m[zo + co] : T(0);
-      hm = b ? m[zo + ho] : T(0);
-      if (kFirst) {
-        cu = a && uin ? uin[zo + co] : T(0);  // the old image
-        hu = T(0);
-      } else {
-        cu = a ? uin[zo + co] : T(0);
-        hu = b ? uin[zo + ho] : T(0);
+      const bool in = !k3D || (z >= 0 && z < g.nz);
+#pragma unroll
+      for (int j = 0; j < kR; j++) {
+        const long long i = co + j * g.nx;
+        const bool a = in && j < rows && ASD_IN(i, nvox);
+        cm[j] = a ? m[i] : T(0);
+        cu[j] = a && (!kFirst || uin) ? uin[i] : T(0);  // kFirst: the old image
       }
+      const bool a = in && hin && ASD_IN(ho, nvox);
+      hm = a ? m[ho] : T(0);
+      hu = a && !kFirst ? uin[ho] : T(0);
+      co += plane;
+      ho += plane;
     };
-    // the fetched slice's updated values (cells outside the image are zeros:
-    // so is their u) into P[q]; returns the tile cell's
-    auto place = [&](int q) {
-      const T c = kFirst || !cin ? cm : cm - coef * cu;
-      const T h = kFirst || !hin ? hm : hm - coef * hu;
-      P[q][ly + 1][lx + 1] = c;
-      if (halo) P[q][hy][hx] = h;
-      return c;
+    // the fetched slice's updated values into P[q] and n (cells outside the
+    // image are zeros, and so is their u)
+    auto place = [&](int q, T (&n)[kR]) {
+#pragma unroll
+      for (int j = 0; j < kR; j++) {
+        n[j] = kFirst || j >= rows ? cm[j] : cm[j] - coef * cu[j];
+        P[q][ly + j + 1][lx + 1] = n[j];
+      }
+      if (halo) P[q][hy][hx] = kFirst || !hin ? hm : hm - coef * hu;
     };
-    // reciprocal root of cell (y, x) of P[q], over the slice P[q0] (3-D);
-    // s: the sum of its three differences
-    auto root = [&](int q, int q0, int y, int x, T &s) {
-      const T c = P[q][y][x];
-      const T dx = c - P[q][y][x - 1], dy = c - P[q][y - 1][x];
+    // reciprocal root of a cell from its differences; s: their sum
+    auto root = [&](T dx, T dy, T dz, T &s) {
       T den = tv_eps<T>() + dx * dx + dy * dy;
       s = dx + dy;
       if (k3D) {
-        const T dz = c - P[q0][y][x];
         den += dz * dz;
         s += dz;
       }
       return tv_recip_root(den);
     };
-    auto roots = [&](int r, int q, int q0, T &s) {
-      const T own = root(q, q0, ly + 1, lx + 1, s);
-      R[r][ly][lx] = own;
+    // roots of the slice n in P[q] over the slice `prev` in P[q0], into R[r]
+    auto roots = [&](int r, int q, int q0, const T (&n)[kR], const T (&prev)[kR], T (&own)[kR],
+                     T (&s)[kR]) {
+#pragma unroll
+      for (int j = 0; j < kR; j++) {
+        const T up = j ? n[j - 1] : P[q][ly][lx + 1];
+        own[j] = root(n[j] - P[q][ly + j + 1][lx], n[j] - up, n[j] - prev[j], s[j]);
+        R[r][ly + j][lx] = own[j];
+      }
       if (rext) {
         T dummy;
-        R[r][ey - 1][ex - 1] = root(q, q0, ey, ex, dummy);
+        const T c = P[q][ey][ex];
+        R[r][ey - 1][ex - 1] = root(c - P[q][ey][ex - 1], c - P[q][ey - 1][ex],
+                                    k3D ? c - P[q0][ey][ex] : T(0), dummy);
       }
-      return own;
     };
     float accf[2] = {0.f, 0.f};
     auto add = [&](int k, T v) {
@@ -267,57 +294,74 @@ __global__ void __launch_bounds__(kTvT, sizeof(T) == 8 ? 2 : 3)
       else
         accf[k] += (float)v;
     };
-    // u of the tile cell in P[q], R[r] and what the slice above it adds
-    auto emit = [&](long long zo, int q, int r, T s, T own, T above) {
-      const T c = P[q][ly + 1][lx + 1];
-      T u = s * own;
-      u += (c - P[q][ly + 2][lx + 1]) * R[r][ly + 1][lx];
-      u += (c - P[q][ly + 1][lx + 2]) * R[r][ly][lx + 1];
-      u += above;
-      if (!cin || !ASD_IN(zo + co, nvox)) return;
-      uout[zo + co] = u;
-      if (!kFirst) mout[zo + co] = c;
-      add(0, u * u);
-    };
     auto distance = [&]() {
-      if (kFirst && cin) {
-        const T d = cm - cu;
-        add(1, d * d);
-      }
+      if (kFirst)
+#pragma unroll
+        for (int j = 0; j < kR; j++)
+          if (j < rows) {
+            const T d = cm[j] - cu[j];
+            add(1, d * d);
+          }
     };
-    fetch(k3D ? z0 - 1 : 0);
+    // u of the slice c in P[q], R[r]; `above`: the term of the slice above
+    auto emit = [&](int q, int r, const T (&c)[kR], const T (&own)[kR], const T (&s)[kR],
+                    const T (&above)[kR]) {
+#pragma unroll
+      for (int j = 0; j < kR; j++) {
+        const T yp = j + 1 < kR ? c[j + 1 < kR ? j + 1 : j] : P[q][ly + kR + 1][lx + 1];
+        const T ry = j + 1 < kR ? own[j + 1 < kR ? j + 1 : j] : R[r][ly + kR][lx];
+        T u = s[j] * own[j];
+        u += (c[j] - yp) * ry;
+        u += (c[j] - P[q][ly + j + 1][lx + 2]) * R[r][ly + j][lx + 1];
+        u += above[j];
+        const long long i = wo + j * g.nx;
+        if (j >= rows || !ASD_IN(i, nvox)) continue;
+        uout[i] = u;
+        if (!kFirst) mout[i] = c[j];
+        add(0, u * u);
+      }
+      wo += plane;
+    };
+    T c[kR], own[kR], s[kR], n[kR], own1[kR], s1[kR], above[kR];
+    fetch(z0 - 1);
     if (!sized) coef = (T)tv_step_size(pin, np, step, alpha, scal);  // has a barrier
     sized = true;
     if (item != (int)blockIdx.x) __syncthreads();  // P and R are reused
     if (!k3D) {
       distance();
-      place(0);
+      place(0, c);
       __syncthreads();
-      T s;
-      const T own = roots(0, 0, 0, s);
+      roots(0, 0, 0, c, c, own, s);
       __syncthreads();
-      emit(0, 0, 0, s, own, T(0));
+#pragma unroll
+      for (int j = 0; j < kR; j++) above[j] = T(0);
+      emit(0, 0, c, own, s, above);
     } else {
-      place((z0 + 2) % 3);  // slice z in P[z % 3], its roots in R[z & 1]
+      place((z0 + 2) % 3, n);  // slice z in P[z % 3], its roots in R[z & 1]
       fetch(z0);
       distance();
-      T c = place(z0 % 3);
+      place(z0 % 3, c);
       fetch(z0 + 1);
       __syncthreads();
-      T s, own = roots(z0 & 1, z0 % 3, (z0 + 2) % 3, s);
+      roots(z0 & 1, z0 % 3, (z0 + 2) % 3, c, n, own, s);
       int q = z0 % 3;
+#pragma unroll 1
       for (int z = z0; z < z1; z++) {
         const int q1 = q == 2 ? 0 : q + 1;
         if (z + 1 < z1) distance();  // slice z + 1 is in flight
-        const T n = place(q1);
+        place(q1, n);
         if (z + 1 < z1) fetch(z + 2);
         __syncthreads();
-        T s1;
-        const T own1 = roots((z + 1) & 1, q1, q, s1);
-        emit((long long)z * plane, q, z & 1, s, own, (c - n) * own1);
-        c = n;
-        s = s1;
-        own = own1;
+        roots((z + 1) & 1, q1, q, n, c, own1, s1);
+#pragma unroll
+        for (int j = 0; j < kR; j++) above[j] = (c[j] - n[j]) * own1[j];
+        emit(q, z & 1, c, own, s, above);
+#pragma unroll
+        for (int j = 0; j < kR; j++) {
+          c[j] = n[j];
+          own[j] = own1[j];
+          s[j] = s1[j];
+        }
         q = q1;
       }
     }
@@ -335,7 +379,7 @@ __global__ void __launch_bounds__(kTvT, sizeof(T) == 8 ? 2 : 3)
     if (sizeof(T) == 8)
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
-    if (lx == 0) red[k][ly] = sum[k];
+    if (lx == 0) red[k][wy] = sum[k];
   }
   __syncthreads();
   if (t < kTvT / 32) {
@@ -343,7 +387,7 @@ __global__ void __launch_bounds__(kTvT, sizeof(T) == 8 ? 2 : 3)
     for (int k = 0; k < (kFirst ? 2 : 1); k++) {
       double a = red[k][t];
 #pragma unroll
-      for (int o = kTvT / 64; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffu, a, o);
+      for (int o = kTvT / 64; o > 0; o >>= 1) a += __shfl_xor_sync(0xffu, a, o);
       if (t == 0) pout[k * kTvBlocks + blockIdx.x] = a;
     }
   }
@@ -366,27 +410,36 @@ __global__ void __launch_bounds__(kTvT)
   }
 }
 
-// Slices per item and blocks of a 3-D step: the slab whose rounds of items
-// over the resident blocks cost least (an item costs its slices and about
-// two more for the slices it shares with its neighbours).
-template <class T>
+// Slices per item and blocks of a 3-D step.  An item costs its slices and
+// about one (FP64: the roots of the slice past its end) or two (FP32: the
+// loads at both ends) more.  FP64 steps are bound by the units an SM's blocks
+// share, so the busiest SM's slices count (128^3: 7 slices, two items on
+// every SM; 15 slices and one item: 114 us a step, 8 and an uneven share:
+// 122 us); FP32 steps by latency, so a block's slices do (256^3: 29 slices in
+// 576 blocks; 37 in 448 blocks: 72 us, 32 in 512: 64 us).
+template <class T, bool k3D>
 TvGrid tv_grid(int nx, int ny, int nz, int &blocks) {
-  TvGrid g{nx, ny, nz, (nx + kTvX - 1) / kTvX, (ny + kTvY - 1) / kTvY, 1, 0};
+  constexpr int kY = kTvY<k3D>;
+  TvGrid g{nx, ny, nz, (nx + kTvX - 1) / kTvX, (ny + kY - 1) / kY, 1, 0};
   const long long tiles = (long long)g.tx * g.ty;
-  const long long resident = 152LL * (sizeof(T) == 8 ? 2 : 3);
-  long long best = 0, count = tiles;
-  if (nz > 1)
-    for (int s = 4; s <= 64; s *= 2) {
-      const long long n = tiles * ((nz + s - 1) / s);
-      const long long cost = ((n + resident - 1) / resident) * (std::min(s, nz) + 2);
+  const long long resident = k3D ? 152LL * kTvResident<T, k3D> : kTvBlocks;
+  long long count = tiles;
+  if (k3D) {
+    long long best = 0;
+    for (int s = 4; s <= 64; s++) {
+      const long long n = tiles * ((nz + s - 1) / s), b = std::min(n, resident);
+      const long long items = (n + b - 1) / b, per_sm = (b + 151) / 152;
+      const long long cost = sizeof(T) == 8 ? items * per_sm * (std::min(s, nz) + 1)
+                                            : items * (std::min(s, nz) + 2);
       if (best == 0 || cost < best) {
         best = cost;
         g.slab = s;
         count = n;
       }
     }
+  }
   g.items = (int)count;
-  blocks = (int)std::min<long long>(count, nz > 1 ? resident : kTvBlocks);
+  blocks = (int)std::min(count, resident);
   return g;
 }
 
@@ -397,7 +450,7 @@ cudaError_t tv_minimize_dim(T *img, const T *old, T *wa, T *wb, T *wc, double *s
                             double *partials, int nx, int ny, int nz, double alpha, int n_iter,
                             int pos, cudaStream_t st) {
   int blocks = 0;
-  const TvGrid g = tv_grid<T>(nx, ny, nz, blocks);
+  const TvGrid g = tv_grid<T, k3D>(nx, ny, nz, blocks);
   const long long n = (long long)nx * ny * nz;
   const dim3 grid(blocks), last((unsigned)std::min<long long>((n + kTvT - 1) / kTvT, 152 * 8));
   double *p[2] = {partials, partials + 2 * kTvBlocks};
