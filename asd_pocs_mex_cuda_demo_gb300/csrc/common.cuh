@@ -188,6 +188,10 @@ struct Inst {
   float *cor;                // correction of the current view: element r at
   int cor_stride;            //   cor[r * cor_stride] (1, or kShareSlots when
                              //   a shared-geometry group interleaves them)
+  int rays_t;                // 1: cor and tabC hold the rays of a detector
+                             //   column one after the other (element
+                             //   ia * nb + ib), as the z-column backward
+                             //   step reads them; 0: element ib * na + ia
   float *m_il;               // shared-geometry groups: the group's images
                              //   during the SART sweep, voxel-major, slot
                              //   minor (m_il[v * kShareSlots + slot]); the

@@ -21,6 +21,12 @@ cudaError_t launch_atx(float *x, const float *y, float *sc, const ViewGeo &g,
 // to launch_atx; `scratch` holds the view's ray tables
 // (atx_zcol_scratch_bytes(d) bytes, 256-byte aligned).
 size_t atx_zcol_scratch_bytes(const Dims &d);
+// Whether the z-column form takes these sizes (nz > 1, and its ray indices
+// with their padding fit an int).
+bool zcol_fits(const Dims &d);
+// Zeros that must follow the na * nb rays of Inst::cor and Inst::tabC where
+// the z-column step reads them (Inst::rays_t).
+size_t ray_table_pad(const Dims &d);
 cudaError_t launch_atx_zcol(float *x, const float *y, float *sc, const ViewGeo &g,
                             const Dims &d, void *scratch, cudaStream_t st);
 
@@ -51,8 +57,8 @@ cudaError_t launch_store_sinogram(const float *src, void *dst, size_t n, int fmt
 cudaError_t launch_sart_ax(const Inst *insts, int batch, const Dims &d,
                            int view, cudaStream_t st, bool exact = false,
                            const int *zmap = nullptr);
-// Cone beams (nz > 1) walk voxel columns (k_sart_atx_zcol) in segments of
-// `zseg` voxels (0: the default) unless `zcol` is false (the per-voxel form;
+// Cone beams (nz > 1) run in voxel columns (k_sart_atx_zcol), `zseg` slices a
+// block (rounded up to whole lanes; 0: the default), unless `zcol` is false (the per-voxel form;
 // bit-identical).  `zmap` as for launch_sart_ax.
 cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
                             int view, cudaStream_t st, bool zcol = true, int zseg = 0,

@@ -43,13 +43,12 @@ int atx_blocks(const Dims &d) {
 // it.  (Two warps per ray: 14 % slower for a batch of 64 and 27 % for 256^3.)
 constexpr int kAxBlock = kAxWarps * 32;  // threads per block
 
-// This lane's partial sums of ray r over its columns (no cross-lane sum).
+// This lane's partial sums of ray (ia, ib) over its columns (no cross-lane sum).
 template <class Loader>
 __device__ __forceinline__ void ax_lane_partial(const ViewGeo &G, const Dims &D,
-                                                long long r, Loader ld, float &ys,
+                                                int ia, int ib, Loader ld, float &ys,
                                                 float &ss) {
   const int lane = threadIdx.x & 31;
-  const int ia = (int)(r % D.na), ib = (int)(r / D.na);
   const float zd = G.z_det[ib];
   const RayMarch R = ray_setup(G, D, G.y_det[ia], zd);
   ys = 0.f;
@@ -69,9 +68,10 @@ __global__ void __launch_bounds__(kAxBlock)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long r = (long long)blockIdx.x * kAxWarps + warp;
   if (r >= nray(D)) return;  // the whole warp
+  const unsigned ru = (unsigned)r, na = (unsigned)D.na;  // rays < 2^31
   float ys, ss;
-  ax_lane_partial(G, D, r, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? __ldg(x + i) : 0.f; },
-                  ys, ss);
+  ax_lane_partial(G, D, (int)(ru % na), (int)(ru / na),
+                  [&](unsigned i) { return ASD_IN(i, nvox(D)) ? __ldg(x + i) : 0.f; }, ys, ss);
   ys = warp_sum(ys);
   ss = warp_sum(ss);
   if (lane == 0) {
@@ -403,6 +403,7 @@ struct RayOut {
   float p;    // sinogram value
   double dd;  // Inst::ddr
 };
+// r: the ray's index ib * na + ia
 __device__ __forceinline__ RayOut ray_out_load(const Inst &I, int view, long long r,
                                                long long nr) {
   const long long pi = (long long)view * nr + r;
@@ -411,29 +412,28 @@ __device__ __forceinline__ RayOut ray_out_load(const Inst &I, int view, long lon
   o.dd = ASD_IN(r, nr) ? I.ddr[r] : 0.0;
   return o;
 }
-__device__ __forceinline__ void ray_out_store(const Inst &I, int view, long long r,
+// q: where cor keeps the ray
+__device__ __forceinline__ void ray_out_store(const Inst &I, int view, long long r, long long q,
                                               long long nr, const RayOut &o, float yv,
                                               float srv) {
   const float c0 = o.p - yv;
   const float cr = c0 / (srv == 0.f ? 1.f : srv);
-  if (!ASD_IN(r, nr)) return;
-  I.cor[r * I.cor_stride] = cr;
+  if (!ASD_IN(r, nr) || !ASD_IN(q, nr)) return;
+  I.cor[q * I.cor_stride] = cr;
   I.ddr[r] = o.dd + (double)(c0 * c0);
   if (!isfinite(cr)) I.s->cor_bad = view + 1;
 }
 
-// The view's ray slopes for the backward step that follows (3-D), rays r0 to
-// r0 + kAxWarps - 1 of the block, by the first lanes of its first warp.
+// The view's slopes of ray (ia, ib) for the backward step that follows (3-D).
 __device__ __forceinline__ void ray_slopes(const Inst &I, const ViewGeo &G, const Dims &D,
-                                           int view, long long r0, long long nr) {
-  const long long r = r0 + threadIdx.x;
-  if (threadIdx.x >= kAxWarps || r >= nr || !ASD_IN(r, nr)) return;
-  const int ia = (int)(r % D.na), ib = (int)(r / D.na);
-  I.tabC[r] = ray_tab_c(I.tabA[(long long)view * D.na + ia], G.z_det[ib]);
+                                           int view, int ia, int ib, long long q) {
+  if (ASD_IN(q, nray(D)))
+    I.tabC[q] = ray_tab_c(I.tabA[(long long)view * D.na + ia], G.z_det[ib]);
 }
 
 // For 3D geometry also writes the view's ray slopes (Inst::tabc_mode: a
 // shared table's writer does so even after its own iterations have ended).
+// Rays are taken in the order that cor and tabC keep them.
 template <bool k3D>
 __global__ void __launch_bounds__(kAxBlock)
     k_sart_ax(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap) {
@@ -444,20 +444,34 @@ __global__ void __launch_bounds__(kAxBlock)
   const bool tabc = k3D && (I.tabc_mode == kTabcShared || (!done && I.tabc_mode == kTabcOwn));
   if (done && !tabc) return;
   const Dims D = I.d;
-  const long long nr = nray(D), r0 = (long long)blockIdx.x * kAxWarps;
+  const bool rt = k3D && I.rays_t;
+  const long long nr = nray(D), q0 = (long long)blockIdx.x * kAxWarps;
+  // ray q of the order: (ia, ib), rays < 2^31
+  auto ray = [&](long long q, int &ia, int &ib) {
+    const unsigned n = (unsigned)(rt ? D.nb : D.na), hi = (unsigned)q / n, lo = (unsigned)q % n;
+    ia = (int)(rt ? hi : lo);
+    ib = (int)(rt ? lo : hi);
+  };
+  int ia, ib;
   const ViewGeo G = view_of(I, view);
-  if (tabc) ray_slopes(I, G, D, view, r0, nr);
+  if (tabc && threadIdx.x < kAxWarps && q0 + threadIdx.x < nr) {
+    ray(q0 + threadIdx.x, ia, ib);
+    ray_slopes(I, G, D, view, ia, ib, q0 + threadIdx.x);
+  }
   const int lane = threadIdx.x & 31;
-  const long long r = r0 + (threadIdx.x >> 5);
-  if (done || r >= nr) return;  // the whole warp
+  const long long q = q0 + (threadIdx.x >> 5);
+  if (done || q >= nr) return;  // the whole warp
+  ray(q, ia, ib);
+  const long long r = (long long)ib * D.na + ia;
   RayOut o{0.f, 0.0};
   if (lane == 0) o = ray_out_load(I, view, r, nr);
   const float *m = I.m;
   float ys, ss;
-  ax_lane_partial(G, D, r, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; }, ys, ss);
+  ax_lane_partial(G, D, ia, ib, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; }, ys,
+                  ss);
   ys = warp_sum(ys);
   ss = warp_sum(ss);
-  if (lane == 0) ray_out_store(I, view, r, nr, o, ys * G.scale, ss * G.scale);
+  if (lane == 0) ray_out_store(I, view, r, q, nr, o, ys * G.scale, ss * G.scale);
 }
 
 // k_sart_ax with the exact projection (siddon_warp_rays): a warp per 32 rays,
@@ -476,17 +490,16 @@ __global__ void __launch_bounds__(kAxBlock)
   const ViewGeo G = view_of(I, view);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long r0 = ((long long)blockIdx.x * kAxWarps + warp) * 32, r = r0 + lane;
-  if (tabc && r < nr && ASD_IN(r, nr)) {
-    const int ia = (int)(r % D.na), ib = (int)(r / D.na);
-    I.tabC[r] = ray_tab_c(I.tabA[(long long)view * D.na + ia], G.z_det[ib]);
-  }
+  const int ia = (int)(r % D.na), ib = (int)(r / D.na);
+  const long long q = I.rays_t ? (long long)ia * D.nb + ib : r;
+  if (tabc && r < nr) ray_slopes(I, G, D, view, ia, ib, q);
   if (done || r0 >= nr) return;  // the whole warp
   float yv = 0.f, sv = 0.f;
   const float *m = I.m;
   siddon_warp_rays(G, D, r0, nr, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; },
                    yv, sv);
   if (r < nr)
-    ray_out_store(I, view, r, nr, ray_out_load(I, view, r, nr), yv * G.scale, sv * G.scale);
+    ray_out_store(I, view, r, q, nr, ray_out_load(I, view, r, nr), yv * G.scale, sv * G.scale);
 }
 
 // Planar chord for a window whose rays share dominant axis AX (1: x, 2: y;
@@ -713,248 +726,392 @@ __global__ void __launch_bounds__(kAtxThreads, 4)
 }
 
 // ---------------------------------------------------------------------------
-// Cone-beam backward step per voxel column (z-column form).  A thread owns a
-// segment of kZSeg voxels of one (x, y) column and walks it down z.  What
-// does not depend on z is computed once per segment (zcol_setup): the
-// footprint window's columns and magnification, the shadow's columns and its
-// corners' magnifications, and for each detector column of the shadow the
-// in-plane part of the x and y face tests (col_faces, kept in shared memory,
-// a thread reading only its own slots).  Each voxel then finds its rows
-// (zcol_rows) and evaluates only the z parts of the face tests
-// (chord3_col).  Pairs run as one sequence per voxel, rows outer (the
-// reference's order), a warp walking its longest sequence; the voxels of a
-// warp are 32 neighbours along x at the same z, so image reads and writes
-// are coalesced.  Views that do not allow narrowing (an axis-parallel ray, a
-// residual that is not finite) take the per-voxel form with the reference's
-// whole window.  Columns whose shadow is wider than kZColA detector columns
-// evaluate their chords from the ray tables (chord3_bf).
-// Grid: (x tiles of 32, y tiles of 8 x segments, instances).
+// Cone-beam backward step in voxel columns (z-column form).  The lanes of a
+// warp are consecutive voxels of one (x, y) column (lanes in groups of L for
+// volumes of few slices), so what does not depend on z is the same for all of
+// them: the footprint window's columns and magnification, the shadow's
+// columns and corner magnifications (zcol_setup) and, for each detector
+// column of the shadow, the in-plane part of the x and y face tests
+// (col_faces).  A block computes these once for its W columns, one thread per
+// (column, detector column), and keeps them in shared memory.  Each voxel then
+// finds its rows (zcol_shadow, or zcol_rows where a window clips the shadow)
+// and evaluates the z parts of its pairs' face tests (col_hits).  Residuals
+// and slopes are stored with the rays of a detector column one after the
+// other (Inst::rays_t), so the warp's reads of a detector column are
+// consecutive.
+//
+// The pairs of up to kZcCols detector columns by kZcRows rows are unrolled.
+// Most pairs hit the two in-plane faces; the others (about one pair in seven
+// crosses a z face) go to a list of the warp, whose items are then dealt to
+// the lanes, so that a warp runs the z faces about once per voxel and not for
+// every pair.  The chords go through shared memory and are accumulated in the reference's
+// order (rows outer).  Voxels with more pairs, columns with three or more
+// in-plane hits and shadows wider than kZcSlots take a plain loop, views that
+// do not allow narrowing (an axis-parallel ray, a residual that is not
+// finite) the per-voxel form over the reference's window.
+// Sums pass through a tile of W columns by L voxels, so the image is read and
+// written W voxels at a time.
+// Instruction issue bounds it (80 % of cycles, 816 warp instructions per 32
+// voxels): 0.447 ms for one 256^3 view on a 512^2 detector (ncu), against
+// 0.618 with a thread per segment of a column, which computed the in-plane
+// part once per 8 voxels and the z faces for every pair, and 0.90 per voxel.
+// Grid: x tiles of W x y x segments of `seg` slices, instances.
 // ---------------------------------------------------------------------------
-constexpr int kZSeg = 32;   // longest default segment: voxels of a column per thread
-// Default segment for `voxels` voxels in a launch: the longest of 32, 16,
-// 8, 4 that still gives the launch 2^21 threads (a few per SM slot).
-// Measured on single volumes: 256^3 is fastest with 8 (0.566 ms against
-// 0.639 with 32), 64^3 - 128^3 with 4 (64^3: 0.026 ms against 0.107).
-__host__ __device__ inline int zcol_default_seg(long long voxels) {
-  int seg = kZSeg;
-  while (seg > 4 && voxels / seg < (1LL << 21)) seg /= 2;
-  return seg;
-}
-constexpr int kZColA = 6;   // detector columns of a shadow kept per thread
+constexpr int kZcThreads = 256, kZcWarps = kZcThreads / 32;
+constexpr int kZcSlots = 6;             // detector columns of a shadow kept
+constexpr int kZcCols = 4, kZcRows = 3; // most unrolled pairs
 
+// Elements after the na * nb rays of cor and tabC that the unrolled pairs may
+// read (zeros).
+__host__ __device__ __forceinline__ long long zcol_pad(const Dims &d) {
+  return (long long)(kZcCols - 1) * d.nb + kZcRows;
+}
+
+template <int W>
 struct ZColShared {
-  float4 pts[kZColA][kAtxThreads];   // F1, F2 in-plane points
-  float4 nh[kZColA][kAtxThreads];    // F1, F2 z-half terms (n1, h1, n2, h2)
-  unsigned bits[kZColA][kAtxThreads];
+  float4 z[kZcSlots][W];    // n1, n2, e12, bits
+  float4 pts[kZcSlots][W];  // F1, F2 in-plane points
+  float4 col[W];            // rx, ry, qmin, qmax
+  float tb[W];              // window magnification
+  int lo[W];                // first detector column
+  int count[W];             // detector columns
+  int flags[W];             // kZc*
+  float2 l[kZcCols * kZcRows][kZcThreads];  // a voxel's chords and their products
+  unsigned short list[kZcWarps][32 * kZcCols * kZcRows];  // a warp's z-face pairs
+  float acc[32][W + 1], accl[32][W + 1];
 };
+constexpr int kZcOk = 1, kZcWindow = 2, kZcInside = 4, kZcSpecial = 8;
 
-// Grid of segments of `seg` voxels (a launch shape: the sums of a voxel do not
-// depend on it).
-__host__ __device__ inline dim3 zcol_grid(int nx, int ny, int nz, int batch,
-                                          int seg = kZSeg) {
-  return dim3((nx + kTileX - 1) / kTileX,
-              ((ny + kTileY - 1) / kTileY) * ((nz + seg - 1) / seg), batch);
+// Launch shape: columns of a block (32 or 8), lanes of a column (32, 16 or
+// 8) and slices of a block.  Lanes: the count that wastes least on the last
+// voxels.  8 columns a block where 32 leave the launch under two blocks per
+// resident slot; slices so that a launch has about four.
+struct ZColShape {
+  int W, L, seg;
+  int lsh() const { return L == 32 ? 5 : L == 16 ? 4 : 3; }
+};
+inline ZColShape zcol_shape(const Dims &d, int batch, int seg) {
+  ZColShape s{32, 32, 0};
+  auto padded = [&](int L) { return (d.nz + L - 1) / L * L; };
+  for (int L : {16, 8})
+    if (padded(L) * 20 < padded(s.L) * 19) s.L = L;
+  const long long lines = (long long)d.ny * batch;
+  if ((d.nx + 31) / 32 * lines * ((d.nz + 31) / 32) < 152 * 8) {
+    s.W = 8;
+    s.L = 32;
+  }
+  const int chunks = (d.nz + s.L - 1) / s.L;
+  const long long tiles = (d.nx + s.W - 1) / s.W * lines;
+  const long long split = std::min<long long>(chunks, (152 * 16 + tiles - 1) / tiles);
+  const long long per = seg > 0 ? (seg + s.L - 1) / s.L : (chunks + split - 1) / split;
+  s.seg = (int)per * s.L;
+  return s;
+}
+inline dim3 zcol_grid(const Dims &d, int batch, const ZColShape &s) {
+  return dim3((unsigned)((d.nx + s.W - 1) / s.W) * (unsigned)d.ny *
+                  (unsigned)((d.nz + s.seg - 1) / s.seg),
+              1, batch);
 }
 
-// This thread's column and segment [z0, z1) for an instance of sizes D;
-// false when the block lies outside the instance's own grid.
-__device__ __forceinline__ bool zcol_thread(const Dims &D, int seg, int &ix, int &iy,
-                                            int &z0, int &z1) {
-  const int ty = (D.ny + kTileY - 1) / kTileY, ns = (D.nz + seg - 1) / seg;
-  if ((int)blockIdx.x * kTileX >= D.nx || (int)blockIdx.y >= ty * ns) return false;
-  const int sg = blockIdx.y / ty, yt = blockIdx.y - sg * ty;
-  ix = blockIdx.x * kTileX + threadIdx.x % kTileX;
-  iy = yt * kTileY + threadIdx.x / kTileX;
-  z0 = sg * seg;
-  z1 = min(z0 + seg, D.nz);
-  return true;
+// Sums of a warp's voxels with at most kZcCols detector columns (mA of them
+// in the warp) and kZcRows rows each: the lane's pairs are columns s < cA and
+// rows kb < cB from ray r0 (the others read rays nearby or the padding after
+// the tables, whose values are finite, and have chord 0).  (c, zc0 + zl) of
+// lane `src` come from v0 + src.
+template <int W>
+__device__ __forceinline__ void zcol_pairs(const ViewGeo &G, const Dims &D,
+                                           const float4 *__restrict__ tabC,
+                                           const float *__restrict__ yt, ZColShared<W> &sh, int v0,
+                                           int zc0, int lsh, int c, int r0, int mA, int cA, int cB,
+                                           float rz, float hz, bool steep, float &acc,
+                                           float &accl) {
+  constexpr int B = kZcRows;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const unsigned below = (1u << lane) - 1u;  // lanes before this one
+  const long long room = nray(D) + zcol_pad(D);
+  unsigned short *const list = sh.list[warp];
+  unsigned todo = 0u, bit = 1u;  // pairs that do not hit both F1 and F2
+#pragma unroll 1
+  for (int s = 0; s < mA; s++) {
+    const float4 q = sh.z[s][c];
+    const unsigned bits = __float_as_uint(q.w);
+    const int r = r0 + s * D.nb, rows = s < cA ? cB : 0;
+    float4 Cs[B];
+    float y[B];
+#pragma unroll
+    for (int kb = 0; kb < B; kb++) {
+      const bool in = ASD_IN(r + kb, room);
+      Cs[kb] = in ? __ldg(tabC + r + kb) : make_float4(0.f, 0.f, 0.f, 0.f);
+      y[kb] = in ? __ldg(yt + r + kb) : 0.f;
+    }
+#pragma unroll
+    for (int kb = 0; kb < B; kb++) {
+      const bool on = kb < rows;
+      const ColHits h = col_hits(bits, q.x, q.y, Cs[kb], rz, hz);
+      const float e2 = h.z2 - h.z1, l2 = q.z + e2 * e2;
+      const bool both = on && h.h1 && h.h2 && l2 >= kRootMin;
+      const float l = both ? root_rn(l2) : 0.f;
+      sh.l[s * B + kb][t] = make_float2(l, l * y[kb]);
+      todo |= on && !both && (steep || h.h1 || h.h2) ? bit : 0u;
+      bit <<= 1;
+    }
+  }
+  // the other pairs into the warp's list, a lane's next one at a time
+  int listed = 0;
+  unsigned vote;
+  while ((vote = __ballot_sync(0xffffffffu, todo != 0u)) != 0u) {
+    if (todo) {
+      list[listed + __popc(vote & below)] = (unsigned short)(lane | (__ffs((int)todo) - 1) << 5);
+      todo &= todo - 1u;
+    }
+    listed += __popc(vote);
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int i = lane; i - lane < listed; i += 32) {
+    const int code = i < listed ? list[i] : 0, src = code & 31, k = code >> 5;
+    const int rs = __shfl_sync(0xffffffffu, r0, src);
+    if (i >= listed) continue;
+    const int s = k / B, vs = v0 + src, cs = vs >> lsh;
+    const int r = rs + s * D.nb + k % B;
+    if (!ASD_IN(r, nray(D))) continue;
+    const float zr = 0.0f - zcol_height(G, D, zc0 + (vs & ((1 << lsh) - 1)));
+    const float4 q = sh.z[s][cs], p = sh.col[cs], Cs = __ldg(tabC + r);
+    const float yv = __ldg(yt + r);
+    const ColHits h = col_hits(__float_as_uint(q.w), q.x, q.y, Cs, zr, hz);
+    const float e2 = h.z2 - h.z1;
+    const float l2 = h.h1 && h.h2 ? q.z + e2 * e2
+                                  : chord3_zface2(sh.pts[s][cs], h, Cs, p.x, p.y, zr, hz);
+    const float l = l2 > 0.f ? sqrtf(l2) : 0.f;
+    sh.l[k][warp * 32 + src] = make_float2(l, l * yv);
+  }
+  __syncwarp();
+  // rows outer, columns inner; 0 for a pair that is not there
+#pragma unroll
+  for (int kb = 0; kb < B; kb++)
+#pragma unroll 1
+    for (int s = 0; s < mA; s++) {
+      const float2 p = sh.l[s * B + kb][t];
+      acc += p.y;
+      accl += p.x;
+    }
 }
 
-// Walks this thread's segment.  pair(r, l, on) takes the chord l of ray r
-// (pairs in the reference's order; on == false for a lane past its own
-// pairs), voxel(idx) ends a voxel; begin(idx) starts it (prefetches).
-template <class Begin, class Pair, class Voxel>
+// Footprint sums of this block's columns; out(idx, acc, accl) takes a
+// voxel's.  Every thread of the block calls it.
+template <int W, class Out>
 __device__ __forceinline__ void atx_zcol_walk(const ViewGeo &G, const Dims &D,
                                               const float4 *__restrict__ tabA,
                                               const float4 *__restrict__ tabC,
-                                              bool narrow, int ix, int iy, int z0, int z1,
-                                              ZColShared &sh, Begin begin, Pair pair,
-                                              Voxel voxel) {
-  const bool valid = ix < D.nx && iy < D.ny;
+                                              const float *__restrict__ yt, bool narrow, int lsh,
+                                              int seg, ZColShared<W> &sh, Out out) {
+  const int L = 1 << lsh;
+  const int xt = (D.nx + W - 1) / W, ns = (D.nz + seg - 1) / seg;
+  if ((long long)blockIdx.x >= (long long)xt * D.ny * ns) return;
+  const int x0 = (int)(blockIdx.x % xt) * W, iy = (int)(blockIdx.x / xt % D.ny);
+  const int zb0 = (int)(blockIdx.x / xt / D.ny) * seg, zb1 = min(zb0 + seg, D.nz);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const float hz = G.dz / 2.0f;
-  if (!narrow) {
-    // the per-voxel form over the reference's window (no warp-wide steps)
-    if (!valid) return;
-    for (int iz = z0; iz < z1; iz++) {
-      const unsigned idx = ((unsigned)iz * D.ny + iy) * D.nx + ix;
-      if (!ASD_IN(idx, nvox(D))) continue;
-      begin(idx);
-      const VoxelWin w = voxel_window(G, D, ix, iy, iz);
-      const float rx = G.cos_phi * (-G.SO) - w.xc, ry = G.sin_phi * (-G.SO) - w.yc;
-      const float rz = 0.0f - w.zc;
-      for (int ib = w.b0; ib <= w.b1; ib++) {
-        const float c = (ASD_IN(ib, D.nb) ? __ldg(G.z_det + ib) : 0.f) - 0.0f;
-        for (int ia = w.a0; ia <= w.a1; ia++) {
-          const int r = ib * D.na + ia;
-          if (!(ASD_IN(ia, D.na) && ASD_IN(r, nray(D)))) continue;
-          pair(r, chord3_bf(__ldg(tabA + ia), __ldg(tabC + r), c, rx, ry, rz, G.dz), true);
+  const long long M = nray(D);
+  if (narrow) {
+    const int c = t % W;
+    ZCol col;
+    int cnt = 0;
+    bool wide = false;
+    col.lo = 0;
+    if (x0 + c < D.nx) {
+      col = zcol_setup(G, D, x0 + c, iy, true);
+      cnt = col.lo <= col.hi ? col.hi - col.lo + 1 : 0;
+      wide = cnt > kZcSlots;
+    }
+    if (t < W && x0 + c < D.nx) {
+      sh.col[c] = make_float4(col.rx, col.ry, col.qmin, col.qmax);
+      sh.tb[c] = col.tb;
+      sh.flags[c] = (col.ok ? kZcOk : 0) | (col.a0 <= col.a1 ? kZcWindow : 0) |
+                    (zcol_shadow_inside(G, D, col, zb0, zb1) ? kZcInside : 0) |
+                    (wide ? kZcSpecial : 0);
+    } else if (t < W) {
+      sh.col[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+      sh.tb[c] = 0.f;
+      sh.flags[c] = kZcInside;
+    }
+    if (t < W) {
+      sh.lo[c] = col.lo;
+      sh.count[c] = cnt;
+    }
+    __syncthreads();
+    for (int k = t / W; k < cnt && !wide; k += kZcThreads / W) {
+      if (!ASD_IN(col.lo + k, D.na)) continue;
+      const ColFaces f = col_faces(__ldg(tabA + col.lo + k), col.rx, col.ry);
+      sh.pts[k][c] = make_float4(f.p1x, f.p1y, f.p2x, f.p2y);
+      sh.z[k][c] = make_float4(f.n1, f.n2, f.e12, __uint_as_float(f.bits));
+      if (f.bits & kCfMany) atomicOr(&sh.flags[c], kZcSpecial);
+    }
+    __syncthreads();
+  }
+  // both z faces of a voxel can be hit, and so count without an in-plane
+  // face, only if a ray climbs dz within a pixel; less than half of that
+  // anywhere on the detector and the question never comes up
+  const bool steep = !(D.nb * G.dz_det < G.dz * G.SD);
+  const int zl = lane & (L - 1);
+  for (int zc0 = zb0; zc0 < zb1; zc0 += L) {
+    // what depends on the lane's height only
+    const int iz = zc0 + zl;
+    const float zc = zcol_height(G, D, iz), rz = 0.0f - zc;
+    float zlo, zhi;
+    zcol_faces(G, zc, zlo, zhi);
+    for (int v0 = warp * 32; v0 < W * L; v0 += kZcThreads) {  // warp-uniform
+      const int c = (v0 + lane) >> lsh;
+      const int ix = x0 + c;
+      const bool valid = ix < D.nx && iz < zb1;
+      float acc = 0.f, accl = 0.f;
+      if (!narrow) {
+        // the per-voxel form over the reference's window
+        if (valid) {
+          const VoxelWin w = voxel_window(G, D, ix, iy, iz);
+          const float rx = G.cos_phi * (-G.SO) - w.xc, ry = G.sin_phi * (-G.SO) - w.yc;
+          for (int ib = w.b0; ib <= w.b1; ib++) {
+            const float cz = (ASD_IN(ib, D.nb) ? __ldg(G.z_det + ib) : 0.f) - 0.0f;
+            for (int ia = w.a0; ia <= w.a1; ia++) {
+              const int r = ia * D.nb + ib;
+              if (!(ASD_IN(ia, D.na) && ASD_IN(r, M))) continue;
+              const float l =
+                  chord3_bf(__ldg(tabA + ia), __ldg(tabC + r), cz, rx, ry, rz, G.dz);
+              acc += l * __ldg(yt + r);
+              accl += l;
+            }
+          }
+        }
+      } else {
+        const float4 cd = sh.col[c];  // rx, ry, qmin, qmax
+        const int flags = sh.flags[c];
+        int blo, bhi;
+        if (any_lane(!(flags & kZcInside))) {
+          float zr;
+          ZCol col;
+          col.qmin = cd.z;
+          col.qmax = cd.w;
+          col.tb = sh.tb[c];
+          col.ok = flags & kZcOk;
+          col.a0 = 0;
+          col.a1 = (flags & kZcWindow) ? 0 : -1;
+          if (!zcol_rows(G, D, col, iz, zr, blo, bhi)) bhi = blo - 1;
+        } else {
+          float s0, s1;
+          zcol_shadow(D, cd.z, cd.w, zlo, zhi, s0, s1);
+          blo = max((int)ceilf(s0), 0);
+          bhi = min((int)floorf(s1), D.nb - 1);
+        }
+        const int cB = valid && blo <= bhi ? bhi - blo + 1 : 0;
+        const int cA = cB > 0 ? sh.count[c] : 0;
+        const int mA = __reduce_max_sync(0xffffffffu, cA);
+        const int mB = __reduce_max_sync(0xffffffffu, cA > 0 ? cB : 0);
+        const int lo = sh.lo[c];
+        const int r0 = lo * D.nb + min(blo, D.nb - 1);  // the first pair's ray
+        const bool special = cA > 0 && (flags & kZcSpecial);
+        if (mA <= kZcCols && mB <= kZcRows && !any_lane(special)) {
+          zcol_pairs<W>(G, D, tabC, yt, sh, v0, zc0, lsh, c, r0, mA, cA, cB, rz, hz, steep, acc,
+                        accl);
+        } else {
+          for (int kb = 0; kb < cB; kb++)
+            for (int s = 0; s < cA; s++) {
+              const int r = r0 + s * D.nb + kb;
+              if (!ASD_IN(r, M) || !ASD_IN(lo + s, D.na)) continue;
+              const float4 Cs = __ldg(tabC + r);
+              float l;
+              if (flags & kZcSpecial) {
+                l = chord3_bf(__ldg(tabA + lo + s), Cs, 0.0f, cd.x, cd.y, rz, G.dz);
+              } else {
+                const float4 q = sh.z[s][c], p = sh.pts[s][c];
+                const ColFaces f{p.x, p.y, p.z, p.w, q.x, q.y, q.z, __float_as_uint(q.w)};
+                l = chord3_col(f, Cs, cd.x, cd.y, rz, hz);
+              }
+              acc += l * __ldg(yt + r);
+              accl += l;
+            }
         }
       }
-      voxel(idx);
+      sh.acc[zl][c] = acc;
+      sh.accl[zl][c] = accl;
     }
-    return;
-  }
-  const int t = threadIdx.x;
-  ZCol col;
-  int cntA = 0;
-  bool wide = false;
-  col.lo = 0;
-  col.rx = col.ry = 0.f;
-  if (valid) {
-    col = zcol_setup(G, D, ix, iy, true);
-    cntA = col.lo <= col.hi ? col.hi - col.lo + 1 : 0;
-    wide = cntA > kZColA;
-    if (!wide)
-      for (int k = 0; k < cntA; k++) {
-        if (!ASD_IN(col.lo + k, D.na)) continue;
-        const ColFaces f = col_faces(__ldg(tabA + col.lo + k), col.rx, col.ry);
-        sh.pts[k][t] = make_float4(f.p1x, f.p1y, f.p2x, f.p2y);
-        sh.nh[k][t] = make_float4(f.n1, f.h1, f.n2, f.h2);
-        sh.bits[k][t] = f.bits;
-      }
-  }
-  for (int iz = z0; iz < z1; iz++) {
-    const unsigned idx = ((unsigned)iz * D.ny + iy) * D.nx + ix;
-    const bool vin = valid && ASD_IN(idx, nvox(D));
-    if (vin) begin(idx);
-    float zc = 0.f;
-    int blo = 0, bhi = -1;
-    const bool has = valid && zcol_rows(G, D, col, iz, zc, blo, bhi);
-    const int cntB = has && blo <= bhi ? bhi - blo + 1 : 0;
-    const int cnt = cntA * cntB;
-    const int kN = __reduce_max_sync(0xffffffffu, cnt);
-    const float rz = 0.0f - zc;
-    int ka = 0, ib = blo;
-    for (int k = 0; k < kN; k++) {
-      const bool on = k < cnt;
-      const int kk = on ? ka : 0;
-      const int ia = on ? col.lo + ka : 0;
-      const int r = (on ? ib : 0) * D.na + ia;
-      const bool rin = ASD_IN(r, nray(D)) && ASD_IN(ia, D.na);
-      const float4 Cs = rin ? __ldg(tabC + r) : make_float4(0.f, 0.f, 0.f, 0.f);
-      float l;
-      if (!wide) {
-        const float4 p = sh.pts[kk][t], q = sh.nh[kk][t];
-        const ColFaces f{p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w, sh.bits[kk][t]};
-        if (f.bits & kCfMany)
-          l = (f.bits & kCfXF) ? chord3_axis<true>(__ldg(tabA + ia), Cs, col.rx, col.ry, rz, G.dz)
-                               : chord3_axis<false>(__ldg(tabA + ia), Cs, col.rx, col.ry, rz, G.dz);
-        else
-          l = chord3_col(f, Cs, col.rx, col.ry, rz, hz);
-      } else {
-        l = chord3_bf(__ldg(tabA + ia), Cs, 0.0f, col.rx, col.ry, rz, G.dz);
-      }
-      pair(r, l, on && rin);
-      if (++ka == cntA) {
-        ka = 0;
-        ib++;
-      }
+    __syncthreads();
+    for (int i = t; i < W * L; i += kZcThreads) {
+      const int zl = i / W, c = i % W, iz = zc0 + zl, ix = x0 + c;
+      const unsigned idx = ((unsigned)iz * D.ny + iy) * D.nx + ix;
+      if (ix < D.nx && iz < zb1 && ASD_IN(idx, nvox(D))) out(idx, sh.acc[zl][c], sh.accl[zl][c]);
     }
-    if (vin) voxel(idx);
+    __syncthreads();
   }
 }
 
 // SART backward step of cone-beam instances (see k_sart_atx) in z columns.
-__global__ void __launch_bounds__(kAtxThreads, 4)
-    k_sart_atx_zcol(const Inst *__restrict__ insts, int view, int seg,
+template <int W>
+__global__ void __launch_bounds__(kZcThreads, 4)
+    k_sart_atx_zcol(const Inst *__restrict__ insts, int view, int lsh, int seg,
                     const int *__restrict__ zmap) {
-  __shared__ ZColShared sh;
+  __shared__ ZColShared<W> sh;
   pdl_enter();
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
   if (view >= I.nv || ((volatile int *)&I.s->done)[0]) return;
   const Dims D = I.d;
-  int ix, iy, z0, z1;
-  if (!zcol_thread(D, seg, ix, iy, z0, z1)) return;
   const ViewGeo G = view_of(I, view);
-  const float4 *tabA = I.tabA + (long long)view * D.na;
   const bool narrow = !(I.vflags[view] & kViewAxisParallel) && I.s->cor_bad != view + 1;
   const float beta = I.s->beta_f;
   float *m = I.m;
-  const float *__restrict__ cor = I.cor;
-  float acc = 0.f, accl = 0.f, mv = 0.f;
-  atx_zcol_walk(
-      G, D, tabA, I.tabC, narrow, ix, iy, z0, z1, sh,
-      [&](unsigned idx) {
-        mv = m[idx];
-        acc = 0.f;
-        accl = 0.f;
-      },
-      [&](int r, float l, bool on) {
-        const float yv = on ? __ldg(cor + r) : 0.f;
-        if (on) {
-          acc += l * yv;
-          accl += l;
-        }
-      },
-      [&](unsigned idx) {
-        const float bp = acc * G.scale, scv = accl * G.scale;
-        const float mn = mv + beta * __fdividef(bp, scv == 0.f ? 1.f : scv);
-        m[idx] = mn < 0.f ? 0.f : mn;
-      });
+  atx_zcol_walk<W>(G, D, I.tabA + (long long)view * D.na, I.tabC, I.cor, narrow, lsh, seg, sh,
+                   [&](unsigned idx, float acc, float accl) {
+                     const float bp = acc * G.scale, scv = accl * G.scale;
+                     const float mn = m[idx] + beta * __fdividef(bp, scv == 0.f ? 1.f : scv);
+                     m[idx] = mn < 0.f ? 0.f : mn;
+                   });
 }
 
-// Ray tables of one view for the standalone backward step (launcher path):
-// tabA[na], tabC[na*nb] and, in flag[0], whether the view forbids narrowing
+// Ray tables of one view for the standalone backward step (launcher path), in
+// the z-column step's ray order (ia * nb + ib): tabA[na], tabC[na*nb], the
+// view's values yt[na*nb] and, in flag[0], whether the view forbids narrowing
 // (flag[0] set unless every ray has both in-plane components, the bins lie
 // on the uniform grid and every value is finite; flag[0] must be 0 before
 // the launch).
 __global__ void __launch_bounds__(256)
-    k_view_tab3(const float *__restrict__ yv, float4 *tabA, float4 *tabC, int *flag,
+    k_view_tab3(const float *__restrict__ yv, float4 *tabA, float4 *tabC, float *yt, int *flag,
                 ViewGeo G, Dims D) {
   const long long nr = (long long)D.na * D.nb;
-  const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   bool ok = true;
-  if (r < nr) {
-    const int ia = (int)(r % D.na), ib = (int)(r / D.na);
+  if (q >= nr && q < nr + zcol_pad(D)) {
+    tabC[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    yt[q] = 0.f;
+  }
+  if (q < nr) {
+    const int ia = (int)(q / D.nb), ib = (int)(q % D.nb);
+    const long long r = (long long)ib * D.na + ia;
     const float yd = G.y_det[ia], zd = G.z_det[ib];
     const float4 A = ray_tab_a(G, yd);
     if (ib == 0 && ASD_IN(ia, D.na)) tabA[ia] = A;
-    if (ASD_IN(r, nr)) tabC[r] = ray_tab_c(A, zd);
+    const float v = ASD_IN(r, nr) ? yv[r] : 0.f;
+    if (ASD_IN(q, nr)) {
+      tabC[q] = ray_tab_c(A, zd);
+      yt[q] = v;
+    }
     ok = A.x != 0.0f && A.y != 0.0f && on_grid(yd, ia, D.na, G.dy_det) &&
-         on_grid(zd, ib, D.nb, G.dz_det) && isfinite(yv[r]) && G.dy_det > 0.0f &&
-         G.dz_det > 0.0f;
+         on_grid(zd, ib, D.nb, G.dz_det) && isfinite(v) && G.dy_det > 0.0f && G.dz_det > 0.0f;
   }
   if (!__all_sync(0xffffffffu, ok) && (threadIdx.x & 31) == 0) atomicOr(flag, 1);
 }
 
 // Standalone cone-beam backward step (Ax_cone_gpu.cu:214-271) in z columns,
 // from the tables of k_view_tab3.
-__global__ void __launch_bounds__(kAtxThreads, 4)
-    k_atx_zcol(float *__restrict__ x, const float *__restrict__ yv, float *__restrict__ sc,
-               const float4 *__restrict__ tabA, const float4 *__restrict__ tabC,
-               const int *__restrict__ flag, ViewGeo G, Dims D, int seg) {
-  __shared__ ZColShared sh;
-  int ix, iy, z0, z1;
-  if (!zcol_thread(D, seg, ix, iy, z0, z1)) return;
-  const bool narrow = flag[0] == 0;
-  float acc = 0.f, accl = 0.f;
-  atx_zcol_walk(
-      G, D, tabA, tabC, narrow, ix, iy, z0, z1, sh,
-      [&](unsigned) {
-        acc = 0.f;
-        accl = 0.f;
-      },
-      [&](int r, float l, bool on) {
-        const float v = on ? __ldg(yv + r) : 0.f;
-        if (on) {
-          acc += l * v;
-          accl += l;
-        }
-      },
-      [&](unsigned idx) {
-        x[idx] = acc * G.scale;
-        sc[idx] = accl * G.scale;
-      });
+template <int W>
+__global__ void __launch_bounds__(kZcThreads, 4)
+    k_atx_zcol(float *__restrict__ x, float *__restrict__ sc, const float4 *__restrict__ tabA,
+               const float4 *__restrict__ tabC, const float *__restrict__ yt,
+               const int *__restrict__ flag, ViewGeo G, Dims D, int lsh, int seg) {
+  __shared__ ZColShared<W> sh;
+  atx_zcol_walk<W>(G, D, tabA, tabC, yt, flag[0] == 0, lsh, seg, sh,
+                   [&](unsigned idx, float acc, float accl) {
+                     x[idx] = acc * G.scale;
+                     sc[idx] = accl * G.scale;
+                   });
 }
 
 // ---------------------------------------------------------------------------
@@ -1371,7 +1528,10 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
   const ViewGeo G = view_of(I0, view);
   // cone beam: the plan's one ray-slope table, refreshed by group 0 every
   // view whether or not its instances still run
-  if (k3D && blockIdx.z == 0) ray_slopes(I0, G, D, view, r0, nr);
+  if (k3D && blockIdx.z == 0 && threadIdx.x < kAxWarps && r0 + threadIdx.x < nr) {
+    const long long rs = r0 + threadIdx.x;
+    ray_slopes(I0, G, D, view, (int)(rs % D.na), (int)(rs / D.na), rs);
+  }
   if (r >= nr) return;  // the whole warp
   // lane b: instance gi + b
   const Inst &Ib = insts[gi + min(lane, gn - 1)];
@@ -1454,7 +1614,7 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
 #pragma unroll
   for (int b = 0; b < kS; b++)
     if (lane == b) yb = v[b];
-  if (live) ray_out_store(Ib, view, r, nr, o, yb * G.scale, v[kS] * G.scale);
+  if (live) ray_out_store(Ib, view, r, r, nr, o, yb * G.scale, v[kS] * G.scale);
 }
 
 // Rounds an FP32 sinogram to FP16 / BF16 storage (round to nearest, ties to
@@ -1545,26 +1705,37 @@ cudaError_t launch_store_sinogram(const float *src, void *dst, size_t n, int fmt
   return cudaGetLastError();
 }
 
+static size_t zcol_align(size_t b) { return (b + 255) & ~(size_t)255; }
+
+bool zcol_fits(const Dims &d) {
+  return d.nz > 1 && ((long long)d.na + kZcCols) * d.nb + kZcRows < (1LL << 31);
+}
+
+size_t ray_table_pad(const Dims &d) { return zcol_fits(d) ? (size_t)zcol_pad(d) : 0; }
+
 size_t atx_zcol_scratch_bytes(const Dims &d) {
-  const size_t a = ((size_t)d.na * sizeof(float4) + 255) & ~(size_t)255;
-  const size_t c = ((size_t)d.na * d.nb * sizeof(float4) + 255) & ~(size_t)255;
-  return a + c + 256;
+  const size_t M = (size_t)d.na * d.nb + (size_t)zcol_pad(d);
+  return zcol_align((size_t)d.na * sizeof(float4)) + zcol_align(M * sizeof(float4)) +
+         zcol_align(M * sizeof(float)) + 256;
 }
 
 cudaError_t launch_atx_zcol(float *x, const float *y, float *sc, const ViewGeo &g,
                             const Dims &d, void *scratch, cudaStream_t st) {
+  const long long nr = (long long)d.na * d.nb + zcol_pad(d);
   char *b = (char *)scratch;
   float4 *tabA = (float4 *)b;
-  float4 *tabC = (float4 *)(b + (((size_t)d.na * sizeof(float4) + 255) & ~(size_t)255));
-  int *flag = (int *)(b + atx_zcol_scratch_bytes(d) - 256);
+  float4 *tabC = (float4 *)(b + zcol_align((size_t)d.na * sizeof(float4)));
+  float *yt = (float *)((char *)tabC + zcol_align((size_t)nr * sizeof(float4)));
+  int *flag = (int *)((char *)yt + zcol_align((size_t)nr * sizeof(float)));
   cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
-  const long long nr = (long long)d.na * d.nb;
-  k_view_tab3<<<(unsigned)((nr + 255) / 256), 256, 0, st>>>(y, tabA, tabC, flag, g, d);
-  const int seg = zcol_default_seg((long long)d.nx * d.ny * d.nz);
-  k_atx_zcol<<<zcol_grid(d.nx, d.ny, d.nz, 1, seg), kAtxThreads, 0, st>>>(x, y, sc, tabA,
-                                                                          tabC, flag, g, d,
-                                                                          seg);
+  k_view_tab3<<<(unsigned)((nr + 255) / 256), 256, 0, st>>>(y, tabA, tabC, yt, flag, g, d);
+  const ZColShape s = zcol_shape(d, 1, 0);
+  const dim3 grid = zcol_grid(d, 1, s);
+  if (s.W == 32)
+    k_atx_zcol<32><<<grid, kZcThreads, 0, st>>>(x, sc, tabA, tabC, yt, flag, g, d, s.lsh(), s.seg);
+  else
+    k_atx_zcol<8><<<grid, kZcThreads, 0, st>>>(x, sc, tabA, tabC, yt, flag, g, d, s.lsh(), s.seg);
   return cudaGetLastError();
 }
 
@@ -1604,11 +1775,11 @@ cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
                             const int *zmap) {
   cudaError_t e;
   const dim3 grid = group_grid(d.nx, d.ny, d.nz, batch);
-  zseg = zseg > 0 ? zseg : zcol_default_seg((long long)d.nx * d.ny * d.nz * batch);
-  if (d.nz > 1 && zcol)
-    e = launch_iter(k_sart_atx_zcol, zcol_grid(d.nx, d.ny, d.nz, batch, zseg),
-                    dim3(kAtxThreads), st, insts, view, zseg, zmap);
-  else if (d.nz > 1 || d.nb > 1)
+  if (d.nz > 1 && zcol) {
+    const ZColShape s = zcol_shape(d, batch, zseg);
+    e = launch_iter(s.W == 32 ? k_sart_atx_zcol<32> : k_sart_atx_zcol<8>, zcol_grid(d, batch, s),
+                    dim3(kZcThreads), st, insts, view, s.lsh(), s.seg, zmap);
+  } else if (d.nz > 1 || d.nb > 1)
     e = launch_iter(k_sart_atx<false>, grid, dim3(kAtxThreads), st, insts, view, zmap);
   else
     e = launch_iter(k_sart_atx<true>, grid, dim3(kAtxThreads), st, insts, view, zmap);

@@ -1,0 +1,58 @@
+"""The cone-beam backward step in voxel columns against its per-voxel form,
+bit for bit, over the sizes and geometries where its lane and block layout and
+its pair paths change: asdpocs_atx_device takes the per-voxel form while its
+stream is captured, so one call is made plainly and one in a graph."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+pytestmark = pytest.mark.gpu
+
+# nx, ny, nz, na, nb, SO, OD (voxels), detector pitch (voxels), dz
+CASES = [
+    (20, 20, 20, 40, 30, 90.0, 45.0, 0.9, 1.0),       # 8 columns a block
+    (41, 37, 33, 64, 70, 90.0, 45.0, 0.9, 1.0),       # ragged, one slice past a warp
+    (40, 640, 10, 900, 24, 900.0, 450.0, 1.1, 1.0),   # 32 columns, 16 lanes
+    (33, 1300, 7, 1500, 20, 1800.0, 900.0, 1.3, 1.0),  # 8 lanes
+    (64, 640, 24, 700, 48, 900.0, 450.0, 1.1, 1.0),   # 8 lanes, several chunks
+    (24, 24, 40, 90, 150, 90.0, 45.0, 0.4, 1.0),      # shadows of 4 columns and more rows
+    (16, 16, 24, 200, 260, 60.0, 60.0, 0.18, 1.0),    # shadows wider than the slots
+    (24, 24, 40, 40, 120, 20.0, 10.0, 0.9, 1.0),      # steep rays, corners near the source
+    (24, 20, 30, 48, 60, 90.0, 45.0, 0.9, 0.7),       # slices that are not 1
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=[str(c[:5]) for c in CASES])
+@pytest.mark.parametrize("angle", [0.0, 45.0, 90.0, 201.3])
+def test_columns_equal_voxels(gpu, case, angle):
+    import torch
+
+    nx, ny, nz, na, nb, SO, OD, det, dz = case
+    rng = np.random.default_rng(nx + nz)
+    f = np.float32
+    yd = ((np.arange(na) - na / 2.0 + 0.5) * det).astype(f)
+    zd = ((np.arange(nb) - nb / 2.0 + 0.5) * det).astype(f)
+    phi = f(np.deg2rad(angle))
+    T = lambda a: torch.tensor(a, device=gpu)  # noqa: E731
+    y, ydd, zdd = T(rng.standard_normal(na * nb).astype(f)), T(yd), T(zd)
+    out = [torch.full((nx * ny * nz,), np.nan, device=gpu) for _ in range(4)]
+    P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+
+    def call(x, sc):
+        check(load().asdpocs_atx_device(
+            P(x), P(y), P(sc), float(np.cos(phi)), float(np.sin(phi)), P(ydd), P(zdd), SO, OD, 0.7,
+            det, det, dz, nx, ny, nz, na, nb,
+            C.c_void_p(torch.cuda.current_stream().cuda_stream or None)))
+
+    call(out[0], out[1])
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        call(out[2], out[3])
+    g.replay()
+    torch.cuda.synchronize()
+    for a, b in ((0, 2), (1, 3)):
+        assert torch.equal(out[a].view(torch.int32), out[b].view(torch.int32))
+    assert float(out[1].abs().max()) > 0
