@@ -759,7 +759,8 @@ __global__ void __launch_bounds__(kAtxThreads, 4)
 // ---------------------------------------------------------------------------
 constexpr int kZcThreads = 256, kZcWarps = kZcThreads / 32;
 constexpr int kZcSlots = 6;             // detector columns of a shadow kept
-constexpr int kZcCols = 4, kZcRows = 3; // most unrolled pairs
+constexpr int kZcCols = 4, kZcRows = 3; // most listed pairs
+static_assert(kZcRows <= 4 && kZcCols <= 8, "a pair's bit is 4 s + kb");
 
 // Elements after the na * nb rays of cor and tabC that the unrolled pairs may
 // read (zeros).
@@ -830,19 +831,21 @@ __device__ __forceinline__ void zcol_pairs(const ViewGeo &G, const Dims &D,
   const unsigned below = (1u << lane) - 1u;  // lanes before this one
   const long long room = nray(D) + zcol_pad(D);
   unsigned short *const list = sh.list[warp];
-  unsigned todo = 0u, bit = 1u;  // pairs that do not hit both F1 and F2
+  unsigned todo = 0u, bit = 1u;  // pairs that do not hit both F1 and F2: bit 4 s + kb
 #pragma unroll 1
   for (int s = 0; s < mA; s++) {
     const float4 q = sh.z[s][c];
     const unsigned bits = __float_as_uint(q.w);
     const int r = r0 + s * D.nb, rows = s < cA ? cB : 0;
+    const float4 *const pc = tabC + r;
+    const float *const py = yt + r;
     float4 Cs[B];
     float y[B];
 #pragma unroll
     for (int kb = 0; kb < B; kb++) {
       const bool in = ASD_IN(r + kb, room);
-      Cs[kb] = in ? __ldg(tabC + r + kb) : make_float4(0.f, 0.f, 0.f, 0.f);
-      y[kb] = in ? __ldg(yt + r + kb) : 0.f;
+      Cs[kb] = in ? __ldg(pc + kb) : make_float4(0.f, 0.f, 0.f, 0.f);
+      y[kb] = in ? __ldg(py + kb) : 0.f;
     }
 #pragma unroll
     for (int kb = 0; kb < B; kb++) {
@@ -851,10 +854,10 @@ __device__ __forceinline__ void zcol_pairs(const ViewGeo &G, const Dims &D,
       const float e2 = h.z2 - h.z1, l2 = q.z + e2 * e2;
       const bool both = on && h.h1 && h.h2 && l2 >= kRootMin;
       const float l = both ? root_rn(l2) : 0.f;
-      sh.l[s * B + kb][t] = make_float2(l, l * y[kb]);
-      todo |= on && !both && (steep || h.h1 || h.h2) ? bit : 0u;
-      bit <<= 1;
+      sh.l[kb * mA + s][t] = make_float2(l, l * y[kb]);
+      todo |= on && !both && (steep || h.h1 || h.h2) ? bit << kb : 0u;
     }
+    bit <<= 4;
   }
   // the other pairs into the warp's list, a lane's next one at a time
   int listed = 0;
@@ -872,8 +875,8 @@ __device__ __forceinline__ void zcol_pairs(const ViewGeo &G, const Dims &D,
     const int code = i < listed ? list[i] : 0, src = code & 31, k = code >> 5;
     const int rs = __shfl_sync(0xffffffffu, r0, src);
     if (i >= listed) continue;
-    const int s = k / B, vs = v0 + src, cs = vs >> lsh;
-    const int r = rs + s * D.nb + k % B;
+    const int s = k >> 2, kb = k & 3, vs = v0 + src, cs = vs >> lsh;
+    const int r = rs + s * D.nb + kb;
     if (!ASD_IN(r, nray(D))) continue;
     const float zr = 0.0f - zcol_height(G, D, zc0 + (vs & ((1 << lsh) - 1)));
     const float4 q = sh.z[s][cs], p = sh.col[cs], Cs = __ldg(tabC + r);
@@ -883,28 +886,30 @@ __device__ __forceinline__ void zcol_pairs(const ViewGeo &G, const Dims &D,
     const float l2 = h.h1 && h.h2 ? q.z + e2 * e2
                                   : chord3_zface2(sh.pts[s][cs], h, Cs, p.x, p.y, zr, hz);
     const float l = l2 > 0.f ? sqrtf(l2) : 0.f;
-    sh.l[k][warp * 32 + src] = make_float2(l, l * yv);
+    sh.l[kb * mA + s][warp * 32 + src] = make_float2(l, l * yv);
   }
   __syncwarp();
   // rows outer, columns inner; 0 for a pair that is not there
-#pragma unroll
-  for (int kb = 0; kb < B; kb++)
+  const float2 *p = &sh.l[0][t];
 #pragma unroll 1
-    for (int s = 0; s < mA; s++) {
-      const float2 p = sh.l[s * B + kb][t];
-      acc += p.y;
-      accl += p.x;
+  for (int k = 0; k < mA; k++, p += B * kZcThreads)
+#pragma unroll
+    for (int j = 0; j < B; j++) {
+      acc += p[j * kZcThreads].y;
+      accl += p[j * kZcThreads].x;
     }
 }
 
-// Footprint sums of this block's columns; out(idx, acc, accl) takes a
-// voxel's.  Every thread of the block calls it.
-template <int W, class Out>
+// Footprint sums of this block's columns; out(idx, acc, accl, was) takes a
+// voxel's, was = old(idx) loaded before the block waits for its
+// sums.  Every thread of the
+// block calls it.
+template <int W, class Old, class Out>
 __device__ __forceinline__ void atx_zcol_walk(const ViewGeo &G, const Dims &D,
                                               const float4 *__restrict__ tabA,
                                               const float4 *__restrict__ tabC,
                                               const float *__restrict__ yt, bool narrow, int lsh,
-                                              int seg, ZColShared<W> &sh, Out out) {
+                                              int seg, ZColShared<W> &sh, Old old, Out out) {
   const int L = 1 << lsh;
   const int xt = (D.nx + W - 1) / W, ns = (D.nz + seg - 1) / seg;
   if ((long long)blockIdx.x >= (long long)xt * D.ny * ns) return;
@@ -955,6 +960,13 @@ __device__ __forceinline__ void atx_zcol_walk(const ViewGeo &G, const Dims &D,
   const bool steep = !(D.nb * G.dz_det < G.dz * G.SD);
   const int zl = lane & (L - 1);
   for (int zc0 = zb0; zc0 < zb1; zc0 += L) {
+    // this thread's voxels of the chunk: every kZcThreads-th
+    constexpr int kMine = W * 32 / kZcThreads;
+    auto voxel = [&](int i, unsigned &idx) {
+      const int v = t + i * kZcThreads, vz = zc0 + v / W, vx = x0 + v % W;
+      idx = ((unsigned)vz * D.ny + iy) * D.nx + vx;
+      return v < W * L && vx < D.nx && vz < zb1 && ASD_IN(idx, nvox(D));
+    };
     // what depends on the lane's height only
     const int iz = zc0 + zl;
     const float zc = zcol_height(G, D, iz), rz = 0.0f - zc;
@@ -1034,11 +1046,18 @@ __device__ __forceinline__ void atx_zcol_walk(const ViewGeo &G, const Dims &D,
       sh.acc[zl][c] = acc;
       sh.accl[zl][c] = accl;
     }
+    float was[kMine];
+#pragma unroll
+    for (int i = 0; i < kMine; i++) {
+      unsigned idx;
+      was[i] = voxel(i, idx) ? old(idx) : 0.f;
+    }
     __syncthreads();
-    for (int i = t; i < W * L; i += kZcThreads) {
-      const int zl = i / W, c = i % W, iz = zc0 + zl, ix = x0 + c;
-      const unsigned idx = ((unsigned)iz * D.ny + iy) * D.nx + ix;
-      if (ix < D.nx && iz < zb1 && ASD_IN(idx, nvox(D))) out(idx, sh.acc[zl][c], sh.accl[zl][c]);
+#pragma unroll
+    for (int i = 0; i < kMine; i++) {
+      unsigned idx;
+      const int v = t + i * kZcThreads;
+      if (voxel(i, idx)) out(idx, sh.acc[v / W][v % W], sh.accl[v / W][v % W], was[i]);
     }
     __syncthreads();
   }
@@ -1059,9 +1078,10 @@ __global__ void __launch_bounds__(kZcThreads, 4)
   const float beta = I.s->beta_f;
   float *m = I.m;
   atx_zcol_walk<W>(G, D, I.tabA + (long long)view * D.na, I.tabC, I.cor, narrow, lsh, seg, sh,
-                   [&](unsigned idx, float acc, float accl) {
+                   [&](unsigned idx) { return m[idx]; },
+                   [&](unsigned idx, float acc, float accl, float was) {
                      const float bp = acc * G.scale, scv = accl * G.scale;
-                     const float mn = m[idx] + beta * __fdividef(bp, scv == 0.f ? 1.f : scv);
+                     const float mn = was + beta * __fdividef(bp, scv == 0.f ? 1.f : scv);
                      m[idx] = mn < 0.f ? 0.f : mn;
                    });
 }
@@ -1108,7 +1128,8 @@ __global__ void __launch_bounds__(kZcThreads, 4)
                const int *__restrict__ flag, ViewGeo G, Dims D, int lsh, int seg) {
   __shared__ ZColShared<W> sh;
   atx_zcol_walk<W>(G, D, tabA, tabC, yt, flag[0] == 0, lsh, seg, sh,
-                   [&](unsigned idx, float acc, float accl) {
+                   [](unsigned) { return 0.f; },
+                   [&](unsigned idx, float acc, float accl, float) {
                      x[idx] = acc * G.scale;
                      sc[idx] = accl * G.scale;
                    });
