@@ -62,21 +62,77 @@ __device__ __forceinline__ void ax_lane_partial(const ViewGeo &G, const Dims &D,
     ray_columns_fast<1>(R, lane, 32, ld, ys, ss);
 }
 
+// Cone beams: a warp takes kAxRows neighbouring rows of a detector column,
+// whose rays share their in-plane march.
+constexpr int kAxRows = 4;
+// Warps of a view: (rows of kAxRows) x columns, the rows of a column first.
+__host__ __device__ __forceinline__ long long ax_warps3(const Dims &d) {
+  return (long long)((d.nb + kAxRows - 1) / kAxRows) * d.na;
+}
+// Detector column and first row of warp w (w < ax_warps3, rays < 2^31).
+__device__ __forceinline__ void ax_rows(const Dims &D, long long w, int &ia, int &ib0) {
+  const unsigned n = (unsigned)((D.nb + kAxRows - 1) / kAxRows);
+  ia = (int)((unsigned)w / n);
+  ib0 = (int)((unsigned)w % n) * kAxRows;
+}
+// Totals of rays (ia, ib0 + k); rows past the detector repeat its last one.
+template <class Loader>
+__device__ __forceinline__ void ax_rows_sum(const ViewGeo &G, const Dims &D, int ia, int ib0,
+                                            Loader ld, float (&ys)[kAxRows],
+                                            float (&ss)[kAxRows]) {
+  const float yd = G.y_det[ia];
+  RayMarch R = ray_setup(G, D, yd, G.z_det[ib0]);
+  float slope2[kAxRows], lfac[kAxRows];
+#pragma unroll
+  for (int k = 0; k < kAxRows; k++) {
+    const RayMarch Rk = ray_setup(G, D, yd, G.z_det[min(ib0 + k, D.nb - 1)]);
+    slope2[k] = Rk.slope2;
+    lfac[k] = Rk.lfac;
+    ys[k] = ss[k] = 0.f;
+  }
+  ray_columns_rows<kAxRows>(R, slope2, lfac, threadIdx.x & 31, 32, ld, ys, ss);
+#pragma unroll
+  for (int k = 0; k < kAxRows; k++) {
+    ys[k] = warp_sum(ys[k]);
+    ss[k] = warp_sum(ss[k]);
+  }
+}
+
+template <bool kVol>
 __global__ void __launch_bounds__(kAxBlock)
     k_ax(const float *__restrict__ x, float *__restrict__ y,
          float *__restrict__ sr, ViewGeo G, Dims D) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long r = (long long)blockIdx.x * kAxWarps + warp;
-  if (r >= nray(D)) return;  // the whole warp
-  const unsigned ru = (unsigned)r, na = (unsigned)D.na;  // rays < 2^31
-  float ys, ss;
-  ax_lane_partial(G, D, (int)(ru % na), (int)(ru / na),
-                  [&](unsigned i) { return ASD_IN(i, nvox(D)) ? __ldg(x + i) : 0.f; }, ys, ss);
-  ys = warp_sum(ys);
-  ss = warp_sum(ss);
-  if (lane == 0) {
-    y[r] = ys * G.scale;
-    sr[r] = ss * G.scale;
+  const long long w = (long long)blockIdx.x * kAxWarps + warp;
+  if (w >= (kVol ? ax_warps3(D) : nray(D))) return;  // the whole warp
+  auto ld = [&](unsigned i) { return ASD_IN(i, nvox(D)) ? __ldg(x + i) : 0.f; };
+  if constexpr (kVol) {
+    int ia, ib0;
+    ax_rows(D, w, ia, ib0);
+    float ys[kAxRows], ss[kAxRows];
+    ax_rows_sum(G, D, ia, ib0, ld, ys, ss);
+    // lane k: row ib0 + k
+    float yv = ys[0], sv = ss[0];
+#pragma unroll
+    for (int k = 1; k < kAxRows; k++) {
+      yv = lane == k ? ys[k] : yv;
+      sv = lane == k ? ss[k] : sv;
+    }
+    if (lane < kAxRows && ib0 + lane < D.nb) {
+      const long long r = (long long)(ib0 + lane) * D.na + ia;
+      y[r] = yv * G.scale;
+      sr[r] = sv * G.scale;
+    }
+  } else {
+    const unsigned ru = (unsigned)w, na = (unsigned)D.na;  // rays < 2^31
+    float ys, ss;
+    ax_lane_partial(G, D, (int)(ru % na), (int)(ru / na), ld, ys, ss);
+    ys = warp_sum(ys);
+    ss = warp_sum(ss);
+    if (lane == 0) {
+      y[w] = ys * G.scale;
+      sr[w] = ss * G.scale;
+    }
   }
 }
 
@@ -433,8 +489,9 @@ __device__ __forceinline__ void ray_slopes(const Inst &I, const ViewGeo &G, cons
 
 // For 3D geometry also writes the view's ray slopes (Inst::tabc_mode: a
 // shared table's writer does so even after its own iterations have ended).
-// Rays are taken in the order that cor and tabC keep them.
-template <bool k3D>
+// Volumes: a warp takes kAxRows rows of a detector column (lane k their k-th
+// ray's value, residual and slopes), else one ray.
+template <bool k3D, bool kVol>
 __global__ void __launch_bounds__(kAxBlock)
     k_sart_ax(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap) {
   pdl_enter();
@@ -444,34 +501,45 @@ __global__ void __launch_bounds__(kAxBlock)
   const bool tabc = k3D && (I.tabc_mode == kTabcShared || (!done && I.tabc_mode == kTabcOwn));
   if (done && !tabc) return;
   const Dims D = I.d;
-  const bool rt = k3D && I.rays_t;
-  const long long nr = nray(D), q0 = (long long)blockIdx.x * kAxWarps;
-  // ray q of the order: (ia, ib), rays < 2^31
-  auto ray = [&](long long q, int &ia, int &ib) {
-    const unsigned n = (unsigned)(rt ? D.nb : D.na), hi = (unsigned)q / n, lo = (unsigned)q % n;
-    ia = (int)(rt ? hi : lo);
-    ib = (int)(rt ? lo : hi);
-  };
-  int ia, ib;
-  const ViewGeo G = view_of(I, view);
-  if (tabc && threadIdx.x < kAxWarps && q0 + threadIdx.x < nr) {
-    ray(q0 + threadIdx.x, ia, ib);
-    ray_slopes(I, G, D, view, ia, ib, q0 + threadIdx.x);
-  }
   const int lane = threadIdx.x & 31;
-  const long long q = q0 + (threadIdx.x >> 5);
-  if (done || q >= nr) return;  // the whole warp
-  ray(q, ia, ib);
-  const long long r = (long long)ib * D.na + ia;
+  const long long nr = nray(D), w = (long long)blockIdx.x * kAxWarps + (threadIdx.x >> 5);
+  if (w >= (kVol ? ax_warps3(D) : nr)) return;  // the whole warp
+  const ViewGeo G = view_of(I, view);
+  int ia, ib;  // the warp's first ray
+  if (kVol) {
+    ax_rows(D, w, ia, ib);
+  } else {
+    ia = (int)((unsigned)w % (unsigned)D.na);
+    ib = (int)((unsigned)w / (unsigned)D.na);
+  }
+  // lane's own ray
+  const int mine = ib + lane;
+  const bool own = lane < (kVol ? kAxRows : 1) && mine < D.nb;
+  const long long r = (long long)mine * D.na + ia;
+  const long long q = k3D && I.rays_t ? (long long)ia * D.nb + mine : r;
+  if (tabc && own) ray_slopes(I, G, D, view, ia, mine, q);
+  if (done) return;
   RayOut o{0.f, 0.0};
-  if (lane == 0) o = ray_out_load(I, view, r, nr);
+  if (own) o = ray_out_load(I, view, r, nr);
   const float *m = I.m;
-  float ys, ss;
-  ax_lane_partial(G, D, ia, ib, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; }, ys,
-                  ss);
-  ys = warp_sum(ys);
-  ss = warp_sum(ss);
-  if (lane == 0) ray_out_store(I, view, r, q, nr, o, ys * G.scale, ss * G.scale);
+  auto ld = [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; };
+  float yv, sv;
+  if constexpr (kVol) {
+    float ys[kAxRows], ss[kAxRows];
+    ax_rows_sum(G, D, ia, ib, ld, ys, ss);
+    yv = ys[0];
+    sv = ss[0];
+#pragma unroll
+    for (int k = 1; k < kAxRows; k++) {
+      yv = lane == k ? ys[k] : yv;
+      sv = lane == k ? ss[k] : sv;
+    }
+  } else {
+    ax_lane_partial(G, D, ia, ib, ld, yv, sv);
+    yv = warp_sum(yv);
+    sv = warp_sum(sv);
+  }
+  if (own) ray_out_store(I, view, r, q, nr, o, yv * G.scale, sv * G.scale);
 }
 
 // k_sart_ax with the exact projection (siddon_warp_rays): a warp per 32 rays,
@@ -1583,16 +1651,19 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
           for (int u = 0; u < kU; u++)
             column_pieces_planar(R, iu0 + u * 32, id[u], w[u], f[u]);
         } else {
-          Column3 c[kU];
+          ColumnV cv[kU];
+          ColumnZ cz[kU];
           bool some = false;
 #pragma unroll
           for (int u = 0; u < kU; u++) {
-            c[u] = column_cells3(R, iu0 + u * 32);
-            some = some || ((c[u].vlo || c[u].vhi) && (c[u].zlo || c[u].zhi));
+            cv[u] = column_v(R, iu0 + u * 32);
+            cz[u] = column_z(R, R.slope2, cv[u]);
+            some = some || ((cv[u].lo || cv[u].hi) && (cz[u].lo || cz[u].hi));
           }
           if (!any_lane(some)) continue;
 #pragma unroll
-          for (int u = 0; u < kU; u++) column_pieces3(R, iu0 + u * 32, c[u], id[u], w[u], f[u]);
+          for (int u = 0; u < kU; u++)
+            column_pieces3(R, R.lfac, iu0 + u * 32, cv[u], cz[u], id[u], w[u], f[u]);
         }
         float4 x[kU][kP][kQ];
 #pragma unroll
@@ -1697,12 +1768,20 @@ __global__ void __launch_bounds__(256)
 
 }  // namespace
 
+// Blocks of the forward kernels that take an instance at a time.
+static unsigned ax_blocks(const Dims &d) {
+  const long long warps = d.nz > 1 ? ax_warps3(d) : (long long)d.na * d.nb;
+  return (unsigned)((warps + kAxWarps - 1) / kAxWarps);
+}
+
 cudaError_t launch_ax(const float *x, float *y, float *sr, const ViewGeo &g,
                       const Dims &d, cudaStream_t st) {
   const long long nr = (long long)d.na * d.nb;
   if (nr == 0) return cudaSuccess;
-  const unsigned blocks = (unsigned)((nr + kAxWarps - 1) / kAxWarps);
-  k_ax<<<blocks, kAxBlock, 0, st>>>(x, y, sr, g, d);
+  if (d.nz > 1)
+    k_ax<true><<<ax_blocks(d), kAxBlock, 0, st>>>(x, y, sr, g, d);
+  else
+    k_ax<false><<<ax_blocks(d), kAxBlock, 0, st>>>(x, y, sr, g, d);
   return cudaGetLastError();
 }
 
@@ -1764,8 +1843,7 @@ cudaError_t launch_sart_ax(const Inst *insts, int batch, const Dims &d,
                            int view, cudaStream_t st, bool exact, const int *zmap) {
   cudaError_t e;
   const long long nr = (long long)d.na * d.nb;
-  const unsigned blocks = (unsigned)((nr + kAxWarps - 1) / kAxWarps);
-  const dim3 grid(blocks, 1, batch);
+  const dim3 grid(ax_blocks(d), 1, batch);
   const dim3 grid_ex((unsigned)((nr + kSidRays - 1) / kSidRays), 1, batch);
   const bool p3 = d.nz > 1 || d.nb > 1;
   if (exact) {
@@ -1774,10 +1852,12 @@ cudaError_t launch_sart_ax(const Inst *insts, int batch, const Dims &d,
     else
       e = launch_iter(k_sart_ax_exact<false>, grid_ex, dim3(kAxBlock), st, insts, view, zmap);
   } else {
-    if (p3)
-      e = launch_iter(k_sart_ax<true>, grid, dim3(kAxBlock), st, insts, view, zmap);
+    if (d.nz > 1)
+      e = launch_iter(k_sart_ax<true, true>, grid, dim3(kAxBlock), st, insts, view, zmap);
+    else if (p3)
+      e = launch_iter(k_sart_ax<true, false>, grid, dim3(kAxBlock), st, insts, view, zmap);
     else
-      e = launch_iter(k_sart_ax<false>, grid, dim3(kAxBlock), st, insts, view, zmap);
+      e = launch_iter(k_sart_ax<false, false>, grid, dim3(kAxBlock), st, insts, view, zmap);
   }
   return e;
 }
