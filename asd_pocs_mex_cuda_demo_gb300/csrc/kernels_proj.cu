@@ -63,8 +63,11 @@ __device__ __forceinline__ void ax_lane_partial(const ViewGeo &G, const Dims &D,
 }
 
 // Cone beams: a warp takes kAxRows neighbouring rows of a detector column,
-// whose rays share their in-plane march.
-constexpr int kAxRows = 4;
+// whose rays share their in-plane march.  One 256^3 view of a reconstruction,
+// 512^2 detector: 283 us with one row a warp, 243 with two, 227 with four,
+// 243 with eight; four rows at 7 blocks per SM (72 registers instead of the
+// 95 it would take; issue 77 %) 206 us, 6 blocks 208, 8 blocks 213.
+constexpr int kAxRows = 4, kAxRowBlocks = 7;
 // Warps of a view: (rows of kAxRows) x columns, the rows of a column first.
 __host__ __device__ __forceinline__ long long ax_warps3(const Dims &d) {
   return (long long)((d.nb + kAxRows - 1) / kAxRows) * d.na;
@@ -99,7 +102,7 @@ __device__ __forceinline__ void ax_rows_sum(const ViewGeo &G, const Dims &D, int
 }
 
 template <bool kVol>
-__global__ void __launch_bounds__(kAxBlock)
+__global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
     k_ax(const float *__restrict__ x, float *__restrict__ y,
          float *__restrict__ sr, ViewGeo G, Dims D) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -492,7 +495,7 @@ __device__ __forceinline__ void ray_slopes(const Inst &I, const ViewGeo &G, cons
 // Volumes: a warp takes kAxRows rows of a detector column (lane k their k-th
 // ray's value, residual and slopes), else one ray.
 template <bool k3D, bool kVol>
-__global__ void __launch_bounds__(kAxBlock)
+__global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
     k_sart_ax(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap) {
   pdl_enter();
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
@@ -1527,6 +1530,7 @@ __global__ void __launch_bounds__(kAtxThreads, kPlanar ? 4 : 5)
   pdl_enter();
   const int g0 = gtab ? gtab[blockIdx.z].x : (int)blockIdx.z * kShareGroup;
   const int gn = gtab ? gtab[blockIdx.z].y : min(kShareGroup, batch - g0);
+  if (view >= insts[g0].nv) return;  // a group with fewer views
   if (threadIdx.x == 0) {
     s_active = 0u;
     s_finite = 1;

@@ -736,3 +736,15 @@ def test_launch_shapes_do_not_change_results(gpu):
             out = recon(paras, [phi] * batch, Ps, **dict(sh))
             for a, b in zip(ref, out):
                 assert np.array_equal(a, b), (batch, sh)
+
+
+def test_phase_timing_of_a_plan_with_different_view_counts(gpu):
+    """asdpocs_plan_time_phase launches every view up to the plan's largest
+    count for every group; a group that has fewer takes no part in the rest."""
+    insts = [_uneven(s, 48, 96, nv, 1, 2, gseed=nv) for s, nv in ((1, 9), (2, 9), (3, 40), (4, 40))]
+    with pkg.Plan([p for _, _, p in insts], [p["phi_vec"] for _, _, p in insts]) as pl:
+        for k, (_, P, _) in enumerate(insts):
+            pl.set_sinogram(k, P.ravel(order="F"))
+        pl.reset()
+        for phase in range(4):
+            assert pl.time_phase(phase, 40) > 0.0
