@@ -169,6 +169,20 @@ struct Scalars {
   int cor_bad;      // 1 + the last view with a residual that is not finite
 };
 
+// Instances per group of the shared-geometry kernels; their residuals are
+// stored interleaved, cor[r * kShareSlots + slot].
+constexpr int kShareSlots = 8;
+
+// What the projector steps of a shared-geometry group need of its instances,
+// gathered once per sweep (k_group_pack): neither the step sizes nor which
+// instances run change within one.
+struct GroupState {
+  float beta[kShareSlots];
+  unsigned active;  // running slots
+  int bad;          // 1 + the last view with a residual that is not finite
+  int pad[6];
+};
+
 struct Inst {
   Dims d;                    // this instance's volume and detector sizes
   int nv;                    // and number of views (a plan's grids are sized
@@ -196,6 +210,7 @@ struct Inst {
                              //   during the SART sweep, voxel-major, slot
                              //   minor (m_il[v * kShareSlots + slot]); the
                              //   group's base, or nullptr
+  GroupState *grp;           // the group's state, or nullptr
   float4 *tabA;              // ray slopes of every view, nv*na (ray_tab_a)
   int *vflags;               // per view: kViewAxisParallel | kViewNotX | kViewNotY
   float4 *tabC;              // 3D ray slopes of the current view, na*nb
@@ -226,10 +241,6 @@ __host__ __device__ inline size_t sino_elem_bytes(int fmt) {
 }
 
 constexpr int kMaxPartials = 1 << 22;  // blocks per reduction (sanity bound)
-
-// Instances per group of the shared-geometry kernels; their residuals are
-// stored interleaved, cor[r * kShareSlots + slot].
-constexpr int kShareSlots = 8;
 
 // Inst::tabc_mode.  kTabcOwn: the instance writes its own table while it
 // runs.  Instances sharing geometry share one table: its writer
@@ -279,25 +290,26 @@ __device__ __forceinline__ bool tile_voxel(int nx, int ny, int nz, int &ix,
 // group.  Grids are (x tiles, y groups * nz, instances).
 constexpr int kTilesPerBlock = 4;
 
-__host__ __device__ inline dim3 group_grid(int nx, int ny, int nz, int batch) {
+__host__ __device__ inline dim3 group_grid(int nx, int ny, int nz, int batch,
+                                           int tiles = kTilesPerBlock) {
   const int ty = (ny + kTileY - 1) / kTileY;
-  const int gy = (ty + kTilesPerBlock - 1) / kTilesPerBlock;
+  const int gy = (ty + tiles - 1) / tiles;
   return dim3((nx + kTileX - 1) / kTileX, gy * nz, batch);
 }
 
-// Origin of tile t (0 <= t < kTilesPerBlock) of this block's group; false
-// when the group has fewer tiles (block-uniform).
+// Origin of tile t (0 <= t < tiles) of this block's group; false when the
+// group has fewer tiles (block-uniform).
 __device__ __forceinline__ bool group_tile(int ny, int nz, int t, int &x0,
-                                           int &y0, int &z) {
+                                           int &y0, int &z, int tiles = kTilesPerBlock) {
   const int ty = (ny + kTileY - 1) / kTileY;
   int g = blockIdx.y;
   z = 0;
   if (nz > 1) {
-    const int gy = (ty + kTilesPerBlock - 1) / kTilesPerBlock;
+    const int gy = (ty + tiles - 1) / tiles;
     z = g / gy;
     g -= z * gy;
   }
-  const int tyi = g * kTilesPerBlock + t;
+  const int tyi = g * tiles + t;
   x0 = blockIdx.x * kTileX;
   y0 = tyi * kTileY;
   return tyi < ty;

@@ -331,7 +331,7 @@ cudaError_t build_chord_tables(const Inst *d_inst, const Dims &d, int nv,
   if (e == cudaSuccess) e = launch_atx_chords(d_inst, d, nv, 0, nullptr, kmax, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(hk, kmax, sizeof(hk), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  const int K = hk[0];
+  const int K = hk[0] + (hk[0] & 1);  // slots are read in pairs
   const size_t bytes = atx_chord_words(d, nv, K) * sizeof(int);
   int *tab = nullptr;
   if (e == cudaSuccess && K > 0 && K <= atx_chord_max_slots() && bytes <= max_bytes &&
@@ -802,6 +802,7 @@ InstLayout layout_instance(const asdpocs_geometry &g, int max_iter,
   const size_t pad = ray_table_pad(d);
   o.cor = off; off += geo ? align256((cor_floats + pad) * 4) : 0;
   o.m_il = off; off += geo ? align256(il_floats * 4) : 0;
+  o.grp = off; off += geo ? align256(il_floats / (N * kShareSlots) * sizeof(GroupState)) : 0;
   o.tabA = off; off += geo ? align256((size_t)g.na * g.nv * 16) : 0;
   o.vflags = off; off += geo ? align256((size_t)g.nv * 4) : 0;
   o.tabC = off; off += geo ? align256(proj3d ? (M + pad) * 16 : 16) : 0;
@@ -846,6 +847,7 @@ cudaError_t bind_geometry(Inst &I, char *b, const InstLayout &o,
   I.cor_stride = 1;
   I.rays_t = 0;
   I.m_il = nullptr;
+  I.grp = nullptr;
   I.tabA = (float4 *)(b + o.tabA);
   I.vflags = (int *)(b + o.vflags);
   I.tabC = (float4 *)(b + o.tabC);
@@ -1536,12 +1538,14 @@ int asdpocs_plan_create(asdpocs_plan *out, int batch,
       I.cor = (float *)(b + base[g] + lay[g].cor) + (p->slot[i] - p->slot[g]);
       I.cor_stride = kShareSlots;
       I.m_il = (float *)(b + base[g] + lay[g].m_il);
+      I.grp = (GroupState *)(b + base[g] + lay[g].grp);
     }
     if (p->shared) {
       const int g = i - i % kShareSlots;
       I.cor = (float *)(b + base[g] + lay[g].cor) + i % kShareSlots;
       I.cor_stride = kShareSlots;
       I.m_il = (float *)(b + base[g] + lay[g].m_il);
+      I.grp = (GroupState *)(b + base[g] + lay[g].grp);
       // one ray-slope table per sub-batch: its first instance refreshes it
       // every view (the sub-batches run different views at a time)
       const int f = plan_sub_first(p, i);
@@ -1890,7 +1894,19 @@ int asdpocs_plan_time_phase(asdpocs_plan p, int phase, int reps,
       default: return launch_after_sweep(p->d_inst, p->batch, p->d, p->st);
     }
   };
-  cudaError_t e = cudaSuccess;
+  // the groups' states, as an iteration's first kernel leaves them
+  auto pack = [&]() {
+    cudaError_t e = cudaSuccess;
+    if (p->mixed) {
+      for (const SubBatch &s : p->subs)
+        if (e == cudaSuccess)
+          e = launch_group_pack(p->d_inst, 0, s.d, 0, p->st, s.gall, (int)s.groups_host.size());
+    } else if (p->shared) {
+      e = launch_group_pack(p->d_inst, p->batch, p->d, 0, p->st);
+    }
+    return e;
+  };
+  cudaError_t e = phase < 2 ? pack() : cudaSuccess;
   float ms = 0.f;
   if (phase == 1) {
     // the backward step reads what the forward step of its view leaves (the
@@ -1909,7 +1925,7 @@ int asdpocs_plan_time_phase(asdpocs_plan p, int phase, int reps,
       ms += t;
     }
   } else {
-    e = launch(0);  // warm-up
+    if (e == cudaSuccess) e = launch(0);  // warm-up
     if (e == cudaSuccess) e = cudaEventRecord(e0, p->st);
     for (int i = 0; i < reps && e == cudaSuccess; i++) e = launch(i);
     if (e == cudaSuccess) e = cudaEventRecord(e1, p->st);

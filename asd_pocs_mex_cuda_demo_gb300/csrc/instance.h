@@ -10,7 +10,7 @@ namespace asd {
 // (each 256-byte aligned), at the instance's own sizes; `bytes` is the
 // block's size.
 struct InstLayout {
-  size_t P, m, m_pre, m_res, m_k1, I0, tvb, tvc, cor, m_il, ydet, zdet, trig,
+  size_t P, m, m_pre, m_res, m_k1, I0, tvb, tvc, cor, m_il, grp, ydet, zdet, trig,
       rmse, part, cnt, ddr, scal, tabA, tabC, vflags, bytes;
   int p_fmt;  // sinogram storage (ASDPOCS_STORE_*)
 };

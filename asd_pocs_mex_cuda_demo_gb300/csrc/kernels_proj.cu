@@ -471,16 +471,16 @@ __device__ __forceinline__ RayOut ray_out_load(const Inst &I, int view, long lon
   o.dd = ASD_IN(r, nr) ? I.ddr[r] : 0.0;
   return o;
 }
-// q: where cor keeps the ray
-__device__ __forceinline__ void ray_out_store(const Inst &I, int view, long long r, long long q,
-                                              long long nr, const RayOut &o, float yv,
-                                              float srv) {
+// q: where cor keeps the ray; bad: Scalars::cor_bad or GroupState::bad
+__device__ __forceinline__ void ray_out_store(const Inst &I, int *bad, int view, long long r,
+                                              long long q, long long nr, const RayOut &o,
+                                              float yv, float srv) {
   const float c0 = o.p - yv;
   const float cr = c0 / (srv == 0.f ? 1.f : srv);
   if (!ASD_IN(r, nr) || !ASD_IN(q, nr)) return;
   I.cor[q * I.cor_stride] = cr;
   I.ddr[r] = o.dd + (double)(c0 * c0);
-  if (!isfinite(cr)) I.s->cor_bad = view + 1;
+  if (!isfinite(cr)) *bad = view + 1;
 }
 
 // The view's slopes of ray (ia, ib) for the backward step that follows (3-D).
@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
     yv = warp_sum(yv);
     sv = warp_sum(sv);
   }
-  if (own) ray_out_store(I, view, r, q, nr, o, yv * G.scale, sv * G.scale);
+  if (own) ray_out_store(I, &I.s->cor_bad, view, r, q, nr, o, yv * G.scale, sv * G.scale);
 }
 
 // k_sart_ax with the exact projection (siddon_warp_rays): a warp per 32 rays,
@@ -570,7 +570,8 @@ __global__ void __launch_bounds__(kAxBlock)
   siddon_warp_rays(G, D, r0, nr, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; },
                    yv, sv);
   if (r < nr)
-    ray_out_store(I, view, r, q, nr, ray_out_load(I, view, r, nr), yv * G.scale, sv * G.scale);
+    ray_out_store(I, &I.s->cor_bad, view, r, q, nr, ray_out_load(I, view, r, nr), yv * G.scale,
+                  sv * G.scale);
 }
 
 // Planar chord for a window whose rays share dominant axis AX (1: x, 2: y;
@@ -592,10 +593,11 @@ __device__ __forceinline__ float chord_sel(const float4 A, float rx, float ry,
 // repeating the window, shadow and face tests of find_l for every group and
 // iteration.  Per view the table holds, for voxel vi = iy * nx + ix of the
 // N = nx * ny voxels:
-//   hdr[vi]          (count << 24) | first ray, 0 for no pair
-//   sum[vi]          the voxel's chord sum (float bits)
-//   ch[k * N + vi]   chord of pair k < count (ray first + k)
-// in that order, (2 + chK) * N words per view.  The pairs, their chords and
+//   head[vi]         (count << 24) | first ray, 0 for no pair; and the
+//                    normalisation 1 / (chord sum) (float bits)
+//   pair[p * N + vi] chords of pairs 2 p and 2 p + 1 < count (rays first + k)
+// in that order, (2 + chK) * N words per view (chK is even, so that heads and
+// pairs are 8-byte aligned).  The pairs, their chords and
 // the chord sum are those of the narrow form of the backward steps
 // (sart_atx_tiles, atx_shared_voxel), in the same order and from the same
 // functions, so they give the same bits with or without the table.  Views
@@ -611,52 +613,89 @@ __host__ __device__ __forceinline__ size_t chord_view_words(const Dims &d, int K
   return (size_t)(2 + K) * (size_t)d.nx * (size_t)d.ny;
 }
 
-// Backward step over this block's tile group from the view's chord table
-// (2-D, narrow form; see sart_atx_tiles): the image value, header, chord sum
-// and first kChordPre chords of a voxel are loaded together, then its
-// residuals (L1) in the pairs' order.
-__device__ __forceinline__ void sart_atx_tiles_tab(const Inst &I, const ViewGeo &G,
-                                                   const Dims &D, const int *__restrict__ tab,
-                                                   int K) {
+// SART update of a voxel (ASD_POCS_cuda.m:127-131): m += beta * Atx(cor) / sumC
+// and positivity, the projector's common scale cancelled: accl is the voxel's
+// chord sum, acc its weighted sum.  Every backward kernel uses these two, so
+// a voxel's result does not depend on the kernel.  The reciprocal is the
+// hardware's (1 ulp); max.NaN keeps NaN, as m(m<0)=0 does.
+__device__ __forceinline__ float sart_norm(float accl) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(accl == 0.f ? 1.f : accl));
+  return r;
+}
+__device__ __forceinline__ float sart_update(float m, float beta, float acc, float norm) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(__fmaf_rn(beta, acc * norm, m)), "f"(0.f));
+  return r;
+}
+// Pair of a 2-D voxel: one rounding.
+__device__ __forceinline__ void pair2(float &acc, float l, float y) { acc = __fmaf_rn(l, y, acc); }
+
+// A voxel's table entries that do not depend on its header: head and the
+// first kChordPre chords.
+struct ChordPre {
+  int cnt, first;
+  float norm;
+  float l[kChordPre];  // 0 past cnt
+};
+__device__ __forceinline__ ChordPre chord_load(const int *__restrict__ tab, size_t N, int K,
+                                               unsigned vi) {
+  static_assert(kChordPre % 2 == 0, "slots are read in pairs");
+  ChordPre c;
+  const int2 h = __ldg((const int2 *)tab + vi);
+  const float2 *__restrict__ pair = (const float2 *)(tab + 2 * N) + vi;
+#pragma unroll
+  for (int p = 0; p < kChordPre / 2; p++) {
+    const float2 v = 2 * p < K ? __ldg(pair + (size_t)p * N) : make_float2(0.f, 0.f);
+    c.l[2 * p] = v.x;
+    c.l[2 * p + 1] = v.y;
+  }
+  c.cnt = (int)((unsigned)h.x >> 24);
+  c.first = h.x & 0xffffff;
+  c.norm = __int_as_float(h.y);
+#pragma unroll
+  for (int k = 0; k < kChordPre; k++) c.l[k] = k < c.cnt ? c.l[k] : 0.f;
+  return c;
+}
+__device__ __forceinline__ float chord_slot(const int *__restrict__ tab, size_t N, unsigned vi,
+                                            int k) {
+  return __ldg((const float *)(tab + 2 * N) + (size_t)(k / 2) * 2 * N + 2 * vi + (k & 1));
+}
+
+// Backward step over this block's `tiles` tiles from the view's chord table
+// (2-D, narrow form; see sart_atx_tiles): the image value, header and first
+// kChordPre chords of a voxel are loaded together, then its residuals (L1) in
+// the pairs' order.  Pairs past a voxel's own add 0 times a residual, which is
+// finite here.
+__device__ __forceinline__ void sart_atx_tiles_tab(const Inst &I, const Dims &D,
+                                                   const int *__restrict__ tab, int K,
+                                                   int tiles) {
   const float beta = I.s->beta_f;
   float *m = I.m;
   const float *__restrict__ cor = I.cor;
   const size_t N = (size_t)D.nx * D.ny;
-  for (int t = 0; t < kTilesPerBlock; t++) {
+  const long long M = nray(D);
+  for (int t = 0; t < tiles; t++) {
     int x0, y0, iz;
-    if (!group_tile(D.ny, D.nz, t, x0, y0, iz)) break;
+    if (!group_tile(D.ny, D.nz, t, x0, y0, iz, tiles)) break;
     const int ix = x0 + threadIdx.x % kTileX, iy = y0 + threadIdx.x / kTileX;
     const bool valid = ix < D.nx && iy < D.ny;
     const unsigned vi = valid ? (unsigned)iy * D.nx + ix : 0u;
-    const float *__restrict__ ch = (const float *)(tab + 2 * N) + vi;
-    int h = 0;
-    float accl = 0.f, mv = 0.f;
-    float pre[kChordPre];
-#pragma unroll
-    for (int k = 0; k < kChordPre; k++) pre[k] = 0.f;
-    if (valid && ASD_IN(vi, N)) {
-      h = __ldg(tab + vi);
-      accl = __int_as_float(__ldg(tab + N + vi));
-#pragma unroll
-      for (int k = 0; k < kChordPre; k++)
-        if (k < K) pre[k] = __ldg(ch + (size_t)k * N);  // slot k < K exists
-      mv = m[vi];
-    }
-    const int cnt = (int)((unsigned)h >> 24), first = h & 0xffffff;
-    const int kA = __reduce_max_sync(0xffffffffu, cnt);
-    const long long M = nray(D);
+    if (!ASD_IN(vi, N)) continue;
+    const ChordPre c = chord_load(tab, N, K, vi);
+    const float mv = m[vi];
+    const int kA = __reduce_max_sync(0xffffffffu, valid ? c.cnt : 0);
     float acc = 0.f;
 #pragma unroll
-    for (int ka = 0; ka < kChordPre; ka++)
-      if (ka < kA && ka < cnt && ASD_IN(first + ka, M)) acc += pre[ka] * __ldg(cor + first + ka);
-    for (int ka = kChordPre; ka < kA; ka++)
-      if (ka < cnt && ASD_IN(ka, K) && ASD_IN(first + ka, M))
-        acc += __ldg(ch + (size_t)ka * N) * __ldg(cor + first + ka);
-    if (valid && ASD_IN(vi, N)) {
-      const float bp = acc * G.scale, scv = accl * G.scale;
-      const float mn = mv + beta * __fdividef(bp, scv == 0.f ? 1.f : scv);
-      m[vi] = mn < 0.f ? 0.f : mn;
+    for (int ka = 0; ka < kChordPre; ka++) {
+      if (ka >= kA) break;
+      const int r = c.first + (ka < c.cnt ? ka : 0);
+      if (ASD_IN(r, M)) pair2(acc, c.l[ka], __ldg(cor + r));
     }
+    for (int ka = kChordPre; ka < kA; ka++)
+      if (ka < c.cnt && ASD_IN(ka, K) && ASD_IN(c.first + ka, M))
+        pair2(acc, chord_slot(tab, N, vi, ka), __ldg(cor + c.first + ka));
+    if (valid) m[vi] = sart_update(mv, beta, acc, c.norm);
   }
 }
 
@@ -664,16 +703,16 @@ template <bool kPlanar, int AX>
 __device__ __forceinline__ void sart_atx_tiles(const Inst &I, const ViewGeo &G,
                                                const Dims &D,
                                                const float4 *__restrict__ tabA,
-                                               bool narrow) {
+                                               bool narrow, int tiles) {
   const float beta = I.s->beta_f;
   const bool planar_ok = !kPlanar || G.z_det[0] == 0.0f;
   float *m = I.m;
   const float *__restrict__ cor = I.cor;
   const float4 *__restrict__ tabC = I.tabC;
   const float rx0 = G.cos_phi * (-G.SO), ry0 = G.sin_phi * (-G.SO);
-  for (int t = 0; t < kTilesPerBlock; t++) {
+  for (int t = 0; t < tiles; t++) {
     int x0, y0, iz;
-    if (!group_tile(D.ny, D.nz, t, x0, y0, iz)) break;
+    if (!group_tile(D.ny, D.nz, t, x0, y0, iz, tiles)) break;
     const int ix = x0 + threadIdx.x % kTileX, iy = y0 + threadIdx.x / kTileX;
     const bool valid = ix < D.nx && iy < D.ny;
     float acc = 0.f, accl = 0.f;
@@ -721,7 +760,7 @@ __device__ __forceinline__ void sart_atx_tiles(const Inst &I, const ViewGeo &G,
             const float yv = on && ASD_IN(ia, nray(D)) ? __ldg(cor + ia) : 0.f;
             const float l = chord_sel<AX>(A, rx, ry, G.dz);
             if (on) {
-              acc += l * yv;
+              pair2(acc, l, yv);
               accl += l;
             }
           }
@@ -756,11 +795,8 @@ __device__ __forceinline__ void sart_atx_tiles(const Inst &I, const ViewGeo &G,
       }
     }
     const unsigned idx = ((unsigned)iz * D.ny + iy) * D.nx + ix;
-    if (valid && ASD_IN(idx, nvox(D))) {
-      const float bp = acc * G.scale, scv = accl * G.scale;
-      const float mn = m[idx] + beta * __fdividef(bp, scv == 0.f ? 1.f : scv);
-      m[idx] = mn < 0.f ? 0.f : mn;
-    }
+    if (valid && ASD_IN(idx, nvox(D)))
+      m[idx] = sart_update(m[idx], beta, acc, sart_norm(accl));
   }
 }
 
@@ -775,25 +811,26 @@ __device__ __forceinline__ void sart_atx_tiles(const Inst &I, const ViewGeo &G,
 // axis-specialised chord.
 template <bool kPlanar>
 __global__ void __launch_bounds__(kAtxThreads, 4)
-    k_sart_atx(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap) {
+    k_sart_atx(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap,
+               int tiles) {
   pdl_enter();
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
   if (view >= I.nv || ((volatile int *)&I.s->done)[0]) return;
   const Dims D = I.d;
-  if (own_block(group_grid(D.nx, D.ny, D.nz, 1)).bid < 0) return;
+  if (own_block(group_grid(D.nx, D.ny, D.nz, 1, tiles)).bid < 0) return;
   const ViewGeo G = view_of(I, view);
   const float4 *tabA = I.tabA + (long long)view * D.na;
   const int vf = I.vflags[view];
   const bool narrow = !(vf & kViewAxisParallel) && I.s->cor_bad != view + 1 &&
                       (!kPlanar || G.z_det[0] == 0.0f);
   if (kPlanar && narrow && I.chtab)
-    sart_atx_tiles_tab(I, G, D, I.chtab + (size_t)view * chord_view_words(D, I.chK), I.chK);
+    sart_atx_tiles_tab(I, D, I.chtab + (size_t)view * chord_view_words(D, I.chK), I.chK, tiles);
   else if (!(vf & (kViewAxisParallel | kViewNotX)))
-    sart_atx_tiles<kPlanar, 1>(I, G, D, tabA, narrow);
+    sart_atx_tiles<kPlanar, 1>(I, G, D, tabA, narrow, tiles);
   else if (!(vf & (kViewAxisParallel | kViewNotY)))
-    sart_atx_tiles<kPlanar, 2>(I, G, D, tabA, narrow);
+    sart_atx_tiles<kPlanar, 2>(I, G, D, tabA, narrow, tiles);
   else
-    sart_atx_tiles<kPlanar, 0>(I, G, D, tabA, narrow);
+    sart_atx_tiles<kPlanar, 0>(I, G, D, tabA, narrow, tiles);
 }
 
 // ---------------------------------------------------------------------------
@@ -1151,9 +1188,7 @@ __global__ void __launch_bounds__(kZcThreads, 4)
   atx_zcol_walk<W>(G, D, I.tabA + (long long)view * D.na, I.tabC, I.cor, narrow, lsh, seg, sh,
                    [&](unsigned idx) { return m[idx]; },
                    [&](unsigned idx, float acc, float accl, float was) {
-                     const float bp = acc * G.scale, scv = accl * G.scale;
-                     const float mn = was + beta * __fdividef(bp, scv == 0.f ? 1.f : scv);
-                     m[idx] = mn < 0.f ? 0.f : mn;
+                     m[idx] = sart_update(was, beta, acc, sart_norm(accl));
                    });
 }
 
@@ -1221,31 +1256,23 @@ constexpr int kShareGroup = kShareSlots;
 // than 2 for cone-beam groups, the same for fan beams)
 constexpr int kPairChunk = 1;
 
-// SART update of one voxel for the group (ASD_POCS_cuda.m:128-134):
-// m += beta * (Atx(cor) * scale) / (sumC * scale), sumC == 0 -> 1, then
-// positivity.  accl is the voxel's chord sum, acc[b] slot b's weighted sum.
-__device__ __forceinline__ void atx_shared_apply(const ViewGeo &G, unsigned vi,
-                                                 float accl, const float *acc,
-                                                 unsigned active, int gn, float *m_il,
-                                                 const float *s_beta) {
-  const float scv = accl * G.scale;
-  // the group's images, interleaved: kShareGroup / 4 float4 per voxel
-  float4 *mg = (float4 *)m_il + (size_t)vi * (kShareGroup / 4);
+// SART update of one voxel for the group's running instances (sart_update):
+// m4 the group's images at the voxel, acc[b] slot b's weighted sum.
+__device__ __forceinline__ void atx_shared_apply(float norm, const float *acc,
+                                                 const GroupState &gs, unsigned active,
+                                                 const float4 (&m4)[kShareGroup / 4],
+                                                 float4 *mg) {
 #pragma unroll
   for (int q = 0; q < kShareGroup / 4; q++) {
     if (!((active >> (4 * q)) & 0xFu)) continue;
-    float4 m4 = mg[q];
-    float *mv = &m4.x;
+    const float4 b4 = __ldg((const float4 *)gs.beta + q);
+    float4 v = m4[q];
+    const float *be = &b4.x;
+    float *mv = &v.x;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int b = 4 * q + j;
-      if (b < gn && ((active >> b) & 1u)) {
-        const float bp = acc[b] * G.scale;
-        const float mn = mv[j] + s_beta[b] * __fdividef(bp, scv == 0.f ? 1.f : scv);
-        mv[j] = mn < 0.f ? 0.f : mn;
-      }
-    }
-    mg[q] = m4;
+    for (int j = 0; j < 4; j++)
+      if ((active >> (4 * q + j)) & 1u) mv[j] = sart_update(mv[j], be[j], acc[4 * q + j], norm);
+    mg[q] = v;
   }
 }
 
@@ -1254,8 +1281,7 @@ template <bool kPlanar, int AX>
 __device__ __forceinline__ void atx_shared_voxel(
     const ViewGeo &G, const Dims &D, const float4 *__restrict__ corg,
     const float4 *__restrict__ tabA, const float4 *__restrict__ tabC,
-    bool planar_ok, bool narrow, unsigned active, int gn, float *m_il,
-    const float *s_beta) {
+    bool planar_ok, bool narrow, const GroupState &gs, unsigned active, float *m_il) {
   int ix, iy, iz;
   const bool valid = tile_voxel(D, ix, iy, iz);
   VoxelWin w;
@@ -1356,10 +1382,14 @@ __device__ __forceinline__ void atx_shared_voxel(
               const float4 c4 = ASD_IN(idx[j], nray(D))
                                     ? __ldg(corg + (long long)idx[j] * (kShareGroup / 4) + q)
                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-              acc[4 * q] += l[j] * c4.x;
-              acc[4 * q + 1] += l[j] * c4.y;
-              acc[4 * q + 2] += l[j] * c4.z;
-              acc[4 * q + 3] += l[j] * c4.w;
+              const float *cv = &c4.x;
+#pragma unroll
+              for (int b = 0; b < 4; b++) {
+                if (kPlanar)
+                  pair2(acc[4 * q + b], l[j], cv[b]);
+                else
+                  acc[4 * q + b] += l[j] * cv[b];
+              }
             }
           }
         }
@@ -1369,7 +1399,11 @@ __device__ __forceinline__ void atx_shared_voxel(
   if (!valid) return;
   const unsigned vi = ((unsigned)iz * D.ny + iy) * D.nx + ix;
   if (!ASD_IN(vi, nvox(D))) return;
-  atx_shared_apply(G, vi, accl, acc, active, gn, m_il, s_beta);
+  float4 *mg = (float4 *)m_il + (size_t)vi * (kShareGroup / 4);
+  float4 m4[kShareGroup / 4];
+#pragma unroll
+  for (int q = 0; q < kShareGroup / 4; q++) m4[q] = mg[q];
+  atx_shared_apply(sart_norm(accl), acc, gs, active, m4, mg);
 }
 
 // Pairs of this voxel: the reference's window narrowed to the voxel's shadow.
@@ -1403,16 +1437,17 @@ __device__ __forceinline__ void chords_voxel(const ViewGeo &G, const Dims &D,
   const float rx = G.cos_phi * (-G.SO) - w.xc;
   const float ry = G.sin_phi * (-G.SO) - w.yc;
   if (!ASD_IN(vi, N)) return;
-  float *ch = (float *)(tab + 2 * N) + vi;
+  float *ch = (float *)(tab + 2 * N) + 2 * vi;
   float accl = 0.f;
   for (int ka = 0; ka < cnt; ka++) {
     if (!(ASD_IN(lo + ka, D.na) && ASD_IN(ka, K))) continue;
     const float l = chord_sel<AX>(__ldg(tabA + lo + ka), rx, ry, G.dz);
     accl += l;
-    ch[(size_t)ka * N] = l;
+    ch[(size_t)(ka / 2) * 2 * N + (ka & 1)] = l;
   }
-  tab[vi] = cnt ? (int)(((unsigned)cnt << 24) | (unsigned)(w.b0 * D.na + lo)) : 0;
-  tab[N + vi] = __float_as_int(accl);
+  ((int2 *)tab)[vi] =
+      make_int2(cnt ? (int)(((unsigned)cnt << 24) | (unsigned)(w.b0 * D.na + lo)) : 0,
+                __float_as_int(sart_norm(accl)));
 }
 
 // Counting (K == 0: the largest pair count into kmax[0]) or filling pass over
@@ -1439,137 +1474,88 @@ __global__ void __launch_bounds__(kAtxThreads)
     chords_voxel<0>(G, D, tabA, valid, ix, iy, K, tab, kmax);
 }
 
-// The voxel of this thread for the group, from the view's chord table: the
-// pairs, chords and accumulation order of atx_shared_voxel's narrow form,
-// and its update (atx_shared_apply).  Everything that does not depend on the
-// header -- the group's image values, the chord sum and the first
-// kChordPre chord slots -- is loaded together up front, so a warp waits for
-// DRAM once; the residuals it then reads are the view's few kB, in L1.
-// (A kernel of its own for this path, 48 registers and 5 blocks per SM with
-// the direct form out of line, measured 14 % slower: more long-scoreboard
-// stalls, fewer L1 hits.)
-
-__device__ __forceinline__ void atx_shared_voxel_tab(
-    const ViewGeo &G, const Dims &D, const float4 *__restrict__ corg,
-    const int *__restrict__ tab, int K, unsigned active, int gn, float *m_il,
-    const float *s_beta) {
-  int ix, iy, iz;
-  const bool valid = tile_voxel(D, ix, iy, iz);
-  const size_t N = (size_t)D.nx * D.ny;
-  const unsigned vi = valid ? (unsigned)iy * D.nx + ix : 0u;
-  const float *__restrict__ ch = (const float *)(tab + 2 * N) + vi;
-  float4 *mg = (float4 *)m_il + (size_t)vi * (kShareGroup / 4);
-  int h = 0;
-  float accl = 0.f;
-  float pre[kChordPre];
-  float4 m4[kShareGroup / 4];
-#pragma unroll
-  for (int k = 0; k < kChordPre; k++) pre[k] = 0.f;
-  if (valid && ASD_IN(vi, N)) {
-    h = __ldg(tab + vi);
-    accl = __int_as_float(__ldg(tab + N + vi));
-#pragma unroll
-    for (int k = 0; k < kChordPre; k++)
-      if (k < K) pre[k] = __ldg(ch + (size_t)k * N);  // slot k < K exists
-#pragma unroll
-    for (int q = 0; q < kShareGroup / 4; q++)
-      if ((active >> (4 * q)) & 0xFu) m4[q] = mg[q];
-  }
-  const int cnt = (int)((unsigned)h >> 24), first = h & 0xffffff;
-  const int kA = __reduce_max_sync(0xffffffffu, cnt);
-  float acc[kShareGroup];
-#pragma unroll
-  for (int b = 0; b < kShareGroup; b++) acc[b] = 0.f;
-  auto pair = [&](int ka, float l) {
-    const long long r = first + ka;
-    if (!ASD_IN(r, nray(D))) return;
-#pragma unroll
-    for (int q = 0; q < kShareGroup / 4; q++) {
-      if (!((active >> (4 * q)) & 0xFu)) continue;
-      const float4 c4 = __ldg(corg + r * (kShareGroup / 4) + q);
-      acc[4 * q] += l * c4.x;
-      acc[4 * q + 1] += l * c4.y;
-      acc[4 * q + 2] += l * c4.z;
-      acc[4 * q + 3] += l * c4.w;
-    }
-  };
-#pragma unroll
-  for (int ka = 0; ka < kChordPre; ka++)
-    if (ka < kA && ka < cnt) pair(ka, pre[ka]);
-  for (int ka = kChordPre; ka < kA; ka++)
-    if (ka < cnt && ASD_IN(ka, K)) pair(ka, __ldg(ch + (size_t)ka * N));
-  if (!valid || !ASD_IN(vi, N)) return;
-  // atx_shared_apply with the image values already loaded
-  const float scv = accl * G.scale;
-#pragma unroll
-  for (int q = 0; q < kShareGroup / 4; q++) {
-    if (!((active >> (4 * q)) & 0xFu)) continue;
-    float *mv = &m4[q].x;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int b = 4 * q + j;
-      if (b < gn && ((active >> b) & 1u)) {
-        const float bp = acc[b] * G.scale;
-        const float mn = mv[j] + s_beta[b] * __fdividef(bp, scv == 0.f ? 1.f : scv);
-        mv[j] = mn < 0.f ? 0.f : mn;
-      }
-    }
-    mg[q] = m4[q];
-  }
-}
-
-// 4 blocks per SM for fan beams; 5 for cone beams (measured 3 % faster at
-// 128^3, 6 % slower for fan beams, whose extra spills cost more)
+// Backward step for a group of instances sharing geometry.  With a chord
+// table (2-D) a thread's loads that depend on nothing but its position -- the
+// table's head and first kChordPre chords, the group's image values -- go out
+// together with the group's state, so that it waits for memory once before
+// the residuals (the view's few kB, in L1), and no barrier is needed.  Pairs
+// past a voxel's own add 0 times a residual, which is finite here.
+// Memory latency bounds it (28 % issue).  A launch of 64 instances, 512^2:
+// 53.5 us with the group's scalars gathered through shared memory between two
+// barriers, one load per chord and a division per instance; 42.7 us now at 4
+// blocks per SM, 41.3 at 5, 42.5 at 6; with the direct form out of line 43.8
+// (5 blocks) to 54.8 (8 blocks).
 template <bool kPlanar>
-__global__ void __launch_bounds__(kAtxThreads, kPlanar ? 4 : 5)
+__global__ void __launch_bounds__(kAtxThreads, 5)
     k_sart_atx_shared(const Inst *__restrict__ insts, int batch, int view,
                       const int2 *__restrict__ gtab) {
-  __shared__ float s_beta[kShareGroup];
-  __shared__ unsigned s_active;
-  __shared__ int s_finite;
+  (void)batch;
   pdl_enter();
   const int g0 = gtab ? gtab[blockIdx.z].x : (int)blockIdx.z * kShareGroup;
-  const int gn = gtab ? gtab[blockIdx.z].y : min(kShareGroup, batch - g0);
-  if (view >= insts[g0].nv) return;  // a group with fewer views
-  if (threadIdx.x == 0) {
-    s_active = 0u;
-    s_finite = 1;
-  }
-  __syncthreads();
-  if (threadIdx.x < gn) {
-    const Inst &Ib = insts[g0 + threadIdx.x];
-    const bool live = ((volatile int *)&Ib.s->done)[0] == 0;
-    s_beta[threadIdx.x] = Ib.s->beta_f;
-    if (live) {
-      atomicOr(&s_active, 1u << threadIdx.x);
-      if (Ib.s->cor_bad == view + 1) atomicAnd(&s_finite, 0);
-    }
-  }
-  __syncthreads();
-  const unsigned active = s_active;
-  if (!active) return;
   const Inst &I0 = insts[g0];
-  const Dims D = I0.d;  // every instance of a shared-geometry plan
-  const ViewGeo G = view_of(I0, view);
+  if (view >= I0.nv) return;  // a group with fewer views
+  const Dims D = I0.d;  // every instance of the group
+  const GroupState &gs = *I0.grp;
   // the group's residuals, interleaved: ray r of slot b at corg[r*kShareGroup + b]
   const float4 *__restrict__ corg = (const float4 *)I0.cor;
+  const int vf = I0.vflags[view];
+  if (kPlanar && I0.chtab) {
+    int ix, iy, iz;
+    const bool valid = tile_voxel(D, ix, iy, iz);
+    const size_t N = (size_t)D.nx * D.ny;
+    const int K = I0.chK;
+    const int *__restrict__ tab = I0.chtab + (size_t)view * chord_view_words(D, K);
+    const unsigned vi = valid ? (unsigned)iy * D.nx + ix : 0u;
+    float4 *mg = (float4 *)I0.m_il + (size_t)vi * (kShareGroup / 4);
+    const ChordPre c = chord_load(tab, N, K, vi);
+    float4 m4[kShareGroup / 4];
+#pragma unroll
+    for (int q = 0; q < kShareGroup / 4; q++) m4[q] = mg[q];
+    const unsigned active = gs.active;
+    if (!active) return;
+    if (!(vf & kViewAxisParallel) && gs.bad != view + 1 && I0.g.z_det[0] == 0.0f) {
+      const int kA = __reduce_max_sync(0xffffffffu, valid ? c.cnt : 0);
+      const long long M = nray(D);
+      float acc[kShareGroup];
+#pragma unroll
+      for (int b = 0; b < kShareGroup; b++) acc[b] = 0.f;
+      auto pair = [&](int r, float l) {
+        if (!ASD_IN(r, M)) return;
+        const float4 *p = corg + (size_t)r * (kShareGroup / 4);
+#pragma unroll
+        for (int q = 0; q < kShareGroup / 4; q++) {
+          if (!((active >> (4 * q)) & 0xFu)) continue;
+          const float4 c4 = __ldg(p + q);
+          pair2(acc[4 * q], l, c4.x);
+          pair2(acc[4 * q + 1], l, c4.y);
+          pair2(acc[4 * q + 2], l, c4.z);
+          pair2(acc[4 * q + 3], l, c4.w);
+        }
+      };
+#pragma unroll
+      for (int ka = 0; ka < kChordPre; ka++) {
+        if (ka >= kA) break;
+        pair(c.first + (ka < c.cnt ? ka : 0), c.l[ka]);
+      }
+      for (int ka = kChordPre; ka < kA; ka++)
+        if (ka < c.cnt && ASD_IN(ka, K)) pair(c.first + ka, chord_slot(tab, N, vi, ka));
+      if (valid && ASD_IN(vi, N)) atx_shared_apply(c.norm, acc, gs, active, m4, mg);
+      return;
+    }
+  }
+  const unsigned active = gs.active;
+  if (!active) return;
+  const ViewGeo G = view_of(I0, view);
   const float4 *__restrict__ tabA = I0.tabA + (long long)view * D.na;
   const float4 *__restrict__ tabC = I0.tabC;
-  const int vf = I0.vflags[view];
   const bool planar_ok = !kPlanar || G.z_det[0] == 0.0f;
-  const bool narrow = planar_ok && !(vf & kViewAxisParallel) && s_finite;
-  if (kPlanar && narrow && I0.chtab)
-    atx_shared_voxel_tab(G, D, corg, I0.chtab + (size_t)view * chord_view_words(D, I0.chK),
-                         I0.chK, active, gn, I0.m_il, s_beta);
-  else if (!(vf & (kViewAxisParallel | kViewNotX)))
-    atx_shared_voxel<kPlanar, 1>(G, D, corg, tabA, tabC, planar_ok, narrow, active,
-                                 gn, I0.m_il, s_beta);
+  const bool narrow = planar_ok && !(vf & kViewAxisParallel) && gs.bad != view + 1;
+  if (!(vf & (kViewAxisParallel | kViewNotX)))
+    atx_shared_voxel<kPlanar, 1>(G, D, corg, tabA, tabC, planar_ok, narrow, gs, active, I0.m_il);
   else if (!(vf & (kViewAxisParallel | kViewNotY)))
-    atx_shared_voxel<kPlanar, 2>(G, D, corg, tabA, tabC, planar_ok, narrow, active,
-                                 gn, I0.m_il, s_beta);
+    atx_shared_voxel<kPlanar, 2>(G, D, corg, tabA, tabC, planar_ok, narrow, gs, active, I0.m_il);
   else
-    atx_shared_voxel<kPlanar, 0>(G, D, corg, tabA, tabC, planar_ok, narrow, active,
-                                 gn, I0.m_il, s_beta);
+    atx_shared_voxel<kPlanar, 0>(G, D, corg, tabA, tabC, planar_ok, narrow, gs, active, I0.m_il);
 }
 
 // ---------------------------------------------------------------------------
@@ -1626,11 +1612,11 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
     ray_slopes(I0, G, D, view, (int)(rs % D.na), (int)(rs / D.na), rs);
   }
   if (r >= nr) return;  // the whole warp
+  const unsigned active = (I0.grp->active >> (4 * q0)) & ((1u << kS) - 1u);
+  if (!active) return;
   // lane b: instance gi + b
   const Inst &Ib = insts[gi + min(lane, gn - 1)];
-  const bool live = lane < gn && ((volatile int *)&Ib.s->done)[0] == 0;
-  const unsigned active = __ballot_sync(0xffffffffu, live);
-  if (!active) return;
+  const bool live = lane < gn && ((active >> lane) & 1u);
   RayOut o{0.f, 0.0};
   if (live) o = ray_out_load(Ib, view, r, nr);
   float v[kS + 1];  // the instances' sums, then the weights' sum
@@ -1710,7 +1696,7 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
 #pragma unroll
   for (int b = 0; b < kS; b++)
     if (lane == b) yb = v[b];
-  if (live) ray_out_store(Ib, view, r, r, nr, o, yb * G.scale, v[kS] * G.scale);
+  if (live) ray_out_store(Ib, &I0.grp->bad, view, r, r, nr, o, yb * G.scale, v[kS] * G.scale);
 }
 
 // Rounds an FP32 sinogram to FP16 / BF16 storage (round to nearest, ties to
@@ -1746,6 +1732,14 @@ __global__ void __launch_bounds__(256)
   }
   __syncthreads();
   const unsigned active = s_active;
+  if (!unpack && blockIdx.x == 0) {  // the sweep's group state
+    GroupState &gs = *insts[g0].grp;
+    if (threadIdx.x < gn) gs.beta[threadIdx.x] = insts[g0 + threadIdx.x].s->beta_f;
+    if (threadIdx.x == 0) {
+      gs.active = active;
+      gs.bad = 0;
+    }
+  }
   const Dims D = insts[g0].d;
   const long long n = (long long)D.nx * D.ny * D.nz;
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1879,15 +1873,25 @@ cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
                             int view, cudaStream_t st, bool zcol, int zseg,
                             const int *zmap) {
   cudaError_t e;
-  const dim3 grid = group_grid(d.nx, d.ny, d.nz, batch);
+  // fan beams: the fewest tiles a block (1, 2 or 4) that keep the launch within
+  // two blocks per SM, so that the blocks of the next, programmatic launch
+  // still find room (512^2, ten iterations: 10.7 ms with 256 blocks of four
+  // tiles, 11.2 with 512 of two, 11.5 with 1024 of one; 64^2 by itself is
+  // faster spread out)
+  int tiles = d.nz == 1 ? 1 : kTilesPerBlock;
+  dim3 grid = group_grid(d.nx, d.ny, d.nz, batch, tiles);
+  while (tiles < kTilesPerBlock && (long long)grid.x * grid.y * batch > 152 * 2) {
+    tiles *= 2;
+    grid = group_grid(d.nx, d.ny, d.nz, batch, tiles);
+  }
   if (d.nz > 1 && zcol) {
     const ZColShape s = zcol_shape(d, batch, zseg);
     e = launch_iter(s.W == 32 ? k_sart_atx_zcol<32> : k_sart_atx_zcol<8>, zcol_grid(d, batch, s),
                     dim3(kZcThreads), st, insts, view, s.lsh(), s.seg, zmap);
   } else if (d.nz > 1 || d.nb > 1)
-    e = launch_iter(k_sart_atx<false>, grid, dim3(kAtxThreads), st, insts, view, zmap);
+    e = launch_iter(k_sart_atx<false>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
   else
-    e = launch_iter(k_sart_atx<true>, grid, dim3(kAtxThreads), st, insts, view, zmap);
+    e = launch_iter(k_sart_atx<true>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
   return e;
 }
 

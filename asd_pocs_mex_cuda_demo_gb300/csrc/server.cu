@@ -189,6 +189,7 @@ Inst empty_slot(const Lane &L, int s) {
   I.cor = L.tmpl.cor + (size_t)(s / kShareSlots) * M * kShareSlots + s % kShareSlots;
   I.cor_stride = kShareSlots;
   I.m_il = L.tmpl.m_il + (size_t)(s / kShareSlots) * N * kShareSlots;
+  I.grp = L.tmpl.grp + s / kShareSlots;
   I.tabc_mode = s == 0 ? kTabcShared : kTabcNone;
   return I;
 }
@@ -220,6 +221,7 @@ bool lane_create(asdpocs_server sv, Lane &L) {
   memset(&L.tmpl, 0, sizeof L.tmpl);
   SV_CUDA(bind_geometry(L.tmpl, L.geo, gl, L.g, L.phi.data(), L.st));
   L.tmpl.m_il = (float *)(L.geo + gl.m_il);
+  L.tmpl.grp = (GroupState *)(L.geo + gl.grp);
   L.slot_desc.resize(L.S);
   for (int s = 0; s < L.S; s++) L.slot_desc[s] = empty_slot(L, s);
   SV_CUDA(cudaMemcpyAsync(L.d_inst, L.slot_desc.data(), sizeof(Inst) * L.S,
