@@ -57,11 +57,16 @@ __device__ __forceinline__ bool asd_in(long long i, long long n) {
 // plan that runs on one stream are launched with programmatic stream
 // serialization (launch_iter inside a PdlScope), so a kernel's launch and
 // block scheduling overlap the tail of the kernel before it.  Each such
-// kernel calls pdl_enter() before its first global-memory access: it waits
-// there until the preceding kernel has completed and its writes are visible
-// (so every kernel still sees all earlier ones), then lets its own successor
-// be scheduled -- once all of its blocks are resident, so the successor's
-// waiting blocks never take the slots of its own.  In a kernel launched the
+// kernel calls pdl_enter() before its first access to memory that an
+// iteration writes: it waits there until the preceding kernel has completed
+// and its writes are visible (so every kernel still sees all earlier ones),
+// then lets its own successor be scheduled -- once all of its blocks are resident, so the successor's
+// waiting blocks never take the slots of its own.  Before it, a kernel may
+// load what the plan wrote at its creation or before the run (descriptors,
+// geometry, chord tables, sinograms), which hides that latency behind the
+// kernel before.  Every block calls it, also one that then has nothing to do:
+// a grid whose blocks did not wait could end before its predecessor, and its
+// successor waits for it alone.  In a kernel launched the
 // ordinary way both instructions do nothing.  Plans that run sub-batches on
 // concurrent streams (and the serving lanes) launch the ordinary way: there
 // the successor's early, waiting blocks hold SM slots the other stream's
@@ -157,9 +162,8 @@ struct Scalars {
   double dd2;       // ||P - Ax||^2 (Inst::ddr summed) of the last complete sweep (out.dataTolerance)
   double dp;        // ||m - m_pre|| of the last sweep
   double d_tv;      // ||m - m_k1|| at TV entry (imgTVGradMin.cpp:57-60)
-  double tv_coef;   // alpha*d/||v|| of the current TV step
-  float tv_coef_f;  // FP32 copies read by the per-voxel kernels
-  float beta_f;
+  float tv_coef_f;  // alpha*d/||v|| of the current TV step
+  float beta_f;     // FP32 copy read by the per-voxel kernels
   double dg;        // ||m_TV - m_SART||
   int k;            // 1-based iteration about to run / running
   int done;         // stop criterion met or maxnumIter reached

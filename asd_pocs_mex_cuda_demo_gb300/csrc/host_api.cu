@@ -697,6 +697,7 @@ struct asdpocs_plan_s {
   int pdl = -1;         // programmatic dependent launches: -1 = when the plan
                         // runs on one stream, 0 = off, 1 = on
   Inst *d_inst = nullptr;
+  Scalars *d_start = nullptr;  // the instances' scalars at a reset, in d_inst order
   void *arena = nullptr;
   size_t bytes = 0;
   std::vector<asd::SubBatch> subs;
@@ -1503,6 +1504,8 @@ int asdpocs_plan_create(asdpocs_plan *out, int batch,
   }
   const size_t inst_off = off;
   off += align256(sizeof(Inst) * batch);
+  const size_t start_off = off;
+  off += align256(sizeof(Scalars) * batch);
   const size_t zmap_off = off;  // the sub-batches' instance and group lists
   size_t zints = 0, zpairs = 0;
   for (const SubBatch &s : p->subs) {
@@ -1554,6 +1557,7 @@ int asdpocs_plan_create(asdpocs_plan *out, int batch,
     }
   }
   p->d_inst = (Inst *)(b + inst_off);
+  p->d_start = (Scalars *)(b + start_off);
   if (e == cudaSuccess) e = plan_upload(p);
   {
     int *dz = (int *)(b + zmap_off);
@@ -1723,9 +1727,14 @@ int asdpocs_plan_set_reference(asdpocs_plan p, int inst, const float *I0,
 int asdpocs_plan_reset(asdpocs_plan p) {
   clear_error();
   if (!p) return set_error(ASDPOCS_ERR_ARG, "null plan");
+  std::vector<Scalars> start(p->batch);  // in d_inst order
   for (int i = 0; i < p->batch; i++)
-    ASD_CUDA(reset_instance(p->h_inst[i], initial_scalars(p->opt[i], p->has_ref[i]),
-                            p->st));
+    start[p->mixed ? p->slot[i] : i] = initial_scalars(p->opt[i], p->has_ref[i]);
+  ASD_CUDA(cudaMemcpyAsync(p->d_start, start.data(), sizeof(Scalars) * p->batch,
+                           cudaMemcpyHostToDevice, p->st));
+  for (int i = 0; i < p->batch; i += 65535)  // the grid's limit
+    ASD_CUDA(launch_reset(p->d_inst + i, p->d_start + i, std::min(p->batch - i, 65535), p->d,
+                          p->st));
   ASD_CUDA(cudaStreamSynchronize(p->st));
   return 0;
 }

@@ -102,6 +102,11 @@ int reduce_blocks_for(const Dims &d);
 // the end of the sweep four), or tiles x slabs of the cone-beam TV step.
 int tv_partials_for(const Dims &d);
 
+// Start state of `batch` instances (largest sizes d) with the scalars start[i]
+// (device): what reset_instance does, in one launch.  batch <= 65535.
+cudaError_t launch_reset(const Inst *insts, const Scalars *start, int batch, const Dims &d,
+                         cudaStream_t st);
+
 // Copies Inst::s->done of n instances into the device array out[n].
 cudaError_t launch_gather_done(const Inst *insts, int n, int *out,
                                cudaStream_t st);

@@ -540,6 +540,11 @@ __device__ __forceinline__ float *tv_dst(const Inst &I, int step) {
   return (step & 1) ? I.tv_c : I.tv_b;
 }
 
+// Step size alpha d / ||v|| of a TV step whose stencil's squares sum to v2.
+__device__ __forceinline__ float tv_coef(const Scalars &s, double v2) {
+  return (float)(s.alpha * s.d_tv * rsqrt(v2));
+}
+
 // End-of-iteration scalars (ASD_POCS_cuda.m:166-170) by the last block.
 __device__ __forceinline__ void finish_scalars(Scalars *s, double dg2) {
   s->dg = sqrt(dg2);
@@ -568,8 +573,7 @@ __device__ __forceinline__ void sweep_scalars(const Inst &I, const double (&tot)
     s->done = 1;
   } else {
     s->d_tv = sqrt(tot[1]);
-    s->tv_coef = s->alpha * s->d_tv / sqrt(tot[3]);
-    s->tv_coef_f = (float)s->tv_coef;
+    s->tv_coef_f = tv_coef(*s, tot[3]);
   }
 }
 
@@ -660,12 +664,18 @@ __global__ void __launch_bounds__(kThreads)
 //
 // ||v(m')||^2 (or, in the last step, the positivity-change norm) is summed
 // per band of 16 output rows of a strip -- lanes in row order, then an xor
-// butterfly -- and the walk that finishes last sums the band partials of
-// the instance in order; walks of `bands` consecutive bands (chosen by the
-// host from the batch size) therefore give the same bits for every choice.
+// butterfly -- and the band partials of the instance in order.  Launches of one
+// band per walk leave that to every block of the next step, which does it while
+// its first rows are on their way (one 512^2 image: 6.1 us a step, 8.8 with
+// a ticket in every step); in larger launches, whose blocks would repeat
+// it too often, and after the last step the walk that finishes last sums them
+// (64 images: 41.0 us a step, 43.0 the other way).  Walks of `bands`
+// consecutive bands (chosen by the host from the batch size) give the same bits
+// for every choice.
 constexpr int kWalkWarps = 4;
 constexpr int kWalkOut = 60;   // output columns of a strip
 constexpr int kBandRows = 16;  // output rows of a partial
+constexpr int kWalkBlocks = 6; // resident blocks per SM (7 and 8 spill)
 constexpr int kWalkChunk = 4;  // rows per chunk (a band ends at a chunk's end)
 constexpr int kWalkRing = 8;  // rows of m in flight per warp (shared-memory ring)
 static_assert(4 % kWalkChunk == 0 && kBandRows % 4 == 0, "bands and the steady chunks line up");
@@ -718,10 +728,10 @@ __device__ __forceinline__ void cp_async_8(float *smem, const float *gmem, bool 
                : "memory");
 }
 
-template <int kMode, bool kPair>
+template <int kMode, bool kPair, class Coef>
 __device__ __forceinline__ void tv_walk(const Inst &I, int step, int y0, int y1, int xa,
-                                        int strip, int S, float coef, float2 *ring,
-                                        float2 *ring0) {
+                                        int strip, int S, double *partials, Coef step_size,
+                                        float2 *ring, float2 *ring0) {
   const Dims D = I.d;
   const int lane = threadIdx.x & 31;
   const float *src = tv_src(I, step);
@@ -732,7 +742,6 @@ __device__ __forceinline__ void tv_walk(const Inst &I, int step, int y0, int y1,
   const bool outa = outl && ina, outb = outl && inb;
   const int jl0 = y0 - 2, jl1 = min(D.ny, y1 + 2);  // rows of m read
   const int j1 = y1 + 2;                            // rows walked: jl0 .. j1 - 1
-  const float coef_a = ina ? coef : 0.f, coef_b = inb ? coef : 0.f;
   const long long N2 = (long long)D.nx * D.ny;  // bounds-checked builds
   // Rows of m stream through a ring of kWalkRing rows per warp (each lane
   // its two columns), copied asynchronously kWalkRing - 1 rows ahead of the
@@ -766,13 +775,15 @@ __device__ __forceinline__ void tv_walk(const Inst &I, int step, int y0, int y1,
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   for (int k = 0; k < kWalkRing - 1; k++) fetch(jl0 + k, k);
+  const float coef = step_size();
+  const float coef_a = ina ? coef : 0.f, coef_b = inb ? coef : 0.f;
   WalkField f1{0.f, 0.f, 0.f, 0.f}, f2{0.f, 0.f, 0.f, 0.f};
   float acc = 0.f;
   // one partial from the band whose last output row is o
   auto flush = [&](int o) {
 #pragma unroll
     for (int w = 16; w > 0; w >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, w);
-    if (lane == 0) I.partials[(o / kBandRows) * S + strip] = (double)acc;
+    if (lane == 0) partials[(o / kBandRows) * S + strip] = (double)acc;
     acc = 0.f;
   };
   // row j of m in: v(m) and m' of row j - 1, v(m') of row j - 2
@@ -860,7 +871,7 @@ __device__ __forceinline__ void tv_walk(const Inst &I, int step, int y0, int y1,
     if (kMode == 0 && j0 >= y0 + 2 && j0 <= y1 - 3) {
 #pragma unroll
       for (int k = 0; k < kWalkChunk; k++) walk_row(std::false_type(), j0 + k, s0 + k);
-      // bands start at multiples of 32 (so does y0) and steady chunks at
+      // bands (and y0) start at multiples of kBandRows and steady chunks at
       // y0 - 2 plus a multiple of 4: a band can only end at a chunk's end
       if ((j0 + 2) % kBandRows == 0) flush(j0 + 1);
     } else {
@@ -871,40 +882,69 @@ __device__ __forceinline__ void tv_walk(const Inst &I, int step, int y0, int y1,
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");  // the ring's last copies
 }
 
-__global__ void __launch_bounds__(kWalkWarps * 32, 8)
+__global__ void __launch_bounds__(kWalkWarps * 32, kWalkBlocks)
     k_tv_walk2d(const Inst *__restrict__ insts, int step, int bands,
                 const int *__restrict__ zmap) {
   __shared__ float2 ring[kWalkWarps][kWalkRing * 32], ring0[kWalkWarps][kWalkRing * 32];
-  pdl_enter();
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
+  const Dims D = I.d;  // the descriptor, before the wait
+  pdl_enter();
   if (inst_done(I)) return;
   const int ng = I.s->ng;
   if (step >= ng) return;
-  const Dims D = I.d;
   const int S = walk_strips(D.nx), NB = walk_bands(D.ny);
   const int per_strip = (NB + bands - 1) / bands;
   const int walks = S * per_strip;
   const int w = blockIdx.x * kWalkWarps + (threadIdx.x >> 5);
-  if (w >= walks) return;  // warp-uniform
   const int lane = threadIdx.x & 31;
   const int strip = w % S, b0 = (w / S) * bands;
   const int y0 = b0 * kBandRows, y1 = min(D.ny, (b0 + bands) * kBandRows);
   const int xa = strip * kWalkOut - 2 + 2 * lane;
   const bool last = step == ng - 1;
-  const float coef = I.s->tv_coef_f;
   const bool pair = (D.nx & 1) == 0;
+  // steps take turns with two sets of partials: one is read here while the
+  // other is written
+  const int P = S * NB;
+  double *const mine = I.partials + (step & 1 ? P : 0);
+  const double *const prev = I.partials + (step & 1 ? 0 : P);
+  __shared__ float s_coef;
+  // alpha d / ||v||: of the first step from the end of the sweep, then from
+  // the partials of the step before, summed by the block's first warp.  Every
+  // warp of the block calls it once.
+  const bool ticketed = bands > 1;  // the same for every step of an iteration
+  auto total = [&](const double *partials) {
+    double a = 0.0;
+    for (int p = lane; p < P; p += 32) a += ((volatile const double *)partials)[p];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+  };
+  auto step_size = [&]() -> float {
+    if (step == 0 || ticketed) return I.s->tv_coef_f;
+    if (threadIdx.x < 32) {
+      const double a = total(prev);
+      if (lane == 0) s_coef = tv_coef(*I.s, a);
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(kWalkWarps * 32) : "memory");
+    return s_coef;
+  };
+  if (w >= walks) {  // warp-uniform
+    step_size();
+    return;
+  }
   float2 *const rg = ring[threadIdx.x >> 5], *const rg0 = ring0[threadIdx.x >> 5];
   if (!last)
-    pair ? tv_walk<0, true>(I, step, y0, y1, xa, strip, S, coef, rg, rg0)
-         : tv_walk<0, false>(I, step, y0, y1, xa, strip, S, coef, rg, rg0);
+    pair ? tv_walk<0, true>(I, step, y0, y1, xa, strip, S, mine, step_size, rg, rg0)
+         : tv_walk<0, false>(I, step, y0, y1, xa, strip, S, mine, step_size, rg, rg0);
   else if (ng == 1)
-    pair ? tv_walk<1, true>(I, step, y0, y1, xa, strip, S, coef, rg, rg0)
-         : tv_walk<1, false>(I, step, y0, y1, xa, strip, S, coef, rg, rg0);
+    pair ? tv_walk<1, true>(I, step, y0, y1, xa, strip, S, mine, step_size, rg, rg0)
+         : tv_walk<1, false>(I, step, y0, y1, xa, strip, S, mine, step_size, rg, rg0);
   else
-    pair ? tv_walk<2, true>(I, step, y0, y1, xa, strip, S, coef, rg, rg0)
-         : tv_walk<2, false>(I, step, y0, y1, xa, strip, S, coef, rg, rg0);
-  if (last && ng == 1) return;  // nothing to sum: k_finish_iter ends the iteration
-  // the walk that finishes last sums the instance's band partials
+    pair ? tv_walk<2, true>(I, step, y0, y1, xa, strip, S, mine, step_size, rg, rg0)
+         : tv_walk<2, false>(I, step, y0, y1, xa, strip, S, mine, step_size, rg, rg0);
+  // after the last step the walk that finishes last ends the iteration (a
+  // single step leaves that to k_finish_iter)
+  if (last ? ng == 1 : !ticketed) return;
   unsigned ticket = 0;
   if (lane == 0) {
     __threadfence();
@@ -913,20 +953,13 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 8)
   ticket = __shfl_sync(0xffffffffu, ticket, 0);
   if (ticket != (unsigned)walks - 1) return;
   __threadfence();
-  const int P = S * NB;
-  double a = 0.0;
-  for (int p = lane; p < P; p += 32) a += ((volatile const double *)I.partials)[p];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  const double a = total(mine);
   if (lane == 0) {
     *I.counter = 0u;
-    Scalars *s = I.s;
-    if (last) {
-      finish_scalars(s, a);
-    } else {
-      s->tv_coef = s->alpha * s->d_tv / sqrt(a);
-      s->tv_coef_f = (float)s->tv_coef;
-    }
+    if (last)
+      finish_scalars(I.s, a);
+    else
+      I.s->tv_coef_f = tv_coef(*I.s, a);
   }
 }
 
@@ -1422,8 +1455,7 @@ __global__ void __launch_bounds__(kZThreads, kZMinBlocks)
     if (last) {
       finish_scalars(s, tot[0]);
     } else {
-      s->tv_coef = s->alpha * s->d_tv / sqrt(tot[0]);
-      s->tv_coef_f = (float)s->tv_coef;
+      s->tv_coef_f = tv_coef(*s, tot[0]);
     }
   }
 }
@@ -1461,6 +1493,32 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// Start state of every instance of a plan in one launch: the images from the
+// starting image, no residuals, the ticket and the scalars.  As copies, five
+// per instance, a plan of 64 instances of 512^2 took 1.19 ms to reset; the
+// image traffic of one launch takes 0.05.
+__global__ void __launch_bounds__(256)
+    k_reset(const Inst *__restrict__ insts, const Scalars *__restrict__ start) {
+  const Inst &I = insts[blockIdx.y];
+  const Dims D = I.d;
+  const long long n = (long long)D.nx * D.ny * D.nz, nr = (long long)D.na * D.nb;
+  const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+  const long long step = (long long)gridDim.x * 256;
+  // the buffers are 256-byte aligned
+  for (long long i = t; i < n / 4; i += step) {
+    const float4 v = ((const float4 *)I.m_k1)[i];
+    ((float4 *)I.m)[i] = v;
+    ((float4 *)I.m_pre)[i] = v;
+    ((float4 *)I.m_res)[i] = v;
+  }
+  for (long long i = n / 4 * 4 + t; i < n; i += step) I.m[i] = I.m_pre[i] = I.m_res[i] = I.m_k1[i];
+  for (long long r = t; r < nr; r += step) I.ddr[r] = 0.0;
+  if (t == 0) {
+    *I.counter = 0u;
+    *I.s = start[blockIdx.y];
+  }
+}
+
 // Done flags of n instances (the serving queue's poll after an iteration).
 __global__ void k_gather_done(const Inst *__restrict__ insts, int n, int *out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1468,6 +1526,15 @@ __global__ void k_gather_done(const Inst *__restrict__ insts, int n, int *out) {
 }
 
 }  // namespace
+
+cudaError_t launch_reset(const Inst *insts, const Scalars *start, int batch, const Dims &d,
+                         cudaStream_t st) {
+  const long long n = (long long)d.nx * d.ny * d.nz / 4 + 1;
+  const long long most = std::max<long long>(1, 152 * 16 / batch);
+  const dim3 grid((unsigned)std::min<long long>((n + 255) / 256, most), batch);
+  k_reset<<<grid, 256, 0, st>>>(insts, start);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_gather_done(const Inst *insts, int n, int *out,
                                cudaStream_t st) {
@@ -1534,11 +1601,11 @@ cudaError_t launch_tv_step(const Inst *insts, int batch, const Dims &d,
     return launch_iter(k_tv_walk3d, dim3((unsigned)walks, 1, batch), dim3(kZThreads), st,
                        insts, step, slabs, zmap);
   } else {
-    // bands per walk: the batch's walks within about one wave of 32
-    // resident warps per SM; one band (16 rows) per walk for small batches,
+    // bands per walk: the batch's walks within about one wave of
+    // resident warps; one band (16 rows) per walk for small batches,
     // which keeps a single instance's step spread over many warps
     const long long units = (long long)walk_strips(d.nx) * walk_bands(d.ny);
-    const long long cap = 152LL * 32;
+    const long long cap = 152LL * kWalkWarps * kWalkBlocks;
     const long long per = walk > 0 ? walk : (units * batch + cap - 1) / cap;
     const int bands = (int)(per < 1 ? 1 : (per > walk_bands(d.ny) ? walk_bands(d.ny) : per));
     const long long walks = (long long)walk_strips(d.nx) * ((walk_bands(d.ny) + bands - 1) / bands);
