@@ -43,20 +43,23 @@ int atx_blocks(const Dims &d) {
 // it.  (Two warps per ray: 14 % slower for a batch of 64 and 27 % for 256^3.)
 constexpr int kAxBlock = kAxWarps * 32;  // threads per block
 
-// This lane's partial sums of ray (ia, ib) over its columns (no cross-lane sum).
-template <class Loader>
-__device__ __forceinline__ void ax_lane_partial(const ViewGeo &G, const Dims &D,
-                                                int ia, int ib, Loader ld, float &ys,
-                                                float &ss) {
-  const int lane = threadIdx.x & 31;
+// Ray (ia, ib) of a view.
+__device__ __forceinline__ RayMarch ax_ray(const ViewGeo &G, const Dims &D, int ia, int ib,
+                                           bool &planar) {
   const float zd = G.z_det[ib];
-  const RayMarch R = ray_setup(G, D, G.y_det[ia], zd);
+  planar = D.nz == 1 && zd == 0.0f;
+  return ray_setup(G, D, G.y_det[ia], zd);
+}
+// This lane's partial sums of ray R over its columns (no cross-lane sum).
+template <class Loader>
+__device__ __forceinline__ void ax_lane_partial(const RayMarch &R, bool planar, Loader ld,
+                                                float &ys, float &ss) {
+  const int lane = threadIdx.x & 31;
   ys = 0.f;
   ss = 0.f;
-  // fan beams: the loads of two columns per round; cone beams: one (its
-  // three pieces per column already keep loads in flight; two measured 6 %
-  // slower at 256^3)
-  if (D.nz == 1 && zd == 0.0f)
+  // fan beams: the loads of two columns per round; single slices with detector
+  // rows: one (its three pieces per column already keep loads in flight)
+  if (planar)
     ray_columns_planar_fast<2>(R, lane, 32, ld, ys, ss);
   else
     ray_columns_fast<1>(R, lane, 32, ld, ys, ss);
@@ -129,7 +132,9 @@ __global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
   } else {
     const unsigned ru = (unsigned)w, na = (unsigned)D.na;  // rays < 2^31
     float ys, ss;
-    ax_lane_partial(G, D, (int)(ru % na), (int)(ru / na), ld, ys, ss);
+    bool planar;
+    const RayMarch R = ax_ray(G, D, (int)(ru % na), (int)(ru / na), planar);
+    ax_lane_partial(R, planar, ld, ys, ss);
     ys = warp_sum(ys);
     ss = warp_sum(ss);
     if (lane == 0) {
@@ -463,13 +468,16 @@ struct RayOut {
   double dd;  // Inst::ddr
 };
 // r: the ray's index ib * na + ia
+__device__ __forceinline__ float ray_value(const Inst &I, int view, long long r, long long nr) {
+  const long long pi = (long long)view * nr + r;
+  return ASD_IN(pi, nr * I.nv) ? sino_at(I, pi) : 0.f;
+}
+__device__ __forceinline__ double ray_squares(const Inst &I, long long r, long long nr) {
+  return ASD_IN(r, nr) ? I.ddr[r] : 0.0;
+}
 __device__ __forceinline__ RayOut ray_out_load(const Inst &I, int view, long long r,
                                                long long nr) {
-  const long long pi = (long long)view * nr + r;
-  RayOut o;
-  o.p = ASD_IN(pi, nr * I.nv) ? sino_at(I, pi) : 0.f;
-  o.dd = ASD_IN(r, nr) ? I.ddr[r] : 0.0;
-  return o;
+  return RayOut{ray_value(I, view, r, nr), ray_squares(I, r, nr)};
 }
 // q: where cor keeps the ray; bad: Scalars::cor_bad or GroupState::bad
 __device__ __forceinline__ void ray_out_store(const Inst &I, int *bad, int view, long long r,
@@ -497,33 +505,38 @@ __device__ __forceinline__ void ray_slopes(const Inst &I, const ViewGeo &G, cons
 template <bool k3D, bool kVol>
 __global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
     k_sart_ax(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap) {
-  pdl_enter();
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
-  if (view >= I.nv) return;
-  const bool done = ((volatile int *)&I.s->done)[0] != 0;
-  const bool tabc = k3D && (I.tabc_mode == kTabcShared || (!done && I.tabc_mode == kTabcOwn));
-  if (done && !tabc) return;
   const Dims D = I.d;
   const int lane = threadIdx.x & 31;
   const long long nr = nray(D), w = (long long)blockIdx.x * kAxWarps + (threadIdx.x >> 5);
-  if (w >= (kVol ? ax_warps3(D) : nr)) return;  // the whole warp
-  const ViewGeo G = view_of(I, view);
-  int ia, ib;  // the warp's first ray
-  if (kVol) {
-    ax_rows(D, w, ia, ib);
-  } else {
-    ia = (int)((unsigned)w % (unsigned)D.na);
-    ib = (int)((unsigned)w / (unsigned)D.na);
+  const bool have = view < I.nv && w < (kVol ? ax_warps3(D) : nr);  // the whole warp
+  ViewGeo G;
+  int ia = 0, ib = 0;  // the warp's first ray
+  RayMarch R;
+  bool planar = false, own = false;
+  long long r = 0;  // lane's own ray
+  float p = 0.f;
+  if (have) {  // geometry and sinogram, before the wait
+    G = view_of(I, view);
+    if (kVol) {
+      ax_rows(D, w, ia, ib);
+    } else {
+      ia = (int)((unsigned)w % (unsigned)D.na);
+      ib = (int)((unsigned)w / (unsigned)D.na);
+      R = ax_ray(G, D, ia, ib, planar);
+    }
+    own = lane < (kVol ? kAxRows : 1) && ib + lane < D.nb;
+    r = (long long)(ib + lane) * D.na + ia;
+    if (own) p = ray_value(I, view, r, nr);
   }
-  // lane's own ray
-  const int mine = ib + lane;
-  const bool own = lane < (kVol ? kAxRows : 1) && mine < D.nb;
-  const long long r = (long long)mine * D.na + ia;
-  const long long q = k3D && I.rays_t ? (long long)ia * D.nb + mine : r;
-  if (tabc && own) ray_slopes(I, G, D, view, ia, mine, q);
+  pdl_enter();
+  if (!have) return;
+  const bool done = ((volatile int *)&I.s->done)[0] != 0;
+  const bool tabc = k3D && (I.tabc_mode == kTabcShared || (!done && I.tabc_mode == kTabcOwn));
+  const long long q = k3D && I.rays_t ? (long long)ia * D.nb + ib + lane : r;
+  if (tabc && own) ray_slopes(I, G, D, view, ia, ib + lane, q);
   if (done) return;
-  RayOut o{0.f, 0.0};
-  if (own) o = ray_out_load(I, view, r, nr);
+  const double dd = own ? ray_squares(I, r, nr) : 0.0;
   const float *m = I.m;
   auto ld = [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; };
   float yv, sv;
@@ -538,11 +551,12 @@ __global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
       sv = lane == k ? ss[k] : sv;
     }
   } else {
-    ax_lane_partial(G, D, ia, ib, ld, yv, sv);
+    ax_lane_partial(R, planar, ld, yv, sv);
     yv = warp_sum(yv);
     sv = warp_sum(sv);
   }
-  if (own) ray_out_store(I, &I.s->cor_bad, view, r, q, nr, o, yv * G.scale, sv * G.scale);
+  if (own)
+    ray_out_store(I, &I.s->cor_bad, view, r, q, nr, RayOut{p, dd}, yv * G.scale, sv * G.scale);
 }
 
 // k_sart_ax with the exact projection (siddon_warp_rays): a warp per 32 rays,
@@ -663,28 +677,54 @@ __device__ __forceinline__ float chord_slot(const int *__restrict__ tab, size_t 
 }
 
 // Backward step over this block's `tiles` tiles from the view's chord table
-// (2-D, narrow form; see sart_atx_tiles): the image value, header and first
-// kChordPre chords of a voxel are loaded together, then its residuals (L1) in
-// the pairs' order.  Pairs past a voxel's own add 0 times a residual, which is
-// finite here.
+// (2-D, narrow form; see sart_atx_tiles).  The table entries of a voxel of
+// every tile are loaded before the wait for the forward step, the images
+// together after it, then the residuals (L1) in the pairs' order: a block
+// waits for memory once and not once a tile.  Pairs past a voxel's own add 0
+// times a residual, which is finite here.
+struct TabTiles {
+  ChordPre c[kTilesPerBlock];
+};
+__device__ __forceinline__ bool tab_voxel(const Dims &D, int tiles, int t, unsigned &vi) {
+  const int ix = blockIdx.x * kTileX + threadIdx.x % kTileX;
+  const int iy = (blockIdx.y * tiles + t) * kTileY + threadIdx.x / kTileX;
+  const bool in = t < tiles && ix < D.nx && iy < D.ny;
+  vi = in ? (unsigned)iy * D.nx + ix : 0u;
+  return in;
+}
+__device__ __forceinline__ void tab_load(const Dims &D, const int *__restrict__ tab, int K,
+                                         int tiles, TabTiles &T) {
+#pragma unroll
+  for (int t = 0; t < kTilesPerBlock; t++) {
+    if (t >= tiles) break;
+    unsigned vi;
+    tab_voxel(D, tiles, t, vi);
+    T.c[t] = chord_load(tab, (size_t)D.nx * D.ny, K, vi);
+  }
+}
 __device__ __forceinline__ void sart_atx_tiles_tab(const Inst &I, const Dims &D,
                                                    const int *__restrict__ tab, int K,
-                                                   int tiles) {
+                                                   int tiles, const TabTiles &T) {
   const float beta = I.s->beta_f;
   float *m = I.m;
   const float *__restrict__ cor = I.cor;
   const size_t N = (size_t)D.nx * D.ny;
   const long long M = nray(D);
-  for (int t = 0; t < tiles; t++) {
-    int x0, y0, iz;
-    if (!group_tile(D.ny, D.nz, t, x0, y0, iz, tiles)) break;
-    const int ix = x0 + threadIdx.x % kTileX, iy = y0 + threadIdx.x / kTileX;
-    const bool valid = ix < D.nx && iy < D.ny;
-    const unsigned vi = valid ? (unsigned)iy * D.nx + ix : 0u;
-    if (!ASD_IN(vi, N)) continue;
-    const ChordPre c = chord_load(tab, N, K, vi);
-    const float mv = m[vi];
-    const int kA = __reduce_max_sync(0xffffffffu, valid ? c.cnt : 0);
+  float mv[kTilesPerBlock];
+#pragma unroll
+  for (int t = 0; t < kTilesPerBlock; t++) {
+    if (t >= tiles) break;
+    unsigned vi;
+    tab_voxel(D, tiles, t, vi);
+    mv[t] = ASD_IN(vi, N) ? m[vi] : 0.f;
+  }
+#pragma unroll
+  for (int t = 0; t < kTilesPerBlock; t++) {
+    if (t >= tiles) break;
+    unsigned vi;
+    const bool in = tab_voxel(D, tiles, t, vi);
+    const ChordPre &c = T.c[t];
+    const int kA = __reduce_max_sync(0xffffffffu, in ? c.cnt : 0);
     float acc = 0.f;
 #pragma unroll
     for (int ka = 0; ka < kChordPre; ka++) {
@@ -695,7 +735,7 @@ __device__ __forceinline__ void sart_atx_tiles_tab(const Inst &I, const Dims &D,
     for (int ka = kChordPre; ka < kA; ka++)
       if (ka < c.cnt && ASD_IN(ka, K) && ASD_IN(c.first + ka, M))
         pair2(acc, chord_slot(tab, N, vi, ka), __ldg(cor + c.first + ka));
-    if (valid) m[vi] = sart_update(mv, beta, acc, c.norm);
+    if (in && ASD_IN(vi, N)) m[vi] = sart_update(mv[t], beta, acc, c.norm);
   }
 }
 
@@ -810,22 +850,35 @@ __device__ __forceinline__ void sart_atx_tiles(const Inst &I, const ViewGeo &G,
 // ray (the instance's view flags; a block-uniform branch) uses the
 // axis-specialised chord.
 template <bool kPlanar>
-__global__ void __launch_bounds__(kAtxThreads, 4)
+__global__ void __launch_bounds__(kAtxThreads, kPlanar ? 3 : 4)
     k_sart_atx(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap,
                int tiles) {
-  pdl_enter();
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
-  if (view >= I.nv || ((volatile int *)&I.s->done)[0]) return;
   const Dims D = I.d;
-  if (own_block(group_grid(D.nx, D.ny, D.nz, 1, tiles)).bid < 0) return;
+  const bool have =
+      view < I.nv && own_block(group_grid(D.nx, D.ny, D.nz, 1, tiles)).bid >= 0;
+  const int *tab = nullptr;
+  TabTiles T;
+  int vf = 0;
+  if (have) {  // the plan's tables, before the wait
+    vf = I.vflags[view];
+    if (kPlanar && I.chtab && !(vf & kViewAxisParallel) && I.g.z_det[0] == 0.0f) {
+      tab = I.chtab + (size_t)view * chord_view_words(D, I.chK);
+      tab_load(D, tab, I.chK, tiles, T);
+    }
+  }
+  pdl_enter();
+  if (!have || ((volatile int *)&I.s->done)[0]) return;
+  const bool finite = I.s->cor_bad != view + 1;
+  if (tab && finite) {
+    sart_atx_tiles_tab(I, D, tab, I.chK, tiles, T);
+    return;
+  }
   const ViewGeo G = view_of(I, view);
   const float4 *tabA = I.tabA + (long long)view * D.na;
-  const int vf = I.vflags[view];
-  const bool narrow = !(vf & kViewAxisParallel) && I.s->cor_bad != view + 1 &&
-                      (!kPlanar || G.z_det[0] == 0.0f);
-  if (kPlanar && narrow && I.chtab)
-    sart_atx_tiles_tab(I, D, I.chtab + (size_t)view * chord_view_words(D, I.chK), I.chK, tiles);
-  else if (!(vf & (kViewAxisParallel | kViewNotX)))
+  const bool narrow =
+      !(vf & kViewAxisParallel) && finite && (!kPlanar || G.z_det[0] == 0.0f);
+  if (!(vf & (kViewAxisParallel | kViewNotX)))
     sart_atx_tiles<kPlanar, 1>(I, G, D, tabA, narrow, tiles);
   else if (!(vf & (kViewAxisParallel | kViewNotY)))
     sart_atx_tiles<kPlanar, 2>(I, G, D, tabA, narrow, tiles);
@@ -1874,10 +1927,9 @@ cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
                             const int *zmap) {
   cudaError_t e;
   // fan beams: the fewest tiles a block (1, 2 or 4) that keep the launch within
-  // two blocks per SM, so that the blocks of the next, programmatic launch
-  // still find room (512^2, ten iterations: 10.7 ms with 256 blocks of four
-  // tiles, 11.2 with 512 of two, 11.5 with 1024 of one; 64^2 by itself is
-  // faster spread out)
+  // two blocks per SM, so that they sit, their tables loaded, beside the forward
+  // step's (512^2, ten iterations: 8.10 ms with 256 blocks of four tiles, 8.55
+  // with 512 of two; 10.4 without the loads before the wait)
   int tiles = d.nz == 1 ? 1 : kTilesPerBlock;
   dim3 grid = group_grid(d.nx, d.ny, d.nz, batch, tiles);
   while (tiles < kTilesPerBlock && (long long)grid.x * grid.y * batch > 152 * 2) {
