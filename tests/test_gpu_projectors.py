@@ -290,3 +290,57 @@ def test_exact_forward_mode_against_fp64_siddon(gpu, oracle_mod, case):
         worst_march = max(worst_march, rel_l2(ym, ye))
     if nz > 8:
         assert worst_march > 1e-4  # the reference march's documented 3-D deviation
+
+
+@pytest.mark.parametrize("dims", [(512, 512, 1, 888, 1), (65, 31, 1, 97, 1), (40, 24, 1, 57, 3),
+                                  (9, 7, 5, 19, 11)])
+def test_chained_device_projections_wait_for_each_other(gpu, oracle_mod, dims):
+    """Ax then Atx then Ax ..., each on the previous one's output and on
+    detector coordinates that a copy just before it wrote, without a
+    synchronisation in between (each kernel starts while the one before it
+    drains), captured in a graph as well: the same bits as with one."""
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    nx, ny, nz, na, nb = dims
+    L, N, M = load(), nx * ny * nz, na * nb
+    geo = [oracle_mod.gateway_geometry(-a / 180 * np.pi, 541.0, 408.0, 541.0 / 949.0 * na / nx,
+                                       1.0, na, nb) for a in (0.0, 31.0, 90.0, 211.0)]
+    yd = [torch.from_numpy(np.ascontiguousarray(g["y_det"], np.float32)).cuda() for g in geo]
+    zd = [torch.from_numpy(np.ascontiguousarray(g["z_det"], np.float32)).cuda() for g in geo]
+    x0 = torch.from_numpy(np.random.default_rng(3).random(N).astype(np.float32)).cuda()
+    x, sc = torch.empty(N, device="cuda"), torch.empty(N, device="cuda")
+    y, sr = torch.empty(M, device="cuda"), torch.empty(M, device="cuda")
+    py, pz = torch.empty(na, device="cuda"), torch.empty(nb, device="cuda")
+
+    def chain(sync):
+        st = torch.cuda.current_stream().cuda_stream
+        x.copy_(x0)
+        for _ in range(3):
+            for g, a, b in zip(geo, yd, zd):
+                view = (g["cos_phi"], g["sin_phi"], py.data_ptr(), pz.data_ptr(), g["SO"],
+                        g["OD"], g["scale"])
+                py.fill_(float("nan"))
+                torch.add(a, 0.0, out=py)
+                torch.add(b, 0.0, out=pz)
+                check(L.asdpocs_ax_device(x.data_ptr(), y.data_ptr(), sr.data_ptr(), *view,
+                                          1.0, *dims, st))
+                if sync:
+                    torch.cuda.synchronize()
+                check(L.asdpocs_atx_device(x.data_ptr(), y.data_ptr(), sc.data_ptr(), *view,
+                                           g["det"], g["det"], 1.0, *dims, st))
+                if sync:
+                    torch.cuda.synchronize()
+                x.div_(x.abs().max())
+        return x.clone()
+
+    want = chain(True)
+    assert torch.isfinite(want).all() and want.abs().max() == 1
+    assert torch.equal(chain(False), want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = chain(False)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
