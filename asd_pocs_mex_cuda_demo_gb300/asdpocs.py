@@ -287,7 +287,7 @@ class Plan:
 
     def autotune_shapes(self, reps: int = 10) -> dict:
         """Times every launch shape that applies to the plan (TV walk, the
-        shared forward step's loads per round and quads per block, the
+        shared forward step's loads per round and quads per lane, the
         cone-beam backward step's column segment, programmatic launches) on
         its own data and keeps the fastest; no shape changes a result bit.
         Resets the plan.  Returns the chosen shapes and the iteration's

@@ -651,6 +651,11 @@ struct SubBatch {
   // position in d_inst, count) with their device list gall
   bool shared = false;
   std::vector<int2> groups_host;
+  int fewest() const {  // instances of the smallest group
+    int n = kShareSlots;
+    for (const int2 &g : groups_host) n = std::min(n, g.y);
+    return n;
+  }
   const int2 *gall = nullptr;
   std::vector<int2> gtab_host;  // mixed plans: the view sets' group lists
   Dims d{};                  // largest sizes of these instances
@@ -916,7 +921,7 @@ cudaError_t enqueue_iteration(const Inst *d_inst, int batch, const Dims &d,
                               int nv, int ng, bool shared, cudaStream_t st,
                               const IterShape &sh, bool finish,
                               const std::vector<ViewSet> *sets, const int *zall,
-                              const int2 *gall, int ngroups) {
+                              const int2 *gall, int ngroups, int fewest) {
   const PdlScope scope(sh.pdl);
   cudaError_t e = cudaSuccess;
   if (shared) e = launch_group_pack(d_inst, batch, d, 0, st, gall, ngroups);
@@ -938,7 +943,7 @@ cudaError_t enqueue_iteration(const Inst *d_inst, int batch, const Dims &d,
     }
     if (shared) {
       e = launch_sart_ax_shared(d_inst, batch, vd, v, st, sh.ax_u, sh.ax_q, gtab, vg);
-      if (e == cudaSuccess) e = launch_sart_atx_shared(d_inst, batch, vd, v, st, gtab, vg);
+      if (e == cudaSuccess) e = launch_sart_atx_shared(d_inst, batch, vd, v, st, gtab, vg, fewest);
       continue;
     }
     e = launch_sart_ax(d_inst, vb, vd, v, st, sh.exact, zmap);
@@ -971,7 +976,7 @@ static int plan_enqueue_sub(asdpocs_plan p, const SubBatch &s) {
   ASD_CUDA(enqueue_iteration(listed ? p->d_inst : p->d_inst + s.first,
                              listed ? (int)s.members.size() : s.count, s.d, s.nv, s.max_ng,
                              s.shared, s.st, plan_shape(p), s.min_ng < 2, &s.sets, s.zall,
-                             s.gall, (int)s.groups_host.size()));
+                             s.gall, (int)s.groups_host.size(), s.fewest()));
   return 0;
 }
 
@@ -1886,7 +1891,7 @@ int asdpocs_plan_time_phase(asdpocs_plan p, int phase, int reps,
       for (const SubBatch &s : p->subs)
         if (e == cudaSuccess)
           e = launch_sart_atx_shared(p->d_inst, 0, s.d, v, p->st, s.gall,
-                                     (int)s.groups_host.size());
+                                     (int)s.groups_host.size(), s.fewest());
       return e;
     }
     return p->shared ? launch_sart_atx_shared(p->d_inst, p->batch, p->d, v, p->st)

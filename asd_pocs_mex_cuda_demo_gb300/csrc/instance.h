@@ -87,7 +87,7 @@ struct IterShape {
   bool zcol = true;         // cone beams: z-column backward step (else per voxel)
   int zseg = 0;             //   its segment length in voxels (0: the default)
   int ax_u = 0, ax_q = 0;   // shared forward step: columns of loads per round,
-                            //   quads of instances per block (0: the defaults)
+                            //   quads of instances per lane (0: the defaults)
   bool pdl = false;         // programmatic dependent launches (work alone on
                             //   its stream)
   bool exact = false;       // forward steps: exact projection (launch_sart_ax)
@@ -110,13 +110,13 @@ struct ViewSet {
 // [0, nv) (null or empty: every instance of zall in every view, at sizes d).
 // `gall` (shared only; device, `ngroups` entries; null: groups of
 // kShareSlots consecutive instances): the groups of instances sharing
-// geometry, as (first instance, count).
+// geometry, as (first instance, count), `fewest` the least of these counts.
 cudaError_t enqueue_iteration(const Inst *d_inst, int batch, const Dims &d,
                               int nv, int ng, bool shared, cudaStream_t st,
                               const IterShape &shape = IterShape(), bool finish = true,
                               const std::vector<ViewSet> *sets = nullptr,
                               const int *zall = nullptr, const int2 *gall = nullptr,
-                              int ngroups = 0);
+                              int ngroups = 0, int fewest = kShareSlots);
 
 // Backward-step chord tables (Inst::chtab) of instances sharing 2-D geometry
 // and view angles, from d_inst[0], whose view tables are built: a counting

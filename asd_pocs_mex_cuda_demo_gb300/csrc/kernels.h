@@ -117,15 +117,17 @@ cudaError_t launch_gather_done(const Inst *insts, int n, int *out,
 // `gtab` (device, `ngroups` entries; null: groups of kShareSlots
 // consecutive instances): the launch's groups as (first instance, count),
 // each group's instances sharing geometry and view angles; groups of
-// different sizes may share a launch, `d` holding the largest sizes.
+// different sizes may share a launch, `d` holding the largest sizes and
+// `fewest` the least count of a group (or less).
 cudaError_t launch_sart_atx_shared(const Inst *insts, int batch,
                                    const Dims &d, int view, cudaStream_t st,
-                                   const int2 *gtab = nullptr, int ngroups = 0);
+                                   const int2 *gtab = nullptr, int ngroups = 0,
+                                   int fewest = kShareSlots);
 
 // Forward step for a batch whose instances share geometry and view angles:
 // the column march evaluated once per ray for groups of instances whose
 // images are interleaved (Inst::m_il) during the sweep.
-// `u` columns of loads per round and `q` quads of instances per block (1 or
+// `u` columns of loads per round and `q` quads of instances per lane (1 or
 // 2 each; 0: the defaults, 2 x 1 for fan beams, 1 x 2 for cone beams) are
 // launch shapes that do not change results.
 // `gtab`, `ngroups` as for launch_sart_atx_shared.

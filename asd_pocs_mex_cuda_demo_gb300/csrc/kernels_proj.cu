@@ -1555,7 +1555,15 @@ __global__ void __launch_bounds__(kAtxThreads)
 // barriers, one load per chord and a division per instance; 42.7 us now at 4
 // blocks per SM, 41.3 at 5, 42.5 at 6; with the direct form out of line 43.8
 // (5 blocks) to 54.8 (8 blocks).
-template <bool kPlanar>
+// kPairs: a thread still loads its own voxel's table entries, but the image
+// and the residuals are read with two lanes to a voxel, a quad of instances
+// each, in two turns (the entries through shuffles): a load then takes whole
+// 32-byte sectors, 16 of them in 512 contiguous bytes, where a lane that reads
+// its two quads one after the other touches each sector twice.  34.8 us (4
+// blocks 36.3, 3 42.8, 6 with the spills 41.0).  Groups of at most four
+// instances, whose second quad is empty, keep the lane per voxel: 24 instances
+// in groups of four 4.6 ms a run, 5.0 in pairs.
+template <bool kPlanar, bool kPairs>
 __global__ void __launch_bounds__(kAtxThreads, 5)
     k_sart_atx_shared(const Inst *__restrict__ insts, int batch, int view,
                       const int2 *__restrict__ gtab) {
@@ -1576,41 +1584,109 @@ __global__ void __launch_bounds__(kAtxThreads, 5)
     const int K = I0.chK;
     const int *__restrict__ tab = I0.chtab + (size_t)view * chord_view_words(D, K);
     const unsigned vi = valid ? (unsigned)iy * D.nx + ix : 0u;
-    float4 *mg = (float4 *)I0.m_il + (size_t)vi * (kShareGroup / 4);
     const ChordPre c = chord_load(tab, N, K, vi);
-    float4 m4[kShareGroup / 4];
+    const bool use = !(vf & kViewAxisParallel) && I0.g.z_det[0] == 0.0f;
+    if constexpr (kPairs) {
+      // lane 2 j + q: quad q of voxel 16 h + j of the warp's row in turn h
+      static_assert(kShareGroup == 8, "two quads");
+      const int lane = threadIdx.x & 31, q = lane & 1;
+      float4 *const mq = (float4 *)I0.m_il + q;
+      const unsigned mine_vi = valid ? vi : 0xffffffffu;
+      unsigned vh[2];
+      float4 m4[2];
 #pragma unroll
-    for (int q = 0; q < kShareGroup / 4; q++) m4[q] = mg[q];
-    const unsigned active = gs.active;
-    if (!active) return;
-    if (!(vf & kViewAxisParallel) && gs.bad != view + 1 && I0.g.z_det[0] == 0.0f) {
-      const int kA = __reduce_max_sync(0xffffffffu, valid ? c.cnt : 0);
-      const long long M = nray(D);
-      float acc[kShareGroup];
-#pragma unroll
-      for (int b = 0; b < kShareGroup; b++) acc[b] = 0.f;
-      auto pair = [&](int r, float l) {
-        if (!ASD_IN(r, M)) return;
-        const float4 *p = corg + (size_t)r * (kShareGroup / 4);
-#pragma unroll
-        for (int q = 0; q < kShareGroup / 4; q++) {
-          if (!((active >> (4 * q)) & 0xFu)) continue;
-          const float4 c4 = __ldg(p + q);
-          pair2(acc[4 * q], l, c4.x);
-          pair2(acc[4 * q + 1], l, c4.y);
-          pair2(acc[4 * q + 2], l, c4.z);
-          pair2(acc[4 * q + 3], l, c4.w);
-        }
-      };
-#pragma unroll
-      for (int ka = 0; ka < kChordPre; ka++) {
-        if (ka >= kA) break;
-        pair(c.first + (ka < c.cnt ? ka : 0), c.l[ka]);
+      for (int h = 0; h < 2; h++) {
+        vh[h] = __shfl_sync(0xffffffffu, mine_vi, 16 * h + (lane >> 1));
+        m4[h] = vh[h] < N ? mq[(size_t)vh[h] * 2] : make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      for (int ka = kChordPre; ka < kA; ka++)
-        if (ka < c.cnt && ASD_IN(ka, K)) pair(c.first + ka, chord_slot(tab, N, vi, ka));
-      if (valid && ASD_IN(vi, N)) atx_shared_apply(c.norm, acc, gs, active, m4, mg);
-      return;
+      const unsigned active = gs.active;
+      if (!active) return;
+      if (use && gs.bad != view + 1) {
+        const unsigned mine = (active >> (4 * q)) & 0xFu;  // the quad's running instances
+        const int kA = __reduce_max_sync(0xffffffffu, valid ? c.cnt : 0);
+        const long long M = nray(D);
+        const float4 *const cq = corg + q;
+        const int head = c.cnt << 24 | c.first;
+        int hd[2];
+        float acc[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          hd[h] = __shfl_sync(0xffffffffu, head, 16 * h + (lane >> 1));
+#pragma unroll
+          for (int b = 0; b < 4; b++) acc[h][b] = 0.f;
+        }
+        auto pair = [&](float (&a)[4], int r, float l) {
+          if (!mine || !ASD_IN(r, M)) return;
+          const float4 c4 = __ldg(cq + (size_t)r * 2);
+          pair2(a[0], l, c4.x);
+          pair2(a[1], l, c4.y);
+          pair2(a[2], l, c4.z);
+          pair2(a[3], l, c4.w);
+        };
+#pragma unroll
+        for (int ka = 0; ka < kChordPre; ka++) {
+          if (ka >= kA) break;
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const float l = __shfl_sync(0xffffffffu, c.l[ka], 16 * h + (lane >> 1));
+            pair(acc[h], (hd[h] & 0xffffff) + (ka < (int)((unsigned)hd[h] >> 24) ? ka : 0), l);
+          }
+        }
+        for (int ka = kChordPre; ka < kA; ka++)
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+            if (ka < (int)((unsigned)hd[h] >> 24) && ASD_IN(ka, K) && vh[h] < N)
+              pair(acc[h], (hd[h] & 0xffffff) + ka, chord_slot(tab, N, vh[h], ka));
+        const float4 b4 = __ldg((const float4 *)gs.beta + q);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const float norm = __shfl_sync(0xffffffffu, c.norm, 16 * h + (lane >> 1));
+          if (vh[h] >= N || !mine) continue;
+          float4 v = m4[h];
+          if (mine & 1u) v.x = sart_update(v.x, b4.x, acc[h][0], norm);
+          if (mine & 2u) v.y = sart_update(v.y, b4.y, acc[h][1], norm);
+          if (mine & 4u) v.z = sart_update(v.z, b4.z, acc[h][2], norm);
+          if (mine & 8u) v.w = sart_update(v.w, b4.w, acc[h][3], norm);
+          mq[(size_t)vh[h] * 2] = v;
+        }
+        return;
+      }
+    } else {
+      float4 *mg = (float4 *)I0.m_il + (size_t)vi * (kShareGroup / 4);
+      float4 m4[kShareGroup / 4];
+#pragma unroll
+      for (int q = 0; q < kShareGroup / 4; q++) m4[q] = mg[q];
+      const unsigned active = gs.active;
+      if (!active) return;
+      if (use && gs.bad != view + 1) {
+        const int kA = __reduce_max_sync(0xffffffffu, valid ? c.cnt : 0);
+        const long long M = nray(D);
+        float acc[kShareGroup];
+#pragma unroll
+        for (int b = 0; b < kShareGroup; b++) acc[b] = 0.f;
+        auto pair = [&](int r, float l) {
+          if (!ASD_IN(r, M)) return;
+          const float4 *p = corg + (size_t)r * (kShareGroup / 4);
+#pragma unroll
+          for (int q = 0; q < kShareGroup / 4; q++) {
+            if (!((active >> (4 * q)) & 0xFu)) continue;
+            const float4 c4 = __ldg(p + q);
+            pair2(acc[4 * q], l, c4.x);
+            pair2(acc[4 * q + 1], l, c4.y);
+            pair2(acc[4 * q + 2], l, c4.z);
+            pair2(acc[4 * q + 3], l, c4.w);
+          }
+        };
+#pragma unroll
+        for (int ka = 0; ka < kChordPre; ka++) {
+          if (ka >= kA) break;
+          pair(c.first + (ka < c.cnt ? ka : 0), c.l[ka]);
+        }
+        for (int ka = kChordPre; ka < kA; ka++)
+          if (ka < c.cnt && ASD_IN(ka, K)) pair(c.first + ka, chord_slot(tab, N, vi, ka));
+        if (valid && ASD_IN(vi, N)) atx_shared_apply(c.norm, acc, gs, active, m4, mg);
+        return;
+      }
     }
   }
   const unsigned active = gs.active;
@@ -1638,19 +1714,23 @@ __global__ void __launch_bounds__(kAtxThreads, 5)
 // flags are bit-identical to it.
 // ---------------------------------------------------------------------------
 // columns per round of loads in the shared forward step: two for fan beams
-// (measured 6 % faster than one); one for cone beams, whose three pieces per
+// (26.9 us a launch of 64, one 26.3); one for cone beams, whose three pieces per
 // column already keep six loads in flight.  Blocks per SM: 6 for fan beams
 // (72 registers, no spills), 8 for cone beams (64 registers: 10 % faster
 // than 6 at 128^3).
 template <bool k3D>
 constexpr int kAxShareU = k3D ? 1 : 2;
-// quads of a group (4 instances each) per block: one for fan beams (twice
-// the warps, half the accumulators: measured 10 % faster), both for cone
-// beams
+// quads of a group (4 instances each) per lane: one for fan beams, both for
+// cone beams.  One: two lanes to a voxel, so that a load takes whole 32-byte
+// sectors, and two warps to a ray, 16 of its columns each, so that the columns
+// are still dealt to 32 lanes and added in the same order.  A launch of 64
+// instances, 512^2 and 888 bins, waits for memory (37 % issue): 32.8 us with
+// the two quads in blocks of their own, each taking half of every sector, 26.9
+// now; both quads in a lane 29.0.
 template <bool k3D>
 constexpr int kAxShareQ = k3D ? kShareGroup / 4 : 1;
 
-// kU columns per round and kQ quads per block are launch shapes that a plan's
+// kU columns per round and kQ quads per lane are launch shapes that a plan's
 // autotuner may change (asdpocs_plan_autotune_shapes): neither changes the
 // order in which an instance's pieces are added, so every shape gives the
 // same bits.
@@ -1658,42 +1738,44 @@ template <bool k3D, int kU, int kQ>
 __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
     k_sart_ax_shared(const Inst *__restrict__ insts, int batch, int view,
                      const int2 *__restrict__ gtab) {
-  constexpr int kQuads = kShareGroup / 4;
+  constexpr int kQuads = kShareGroup / 4, kS = 4 * kQ;
+  // kW lanes of a voxel (kQ quads each) and, so that a ray's columns are
+  // still dealt to 32 lanes, kW warps of a ray
+  constexpr int kW = kQuads / kQ, kRays = kAxWarps / kW;
+  __shared__ float s_part[kW > 1 ? kRays : 1][kW][kS + 1][32];
   pdl_enter();
-  // this block: kQ of the group's quads (4 instances each), from q0
-  constexpr int kS = 4 * kQ;
-  const int q0 = (int)(blockIdx.z % (kQuads / kQ)) * kQ;
-  const int gz = (int)(blockIdx.z / (kQuads / kQ));                  // the group
+  const int gz = (int)blockIdx.z;                                    // the group
   const int g0 = gtab ? gtab[gz].x : gz * kShareGroup;
-  const int gi = g0 + 4 * q0;                                        // first instance
-  const int gn = min(kS, (gtab ? g0 + gtab[gz].y : batch) - gi);
-  if (gn <= 0) return;
+  const int gn = gtab ? gtab[gz].y : min(kShareGroup, batch - g0);
   const Inst &I0 = insts[g0];
   if (view >= I0.nv) return;
   const Dims D = I0.d;
-  const long long nr = nray(D), r0 = (long long)blockIdx.x * kAxWarps;
+  const long long nr = nray(D), r0 = (long long)blockIdx.x * kRays;
   const int lane = threadIdx.x & 31;
-  const long long r = r0 + (threadIdx.x >> 5);
+  const int rl = (threadIdx.x >> 5) / kW, wr = (threadIdx.x >> 5) % kW;
+  const long long r = r0 + rl;
+  const int q0 = lane % kW;                     // this lane's quads: q0, q0 + kW, ...
+  const int col = wr * (32 / kW) + lane / kW;   // its columns: col, col + 32, ...
   const ViewGeo G = view_of(I0, view);
   // cone beam: the plan's one ray-slope table, refreshed by group 0 every
   // view whether or not its instances still run
-  if (k3D && blockIdx.z == 0 && threadIdx.x < kAxWarps && r0 + threadIdx.x < nr) {
+  if (k3D && blockIdx.z == 0 && threadIdx.x < kRays && r0 + threadIdx.x < nr) {
     const long long rs = r0 + threadIdx.x;
     ray_slopes(I0, G, D, view, (int)(rs % D.na), (int)(rs / D.na), rs);
   }
-  if (r >= nr) return;  // the whole warp
-  const unsigned active = (I0.grp->active >> (4 * q0)) & ((1u << kS) - 1u);
+  const unsigned active = I0.grp->active;
   if (!active) return;
-  // lane b: instance gi + b
-  const Inst &Ib = insts[gi + min(lane, gn - 1)];
-  const bool live = lane < gn && ((active >> lane) & 1u);
+  // lane kW * j + q0 of a ray's first warp: its j-th sum's instance
+  const int slot = 4 * (q0 + kW * ((lane / kW) / 4)) + (lane / kW) % 4;
+  const Inst &Ib = insts[g0 + min(slot, gn - 1)];
+  const bool live = wr == 0 && r < nr && lane < kShareGroup && slot < gn && ((active >> slot) & 1u);
   RayOut o{0.f, 0.0};
   if (live) o = ray_out_load(Ib, view, r, nr);
   float v[kS + 1];  // the instances' sums, then the weights' sum
 #pragma unroll
   for (int b = 0; b <= kS; b++) v[b] = 0.f;
   const float4 *__restrict__ mg = (const float4 *)I0.m_il;
-  {
+  if (r < nr) {  // the whole warp
     const int ia = (int)(r % D.na), ib = (int)(r / D.na);
     const float zd = G.z_det[ib];
     const RayMarch R = ray_setup(G, D, G.y_det[ia], zd);
@@ -1702,7 +1784,7 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
     // (predicated) loads, then the accumulation in column and piece order
     auto march = [&](auto pieces) {
       constexpr int kP = decltype(pieces)::value;
-      for (int iu0 = lane; iu0 - lane < R.nu; iu0 += 32 * kU) {
+      for (int iu0 = col; iu0 - col < R.nu; iu0 += 32 * kU) {
         unsigned id[kU][kP];
         float w[kU][kP];
         bool f[kU][kP];
@@ -1734,8 +1816,8 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
             f[u][j] = f[u][j] && ASD_IN(id[u][j], nvox(D));
 #pragma unroll
             for (int q = 0; q < kQ; q++)
-              x[u][j][q] = (f[u][j] && ((active >> (4 * q)) & 0xFu))
-                               ? __ldg(p + q)
+              x[u][j][q] = (f[u][j] && ((active >> (4 * (q0 + kW * q))) & 0xFu))
+                               ? __ldg(p + kW * q)
                                : make_float4(0.f, 0.f, 0.f, 0.f);
           }
 #pragma unroll
@@ -1760,12 +1842,25 @@ __global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
     else if constexpr (k3D)
       march(std::integral_constant<int, 3>());
   }
+  // the butterfly of warp_sum over the 32 columns: the steps between a ray's
+  // warps through shared memory, the others between lanes
+  if constexpr (kW > 1) {
+    static_assert(kW == 2, "one step between warps");
 #pragma unroll
-  for (int b = 0; b <= kS; b++) v[b] = warp_sum(v[b]);
+    for (int b = 0; b <= kS; b++) s_part[rl][wr][b][lane] = v[b];
+    __syncthreads();
+    if (wr) return;
+#pragma unroll
+    for (int b = 0; b <= kS; b++) v[b] += s_part[rl][1][b][lane];
+  }
+#pragma unroll
+  for (int b = 0; b <= kS; b++)
+#pragma unroll
+    for (int o = 16; o >= kW; o >>= 1) v[b] += __shfl_xor_sync(0xffffffffu, v[b], o);
   float yb = 0.f;
 #pragma unroll
   for (int b = 0; b < kS; b++)
-    if (lane == b) yb = v[b];
+    if (lane / kW == b) yb = v[b];
   if (live) ray_out_store(Ib, &I0.grp->bad, view, r, r, nr, o, yb * G.scale, v[kS] * G.scale);
 }
 
@@ -1968,55 +2063,59 @@ cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
 
 cudaError_t launch_sart_atx_shared(const Inst *insts, int batch,
                                    const Dims &d, int view, cudaStream_t st,
-                                   const int2 *gtab, int ngroups) {
+                                   const int2 *gtab, int ngroups, int fewest) {
   cudaError_t e;
+  if (!gtab) fewest = min(batch, kShareGroup);
   dim3 grid = tile_grid(d.nx, d.ny, d.nz, 1);
   grid.z = gtab ? ngroups : (batch + kShareGroup - 1) / kShareGroup;
   if (d.nz > 1 || d.nb > 1)
-    e = launch_iter(k_sart_atx_shared<false>, grid, dim3(kAtxThreads), st, insts, batch,
+    e = launch_iter(k_sart_atx_shared<false, false>, grid, dim3(kAtxThreads), st, insts, batch,
+                    view, gtab);
+  else if (fewest > 4)
+    e = launch_iter(k_sart_atx_shared<true, true>, grid, dim3(kAtxThreads), st, insts, batch,
                     view, gtab);
   else
-    e = launch_iter(k_sart_atx_shared<true>, grid, dim3(kAtxThreads), st, insts, batch,
+    e = launch_iter(k_sart_atx_shared<true, false>, grid, dim3(kAtxThreads), st, insts, batch,
                     view, gtab);
   return e;
 }
 
 template <bool k3D, int kU, int kQ>
-static cudaError_t sart_ax_shared_as(const Inst *insts, int batch, unsigned blocks,
+static cudaError_t sart_ax_shared_as(const Inst *insts, int batch, long long rays,
                                      unsigned groups, int view, cudaStream_t st,
                                      const int2 *gtab) {
+  constexpr int kRays = kAxWarps / (kShareGroup / 4 / kQ);
   return launch_iter(k_sart_ax_shared<k3D, kU, kQ>,
-                     dim3(blocks, 1, groups * (kShareGroup / 4 / kQ)), dim3(kAxBlock), st,
+                     dim3((unsigned)((rays + kRays - 1) / kRays), 1, groups), dim3(kAxBlock), st,
                      insts, batch, view, gtab);
 }
 
 template <bool k3D>
-static cudaError_t sart_ax_shared_shape(const Inst *insts, int batch, unsigned blocks,
+static cudaError_t sart_ax_shared_shape(const Inst *insts, int batch, long long rays,
                                         unsigned groups, int view, cudaStream_t st, int u,
                                         int q, const int2 *gtab) {
   u = u ? u : kAxShareU<k3D>;
   q = q ? q : kAxShareQ<k3D>;
   if (u == 1 && q == 1)
-    return sart_ax_shared_as<k3D, 1, 1>(insts, batch, blocks, groups, view, st, gtab);
+    return sart_ax_shared_as<k3D, 1, 1>(insts, batch, rays, groups, view, st, gtab);
   if (u == 2 && q == 1)
-    return sart_ax_shared_as<k3D, 2, 1>(insts, batch, blocks, groups, view, st, gtab);
+    return sart_ax_shared_as<k3D, 2, 1>(insts, batch, rays, groups, view, st, gtab);
   if (u == 1 && q == 2)
-    return sart_ax_shared_as<k3D, 1, 2>(insts, batch, blocks, groups, view, st, gtab);
+    return sart_ax_shared_as<k3D, 1, 2>(insts, batch, rays, groups, view, st, gtab);
   if (u == 2 && q == 2)
-    return sart_ax_shared_as<k3D, 2, 2>(insts, batch, blocks, groups, view, st, gtab);
+    return sart_ax_shared_as<k3D, 2, 2>(insts, batch, rays, groups, view, st, gtab);
   return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_sart_ax_shared(const Inst *insts, int batch, const Dims &d,
                                   int view, cudaStream_t st, int u, int q,
                                   const int2 *gtab, int ngroups) {
-  const long long nr = (long long)d.na * d.nb;
-  const unsigned blocks = (unsigned)((nr + kAxWarps - 1) / kAxWarps);
+  const long long rays = (long long)d.na * d.nb;
   const unsigned groups =
       gtab ? (unsigned)ngroups : (unsigned)((batch + kShareGroup - 1) / kShareGroup);
   if (d.nz > 1 || d.nb > 1)
-    return sart_ax_shared_shape<true>(insts, batch, blocks, groups, view, st, u, q, gtab);
-  return sart_ax_shared_shape<false>(insts, batch, blocks, groups, view, st, u, q, gtab);
+    return sart_ax_shared_shape<true>(insts, batch, rays, groups, view, st, u, q, gtab);
+  return sart_ax_shared_shape<false>(insts, batch, rays, groups, view, st, u, q, gtab);
 }
 
 cudaError_t launch_group_pack(const Inst *insts, int batch, const Dims &d,

@@ -325,7 +325,7 @@ int asdpocs_plan_autotune(asdpocs_plan plan, int reps, int *walk, double *ms);
 typedef struct {
   int tv_walk;         /* TV step: bands (2-D) or slabs (3-D) per walk */
   int ax_cols;         /* shared-geometry forward step: columns of loads per round, 1 or 2 */
-  int ax_quads;        /* ... and quads of 4 instances per block, 1 or 2 */
+  int ax_quads;        /* ... and quads of 4 instances per lane, 1 or 2 */
   int zcol_segment;    /* cone-beam backward step: voxels per column segment, 8 .. 64 */
   int pdl;             /* programmatic dependent launches: -1 auto (plans on one stream),
                         * 0 off, 1 on */

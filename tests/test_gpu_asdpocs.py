@@ -748,3 +748,31 @@ def test_phase_timing_of_a_plan_with_different_view_counts(gpu):
         pl.reset()
         for phase in range(4):
             assert pl.time_phase(phase, 40) > 0.0
+
+
+@pytest.mark.parametrize("nx,ny,na", [(1, 3, 1), (15, 9, 23), (17, 8, 31), (33, 7, 64),
+                                      (64, 5, 65)])
+@pytest.mark.parametrize("batch", [4, 5, 8, 13])
+def test_two_lanes_per_voxel_groups_equal_alone_bitwise(gpu, nx, ny, na, batch):
+    """Groups of more than four instances are projected and back-projected
+    with two lanes to a voxel: at ragged rows, odd ray counts, groups whose
+    second quad is partly filled and instances that finish apart, every image
+    equals the one of the instance alone."""
+    phi = phantoms.views(5)
+    rng = np.random.default_rng(nx + batch)
+    paras = [dict(SO=541.0, OD=408.0, vxlsize=541.0 / 949.0 * na / nx, nx=nx, ny=ny, nz=1,
+                  na=na, nb=1, detsize=1.0, phi_vec=phi, maxnumIter=1 + k % 3,
+                  numOfgradients=2, alpha=0.02) for k in range(batch)]
+    Ps = [rng.random(na * len(phi)).astype(np.float32) for _ in range(batch)]
+
+    def run(ks):
+        with pkg.Plan([paras[k] for k in ks], [phi] * len(ks)) as pl:
+            for i, k in enumerate(ks):
+                pl.set_sinogram(i, Ps[k])
+            pl.reset()
+            pl.run()
+            return [pl.image(i) for i in range(len(ks))]
+
+    together = run(range(batch))
+    for k in range(batch):
+        assert np.array_equal(run([k])[0], together[k]), k
