@@ -344,3 +344,57 @@ def test_chained_device_projections_wait_for_each_other(gpu, oracle_mod, dims):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, want)
+
+
+def test_small_host_calls_equal_large_ones(gpu, oracle_mod):
+    """Calls with few bytes of arguments pass them through page-locked memory
+    (up to 512 KiB of inputs, 256 KiB of results): on both sides of the
+    limits, and from several threads at once, the bits of the device entry
+    points."""
+    import threading
+
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    L = load()
+    dims = [(8, 8, 1, 9, 1), (128, 256, 1, 64, 1), (129, 256, 1, 64, 1), (361, 362, 1, 64, 1),
+            (363, 362, 1, 64, 1), (20, 24, 30, 200, 300), (20, 24, 30, 400, 330)]
+    jobs = []
+    for k, (nx, ny, nz, na, nb) in enumerate(dims):
+        rng = np.random.default_rng(k)
+        para = dict(SO=541.0, OD=408.0, vxlsize=541.0 / 949.0 * na / nx, nx=nx, ny=ny, nz=nz,
+                    phi=-0.3 - k, detsize=1.0, na=na, nb=nb)
+        g = oracle_mod.gateway_geometry(para["phi"], 541.0, 408.0, para["vxlsize"], 1.0, na, nb)
+        x = rng.random(nx * ny * nz).astype(np.float32)
+        y = rng.random(na * nb).astype(np.float32)
+        dev = [torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
+               for a in (x, y, g["y_det"], g["z_det"])]
+        out = [torch.empty(n, device="cuda") for n in (y.size, y.size, x.size, x.size)]
+        st = torch.cuda.current_stream().cuda_stream
+        view = (g["cos_phi"], g["sin_phi"], dev[2].data_ptr(), dev[3].data_ptr(), g["SO"],
+                g["OD"], g["scale"])
+        check(L.asdpocs_ax_device(dev[0].data_ptr(), out[0].data_ptr(), out[1].data_ptr(), *view,
+                                  1.0, nx, ny, nz, na, nb, st))
+        check(L.asdpocs_atx_device(out[2].data_ptr(), dev[1].data_ptr(), out[3].data_ptr(), *view,
+                                   g["det"], g["det"], 1.0, nx, ny, nz, na, nb, st))
+        torch.cuda.synchronize()
+        jobs.append((para, x, y, [o.cpu().numpy() for o in out]))
+
+    wrong = []
+
+    def work(order):
+        for k in order:
+            para, x, y, want = jobs[k]
+            got = pkg.Ax_cone_gpu(x, para) + pkg.Atx_cone_gpu(y, para)
+            if not all(np.array_equal(a, b) for a, b in zip(got, want)):
+                wrong.append(dims[k])
+
+    work(range(len(jobs)))
+    threads = [threading.Thread(target=work, args=(np.roll(range(len(jobs)), t),))
+               for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
