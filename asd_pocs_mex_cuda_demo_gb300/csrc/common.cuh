@@ -64,7 +64,10 @@ __device__ __forceinline__ bool asd_in(long long i, long long n) {
 // waiting blocks never take the slots of its own.  Before it, a kernel may
 // load what the plan wrote at its creation or before the run (descriptors,
 // geometry, chord tables, sinograms), which hides that latency behind the
-// kernel before.  Every block calls it, also one that then has nothing to do:
+// kernel before.  It may also load what a kernel before the one it
+// waits for wrote, if the latter does not write it: that one's blocks have all
+// passed their own wait before this kernel starts.  Such loads go to the L2
+// (__ldcg): nothing orders the L1 before the wait.  Every block calls it, also one that then has nothing to do:
 // a grid whose blocks did not wait could end before its predecessor, and its
 // successor waits for it alone.  In a kernel launched the
 // ordinary way both instructions do nothing.  Plans that run sub-batches on

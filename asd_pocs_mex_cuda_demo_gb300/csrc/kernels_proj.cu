@@ -533,7 +533,14 @@ __global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
   bool planar = false, own = false;
   long long r = 0;  // lane's own ray
   float p = 0.f;
+  bool done = true;
+  const float *m = nullptr;
   if (have) {  // geometry and sinogram, before the wait
+    if (!kVol) {
+      m = I.m;
+      // set, if at all, by the kernels between two sweeps
+      if (view > 0) done = __ldcg(&I.s->done) != 0;
+    }
     G = view_of(I, view);
     if (kVol) {
       ax_rows(D, w, ia, ib);
@@ -548,13 +555,13 @@ __global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
   }
   pdl_enter();
   if (!have) return;
-  const bool done = ((volatile int *)&I.s->done)[0] != 0;
+  if (kVol || view == 0) done = ((volatile int *)&I.s->done)[0] != 0;
   const bool tabc = k3D && (I.tabc_mode == kTabcShared || (!done && I.tabc_mode == kTabcOwn));
   const long long q = k3D && I.rays_t ? (long long)ia * D.nb + ib + lane : r;
   if (tabc && own) ray_slopes(I, G, D, view, ia, ib + lane, q);
   if (done) return;
   const double dd = own ? ray_squares(I, r, nr) : 0.0;
-  const float *m = I.m;
+  if (kVol) m = I.m;
   auto ld = [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; };
   float yv, sv;
   if constexpr (kVol) {
@@ -694,13 +701,15 @@ __device__ __forceinline__ float chord_slot(const int *__restrict__ tab, size_t 
 }
 
 // Backward step over this block's `tiles` tiles from the view's chord table
-// (2-D, narrow form; see sart_atx_tiles).  The table entries of a voxel of
-// every tile are loaded before the wait for the forward step, the images
-// together after it, then the residuals (L1) in the pairs' order: a block
-// waits for memory once and not once a tile.  Pairs past a voxel's own add 0
-// times a residual, which is finite here.
+// (2-D, narrow form; see sart_atx_tiles).  Everything but the residuals is
+// loaded before the wait for the forward step: the table entries, and the
+// image, which the forward step only reads and whose last writer had completed
+// before that step began.  After it the residuals of every tile go out
+// together with the word that says whether they are finite: one latency.
+// Pairs past a voxel's own add 0 times a residual, which is finite here.
 struct TabTiles {
   ChordPre c[kTilesPerBlock];
+  float m[kTilesPerBlock];  // the image
 };
 __device__ __forceinline__ bool tab_voxel(const Dims &D, int tiles, int t, unsigned &vi) {
   const int ix = blockIdx.x * kTileX + threadIdx.x % kTileX;
@@ -710,49 +719,50 @@ __device__ __forceinline__ bool tab_voxel(const Dims &D, int tiles, int t, unsig
   return in;
 }
 __device__ __forceinline__ void tab_load(const Dims &D, const int *__restrict__ tab, int K,
-                                         int tiles, TabTiles &T) {
+                                         int tiles, const float *m, TabTiles &T) {
 #pragma unroll
   for (int t = 0; t < kTilesPerBlock; t++) {
     if (t >= tiles) break;
     unsigned vi;
     tab_voxel(D, tiles, t, vi);
-    T.c[t] = chord_load(tab, (size_t)D.nx * D.ny, K, vi);
+    const size_t N = (size_t)D.nx * D.ny;
+    T.c[t] = chord_load(tab, N, K, vi);
+    T.m[t] = ASD_IN(vi, N) ? __ldcg(m + vi) : 0.f;
   }
+}
+__device__ __forceinline__ void tab_residuals(const Dims &D, int tiles, const TabTiles &T,
+                                              const float *cor,
+                                              float (&y)[kTilesPerBlock][kChordPre]) {
+  const long long M = nray(D);
+#pragma unroll
+  for (int t = 0; t < kTilesPerBlock; t++)
+#pragma unroll
+    for (int ka = 0; ka < kChordPre; ka++) {
+      const int r = t < tiles ? T.c[t].first + (ka < T.c[t].cnt ? ka : 0) : 0;
+      y[t][ka] = t < tiles && ASD_IN(r, M) ? cor[r] : 0.f;
+    }
 }
 __device__ __forceinline__ void sart_atx_tiles_tab(const Inst &I, const Dims &D,
                                                    const int *__restrict__ tab, int K,
-                                                   int tiles, const TabTiles &T) {
-  const float beta = I.s->beta_f;
+                                                   int tiles, const TabTiles &T, float beta,
+                                                   const float (&y)[kTilesPerBlock][kChordPre]) {
   float *m = I.m;
-  const float *__restrict__ cor = I.cor;
+  const float *cor = I.cor;
   const size_t N = (size_t)D.nx * D.ny;
   const long long M = nray(D);
-  float mv[kTilesPerBlock];
-#pragma unroll
-  for (int t = 0; t < kTilesPerBlock; t++) {
-    if (t >= tiles) break;
-    unsigned vi;
-    tab_voxel(D, tiles, t, vi);
-    mv[t] = ASD_IN(vi, N) ? m[vi] : 0.f;
-  }
 #pragma unroll
   for (int t = 0; t < kTilesPerBlock; t++) {
     if (t >= tiles) break;
     unsigned vi;
     const bool in = tab_voxel(D, tiles, t, vi);
     const ChordPre &c = T.c[t];
-    const int kA = __reduce_max_sync(0xffffffffu, in ? c.cnt : 0);
     float acc = 0.f;
 #pragma unroll
-    for (int ka = 0; ka < kChordPre; ka++) {
-      if (ka >= kA) break;
-      const int r = c.first + (ka < c.cnt ? ka : 0);
-      if (ASD_IN(r, M)) pair2(acc, c.l[ka], __ldg(cor + r));
-    }
-    for (int ka = kChordPre; ka < kA; ka++)
-      if (ka < c.cnt && ASD_IN(ka, K) && ASD_IN(c.first + ka, M))
-        pair2(acc, chord_slot(tab, N, vi, ka), __ldg(cor + c.first + ka));
-    if (in && ASD_IN(vi, N)) m[vi] = sart_update(mv[t], beta, acc, c.norm);
+    for (int ka = 0; ka < kChordPre; ka++) pair2(acc, c.l[ka], y[t][ka]);
+    for (int ka = kChordPre; ka < c.cnt; ka++)
+      if (ASD_IN(ka, K) && ASD_IN(c.first + ka, M))
+        pair2(acc, chord_slot(tab, N, vi, ka), cor[c.first + ka]);
+    if (in && ASD_IN(vi, N)) m[vi] = sart_update(T.m[t], beta, acc, c.norm);
   }
 }
 
@@ -866,8 +876,16 @@ __device__ __forceinline__ void sart_atx_tiles(const Inst &I, const ViewGeo &G,
 // whose rays share one dominant in-plane axis and include no axis-parallel
 // ray (the instance's view flags; a block-uniform branch) uses the
 // axis-specialised chord.
-template <bool kPlanar>
-__global__ void __launch_bounds__(kAtxThreads, kPlanar ? 3 : 4)
+// Bound by latency: a chain of dependent launches for one slice, too few loads
+// in flight for a batch of slices of their own geometry.  Ten iterations of one
+// 512^2 slice, 60 views: 8.13 ms with the images loaded after the wait and the
+// residuals tile by tile, 7.3 with both as they are now and 2 blocks per SM, 7.5
+// with 4 (spills).  Four iterations of 15 slices: 16.1 ms then, now 17.7 with 2
+// blocks per SM, 13.9 with 3, 12.1 with 4, 11.9 with 5 (24 slices of 256^2: 7.9,
+// 6.4, 5.8, 6.1), so kBlocks is 2 where the launch has no more and 4 elsewhere;
+// two tiles a block at 5 to 8 blocks 12.7 to 13.3 ms, one 17 to 18.
+template <bool kPlanar, int kBlocks>
+__global__ void __launch_bounds__(kAtxThreads, kBlocks)
     k_sart_atx(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap,
                int tiles) {
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
@@ -877,20 +895,32 @@ __global__ void __launch_bounds__(kAtxThreads, kPlanar ? 3 : 4)
   const int *tab = nullptr;
   TabTiles T;
   int vf = 0;
-  if (have) {  // the plan's tables, before the wait
+  bool done = true;
+  float beta = 0.f;
+  const float *cor = nullptr;
+  Scalars *s = nullptr;
+  if (have) {  // before the wait: what the plan or kernels before the forward step wrote
+    s = I.s;
+    cor = I.cor;
+    done = __ldcg(&s->done) != 0;
+    beta = __ldcg(&s->beta_f);
     vf = I.vflags[view];
     if (kPlanar && I.chtab && !(vf & kViewAxisParallel) && I.g.z_det[0] == 0.0f) {
       tab = I.chtab + (size_t)view * chord_view_words(D, I.chK);
-      tab_load(D, tab, I.chK, tiles, T);
+      tab_load(D, tab, I.chK, tiles, I.m, T);
     }
   }
   pdl_enter();
-  if (!have || ((volatile int *)&I.s->done)[0]) return;
-  const bool finite = I.s->cor_bad != view + 1;
-  if (tab && finite) {
-    sart_atx_tiles_tab(I, D, tab, I.chK, tiles, T);
-    return;
+  if (done) return;
+  if (tab) {
+    float y[kTilesPerBlock][kChordPre];
+    tab_residuals(D, tiles, T, cor, y);
+    if (s->cor_bad != view + 1) {
+      sart_atx_tiles_tab(I, D, tab, I.chK, tiles, T, beta, y);
+      return;
+    }
   }
+  const bool finite = s->cor_bad != view + 1;
   const ViewGeo G = view_of(I, view);
   const float4 *tabA = I.tabA + (long long)view * D.na;
   const bool narrow =
@@ -2042,8 +2072,9 @@ cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
   cudaError_t e;
   // fan beams: the fewest tiles a block (1, 2 or 4) that keep the launch within
   // two blocks per SM, so that they sit, their tables loaded, beside the forward
-  // step's (512^2, ten iterations: 8.10 ms with 256 blocks of four tiles, 8.55
-  // with 512 of two; 10.4 without the loads before the wait)
+  // step's (512^2, ten iterations: 8.1 ms with 256 blocks of four tiles, 8.55
+  // with 512 of two; 10.4 without the loads before the wait; 7.3 with the images
+  // among them)
   int tiles = d.nz == 1 ? 1 : kTilesPerBlock;
   dim3 grid = group_grid(d.nx, d.ny, d.nz, batch, tiles);
   while (tiles < kTilesPerBlock && (long long)grid.x * grid.y * batch > 152 * 2) {
@@ -2055,9 +2086,11 @@ cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
     e = launch_iter(s.W == 32 ? k_sart_atx_zcol<32> : k_sart_atx_zcol<8>, zcol_grid(d, batch, s),
                     dim3(kZcThreads), st, insts, view, s.lsh(), s.seg, zmap);
   } else if (d.nz > 1 || d.nb > 1)
-    e = launch_iter(k_sart_atx<false>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
+    e = launch_iter(k_sart_atx<false, 4>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
+  else if ((long long)grid.x * grid.y * batch <= 152 * 2)
+    e = launch_iter(k_sart_atx<true, 2>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
   else
-    e = launch_iter(k_sart_atx<true>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
+    e = launch_iter(k_sart_atx<true, 4>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
   return e;
 }
 
