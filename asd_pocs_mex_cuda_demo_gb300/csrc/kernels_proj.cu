@@ -700,6 +700,29 @@ __device__ __forceinline__ float chord_slot(const int *__restrict__ tab, size_t 
   return __ldg((const float *)(tab + 2 * N) + (size_t)(k / 2) * 2 * N + 2 * vi + (k & 1));
 }
 
+// Asks for the chord table of the next view (the first after the last) in the
+// L2: part `part` of `parts` of it, by one thread.  The tables of all views
+// come from memory each sweep where they do not fit the L2, and the step waits
+// for them: one slice of 512^2 (6.3 MB a view, 377 in all) 7.3 -> 6.6 ms for ten
+// iterations, 6 and 24 slices of 256^2 (9.4 and 38 MB) 2.38 -> 2.24 and 5.76 ->
+// 5.63 ms.  With 50 MB a view the L2 loses lines it still needs (8 slices of
+// 512^2 7.8 -> 9.1 ms), and with 94 MB in all there is nothing to fetch (1.62 ->
+// 1.64 ms).
+constexpr size_t kPrefetchMax = (size_t)40 << 20, kPrefetchAll = (size_t)96 << 20;
+__device__ __forceinline__ void prefetch_table(const Inst &I, const Dims &D, int view,
+                                               unsigned part, unsigned parts) {
+  const size_t bytes = chord_view_words(D, I.chK) * sizeof(int), next = bytes * gridDim.z;
+  if (next > kPrefetchMax || next * I.nv < kPrefetchAll) return;
+  const char *const t = (const char *)I.chtab + (view + 1 < I.nv ? view + 1 : 0) * bytes;
+  const size_t chunk = (bytes / parts + 16) & ~(size_t)15;
+  const char *lo = t + part * chunk, *hi = t + min((part + 1) * chunk, bytes);
+  lo = (const char *)(((uintptr_t)lo + 15) & ~(uintptr_t)15);
+  hi = (const char *)((uintptr_t)hi & ~(uintptr_t)15);
+  if (lo < hi)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lo), "r"((unsigned)(hi - lo))
+                 : "memory");
+}
+
 // Backward step over this block's `tiles` tiles from the view's chord table
 // (2-D, narrow form; see sart_atx_tiles).  Everything but the residuals is
 // loaded before the wait for the forward step: the table entries, and the
@@ -880,12 +903,14 @@ __device__ __forceinline__ void sart_atx_tiles(const Inst &I, const ViewGeo &G,
 // in flight for a batch of slices of their own geometry.  Ten iterations of one
 // 512^2 slice, 60 views: 8.13 ms with the images loaded after the wait and the
 // residuals tile by tile, 7.3 with both as they are now and 2 blocks per SM, 7.5
-// with 4 (spills).  Four iterations of 15 slices: 16.1 ms then, now 17.7 with 2
-// blocks per SM, 13.9 with 3, 12.1 with 4, 11.9 with 5 (24 slices of 256^2: 7.9,
-// 6.4, 5.8, 6.1), so kBlocks is 2 where the launch has no more and 4 elsewhere;
-// two tiles a block at 5 to 8 blocks 12.7 to 13.3 ms, one 17 to 18.
-template <bool kPlanar, int kBlocks>
-__global__ void __launch_bounds__(kAtxThreads, kBlocks)
+// with 4 (spills); with the next table prefetched 6.6 (96 registers; two blocks
+// then leave room for the forward step's, 110 registers 6.8).  Four iterations
+// of 15 slices: 16.1 ms then, now 17.7 with 2 blocks per SM, 13.9 with 3, 12.1
+// with 4, 11.9 with 5 (24 slices of 256^2: 7.9, 6.4, 5.8, 6.1), so kRegs is 96
+// where the launch has no more than two blocks per SM and 64, for four,
+// elsewhere; two tiles a block at 5 to 8 blocks 12.7 to 13.3 ms, one 17 to 18.
+template <bool kPlanar, int kRegs>
+__global__ void __launch_bounds__(kAtxThreads) __maxnreg__(kRegs)
     k_sart_atx(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap,
                int tiles) {
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
@@ -908,6 +933,10 @@ __global__ void __launch_bounds__(kAtxThreads, kBlocks)
     if (kPlanar && I.chtab && !(vf & kViewAxisParallel) && I.g.z_det[0] == 0.0f) {
       tab = I.chtab + (size_t)view * chord_view_words(D, I.chK);
       tab_load(D, tab, I.chK, tiles, I.m, T);
+      if (threadIdx.x == 0) {
+        const OwnBlock b = own_block(group_grid(D.nx, D.ny, D.nz, 1, tiles));
+        prefetch_table(I, D, view, b.bid, b.nblocks);
+      }
     }
   }
   pdl_enter();
@@ -2086,11 +2115,11 @@ cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
     e = launch_iter(s.W == 32 ? k_sart_atx_zcol<32> : k_sart_atx_zcol<8>, zcol_grid(d, batch, s),
                     dim3(kZcThreads), st, insts, view, s.lsh(), s.seg, zmap);
   } else if (d.nz > 1 || d.nb > 1)
-    e = launch_iter(k_sart_atx<false, 4>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
+    e = launch_iter(k_sart_atx<false, 64>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
   else if ((long long)grid.x * grid.y * batch <= 152 * 2)
-    e = launch_iter(k_sart_atx<true, 2>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
+    e = launch_iter(k_sart_atx<true, 96>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
   else
-    e = launch_iter(k_sart_atx<true, 4>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
+    e = launch_iter(k_sart_atx<true, 64>, grid, dim3(kAtxThreads), st, insts, view, zmap, tiles);
   return e;
 }
 
