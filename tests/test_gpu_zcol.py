@@ -1,12 +1,14 @@
 """The cone-beam backward step in voxel columns against its per-voxel form,
 bit for bit, over the sizes and geometries where its lane and block layout and
-its pair paths change: asdpocs_atx_device takes the per-voxel form while its
-stream is captured, so one call is made plainly and one in a graph."""
+its pair paths change: calls on host arrays take columns; asdpocs_atx_device
+takes the per-voxel form for small volumes and while its stream is captured, so
+one call is made plainly, one in a graph and one on host arrays."""
 import ctypes as C
 
 import numpy as np
 import pytest
 
+import asd_pocs_mex_cuda_demo_gb300 as pkg
 from asd_pocs_mex_cuda_demo_gb300._lib import check, load
 
 pytestmark = pytest.mark.gpu
@@ -22,6 +24,7 @@ CASES = [
     (16, 16, 24, 200, 260, 60.0, 60.0, 0.18, 1.0),    # shadows wider than the slots
     (24, 24, 40, 40, 120, 20.0, 10.0, 0.9, 1.0),      # steep rays, corners near the source
     (24, 20, 30, 48, 60, 90.0, 45.0, 0.9, 0.7),       # slices that are not 1
+    (70, 62, 61, 130, 110, 180.0, 90.0, 0.9, 1.0),    # over 2^18 voxels
 ]
 
 
@@ -53,6 +56,10 @@ def test_columns_equal_voxels(gpu, case, angle):
         call(out[2], out[3])
     g.replay()
     torch.cuda.synchronize()
-    for a, b in ((0, 2), (1, 3)):
+    h = [np.full(nx * ny * nz, np.nan, f) for _ in range(2)]
+    pkg.Atx_cone_mf_gpu_new(h[0], y.cpu().numpy(), h[1], float(np.cos(phi)), float(np.sin(phi)),
+                            yd, zd, SO, OD, 0.7, det, det, dz, nx, ny, nz, na, nb)
+    out += [T(a) for a in h]
+    for a, b in ((0, 2), (1, 3), (4, 2), (5, 3)):
         assert torch.equal(out[a].view(torch.int32), out[b].view(torch.int32))
     assert float(out[1].abs().max()) > 0
