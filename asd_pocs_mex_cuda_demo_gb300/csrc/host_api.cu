@@ -2241,7 +2241,12 @@ int ASD_POCS_cuda(const double *P, const double *phi_vec_deg,
     rc = asdpocs_plan_set_reference(p, 0, buf.data(), 0);
   }
   if (!rc) rc = asdpocs_plan_reset(p);
-  if (!rc) rc = asdpocs_plan_run(p, 1);
+  // The plan runs once: a graph is captured only where it saves more launch time
+  // than its instantiation costs (64^2, 24 views: 2 iterations 1.11 ms with it,
+  // 0.94 without, 8 2.43 and 2.37, 12 3.31 and 3.27, 24 5.94 and 6.10; 128^2, 60
+  // views: 8 3.88 and 3.76, 12 5.34 and 5.39; from 256^2 on the GPU is the slower
+  // side and the direct launches win up to 40 iterations and more, by 0.3 ms).
+  if (!rc) rc = asdpocs_plan_run(p, p->max_iter > 10);
   if (!rc) rc = asdpocs_plan_get_image(p, 0, buf.data(), 0);
   if (!rc) {
     for (size_t i = 0; i < N; i++) m_res[i] = buf[i];

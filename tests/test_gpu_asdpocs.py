@@ -806,3 +806,21 @@ def test_large_chord_tables_equal_direct_form(gpu, monkeypatch, batch):
     assert none == 0
     for a, b in zip(tables, direct):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("iters", [1, 10, 11])
+def test_one_call_equals_plan_run(gpu, iters):
+    """ASD_POCS_cuda launches its kernels directly for at most ten iterations
+    and from a graph beyond: the images of a plan run either way."""
+    n, na, phi = 33, 52, phantoms.views(7)
+    para = dict(SO=541.0, OD=408.0, vxlsize=541.0 / 949.0 * na / n, nx=n, ny=n, nz=1, na=na, nb=1,
+                detsize=1.0, phi_vec=phi, maxnumIter=iters, numOfgradients=4, alpha=0.02)
+    P = np.random.default_rng(iters).random((na, len(phi))).astype(np.float32)
+    m, out = pkg.ASD_POCS_cuda(P, para)
+    assert out["IterationNum"] == iters
+    for graph in (False, True):
+        with pkg.Plan(para, phi) as pl:
+            pl.set_sinogram(0, P.ravel(order="F"))
+            pl.reset()
+            pl.run(use_graph=graph)
+            assert np.array_equal(pl.image(0).ravel(), m.ravel(order="F").astype(np.float32))
