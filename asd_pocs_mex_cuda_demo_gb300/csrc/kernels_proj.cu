@@ -146,10 +146,10 @@ __global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
   }
 }
 
-// Exact forward projection (siddon_setup, siddon_columns), a warp per 32
-// rays: lane j sets up ray j (its FP64 arithmetic once per ray, not once per
+// Exact forward projection (siddon_setup, siddon_columns), a warp per `rpw`
+// (1 to 32) rays: lane j sets up ray j (its FP64 arithmetic once per ray, not once per
 // lane: the GPU's FP64 rate is a small fraction of its FP32 rate), then the
-// warp walks the 32 rays in turn, each ray's set-up broadcast from its lane
+// warp walks its rays in turn, each ray's set-up broadcast from its lane
 // and its columns dealt to the lanes, summed by the butterfly; lane j keeps
 // ray j's totals.
 __device__ __forceinline__ DSFloat ds_shfl(DSFloat v, int src) {
@@ -182,11 +182,11 @@ __device__ __forceinline__ SidRay sid_bcast(const SidRay &R, int src) {
   return o;
 }
 
-// Totals of rays r0 + lane (lane < nr - r0) for the whole warp.
+// Totals of rays r0 + lane (lane < rpw, nr - r0) for the whole warp.
 template <class Loader>
 __device__ __forceinline__ void siddon_warp_rays(const ViewGeo &G, const Dims &D,
-                                                 long long r0, long long nr, Loader ld,
-                                                 float &my_y, float &my_s) {
+                                                 long long r0, long long nr, int rpw,
+                                                 Loader ld, float &my_y, float &my_s) {
   const int lane = threadIdx.x & 31;
   SidRay mine;
   const DSFloat z{0.f, 0.f};
@@ -196,8 +196,8 @@ __device__ __forceinline__ void siddon_warp_rays(const ViewGeo &G, const Dims &D
   mine.su = mine.sv = mine.sz = 0u;
   mine.hit = false;
   const long long r = r0 + lane;
-  if (r < nr) mine = siddon_setup(G, D, G.y_det[r % D.na], G.z_det[r / D.na]);
-  const int cnt = (int)min(32LL, nr - r0);
+  if (lane < rpw && r < nr) mine = siddon_setup(G, D, G.y_det[r % D.na], G.z_det[r / D.na]);
+  const int cnt = (int)min((long long)rpw, nr - r0);
   my_y = my_s = 0.f;
   for (int j = 0; j < cnt; j++) {
     const SidRay R = sid_bcast(mine, j);
@@ -212,20 +212,35 @@ __device__ __forceinline__ void siddon_warp_rays(const ViewGeo &G, const Dims &D
   }
 }
 
-constexpr int kSidRays = kAxWarps * 32;  // rays per block of the exact kernels
+// Rays per warp of the exact kernels for `rays` rays in a launch.  A warp's
+// set-up costs the same for one ray as for 32 (the FP64 pipe: about 0.7 us of
+// an SM's time), and its rays follow one another at about 0.02 us a column, so
+// the best count is near the root of rays over columns: largest power of two
+// with rpw^2 <= 5/8 rays / columns.  us a view with 32 rays a warp, one, and
+// this rule: 512^2 and 888 bins 328, 19.6, 19.6; eight of it 340, 65, 60; 64 of
+// it 409, -, 280; 48^2 x 32 on 80 x 60 64, 37, 19; 96^2 x 64 on 160 x 128 96,
+// -, 51; 160^2 x 128 on 256 x 200 215, -, 144.
+static int sid_rays(long long rays, const Dims &d) {
+  int rpw = 32;
+  while (rpw > 1 && 8LL * rpw * rpw * max(d.nx, d.ny) > 5 * rays) rpw /= 2;
+  return rpw;
+}
+static unsigned sid_blocks(long long rays, int rpw) {
+  return (unsigned)((rays + kAxWarps * rpw - 1) / (kAxWarps * rpw));
+}
 
 __global__ void __launch_bounds__(kAxBlock)
     k_ax_siddon(const float *__restrict__ x, float *__restrict__ y,
-                float *__restrict__ sr, ViewGeo G, Dims D) {
+                float *__restrict__ sr, ViewGeo G, Dims D, int rpw) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long nr = (long long)D.na * D.nb;
-  const long long r0 = ((long long)blockIdx.x * kAxWarps + warp) * 32;
+  const long long r0 = ((long long)blockIdx.x * kAxWarps + warp) * rpw;
   if (r0 >= nr) return;  // the whole warp
   float yv, sv;
-  siddon_warp_rays(G, D, r0, nr,
+  siddon_warp_rays(G, D, r0, nr, rpw,
                    [&](unsigned i) { return ASD_IN(i, nvox(D)) ? __ldg(x + i) : 0.f; }, yv, sv);
   const long long r = r0 + lane;
-  if (r < nr) {
+  if (lane < rpw && r < nr) {
     y[r] = yv * G.scale;
     sr[r] = sv * G.scale;
   }
@@ -587,7 +602,8 @@ __global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
 // lane j ray j's residual and normalisation.
 template <bool k3D>
 __global__ void __launch_bounds__(kAxBlock)
-    k_sart_ax_exact(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap) {
+    k_sart_ax_exact(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap,
+                    int rpw) {
   pdl_enter();
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
   if (view >= I.nv) return;
@@ -598,16 +614,17 @@ __global__ void __launch_bounds__(kAxBlock)
   const long long nr = nray(D);
   const ViewGeo G = view_of(I, view);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long r0 = ((long long)blockIdx.x * kAxWarps + warp) * 32, r = r0 + lane;
+  const long long r0 = ((long long)blockIdx.x * kAxWarps + warp) * rpw, r = r0 + lane;
+  const bool own = lane < rpw && r < nr;
   const int ia = (int)(r % D.na), ib = (int)(r / D.na);
   const long long q = I.rays_t ? (long long)ia * D.nb + ib : r;
-  if (tabc && r < nr) ray_slopes(I, G, D, view, ia, ib, q);
+  if (tabc && own) ray_slopes(I, G, D, view, ia, ib, q);
   if (done || r0 >= nr) return;  // the whole warp
   float yv = 0.f, sv = 0.f;
   const float *m = I.m;
-  siddon_warp_rays(G, D, r0, nr, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; },
+  siddon_warp_rays(G, D, r0, nr, rpw, [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; },
                    yv, sv);
-  if (r < nr)
+  if (own)
     ray_out_store(I, &I.s->cor_bad, view, r, q, nr, ray_out_load(I, view, r, nr), yv * G.scale,
                   sv * G.scale);
 }
@@ -703,9 +720,9 @@ __device__ __forceinline__ float chord_slot(const int *__restrict__ tab, size_t 
 // Asks for the chord table of the next view (the first after the last) in the
 // L2: part `part` of `parts` of it, by one thread.  The tables of all views
 // come from memory each sweep where they do not fit the L2, and the step waits
-// for them: one slice of 512^2 (6.3 MB a view, 377 in all) 7.3 -> 6.6 ms for ten
+// for them: one slice of 512^2 (10.5 MB a view, 629 in all) 7.3 -> 6.6 ms for ten
 // iterations, 6 and 24 slices of 256^2 (9.4 and 38 MB) 2.38 -> 2.24 and 5.76 ->
-// 5.63 ms.  With 50 MB a view the L2 loses lines it still needs (8 slices of
+// 5.63 ms.  With 84 MB a view the L2 loses lines it still needs (8 slices of
 // 512^2 7.8 -> 9.1 ms), and with 94 MB in all there is nothing to fetch (1.62 ->
 // 1.64 ms).
 constexpr size_t kPrefetchMax = (size_t)40 << 20, kPrefetchAll = (size_t)96 << 20;
@@ -2068,13 +2085,14 @@ cudaError_t launch_sart_ax(const Inst *insts, int batch, const Dims &d,
   cudaError_t e;
   const long long nr = (long long)d.na * d.nb;
   const dim3 grid(ax_blocks(d), 1, batch);
-  const dim3 grid_ex((unsigned)((nr + kSidRays - 1) / kSidRays), 1, batch);
+  const int rpw = sid_rays(nr * batch, d);
+  const dim3 grid_ex(sid_blocks(nr, rpw), 1, batch);
   const bool p3 = d.nz > 1 || d.nb > 1;
   if (exact) {
     if (p3)
-      e = launch_iter(k_sart_ax_exact<true>, grid_ex, dim3(kAxBlock), st, insts, view, zmap);
+      e = launch_iter(k_sart_ax_exact<true>, grid_ex, dim3(kAxBlock), st, insts, view, zmap, rpw);
     else
-      e = launch_iter(k_sart_ax_exact<false>, grid_ex, dim3(kAxBlock), st, insts, view, zmap);
+      e = launch_iter(k_sart_ax_exact<false>, grid_ex, dim3(kAxBlock), st, insts, view, zmap, rpw);
   } else {
     if (d.nz > 1)
       e = launch_iter(k_sart_ax<true, true>, grid, dim3(kAxBlock), st, insts, view, zmap);
@@ -2090,8 +2108,8 @@ cudaError_t launch_ax_siddon(const float *x, float *y, float *sr, const ViewGeo 
                              const Dims &d, cudaStream_t st) {
   const long long nr = (long long)d.na * d.nb;
   if (nr == 0) return cudaSuccess;
-  k_ax_siddon<<<(unsigned)((nr + kSidRays - 1) / kSidRays), kAxBlock, 0, st>>>(x, y, sr, g,
-                                                                                d);
+  const int rpw = sid_rays(nr, d);
+  k_ax_siddon<<<sid_blocks(nr, rpw), kAxBlock, 0, st>>>(x, y, sr, g, d, rpw);
   return cudaGetLastError();
 }
 

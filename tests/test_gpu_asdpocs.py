@@ -824,3 +824,32 @@ def test_one_call_equals_plan_run(gpu, iters):
             pl.reset()
             pl.run(use_graph=graph)
             assert np.array_equal(pl.image(0).ravel(), m.ravel(order="F").astype(np.float32))
+
+
+@pytest.mark.parametrize("dims,batches", [((16, 12, 1, 31, 1), (1, 5, 40)),
+                                          ((64, 40, 1, 129, 1), (1, 3, 21)),
+                                          ((10, 12, 9, 37, 23), (1, 2, 9))])
+def test_exact_mode_rays_per_warp_do_not_change_results(gpu, dims, batches):
+    """The exact forward kernels give a warp one to 32 rays, by the rays of the
+    launch and the columns of a ray: an instance's image is the same alone and
+    in batches that change that count, at ray counts that leave the last warp
+    partly filled."""
+    nx, ny, nz, na, nb = dims
+    phi = phantoms.views(5)
+    para = dict(SO=541.0, OD=408.0, vxlsize=541.0 / 949.0 * na / nx, nx=nx, ny=ny, nz=nz, na=na,
+                nb=nb, detsize=1.0, phi_vec=phi, maxnumIter=2, numOfgradients=2, alpha=0.02,
+                ax_mode="exact")
+    rng = np.random.default_rng(na)
+    Ps = [rng.random(na * nb * len(phi)).astype(np.float32) for _ in range(max(batches))]
+    first = None
+    for b in batches:
+        with pkg.Plan([para] * b, [phi] * b) as pl:
+            for k in range(b):
+                pl.set_sinogram(k, Ps[k])
+            pl.reset()
+            pl.run()
+            images = [pl.image(k) for k in range(b)]
+        if first is None:
+            first = images[0]
+            assert np.abs(first).max() > 0
+        assert np.array_equal(images[0], first)
