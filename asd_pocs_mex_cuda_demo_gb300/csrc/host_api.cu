@@ -787,7 +787,7 @@ struct asdpocs_plan_s {
   bool zcol = true;     // cone beams: z-column backward step (else per voxel)
   bool exact = false;   // forward steps: exact Siddon projection (ax_mode)
   int tv_walk = 0;      // TV walk length (0: from the batch size)
-  int zseg = 0;         // z-column segment length (0: the default)
+  int zseg = 0;         // slices of a z-column block (0: the default)
   int ax_u = 0, ax_q = 0;  // shared forward step's shape (0: the defaults)
   int pdl = -1;         // programmatic dependent launches: -1 = when the plan
                         // runs on one stream, 0 = off, 1 = on
@@ -2197,7 +2197,7 @@ int asdpocs_plan_autotune_shapes(asdpocs_plan p, int reps, asdpocs_shapes *out) 
     p->ax_u = uq / 4;
     p->ax_q = uq % 4;
   } else if (p->d.nz > 1 && p->zcol) {
-    rc = pick(1, &p->zseg, {0, 4, 8, 16, 32});  // the z-column segment length (0: by size)
+    rc = pick(1, &p->zseg, {0, 32, 64, 128, 256});  // slices of a z-column block (0: by size)
   }
   double t_best = 0.0;
   // programmatic launches only where the plan runs on one stream (PdlScope)

@@ -81,9 +81,9 @@ UNEVEN = dict(
 # (one volume).  The traffic is about one read of each instance's image or
 # volume plus its writes, so it scales with the batch.
 NCU_DRAM_PER_INSTANCE = {
-    "fan2d": {"sart_ax": 60.94e6 / 64, "sart_atx": 40.13e6 / 32,
+    "fan2d": {"sart_ax": 60.94e6 / 64, "sart_atx": 40.18e6 / 32,
               "tv_step": 90.55e6 / 64},
-    "cone3d": {"sart_ax": 71.55e6, "sart_atx": 80.01e6, "tv_step": 91.60e6},
+    "cone3d": {"sart_ax": 70.10e6, "sart_atx": 80.05e6, "tv_step": 91.60e6},
 }
 
 

@@ -326,7 +326,7 @@ typedef struct {
   int tv_walk;         /* TV step: bands (2-D) or slabs (3-D) per walk */
   int ax_cols;         /* shared-geometry forward step: columns of loads per round, 1 or 2 */
   int ax_quads;        /* ... and quads of 4 instances per lane, 1 or 2 */
-  int zcol_segment;    /* cone-beam backward step: voxels per column segment, 8 .. 64 */
+  int zcol_segment;    /* cone-beam backward step: slices of a block, up to 256 */
   int pdl;             /* programmatic dependent launches: -1 auto (plans on one stream),
                         * 0 off, 1 on */
   double iteration_ms; /* autotune: one iteration with the chosen shapes (device time) */
