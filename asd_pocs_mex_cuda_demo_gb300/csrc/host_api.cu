@@ -2188,7 +2188,7 @@ int asdpocs_plan_autotune_shapes(asdpocs_plan p, int reps, asdpocs_shapes *out) 
   if (p->shared) {
     // the shared forward step's shape, on whole iterations: its kernels share
     // the GPU with the other sub-batch's, which a kernel timed alone misses
-    const int dflt = p->d.nz > 1 || p->d.nb > 1 ? 1 * 4 + 2 : 2 * 4 + 1;
+    const int dflt = 1 * 4 + (p->d.nz > 1 || p->d.nb > 1 ? 2 : 1);
     int uq = dflt;
     std::vector<int> cand{dflt};
     for (int c : {1 * 4 + 1, 2 * 4 + 1, 1 * 4 + 2, 2 * 4 + 2})

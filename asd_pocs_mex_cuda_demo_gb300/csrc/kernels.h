@@ -128,7 +128,7 @@ cudaError_t launch_sart_atx_shared(const Inst *insts, int batch,
 // the column march evaluated once per ray for groups of instances whose
 // images are interleaved (Inst::m_il) during the sweep.
 // `u` columns of loads per round and `q` quads of instances per lane (1 or
-// 2 each; 0: the defaults, 2 x 1 for fan beams, 1 x 2 for cone beams) are
+// 2 each; 0: the defaults, 1 x 1 for fan beams, 1 x 2 for cone beams) are
 // launch shapes that do not change results.
 // `gtab`, `ngroups` as for launch_sart_atx_shared.
 cudaError_t launch_sart_ax_shared(const Inst *insts, int batch, const Dims &d,

@@ -1789,20 +1789,20 @@ __global__ void __launch_bounds__(kAtxThreads, 5)
 // epilogue is that of k_sart_ax, so its projection, residual, squares and
 // flags are bit-identical to it.
 // ---------------------------------------------------------------------------
-// columns per round of loads in the shared forward step: two for fan beams
-// (26.9 us a launch of 64, one 26.3); one for cone beams, whose three pieces per
-// column already keep six loads in flight.  Blocks per SM: 6 for fan beams
-// (72 registers, no spills), 8 for cone beams (64 registers: 10 % faster
-// than 6 at 128^3).
-template <bool k3D>
-constexpr int kAxShareU = k3D ? 1 : 2;
+// columns per round of loads in the shared forward step, and 64 registers for 8
+// blocks per SM.  Cone beams: three pieces per column already keep six loads in
+// flight (8 blocks 10 % faster than 6 at 128^3).  Fan beams, a launch of 64
+// instances and four iterations of them (512^2): one column at 8 blocks 25.0 us
+// and 15.2 ms; at 7 26.4 and 15.7, at 10 25.5 and 15.4; two columns at 6 blocks
+// 26.9 and 16.1, at 8 26.6 and 16.1, at 10 25.9 and 15.5.
+constexpr int kAxShareU = 1;
 // quads of a group (4 instances each) per lane: one for fan beams, both for
 // cone beams.  One: two lanes to a voxel, so that a load takes whole 32-byte
 // sectors, and two warps to a ray, 16 of its columns each, so that the columns
 // are still dealt to 32 lanes and added in the same order.  A launch of 64
-// instances, 512^2 and 888 bins, waits for memory (37 % issue): 32.8 us with
-// the two quads in blocks of their own, each taking half of every sector, 26.9
-// now; both quads in a lane 29.0.
+// instances, 512^2 and 888 bins, waits for memory (37 % issue): at two columns
+// a round 32.8 us with the two quads in blocks of their own, each taking half of
+// every sector, 26.9 now; both quads in a lane 29.0.
 template <bool k3D>
 constexpr int kAxShareQ = k3D ? kShareGroup / 4 : 1;
 
@@ -1811,7 +1811,7 @@ constexpr int kAxShareQ = k3D ? kShareGroup / 4 : 1;
 // order in which an instance's pieces are added, so every shape gives the
 // same bits.
 template <bool k3D, int kU, int kQ>
-__global__ void __launch_bounds__(kAxBlock, k3D ? 8 : 6)
+__global__ void __launch_bounds__(kAxBlock, 8)
     k_sart_ax_shared(const Inst *__restrict__ insts, int batch, int view,
                      const int2 *__restrict__ gtab) {
   constexpr int kQuads = kShareGroup / 4, kS = 4 * kQ;
@@ -2174,7 +2174,7 @@ template <bool k3D>
 static cudaError_t sart_ax_shared_shape(const Inst *insts, int batch, long long rays,
                                         unsigned groups, int view, cudaStream_t st, int u,
                                         int q, const int2 *gtab) {
-  u = u ? u : kAxShareU<k3D>;
+  u = u ? u : kAxShareU;
   q = q ? q : kAxShareQ<k3D>;
   if (u == 1 && q == 1)
     return sart_ax_shared_as<k3D, 1, 1>(insts, batch, rays, groups, view, st, gtab);
