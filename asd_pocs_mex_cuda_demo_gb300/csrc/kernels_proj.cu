@@ -1800,7 +1800,7 @@ constexpr int kAxShareU = 1;
 // cone beams.  One: two lanes to a voxel, so that a load takes whole 32-byte
 // sectors, and two warps to a ray, 16 of its columns each, so that the columns
 // are still dealt to 32 lanes and added in the same order.  A launch of 64
-// instances, 512^2 and 888 bins, waits for memory (37 % issue): at two columns
+// instances, 512^2 and 888 bins, waits for memory (42 % issue): at two columns
 // a round 32.8 us with the two quads in blocks of their own, each taking half of
 // every sector, 26.9 now; both quads in a lane 29.0.
 template <bool k3D>
