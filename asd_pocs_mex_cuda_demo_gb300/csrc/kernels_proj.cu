@@ -1012,15 +1012,8 @@ __global__ void __launch_bounds__(kAtxThreads) __maxnreg__(kRegs)
 // Grid: x tiles of W x y x segments of `seg` slices, instances.
 // ---------------------------------------------------------------------------
 constexpr int kZcThreads = 256, kZcWarps = kZcThreads / 32;
-constexpr int kZcSlots = 6;             // detector columns of a shadow kept
-constexpr int kZcCols = 4, kZcRows = 3; // most listed pairs
+constexpr int kZcSlots = 6;  // detector columns of a shadow kept
 static_assert(kZcRows <= 4 && kZcCols <= 8, "a pair's bit is 4 s + kb");
-
-// Elements after the na * nb rays of cor and tabC that the unrolled pairs may
-// read (zeros).
-__host__ __device__ __forceinline__ long long zcol_pad(const Dims &d) {
-  return (long long)(kZcCols - 1) * d.nb + kZcRows;
-}
 
 template <int W>
 struct ZColShared {
@@ -1180,7 +1173,7 @@ __device__ __forceinline__ void atx_zcol_walk(const ViewGeo &G, const Dims &D,
     col.lo = 0;
     if (x0 + c < D.nx) {
       col = zcol_setup(G, D, x0 + c, iy, true);
-      cnt = col.lo <= col.hi ? col.hi - col.lo + 1 : 0;
+      cnt = zcol_count(col);
       wide = cnt > kZcSlots;
     }
     if (t < W && x0 + c < D.nx) {
@@ -1195,7 +1188,7 @@ __device__ __forceinline__ void atx_zcol_walk(const ViewGeo &G, const Dims &D,
       sh.flags[c] = kZcInside;
     }
     if (t < W) {
-      sh.lo[c] = col.lo;
+      sh.lo[c] = zcol_first(col, cnt);
       sh.count[c] = cnt;
     }
     __syncthreads();
@@ -1273,7 +1266,7 @@ __device__ __forceinline__ void atx_zcol_walk(const ViewGeo &G, const Dims &D,
         const int mA = __reduce_max_sync(0xffffffffu, cA);
         const int mB = __reduce_max_sync(0xffffffffu, cA > 0 ? cB : 0);
         const int lo = sh.lo[c];
-        const int r0 = lo * D.nb + min(blo, D.nb - 1);  // the first pair's ray
+        const int r0 = zcol_first_ray(D, lo, blo);
         const bool special = cA > 0 && (flags & kZcSpecial);
         if (mA <= kZcCols && mB <= kZcRows && !any_lane(special)) {
           zcol_pairs<W>(G, D, tabC, yt, sh, v0, zc0, lsh, c, r0, mA, cA, cB, rz, hz, steep, acc,

@@ -88,3 +88,48 @@ def test_bounds_checked_build_sees_no_bad_index(gpu):
     out = json.loads(r.stdout.strip().splitlines()[-1])
     assert len(out["cases"]) == 11
     assert out["count"] == 0, out
+
+
+WIDE = r"""
+import ctypes as C, json, sys
+import numpy as np
+sys.path.insert(0, ROOT)
+import asd_pocs_mex_cuda_demo_gb300 as pkg
+from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+L = load()
+assert b"bounds-checked" in L.asdpocs_version()
+rng = np.random.default_rng(0)
+for (nx, ny, nz, na, nb) in [(128, 128, 72, 257, 200), (160, 160, 48, 400, 120),
+                             (256, 256, 40, 512, 256)]:
+    vx = 541.0 / 949.0 * na / nx
+    base = dict(SO=541.0, OD=408.0, vxlsize=vx, nx=nx, ny=ny, nz=nz, na=na, nb=nb, detsize=1.0)
+    y = rng.standard_normal(na * nb).astype(np.float32)
+    for a in (0.0, 27.0, 45.0, 60.0, 135.0, 222.0, 315.0):
+        x, sc = pkg.Atx_cone_gpu(y, dict(base, phi=-a / 180 * np.pi))
+        assert np.isfinite(x).all() and np.isfinite(sc).all()
+    phi = np.array([0.0, 27.0, 45.0, 135.0])
+    with pkg.Plan([dict(base, phi_vec=phi, maxnumIter=1, numOfgradients=1)], [phi]) as pl:
+        pl.set_sinogram(0, rng.random(na * nb * len(phi)).astype(np.float32))
+        pl.reset()
+        pl.run()
+        assert np.isfinite(np.asarray(pl.image(0))).all()
+cnt = C.c_ulonglong()
+first = (C.c_longlong * 2)()
+check(L.asdpocs_checked_errors(C.byref(cnt), first))
+print(json.dumps({"count": cnt.value, "first": [first[0], first[1]]}))
+"""
+
+
+def test_bounds_checked_build_on_wide_volumes(gpu):
+    """Volumes large enough for 32 columns a block with 8 and 16 lanes each,
+    partly outside the fan."""
+    from asd_pocs_mex_cuda_demo_gb300 import build
+
+    build.build(checked=True)
+    env = dict(os.environ, ASDPOCS_LIB="checked")
+    r = subprocess.run([sys.executable, "-c", f"ROOT = {ROOT!r}\n" + WIDE], env=env,
+                       capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stderr[-3000:]
+    out = json.loads(r.stdout.strip().splitlines()[-1])
+    assert out["count"] == 0, out

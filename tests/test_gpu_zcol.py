@@ -63,3 +63,77 @@ def test_columns_equal_voxels(gpu, case, angle):
     for a, b in ((0, 2), (1, 3), (4, 2), (5, 3)):
         assert torch.equal(out[a].view(torch.int32), out[b].view(torch.int32))
     assert float(out[1].abs().max()) > 0
+
+
+# A warp holds four (8 lanes) and two (16 lanes) voxel columns and the image
+# reaches past the fan, so that columns without rays sit beside columns with
+# some; nx, ny, nz, na, nb, SO, OD.
+CUT = [(128, 128, 72, 257, 200, 541.0, 408.0), (160, 160, 48, 400, 120, 541.0, 408.0)]
+
+
+def _fan(case):
+    nx, na, SO, OD = case[0], case[3], case[5], case[6]
+    return SO / (SO + OD) * na / nx  # voxel size at which the image fills the fan
+
+
+@pytest.mark.parametrize("case", CUT, ids=[str(c[:5]) for c in CUT])
+@pytest.mark.parametrize("angle", [27.0, 45.0, 135.0, 222.0, 315.0])
+def test_columns_beside_the_fan(gpu, case, angle):
+    """Host calls, whose workspace the call before left full of NaN, against
+    the device call and the per-voxel form (captured)."""
+    import torch
+
+    nx, ny, nz, na, nb, SO, OD = case
+    para = dict(SO=SO, OD=OD, vxlsize=_fan(case), nx=nx, ny=ny, nz=nz, na=na, nb=nb,
+                phi=-angle / 180 * np.pi, detsize=1.0)
+    y = np.random.default_rng(int(angle)).standard_normal(na * nb).astype(np.float32)
+    pkg.imgTVGradMin3D(np.full((nx, ny, nz), np.nan), 0.1, 1, 0)
+    x, sc = pkg.Atx_cone_gpu(y, para)
+    f, vx = np.float32, _fan(case)
+    T = lambda a: torch.tensor(np.asarray(a, f), device=gpu)  # noqa: E731
+    import oracle
+    g = oracle.gateway_geometry(para["phi"], SO, OD, vx, 1.0, na, nb)
+    yt, yd, zd = T(y), T(g["y_det"]), T(g["z_det"])
+    out = [torch.full((nx * ny * nz,), np.nan, device=gpu) for _ in range(4)]
+
+    def call(a, b):
+        check(load().asdpocs_atx_device(
+            C.c_void_p(a.data_ptr()), C.c_void_p(yt.data_ptr()), C.c_void_p(b.data_ptr()),
+            g["cos_phi"], g["sin_phi"], C.c_void_p(yd.data_ptr()), C.c_void_p(zd.data_ptr()),
+            g["SO"], g["OD"], g["scale"], g["det"], g["det"], 1.0, nx, ny, nz, na, nb,
+            C.c_void_p(torch.cuda.current_stream().cuda_stream or None)))
+
+    call(out[0], out[1])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(out[2], out[3])
+    graph.replay()
+    torch.cuda.synchronize()
+    want = [o.cpu().numpy() for o in out[2:]]
+    assert np.isfinite(want[0]).all() and (want[1] == 0).any() and (want[1] > 0).any()
+    for got in ((out[0].cpu().numpy(), out[1].cpu().numpy()), (x, sc)):
+        for a, b in zip(got, want):
+            assert np.array_equal(a.ravel(), b)
+
+
+@pytest.mark.parametrize("case", CUT, ids=[str(c[:5]) for c in CUT])
+def test_plan_of_columns_beside_the_fan(gpu, case, monkeypatch):
+    """The same in a plan whose first view is at 0 degrees (odd bins: a ray
+    along the axis, whose slopes are infinite): the per-voxel plan's image."""
+    nx, ny, nz, na, nb, SO, OD = case
+    phi = np.array([0.0, 27.0, 45.0, 135.0, 315.0])
+    para = dict(SO=SO, OD=OD, vxlsize=_fan(case), nx=nx, ny=ny, nz=nz, na=na, nb=nb, detsize=1.0,
+                phi_vec=phi, maxnumIter=2, numOfgradients=2, alpha=0.002)
+    P = np.random.default_rng(nz).random(na * nb * len(phi)).astype(np.float32)
+
+    def image():
+        with pkg.Plan([para], [phi]) as pl:
+            pl.set_sinogram(0, P)
+            pl.reset()
+            pl.run()
+            return np.asarray(pl.image(0))
+
+    got = image()
+    monkeypatch.setenv("ASDPOCS_CONE_ATX", "voxel")
+    want = image()
+    assert np.isfinite(want).all() and np.array_equal(got, want)
