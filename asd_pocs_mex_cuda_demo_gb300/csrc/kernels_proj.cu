@@ -282,8 +282,6 @@ __device__ __forceinline__ void atx_block_sum(const ViewGeo &G, const Dims &D,
                                               YLoad yl, float &acc,
                                               float &accl) {
   using Sh = AtxShared<kPlanar>;
-  // planar kernels verify the geometry they were chosen for (z_det == 0)
-  const bool planar_ok = !kPlanar || G.z_det[0] == 0.0f;
   VoxelWin w;
   w.a0 = 0;
   w.a1 = -1;
@@ -304,8 +302,11 @@ __device__ __forceinline__ void atx_block_sum(const ViewGeo &G, const Dims &D,
     const int b1 = __reduce_max_sync(0xffffffffu, has ? w.b1 : -1);
     if ((threadIdx.x & 31) == 0) sh.win[threadIdx.x / 32] = make_int4(a0, a1, b0, b1);
   }
-  // from here on memory that the stream's previous kernel may have written
+  // from here on memory that the stream's previous kernel may have written (the
+  // detector coordinates among it)
   pdl_enter();
+  // planar kernels verify the geometry they were chosen for (z_det == 0)
+  const float z0 = kPlanar ? G.z_det[0] : 0.0f;
   __syncthreads();
   int4 bw = sh.win[0];
 #pragma unroll
@@ -318,13 +319,13 @@ __device__ __forceinline__ void atx_block_sum(const ViewGeo &G, const Dims &D,
   acc = 0.f;
   accl = 0.f;
   if (bw.y < 0) return;  // no voxel of the block sees the detector
-  const bool staged = planar_ok && nA <= Sh::kA && (long long)nA * nB <= Sh::kC;
+  const bool fits = nA <= Sh::kA && (long long)nA * nB <= Sh::kC;
   // narrowing to the pixel shadow needs finite view values and rays with
   // both in-plane components (an axis-parallel ray's reference chord ignores
   // one coordinate and is 1 for every voxel of the window)
   bool narrow = true;
   bool allx = true, ally = true;  // every ray of the window x- / y-dominant
-  if (staged) {
+  if (fits) {  // z0 is on its way meanwhile
     narrow = G.dy_det > 0.0f && (kPlanar || G.dz_det > 0.0f);
     for (int k = threadIdx.x; k < nA; k += kAtxThreads) {
       const float yd = G.y_det[amin + k];
@@ -365,7 +366,7 @@ __device__ __forceinline__ void atx_block_sum(const ViewGeo &G, const Dims &D,
       __syncthreads();
     }
   }
-  if (!staged) {
+  if (!fits || z0 != 0.0f) {
     if (valid) voxel_backproject(G, D, w, yl, acc, accl);
     return;
   }

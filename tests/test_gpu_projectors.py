@@ -398,3 +398,45 @@ def test_small_host_calls_equal_large_ones(gpu, oracle_mod):
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_back_projection_waits_for_the_detector_rows(gpu, oracle_mod):
+    """A fan-beam Atx whose detector row lies where the kernel before it, which
+    lets its successor start early, writes it: 0, where the planar form holds,
+    and other heights in turn, the bits of synchronised calls."""
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    n, na, L = 64, 128, load()
+    g = oracle_mod.gateway_geometry(-0.4, 541.0, 408.0, 541.0 / 949.0 * na / n, 1.0, na, 1)
+    y = torch.rand(na, device="cuda")
+    yd = torch.from_numpy(np.ascontiguousarray(g["y_det"], np.float32)).cuda()
+    # one ray along a row of 8192 voxels: their sum goes to the detector row
+    long = [torch.full((8192,), v, device="cuda") for v in (0.0, 1e-4, 0.0, 2e-4, 3e-4)]
+    zero, row, sr = (torch.zeros(1, device="cuda") for _ in range(3))
+
+    def run(sync):
+        st, out = torch.cuda.current_stream().cuda_stream, []
+        for k in range(20):
+            x, sc = torch.empty(n * n, device="cuda"), torch.empty(n * n, device="cuda")
+            check(L.asdpocs_ax_device(long[k % 5].data_ptr(), row.data_ptr(), sr.data_ptr(), 1.0,
+                                      0.0, zero.data_ptr(), zero.data_ptr(), 9000.0, 9000.0, 1.0,
+                                      1.0, 8192, 1, 1, 1, 1, st))
+            if sync:
+                torch.cuda.synchronize()
+            check(L.asdpocs_atx_device(x.data_ptr(), y.data_ptr(), sc.data_ptr(), g["cos_phi"],
+                                       g["sin_phi"], yd.data_ptr(), row.data_ptr(), g["SO"],
+                                       g["OD"], g["scale"], g["det"], g["det"], 1.0, n, n, 1, na,
+                                       1, st))
+            if sync:
+                torch.cuda.synchronize()
+            out += [x, sc, row.clone()]
+        torch.cuda.synchronize()
+        return out
+
+    want = run(True)
+    assert len({float(r) for r in want[2::3]}) == 4
+    assert not torch.equal(want[0], want[3])  # the height matters
+    for a, b in zip(run(False), want):
+        assert torch.equal(a, b)
