@@ -58,19 +58,21 @@ __device__ __forceinline__ bool asd_in(long long i, long long n) {
 // serialization (launch_iter inside a PdlScope), so a kernel's launch and
 // block scheduling overlap the tail of the kernel before it.  Each such
 // kernel calls pdl_enter() before its first access to memory that an
-// iteration writes: it waits there until the preceding kernel has completed
-// and its writes are visible (so every kernel still sees all earlier ones),
-// then lets its own successor be scheduled -- once all of its blocks are resident, so the successor's
-// waiting blocks never take the slots of its own.  Before it, a kernel may
-// load what the plan wrote at its creation or before the run (descriptors,
-// geometry, chord tables, sinograms), which hides that latency behind the
-// kernel before.  It may also load what a kernel before the one it
-// waits for wrote, if the latter does not write it: that one's blocks have all
-// passed their own wait before this kernel starts.  Such loads go to the L2
-// (__ldcg): nothing orders the L1 before the wait.  Every block calls it, also one that then has nothing to do:
-// a grid whose blocks did not wait could end before its predecessor, and its
-// successor waits for it alone.  In a kernel launched the
-// ordinary way both instructions do nothing.  Plans that run sub-batches on
+// iteration, or the kernel before it, may write: it waits there until the
+// preceding kernel has completed and its writes are visible (so every kernel
+// still sees all earlier ones), then lets its own successor be scheduled --
+// once all of its blocks are resident, so the successor's waiting blocks never
+// take the slots of its own.  Before it, a kernel may load what the plan wrote
+// at its creation (descriptors, geometry, chord tables), which hides that
+// latency behind the kernel before.  It may also load what a kernel before the
+// one it waits for wrote, if the latter does not write it: that one's blocks
+// have all passed their own wait before this kernel starts.  (So the first
+// kernel of a run loads no sinogram before its wait: the kernel before it may
+// be the one that wrote it.)  Such loads go to the L2 (__ldcg): nothing orders
+// the L1 before the wait.  Every block calls it, also one that then has nothing
+// to do: a grid whose blocks did not wait could end before its predecessor, and
+// its successor waits for it alone.  In a kernel launched the ordinary way both
+// instructions do nothing.  Plans that run sub-batches on
 // concurrent streams (and the serving lanes) launch the ordinary way: there
 // the successor's early, waiting blocks hold SM slots the other stream's
 // kernels would use (measured 22 % slower at batch 64, against 4 % faster
@@ -235,11 +237,13 @@ struct Inst {
   Scalars *s;
 };
 
-// Sinogram value i of an instance, widened to FP32 from its storage.
+// Sinogram value i of an instance, widened to FP32 from its storage.  From the
+// L2: forward steps read it before their wait (pdl_enter).
 __device__ __forceinline__ float sino_at(const Inst &I, long long i) {
-  if (I.p_fmt == ASDPOCS_STORE_F16) return __half2float(((const __half *)I.P)[i]);
-  if (I.p_fmt == ASDPOCS_STORE_BF16) return __bfloat162float(((const __nv_bfloat16 *)I.P)[i]);
-  return ((const float *)I.P)[i];
+  if (I.p_fmt == ASDPOCS_STORE_F16) return __half2float(__ldcg((const __half *)I.P + i));
+  if (I.p_fmt == ASDPOCS_STORE_BF16)
+    return __bfloat162float(__ldcg((const __nv_bfloat16 *)I.P + i));
+  return __ldcg((const float *)I.P + i);
 }
 
 // Bytes of one stored sinogram value.

@@ -551,7 +551,10 @@ __global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
   float p = 0.f;
   bool done = true;
   const float *m = nullptr;
-  if (have) {  // geometry and sinogram, before the wait
+  // The geometry is read before the wait, and after a sweep's first view the
+  // sinogram too: whatever wrote that before the run (a kernel of the caller's
+  // may, through asdpocs_plan_sinogram_ptr) is the kernel that view 0 waits for.
+  if (have) {
     if (!kVol) {
       m = I.m;
       // set, if at all, by the kernels between two sweeps
@@ -567,10 +570,11 @@ __global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
     }
     own = lane < (kVol ? kAxRows : 1) && ib + lane < D.nb;
     r = (long long)(ib + lane) * D.na + ia;
-    if (own) p = ray_value(I, view, r, nr);
+    if (own && view > 0) p = ray_value(I, view, r, nr);
   }
   pdl_enter();
   if (!have) return;
+  if (own && view == 0) p = ray_value(I, view, r, nr);
   if (kVol || view == 0) done = ((volatile int *)&I.s->done)[0] != 0;
   const bool tabc = k3D && (I.tabc_mode == kTabcShared || (!done && I.tabc_mode == kTabcOwn));
   const long long q = k3D && I.rays_t ? (long long)ia * D.nb + ib + lane : r;

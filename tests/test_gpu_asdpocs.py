@@ -853,3 +853,55 @@ def test_exact_mode_rays_per_warp_do_not_change_results(gpu, dims, batches):
             first = images[0]
             assert np.abs(first).max() > 0
         assert np.array_equal(images[0], first)
+
+
+@pytest.mark.parametrize("dims", [(64, 64, 1, 130, 1), (24, 20, 12, 48, 24)])
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+def test_sinogram_written_by_the_kernel_before_the_run(gpu, oracle_mod, dims, storage):
+    """Projections computed on the plan's stream straight into its sinogram
+    (the first view's last, by a kernel that lets its successor start early),
+    or a device sinogram rounded to FP16 there, and the run next on the stream:
+    the images of a run that synchronises first."""
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    nx, ny, nz, na, nb = dims
+    L, N, M, phi = load(), nx * ny * nz, na * nb, phantoms.views(4)
+    vx = 541.0 / 949.0 * na / nx
+    para = dict(SO=541.0, OD=408.0, vxlsize=vx, nx=nx, ny=ny, nz=nz, na=na, nb=nb, detsize=1.0,
+                phi_vec=phi, maxnumIter=1, numOfgradients=1, sino_storage=storage)
+    geo = [oracle_mod.gateway_geometry(-a / 180 * np.pi, 541.0, 408.0, vx, 1.0, na, nb)
+           for a in phi]
+    T = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()  # noqa: E731
+    yd, zd = T(geo[0]["y_det"]), T(geo[0]["z_det"])
+    xs = [torch.rand(N, generator=torch.Generator("cuda").manual_seed(k), device="cuda")
+          for k in range(3)]
+    sr, P = torch.empty(M, device="cuda"), torch.empty(M * len(phi), device="cuda")
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with pkg.Plan(para, phi, stream=st.cuda_stream) as pl:
+        into = L.asdpocs_plan_sinogram_ptr(pl._h, 0) if storage == "f32" else P.data_ptr()
+
+        def images(sync):
+            out = []
+            for x in xs * 2:
+                pl.reset()
+                for v in reversed(range(len(phi))):
+                    g = geo[v]
+                    check(L.asdpocs_ax_device(x.data_ptr(), into + 4 * M * v, sr.data_ptr(),
+                                              g["cos_phi"], g["sin_phi"], yd.data_ptr(),
+                                              zd.data_ptr(), g["SO"], g["OD"], g["scale"], 1.0,
+                                              *dims, st.cuda_stream))
+                if storage != "f32":
+                    pl.set_sinogram(0, P.data_ptr())
+                if sync:
+                    st.synchronize()
+                pl.run(use_graph=False, sync=False)
+                out.append(pl.image(0))
+            return out
+
+        want = images(True)
+        assert np.abs(want[0] - want[1]).max() > 0
+        for a, b in zip(images(False), want):
+            assert np.array_equal(a, b)
