@@ -142,6 +142,21 @@ static cudaMemPool_t scratch_pool() {
   return pools[dev];
 }
 
+// Scratch from that pool, in the order of st; false (nothing pending, so that an
+// error the caller has not yet read stays where it is) where st is being
+// captured or there is no memory.
+static bool scratch_alloc(void **p, size_t bytes, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+  cudaError_t e = cudaStreamIsCapturing(st, &cap);
+  if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) return false;
+  if (e == cudaSuccess) {
+    const cudaMemPool_t pool = scratch_pool();
+    if (pool && cudaMallocFromPoolAsync(p, bytes, pool, st) == cudaSuccess) return true;
+  }
+  cudaGetLastError();  // of the call above that failed
+  return false;
+}
+
 static inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Host arrays of one synchronous projector call.  A copy between pageable
@@ -321,13 +336,9 @@ int asdpocs_atx_device(float *x_d, const float *y_d, float *sc_d,
   // same bits, below that (six views: 48^2 x 30 0.08 ms against 0.10, 64^3 0.155
   // against 0.142), where the stream is being captured (a graph with allocations
   // of its own would run in fewer places) or no memory is left.
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
-  if (zcol_fits(d) && (long long)nx * ny * nz >= kZcolVoxels &&
-      cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+  if (zcol_fits(d) && (long long)nx * ny * nz >= kZcolVoxels) {
     void *scratch = nullptr;
-    const cudaMemPool_t pool = scratch_pool();
-    if (pool && cudaMallocFromPoolAsync(&scratch, atx_zcol_scratch_bytes(d), pool, st) ==
-                    cudaSuccess) {
+    if (scratch_alloc(&scratch, atx_zcol_scratch_bytes(d), st)) {
       const cudaError_t e = launch_atx_zcol(x_d, y_d, sc_d, g, d, scratch, st);
       const cudaError_t f = cudaFreeAsync(scratch, st);
       ASD_CUDA(e);
@@ -335,7 +346,6 @@ int asdpocs_atx_device(float *x_d, const float *y_d, float *sc_d,
       return 0;
     }
   }
-  cudaGetLastError();  // neither failure above is sticky
   ASD_CUDA(launch_atx(x_d, y_d, sc_d, g, d, st));
   return 0;
 }

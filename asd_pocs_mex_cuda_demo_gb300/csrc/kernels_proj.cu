@@ -2066,16 +2066,18 @@ cudaError_t launch_atx_zcol(float *x, const float *y, float *sc, const ViewGeo &
   float4 *tabC = (float4 *)(b + zcol_align((size_t)d.na * sizeof(float4)));
   float *yt = (float *)((char *)tabC + zcol_align((size_t)nr * sizeof(float4)));
   int *flag = (int *)((char *)yt + zcol_align((size_t)nr * sizeof(float)));
+  // launches that report their own errors only, in the ordinary way (neither
+  // kernel waits for the one before it)
+  const PdlScope scope(false);
   cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), st);
-  if (e != cudaSuccess) return e;
-  k_view_tab3<<<(unsigned)((nr + 255) / 256), 256, 0, st>>>(y, tabA, tabC, yt, flag, g, d);
+  if (e == cudaSuccess)
+    e = launch_iter(k_view_tab3, dim3((unsigned)((nr + 255) / 256)), dim3(256), st, y, tabA, tabC,
+                    yt, flag, g, d);
   const ZColShape s = zcol_shape(d, 1, 0);
-  const dim3 grid = zcol_grid(d, 1, s);
-  if (s.W == 32)
-    k_atx_zcol<32><<<grid, kZcThreads, 0, st>>>(x, sc, tabA, tabC, yt, flag, g, d, s.lsh(), s.seg);
-  else
-    k_atx_zcol<8><<<grid, kZcThreads, 0, st>>>(x, sc, tabA, tabC, yt, flag, g, d, s.lsh(), s.seg);
-  return cudaGetLastError();
+  if (e == cudaSuccess)
+    e = launch_iter(s.W == 32 ? k_atx_zcol<32> : k_atx_zcol<8>, zcol_grid(d, 1, s),
+                    dim3(kZcThreads), st, x, sc, tabA, tabC, yt, flag, g, d, s.lsh(), s.seg);
+  return e;
 }
 
 cudaError_t launch_sart_ax(const Inst *insts, int batch, const Dims &d,

@@ -440,3 +440,40 @@ def test_back_projection_waits_for_the_detector_rows(gpu, oracle_mod):
     assert not torch.equal(want[0], want[3])  # the height matters
     for a, b in zip(run(False), want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dims", [(32, 32, 1, 64, 1), (16, 16, 8, 32, 16), (64, 64, 64, 128, 128)])
+def test_back_projection_leaves_the_callers_error(gpu, oracle_mod, dims):
+    """An error of a call of the caller's own that it has not yet read (here a
+    device number that does not exist) is still there after asdpocs_atx_device."""
+    import ctypes
+
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    nx, ny, nz, na, nb = dims
+    rt = ctypes.CDLL("libcudart.so.13")  # the one the library is linked to
+    g = oracle_mod.gateway_geometry(-0.4, 541.0, 408.0, 541.0 / 949.0 * na / nx, 1.0, na, nb)
+    x, sc = torch.empty(nx * ny * nz, device="cuda"), torch.empty(nx * ny * nz, device="cuda")
+    y = torch.rand(na * nb, device="cuda")
+    yd, zd = (torch.from_numpy(np.ascontiguousarray(g[k], np.float32)).cuda()
+              for k in ("y_det", "z_det"))
+    st = torch.cuda.current_stream().cuda_stream
+
+    def call():
+        check(load().asdpocs_atx_device(x.data_ptr(), y.data_ptr(), sc.data_ptr(), g["cos_phi"],
+                                        g["sin_phi"], yd.data_ptr(), zd.data_ptr(), g["SO"],
+                                        g["OD"], g["scale"], g["det"], g["det"], 1.0, *dims, st))
+
+    call()
+    torch.cuda.synchronize()
+    want, err = (x.clone(), sc.clone()), rt.cudaSetDevice(9999)
+    assert err != 0
+    try:
+        call()
+        assert rt.cudaPeekAtLastError() == err
+    finally:
+        rt.cudaGetLastError()
+    torch.cuda.synchronize()
+    assert torch.equal(x, want[0]) and torch.equal(sc, want[1])
