@@ -142,6 +142,15 @@ static cudaMemPool_t scratch_pool() {
   return pools[dev];
 }
 
+// While one lives, this thread's calls may allocate although a stream other than
+// theirs is being captured (by another thread, or by this one): that capture would
+// end as invalid otherwise.
+struct AllocDuringCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  AllocDuringCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~AllocDuringCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Scratch from that pool, in the order of st; false (nothing pending, so that an
 // error the caller has not yet read stays where it is) where st is being
 // captured or there is no memory.
@@ -337,6 +346,7 @@ int asdpocs_atx_device(float *x_d, const float *y_d, float *sc_d,
   // against 0.142), where the stream is being captured (a graph with allocations
   // of its own would run in fewer places) or no memory is left.
   if (zcol_fits(d) && (long long)nx * ny * nz >= kZcolVoxels) {
+    const AllocDuringCapture relaxed;
     void *scratch = nullptr;
     if (scratch_alloc(&scratch, atx_zcol_scratch_bytes(d), st)) {
       const cudaError_t e = launch_atx_zcol(x_d, y_d, sc_d, g, d, scratch, st);

@@ -477,3 +477,51 @@ def test_back_projection_leaves_the_callers_error(gpu, oracle_mod, dims):
         rt.cudaGetLastError()
     torch.cuda.synchronize()
     assert torch.equal(x, want[0]) and torch.equal(sc, want[1])
+
+
+def test_back_projection_beside_another_threads_capture(gpu, oracle_mod):
+    """asdpocs_atx_device on one thread, with the scratch of its z-column form,
+    while another thread captures a stream of its own: the capture stays valid,
+    and the results are those of a call alone."""
+    import threading
+
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    n, na = 64, 128
+    N = n ** 3
+    g = oracle_mod.gateway_geometry(-0.4, 541.0, 408.0, 541.0 / 949.0 * na / n, 1.0, na, na)
+    y = torch.rand(na * na, device="cuda")
+    yd, zd = (torch.from_numpy(np.ascontiguousarray(g[k], np.float32)).cuda()
+              for k in ("y_det", "z_det"))
+    out = [torch.empty(N, device="cuda") for _ in range(4)]
+    a = torch.ones(1000, device="cuda")
+    other, errors = torch.cuda.Stream(), []
+    torch.cuda.synchronize()
+
+    def call(x, sc):
+        try:
+            check(load().asdpocs_atx_device(x.data_ptr(), y.data_ptr(), sc.data_ptr(),
+                                            g["cos_phi"], g["sin_phi"], yd.data_ptr(),
+                                            zd.data_ptr(), g["SO"], g["OD"], g["scale"], g["det"],
+                                            g["det"], 1.0, n, n, n, na, na, other.cuda_stream))
+        except Exception as e:  # the test reports it
+            errors.append(e)
+
+    call(out[0], out[1])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        a.mul_(2.0)
+        for _ in range(2):
+            t = threading.Thread(target=call, args=(out[2], out[3]))
+            t.start()
+            t.join()
+        call(out[2], out[3])  # and on the capturing thread
+        a.add_(1.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert not errors
+    assert float(a[0]) == 3.0
+    assert torch.equal(out[0], out[2]) and torch.equal(out[1], out[3])
