@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kTvT, (kTvResident<T, k3D>))
   const long long plane = (long long)g.nx * g.ny;
   const long long nvox = plane * g.nz;
   T coef = T(0);
-  double sum[2] = {0.0, 0.0};  // u^2, distance^2 (FP32: lane 0 of each warp)
+  double sum[2] = {0.0, 0.0};  // u^2, distance^2
   bool sized = kFirst;
   for (int item = blockIdx.x; item < g.items; item += gridDim.x) {
     const int tile = item % (g.tx * g.ty), z0 = item / (g.tx * g.ty) * g.slab;
@@ -287,25 +287,34 @@ __global__ void __launch_bounds__(kTvT, (kTvResident<T, k3D>))
                                     k3D ? c - P[q0][ey][ex] : T(0), dummy);
       }
     };
-    float accf[2] = {0.f, 0.f};
+    // a slice's rows are added in T; in FP32 the slices then with each addition's
+    // rounding error kept (Dekker 1971), so that an item's sum carries no more
+    // roundings than its rows'
+    float accf[2] = {0.f, 0.f}, lost[2] = {0.f, 0.f};
     auto add = [&](int k, T v) {
-      if (sizeof(T) == 8)
-        sum[k] += (double)v;
-      else
-        accf[k] += (float)v;
+      if constexpr (sizeof(T) == 8) {
+        sum[k] += v;
+      } else {
+        const float a = __fadd_rn(accf[k], v);
+        lost[k] = __fadd_rn(lost[k], __fsub_rn(v, __fsub_rn(a, accf[k])));
+        accf[k] = a;
+      }
     };
     auto distance = [&]() {
-      if (kFirst)
+      if (kFirst) {
+        T d2 = T(0);
 #pragma unroll
-        for (int j = 0; j < kR; j++)
-          if (j < rows) {
-            const T d = cm[j] - cu[j];
-            add(1, d * d);
-          }
+        for (int j = 0; j < kR; j++) {  // zeros past the image
+          const T d = cm[j] - cu[j];
+          d2 += d * d;
+        }
+        add(1, d2);
+      }
     };
     // u of the slice c in P[q], R[r]; `above`: the term of the slice above
     auto emit = [&](int q, int r, const T (&c)[kR], const T (&own)[kR], const T (&s)[kR],
                     const T (&above)[kR]) {
+      T u2 = T(0);
 #pragma unroll
       for (int j = 0; j < kR; j++) {
         const T yp = j + 1 < kR ? c[j + 1 < kR ? j + 1 : j] : P[q][ly + kR + 1][lx + 1];
@@ -318,8 +327,9 @@ __global__ void __launch_bounds__(kTvT, (kTvResident<T, k3D>))
         if (j >= rows || !ASD_IN(i, nvox)) continue;
         uout[i] = u;
         if (!kFirst) mout[i] = c[j];
-        add(0, u * u);
+        u2 += u * u;
       }
+      add(0, u2);
       wo += plane;
     };
     T c[kR], own[kR], s[kR], n[kR], own1[kR], s1[kR], above[kR];
@@ -365,20 +375,15 @@ __global__ void __launch_bounds__(kTvT, (kTvResident<T, k3D>))
         q = q1;
       }
     }
-    if (sizeof(T) == 4) {  // an item's FP32 sums join the FP64 ones per warp
+    if (sizeof(T) == 4)
 #pragma unroll
-      for (int k = 0; k < (kFirst ? 2 : 1); k++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) accf[k] += __shfl_xor_sync(0xffffffffu, accf[k], o);
-        if (lx == 0) sum[k] += (double)accf[k];
-      }
-    }
+      for (int k = 0; k < (kFirst ? 2 : 1); k++)  // an infinite sum has no error to add
+        sum[k] += (double)accf[k] + (isinf(accf[k]) ? 0.0 : (double)lost[k]);
   }
 #pragma unroll
   for (int k = 0; k < (kFirst ? 2 : 1); k++) {
-    if (sizeof(T) == 8)
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+    for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
     if (lx == 0) red[k][wy] = sum[k];
   }
   __syncthreads();

@@ -106,3 +106,42 @@ def test_tv_noalloc_large_image(gpu):
     check(load().asdpocs_tv_device_noalloc(b.data_ptr(), old.data_ptr(), 1000, 1001, 1, 0.1, 4, 1,
                                            s))
     assert rel_l2(b.cpu().numpy(), a.cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("level", [1.4130100011825562, 1.4100697040557861, 1.0])
+def test_tv_fp32_step_length_of_a_long_slab(gpu, level):
+    """One FP32 step moves the image by alpha ||m - old||, whatever the stencil,
+    so the length shows the two sums behind the step size.  The image is constant
+    (equal squares, whose roundings add up instead of cancelling) and a slab has
+    64 slices.  Bound, in units of 2^-24: a thread's four rows and their squares
+    are rounded four times in each sum and the root halves that, 4; the step size,
+    the product and the difference 3; 7 x 6e-8 = 4.2e-7."""
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    nx, ny, nz, alpha = 640, 960, 64, 10.0
+    m = torch.full((nx * ny * nz,), level, dtype=torch.float32, device=gpu)
+    old = torch.zeros_like(m)
+    want = alpha * float(torch.linalg.vector_norm(m.double()))
+    out = m.clone()
+    check(load().asdpocs_tv_device(out.data_ptr(), old.data_ptr(), nx, ny, nz, alpha, 1, 0,
+                                   torch.cuda.current_stream().cuda_stream))
+    got = float(torch.linalg.vector_norm(out.double() - m.double()))
+    assert abs(got / want - 1) < 4.2e-7, got / want - 1
+
+
+def test_tv_fp32_infinite_distance(gpu):
+    """A distance whose square overflows FP32 gives an infinite step, not NaN:
+    voxels with a positive derivative go to -inf and positivity makes them 0."""
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    for dims in ((40, 33, 1), (40, 33, 9)):
+        n = dims[0] * dims[1] * dims[2]
+        m = torch.rand(n, device=gpu, generator=torch.Generator(gpu).manual_seed(1))
+        old = torch.full_like(m, -3e19)
+        check(load().asdpocs_tv_device(m.data_ptr(), old.data_ptr(), *dims, 0.1, 1, 1,
+                                       torch.cuda.current_stream().cuda_stream))
+        assert bool((torch.isinf(m) | (m == 0)).all())
