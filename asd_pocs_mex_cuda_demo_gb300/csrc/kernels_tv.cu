@@ -421,7 +421,11 @@ __global__ void __launch_bounds__(kTvT)
 // share, so the busiest SM's slices count (128^3: 7 slices, two items on
 // every SM; 15 slices and one item: 114 us a step, 8 and an uneven share:
 // 122 us); FP32 steps by latency, so a block's slices do (256^3: 29 slices in
-// 576 blocks; 37 in 448 blocks: 72 us, 32 in 512: 64 us).
+// 576 blocks; 37 in 448 blocks: 72 us, 32 in 512: 64 us).  FP64 volumes of few
+// tiles have an item per slice, so that a step is two slices long: 32^3 15 us a
+// step, 22 with two slices an item, 29 with three, 36 with four, and 27 with the
+// two kernels that each took all voxels at once (64x64x16 the same; 48^3 23, 22,
+// 29, 37 and 74).  FP32 volumes stay at four: 96^3 9.0 us against 9.9 with one.
 template <class T, bool k3D>
 TvGrid tv_grid(int nx, int ny, int nz, int &blocks) {
   constexpr int kY = kTvY<k3D>;
@@ -431,7 +435,7 @@ TvGrid tv_grid(int nx, int ny, int nz, int &blocks) {
   long long count = tiles;
   if (k3D) {
     long long best = 0;
-    for (int s = 4; s <= 64; s++) {
+    for (int s = sizeof(T) == 8 ? 1 : 4; s <= 64; s++) {
       const long long n = tiles * ((nz + s - 1) / s), b = std::min(n, resident);
       const long long items = (n + b - 1) / b, per_sm = (b + 151) / 152;
       const long long cost = sizeof(T) == 8 ? items * per_sm * (std::min(s, nz) + 1)

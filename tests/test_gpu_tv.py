@@ -145,3 +145,12 @@ def test_tv_fp32_infinite_distance(gpu):
         check(load().asdpocs_tv_device(m.data_ptr(), old.data_ptr(), *dims, 0.1, 1, 1,
                                        torch.cuda.current_stream().cuda_stream))
         assert bool((torch.isinf(m) | (m == 0)).all())
+
+
+@pytest.mark.parametrize("shape", [(31, 33, 24), (64, 64, 60), (40, 40, 301), (64, 64, 200)])
+def test_tv3d_fp64_slab_lengths(gpu, oracle_mod, shape):
+    """FP64 volumes whose items have one, two, eight and six slices."""
+    rng = np.random.default_rng(shape[2])
+    img, old = rng.random(shape), rng.random(shape)
+    out = pkg.imgTVGradMin3D(img, 0.1, 3, 1, old)
+    assert rel_l2(out, oracle_mod.tv(img, 0.1, 3, 1, old)) < 1e-12
