@@ -118,7 +118,6 @@ static int ws_acquire(Workspace *&w, size_t bytes, std::unique_lock<std::mutex> 
 // for it to be mapped again (a 64^3 view 194 us, 35 with this pool).  Null where
 // there is none.
 constexpr unsigned long long kScratchKeep = 32 << 20;
-constexpr long long kZcolVoxels = 1 << 18;  // see asdpocs_atx_device
 static cudaMemPool_t scratch_pool() {
   static std::mutex mu;
   static cudaMemPool_t pools[64];
@@ -339,13 +338,12 @@ int asdpocs_atx_device(float *x_d, const float *y_d, float *sc_d,
                                            dy_det, dz_det, dz, y_det_d, z_det_d});
   Dims d{nx, ny, nz, na, nb};
   const cudaStream_t st = (cudaStream_t)stream;
-  // Cone beams of at least 2^18 voxels: the z-column form, its ray tables in
-  // stream-ordered memory (256^3 on a 512^2 detector: 0.39 ms a view against
-  // 0.90 per voxel).  The per-voxel form, which needs no scratch and gives the
-  // same bits, below that (six views: 48^2 x 30 0.08 ms against 0.10, 64^3 0.155
-  // against 0.142), where the stream is being captured (a graph with allocations
-  // of its own would run in fewer places) or no memory is left.
-  if (zcol_fits(d) && (long long)nx * ny * nz >= kZcolVoxels) {
+  // The z-column form, its ray tables in stream-ordered memory, where it is the
+  // faster one (256^3 on a 512^2 detector: 0.39 ms a view against 0.90 per voxel).
+  // The per-voxel form, which needs no scratch and gives the same bits, elsewhere,
+  // where the stream is being captured (a graph with allocations of its own would
+  // run in fewer places) and where no memory is left.
+  if (atx_columns(g, d)) {
     const AllocDuringCapture relaxed;
     void *scratch = nullptr;
     if (scratch_alloc(&scratch, atx_zcol_scratch_bytes(d), st)) {
@@ -484,7 +482,9 @@ int asdpocs_adjoint_check(const float *X, const float *yv, float cos_phi, float 
     return set_error(ASDPOCS_ERR_ARG, "null pointer");
   const size_t N = (size_t)nx * ny * nz, M = (size_t)na * nb;
   const Dims d{nx, ny, nz, na, nb};
-  const size_t zs = zcol_fits(d) ? atx_zcol_scratch_bytes(d) : 0;
+  ViewGeo g = with_constants(
+      ViewGeo{cos_phi, sin_phi, SO, OD, scale, dy_det, dz_det, dz, nullptr, nullptr});
+  const size_t zs = atx_columns(g, d) ? atx_zcol_scratch_bytes(d) : 0;
   const size_t oX = 0, oY = oX + align256(N * 4), oAx = oY + align256(M * 4),
                oSr = oAx + align256(M * 4), oAty = oSr + align256(M * 4),
                oSc = oAty + align256(N * 4), oA = oSc + align256(N * 4),
@@ -498,9 +498,8 @@ int asdpocs_adjoint_check(const float *X, const float *yv, float cos_phi, float 
   ASD_CUDA(cudaMemcpyAsync(b + oY, yv, M * 4, cudaMemcpyHostToDevice, w->st));
   ASD_CUDA(cudaMemcpyAsync(b + oA, y_det, (size_t)na * 4, cudaMemcpyHostToDevice, w->st));
   ASD_CUDA(cudaMemcpyAsync(b + oB, z_det, (size_t)nb * 4, cudaMemcpyHostToDevice, w->st));
-  const ViewGeo g = with_constants(ViewGeo{cos_phi, sin_phi, SO, OD, scale, dy_det, dz_det,
-                                           dz, (const float *)(b + oA),
-                                           (const float *)(b + oB)});
+  g.y_det = (const float *)(b + oA);
+  g.z_det = (const float *)(b + oB);
   ASD_CUDA(launch_ax((const float *)(b + oX), (float *)(b + oAx), (float *)(b + oSr), g, d,
                      w->st));
   if (zs)
@@ -804,10 +803,11 @@ struct asdpocs_plan_s {
   std::vector<int> slot;
   std::vector<Inst> h_dev;  // mixed plans: the descriptors in d_inst order
   std::vector<size_t> phi_off;  // each instance's first angle in phi_vec_deg
-  bool zcol = true;     // cone beams: z-column backward step (else per voxel)
+  asd::ConeForm cone = asd::kConeVoxels;  // cone beams: form of the backward step
+  int seen = 0;         // slices a view crosses, the most of the instances
   bool exact = false;   // forward steps: exact Siddon projection (ax_mode)
   int tv_walk = 0;      // TV walk length (0: from the batch size)
-  int zseg = 0;         // slices of a z-column block (0: the default)
+  int zseg = 0;         // slices of a block or thread of that step (0: the default)
   int ax_u = 0, ax_q = 0;  // shared forward step's shape (0: the defaults)
   int pdl = -1;         // programmatic dependent launches: -1 = when the plan
                         // runs on one stream, 0 = off, 1 = on
@@ -1057,7 +1057,7 @@ cudaError_t enqueue_iteration(const Inst *d_inst, int batch, const Dims &d,
       continue;
     }
     e = launch_sart_ax(d_inst, vb, vd, v, st, sh.exact, zmap);
-    if (e == cudaSuccess) e = launch_sart_atx(d_inst, vb, vd, v, st, sh.zcol, sh.zseg, zmap);
+    if (e == cudaSuccess) e = launch_sart_atx(d_inst, vb, vd, v, st, sh.cone, sh.zseg, sh.seen, zmap);
   }
   if (shared && e == cudaSuccess) e = launch_group_pack(d_inst, batch, d, 1, st, gall, ngroups);
   if (e == cudaSuccess) e = launch_after_sweep(d_inst, batch, d, st, zall);
@@ -1071,8 +1071,9 @@ cudaError_t enqueue_iteration(const Inst *d_inst, int batch, const Dims &d,
 static IterShape plan_shape(asdpocs_plan p) {
   IterShape sh;
   sh.tv_walk = p->tv_walk;
-  sh.zcol = p->zcol;
+  sh.cone = p->cone;
   sh.zseg = p->zseg;
+  sh.seen = p->seen;
   sh.ax_u = p->ax_u;
   sh.ax_q = p->ax_q;
   sh.pdl = p->pdl < 0 ? p->subs.size() == 1 : p->pdl == 1;
@@ -1437,14 +1438,21 @@ static int plan_describe(asdpocs_plan *out, int batch, const asdpocs_geometry *g
       }
     }
   }
-  // ASDPOCS_CONE_ATX=voxel: the per-voxel form of the cone-beam backward step
-  // (same results; kept for comparison)
-  {
+  // the form of the cone-beam backward step, which every instance takes;
+  // ASDPOCS_CONE_ATX=voxel, columns or walk: that one (same results)
+  if (dmax.nz > 1) {
+    for (int i = 0; i < batch; i++) {
+      const asdpocs_geometry &gi = geom[i];
+      const float s = (float)gi.vxlsize, det = (float)gi.detsize / s;
+      const ViewGeo v = with_constants(ViewGeo{1.f, 0.f, (float)gi.SO / s, (float)gi.OD / s, s, det,
+                                               det, 1.0f, nullptr, nullptr});
+      p->seen = std::max(p->seen, seen_slices(v, Dims{gi.nx, gi.ny, gi.nz, gi.na, gi.nb}));
+    }
+    p->cone = cone_form(dmax, batch, p->seen);
     const char *f = getenv("ASDPOCS_CONE_ATX");
-    p->zcol = !(f && strcmp(f, "voxel") == 0);
-    for (int i = 0; i < batch; i++)
-      p->zcol = p->zcol && (geom[i].nz == 1 || zcol_fits(Dims{geom[i].nx, geom[i].ny, geom[i].nz,
-                                                              geom[i].na, geom[i].nb}));
+    if (f && strcmp(f, "voxel") == 0) p->cone = kConeVoxels;
+    if (f && strcmp(f, "walk") == 0) p->cone = kConeWalk;
+    if (f && strcmp(f, "columns") == 0 && zcol_fits(dmax)) p->cone = kConeColumns;
   }
   *out = p;
   return 0;
@@ -1650,7 +1658,7 @@ int asdpocs_plan_create(asdpocs_plan *out, int batch,
   for (int i = 0; i < batch && e == cudaSuccess; i++) {
     Inst &I = p->h_inst[i];
     e = bind_instance(I, b + base[i], lay[i], geom[i], phi_vec_deg + p->phi_off[i], p->st);
-    I.rays_t = !p->shared && p->zcol && geom[i].nz > 1;
+    I.rays_t = !p->shared && p->cone == kConeColumns;
     if (p->mixed) {
       const int g = group_first[i];
       I.cor = (float *)(b + base[g] + lay[g].cor) + (p->slot[i] - p->slot[g]);
@@ -2005,7 +2013,7 @@ int asdpocs_plan_time_phase(asdpocs_plan p, int phase, int reps,
       return e;
     }
     return p->shared ? launch_sart_atx_shared(p->d_inst, p->batch, p->d, v, p->st)
-                     : launch_sart_atx(p->d_inst, p->batch, p->d, v, p->st, sh.zcol, sh.zseg);
+                     : launch_sart_atx(p->d_inst, p->batch, p->d, v, p->st, sh.cone, sh.zseg, sh.seen);
   };
   auto launch = [&](int i) -> cudaError_t {
     switch (phase) {
@@ -2216,8 +2224,10 @@ int asdpocs_plan_autotune_shapes(asdpocs_plan p, int reps, asdpocs_shapes *out) 
     rc = pick(0, &uq, cand);
     p->ax_u = uq / 4;
     p->ax_q = uq % 4;
-  } else if (p->d.nz > 1 && p->zcol) {
+  } else if (p->cone == kConeColumns) {
     rc = pick(1, &p->zseg, {0, 32, 64, 128, 256});  // slices of a z-column block (0: by size)
+  } else if (p->cone == kConeWalk) {
+    rc = pick(1, &p->zseg, {0, 4, 8, 16, 32});  // slices of a thread (0: by size)
   }
   double t_best = 0.0;
   // programmatic launches only where the plan runs on one stream (PdlScope)

@@ -84,8 +84,9 @@ cudaError_t reset_instance(const Inst &I, const Scalars &s, cudaStream_t st);
 // projection (a mode: different results).
 struct IterShape {
   int tv_walk = 0;          // TV walk length (0: the batch-size rule)
-  bool zcol = true;         // cone beams: z-column backward step (else per voxel)
-  int zseg = 0;             //   its segment length in voxels (0: the default)
+  ConeForm cone = kConeVoxels;  // cone beams: form of the backward step,
+  int zseg = 0;             //   its slices of a block or thread (0: the default),
+  int seen = 0;             //   and the slices a view crosses (0: all)
   int ax_u = 0, ax_q = 0;   // shared forward step: columns of loads per round,
                             //   quads of instances per lane (0: the defaults)
   bool pdl = false;         // programmatic dependent launches (work alone on

@@ -24,6 +24,17 @@ size_t atx_zcol_scratch_bytes(const Dims &d);
 // Whether the z-column form takes these sizes (nz > 1, and its ray indices
 // with their padding fit an int).
 bool zcol_fits(const Dims &d);
+// Forms of the cone-beam backward step, the same to the last bit: a thread per
+// voxel (k_sart_atx), warps along voxel columns (k_sart_atx_zcol), a thread per
+// segment of a column (k_sart_atx_zwalk).
+enum ConeForm { kConeVoxels, kConeColumns, kConeWalk };
+// Slices that a view's rays cross, about (2 to nz; at the axis' magnification).
+int seen_slices(const ViewGeo &g, const Dims &d);
+// The form of a launch of `batch` instances of at most these sizes, of which a
+// view crosses at most `seen` slices.
+ConeForm cone_form(const Dims &d, int batch, int seen);
+// Whether one view by itself is faster through launch_atx_zcol than launch_atx.
+bool atx_columns(const ViewGeo &g, const Dims &d);
 // Zeros that must follow the na * nb rays of Inst::cor and Inst::tabC where
 // the z-column step reads them (Inst::rays_t).
 size_t ray_table_pad(const Dims &d);
@@ -57,12 +68,13 @@ cudaError_t launch_store_sinogram(const float *src, void *dst, size_t n, int fmt
 cudaError_t launch_sart_ax(const Inst *insts, int batch, const Dims &d,
                            int view, cudaStream_t st, bool exact = false,
                            const int *zmap = nullptr);
-// Cone beams (nz > 1) run in voxel columns (k_sart_atx_zcol), `zseg` slices a
-// block (rounded up to whole lanes; 0: the default), unless `zcol` is false (the per-voxel form;
-// bit-identical).  `zmap` as for launch_sart_ax.
+// `form` (nz > 1): kConeColumns needs Inst::rays_t 1, the others 0.  `zseg`: slices
+// of a block of columns (rounded up to whole lanes) or of a thread's walk (0: the
+// default).  `seen`: seen_slices, the most of the launch's instances (0: all).
+// `zmap` as for launch_sart_ax.
 cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
-                            int view, cudaStream_t st, bool zcol = true, int zseg = 0,
-                            const int *zmap = nullptr);
+                            int view, cudaStream_t st, ConeForm form = kConeVoxels, int zseg = 0,
+                            int seen = 0, const int *zmap = nullptr);
 
 // ---- TV and scalars (kernels_tv.cu) ----
 // FP64 / FP32 TV minimisation on device buffers (reference semantics), in

@@ -1029,35 +1029,43 @@ struct ZColShared {
   int lo[W];                // first detector column
   int count[W];             // detector columns
   int flags[W];             // kZc*
+  int seen[2];              // slices [seen[0], seen[1]) may have pairs
   float2 l[kZcCols * kZcRows][kZcThreads];  // a voxel's chords and their products
   unsigned short list[kZcWarps][32 * kZcCols * kZcRows];  // a warp's z-face pairs
   float acc[32][W + 1], accl[32][W + 1];
 };
 constexpr int kZcOk = 1, kZcWindow = 2, kZcInside = 4, kZcSpecial = 8;
 
-// Launch shape: columns of a block (32 or 8), lanes of a column (32, 16 or
-// 8) and slices of a block.  Lanes: the count that wastes least on the last
-// voxels.  8 columns a block where 32 leave the launch under two blocks per
-// resident slot; slices so that a launch has about four.
+// Launch shape: columns of a block (32 or 8), lanes of a column (32 to 2) and
+// slices of a block, for a launch whose rays cross `seen` of its slices.  Lanes:
+// what gives the least time for those, a voxel costing a tenth more with 8 lanes
+// than with 32 or 16, two thirds more with 4 and three times as much with 2
+// (512^2 x 100: 0.68 ms a view with 16 lanes, 0.71 with 8, 1.02 with 4; x 24 0.18
+// with 8, x 4 0.067 with 4 and 0.077 with 8).  8 columns a block (and 32 lanes)
+// where 32 leave SMs without a block; slices so that a launch has about four
+// blocks per resident slot.  A view of a plan, 32 columns against 8: 128^2 x 48
+// 31 us and 42, x 64 37 and 44, 64^2 x 32 14 and 12.
 struct ZColShape {
   int W, L, seg;
-  int lsh() const { return L == 32 ? 5 : L == 16 ? 4 : 3; }
+  int lsh() const { return L == 32 ? 5 : L == 16 ? 4 : L == 8 ? 3 : L == 4 ? 2 : 1; }
 };
-inline ZColShape zcol_shape(const Dims &d, int batch, int seg) {
+inline ZColShape zcol_shape(const Dims &d, int batch, int seg, int seen) {
   ZColShape s{32, 32, 0};
-  auto padded = [&](int L) { return (d.nz + L - 1) / L * L; };
-  for (int L : {16, 8})
-    if (padded(L) * 20 < padded(s.L) * 19) s.L = L;
   const long long lines = (long long)d.ny * batch;
-  if ((d.nx + 31) / 32 * lines * ((d.nz + 31) / 32) < 152 * 8) {
-    s.W = 8;
-    s.L = 32;
-  }
-  const int chunks = (d.nz + s.L - 1) / s.L;
+  if ((d.nx + 31) / 32 * lines * ((d.nz + 31) / 32) < 152) s.W = 8;
+  // a part of the slices begins anywhere in a group of lanes
+  auto cost = [&](int L) {
+    const int n = seen < d.nz ? seen + L / 2 : (seen + L - 1) / L * L;
+    return (long long)n * (L >= 16 ? 20 : L == 8 ? 22 : L == 4 ? 33 : 60);
+  };
+  for (int L : {16, 8, 4, 2})
+    if (s.W == 32 && cost(L) < cost(s.L)) s.L = L;
+  const int least = std::max(s.L, 8);  // slices of a block
+  const int chunks = (d.nz + least - 1) / least;
   const long long tiles = (d.nx + s.W - 1) / s.W * lines;
   const long long split = std::min<long long>(chunks, (152 * 16 + tiles - 1) / tiles);
-  const long long per = seg > 0 ? (seg + s.L - 1) / s.L : (chunks + split - 1) / split;
-  s.seg = (int)per * s.L;
+  const long long per = seg > 0 ? (seg + least - 1) / least : (chunks + split - 1) / split;
+  s.seg = (int)per * least;
   return s;
 }
 inline dim3 zcol_grid(const Dims &d, int batch, const ZColShape &s) {
@@ -1170,54 +1178,74 @@ __device__ __forceinline__ void atx_zcol_walk(const ViewGeo &G, const Dims &D,
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const float hz = G.dz / 2.0f;
   const long long M = nray(D);
+  int za = zb0, zb = zb1;  // the slices that may have pairs
   if (narrow) {
-    const int c = t % W;
-    ZCol col;
-    int cnt = 0;
-    bool wide = false;
-    col.lo = 0;
-    if (x0 + c < D.nx) {
-      col = zcol_setup(G, D, x0 + c, iy, true);
-      cnt = zcol_count(col);
-      wide = cnt > kZcSlots;
-    }
-    if (t < W && x0 + c < D.nx) {
-      sh.col[c] = make_float4(col.rx, col.ry, col.qmin, col.qmax);
-      sh.tb[c] = col.tb;
-      sh.flags[c] = (col.ok ? kZcOk : 0) | (col.a0 <= col.a1 ? kZcWindow : 0) |
-                    (zcol_shadow_inside(G, D, col, zb0, zb1) ? kZcInside : 0) |
-                    (wide ? kZcSpecial : 0);
-    } else if (t < W) {
-      sh.col[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-      sh.tb[c] = 0.f;
-      sh.flags[c] = kZcInside;
-    }
-    if (t < W) {
-      sh.lo[c] = zcol_first(col, cnt);
-      sh.count[c] = cnt;
-    }
-    __syncthreads();
-    for (int k = t / W; k < cnt && !wide; k += kZcThreads / W) {
-      if (!ASD_IN(col.lo + k, D.na)) continue;
-      const ColFaces f = col_faces(__ldg(tabA + col.lo + k), col.rx, col.ry);
-      sh.pts[k][c] = make_float4(f.p1x, f.p1y, f.p2x, f.p2y);
-      sh.z[k][c] = make_float4(f.n1, f.n2, f.e12, __uint_as_float(f.bits));
-      if (f.bits & kCfMany) atomicOr(&sh.flags[c], kZcSpecial);
+    if (t < 32) {  // the columns' set-up, and their slices
+      int s0 = zb1, s1 = zb0;
+      if (t < W) {
+        ZCol col;
+        int cnt = 0, flags = kZcInside;
+        col.rx = col.ry = col.qmin = col.qmax = col.tb = 0.f;
+        if (x0 + t < D.nx) {
+          col = zcol_setup(G, D, x0 + t, iy, true);
+          cnt = zcol_count(col);
+          flags = (col.ok ? kZcOk : 0) | (col.a0 <= col.a1 ? kZcWindow : 0) |
+                  (zcol_shadow_inside(G, D, col, zb0, zb1) ? kZcInside : 0) |
+                  (cnt > kZcSlots ? kZcSpecial : 0);
+          if (cnt > 0) {
+            zcol_seen(G, D, col, s0, s1);
+            s0 = max(s0, zb0);
+            s1 = min(s1, zb1);
+          }
+        }
+        sh.col[t] = make_float4(col.rx, col.ry, col.qmin, col.qmax);
+        sh.tb[t] = col.tb;
+        sh.flags[t] = flags;
+        sh.lo[t] = zcol_first(col, cnt);
+        sh.count[t] = cnt;
+      }
+      s0 = __reduce_min_sync(0xffffffffu, s0);
+      s1 = __reduce_max_sync(0xffffffffu, s1);
+      if (t == 0) {
+        sh.seen[0] = min(s0, s1);
+        sh.seen[1] = s1;
+      }
     }
     __syncthreads();
+    za = sh.seen[0];
+    zb = sh.seen[1];
+    if (za < zb) {
+      const int c = t % W, cnt = sh.count[c], lo = sh.lo[c];
+      const float4 cd = sh.col[c];
+      for (int k = t / W; k < min(cnt, kZcSlots); k += kZcThreads / W) {
+        if (!ASD_IN(lo + k, D.na)) continue;
+        const ColFaces f = col_faces(__ldg(tabA + lo + k), cd.x, cd.y);
+        sh.pts[k][c] = make_float4(f.p1x, f.p1y, f.p2x, f.p2y);
+        sh.z[k][c] = make_float4(f.n1, f.n2, f.e12, __uint_as_float(f.bits));
+        if (f.bits & kCfMany) atomicOr(&sh.flags[c], kZcSpecial);
+      }
+      __syncthreads();
+    }
+  }
+  // the others' sums are 0
+  const int below = za - zb0, rest = below + (zb1 - zb);
+  for (int v = t; v < rest * W; v += kZcThreads) {
+    const int vz = v / W < below ? zb0 + v / W : zb + (v / W - below), vx = x0 + v % W;
+    const unsigned idx = ((unsigned)vz * D.ny + iy) * D.nx + vx;
+    if (vx < D.nx && ASD_IN(idx, nvox(D))) out(idx, 0.f, 0.f, old(idx));
   }
   // both z faces of a voxel can be hit, and so count without an in-plane
   // face, only if a ray climbs dz within a pixel; less than half of that
   // anywhere on the detector and the question never comes up
   const bool steep = !(D.nb * G.dz_det < G.dz * G.SD);
   const int zl = lane & (L - 1);
-  for (int zc0 = zb0; zc0 < zb1; zc0 += L) {
+  for (int zc0 = za; zc0 < zb; zc0 += L) {
     // this thread's voxels of the chunk: every kZcThreads-th
     constexpr int kMine = W * 32 / kZcThreads;
     auto voxel = [&](int i, unsigned &idx) {
       const int v = t + i * kZcThreads, vz = zc0 + v / W, vx = x0 + v % W;
       idx = ((unsigned)vz * D.ny + iy) * D.nx + vx;
-      return v < W * L && vx < D.nx && vz < zb1 && ASD_IN(idx, nvox(D));
+      return v < W * L && vx < D.nx && vz < zb && ASD_IN(idx, nvox(D));
     };
     // what depends on the lane's height only
     const int iz = zc0 + zl;
@@ -1227,7 +1255,7 @@ __device__ __forceinline__ void atx_zcol_walk(const ViewGeo &G, const Dims &D,
     for (int v0 = warp * 32; v0 < W * L; v0 += kZcThreads) {  // warp-uniform
       const int c = (v0 + lane) >> lsh;
       const int ix = x0 + c;
-      const bool valid = ix < D.nx && iz < zb1;
+      const bool valid = ix < D.nx && iz < zb;
       float acc = 0.f, accl = 0.f;
       if (!narrow) {
         // the per-voxel form over the reference's window
@@ -1334,6 +1362,117 @@ __global__ void __launch_bounds__(kZcThreads, 4)
                    [&](unsigned idx, float acc, float accl, float was) {
                      m[idx] = sart_update(was, beta, acc, sart_norm(accl));
                    });
+}
+
+// ---------------------------------------------------------------------------
+// The same step with a thread per segment of a voxel column, walked down z, the
+// 32 lanes of a warp neighbours along x (Inst::rays_t 0).  What does not depend on
+// z is computed by every thread for its segment, in shared memory slots of its
+// own, so no barrier is needed.  It is the better form of volumes of which a view
+// crosses few slices (cone_form).  Pairs run as one sequence per voxel, rows
+// outer, a warp walking its longest.
+// Grid: x tiles of 32, y tiles of 8 x segments of `seg` slices, instances.
+// ---------------------------------------------------------------------------
+struct ZWalkShared {
+  float4 pts[kZcSlots][kAtxThreads];  // F1, F2 in-plane points
+  float4 z[kZcSlots][kAtxThreads];    // n1, n2, e12, bits
+};
+static_assert(sizeof(ZWalkShared) <= 48 << 10, "static shared memory");
+// The longest of 32, 16, 8 and 4 slices that gives the launch 2^21 threads.
+inline int zwalk_seg(long long voxels) {
+  int seg = 32;
+  while (seg > 4 && voxels / seg < (1LL << 21)) seg /= 2;
+  return seg;
+}
+
+__global__ void __launch_bounds__(kAtxThreads, 4)
+    k_sart_atx_zwalk(const Inst *__restrict__ insts, int view, int seg,
+                     const int *__restrict__ zmap) {
+  __shared__ ZWalkShared sh;
+  pdl_enter();
+  const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
+  if (view >= I.nv || ((volatile int *)&I.s->done)[0]) return;
+  const Dims D = I.d;
+  const int ty = (D.ny + kTileY - 1) / kTileY, sg = blockIdx.y / ty;
+  if ((int)blockIdx.x * kTileX >= D.nx || sg * seg >= D.nz) return;
+  const ViewGeo G = view_of(I, view);
+  const float4 *__restrict__ tabA = I.tabA + (long long)view * D.na;
+  const float4 *__restrict__ tabC = I.tabC;
+  const float *__restrict__ cor = I.cor;
+  float *m = I.m;
+  const bool narrow = !(I.vflags[view] & kViewAxisParallel) && I.s->cor_bad != view + 1;
+  const float beta = I.s->beta_f, hz = G.dz / 2.0f;
+  const int t = threadIdx.x;
+  const int ix = blockIdx.x * kTileX + t % kTileX;
+  const int iy = (blockIdx.y - sg * ty) * kTileY + t / kTileX;
+  const int z0 = sg * seg, z1 = min(z0 + seg, D.nz);
+  const bool valid = ix < D.nx && iy < D.ny;
+  ZCol col;
+  int cA = 0;
+  col.lo = 0;
+  col.rx = col.ry = 0.f;
+  if (valid && narrow) {
+    col = zcol_setup(G, D, ix, iy, true);
+    cA = zcol_count(col);
+    for (int k = 0; k < cA && cA <= kZcSlots; k++) {
+      if (!ASD_IN(col.lo + k, D.na)) continue;
+      const ColFaces f = col_faces(__ldg(tabA + col.lo + k), col.rx, col.ry);
+      sh.pts[k][t] = make_float4(f.p1x, f.p1y, f.p2x, f.p2y);
+      sh.z[k][t] = make_float4(f.n1, f.n2, f.e12, __uint_as_float(f.bits));
+    }
+  }
+  for (int iz = z0; iz < z1; iz++) {
+    const unsigned idx = ((unsigned)iz * D.ny + iy) * D.nx + ix;
+    const bool in = valid && ASD_IN(idx, nvox(D));
+    const float was = in ? m[idx] : 0.f;
+    float acc = 0.f, accl = 0.f;
+    if (!narrow) {
+      // the per-voxel form over the reference's window
+      if (in) {
+        const VoxelWin w = voxel_window(G, D, ix, iy, iz);
+        const float rx = G.cos_phi * (-G.SO) - w.xc, ry = G.sin_phi * (-G.SO) - w.yc;
+        for (int ib = w.b0; ib <= w.b1; ib++)
+          for (int ia = w.a0; ia <= w.a1; ia++) {
+            const long long r = (long long)ib * D.na + ia;
+            if (!(ASD_IN(ia, D.na) && ASD_IN(ib, D.nb))) continue;
+            const float l = chord3_bf(__ldg(tabA + ia), __ldg(tabC + r), __ldg(G.z_det + ib) - 0.0f,
+                                      rx, ry, 0.0f - w.zc, G.dz);
+            acc += l * __ldg(cor + r);
+            accl += l;
+          }
+      }
+    } else {
+      float zc = 0.f;
+      int blo = 0, bhi = -1;
+      const bool has = valid && zcol_rows(G, D, col, iz, zc, blo, bhi);
+      const int cnt = has && blo <= bhi ? cA * (bhi - blo + 1) : 0;
+      const int most = __reduce_max_sync(0xffffffffu, cnt);
+      const float rz = 0.0f - zc;
+      int ka = 0, ib = blo;
+      for (int k = 0; k < most; k++) {
+        const bool on = k < cnt;
+        const int ia = on ? col.lo + ka : 0, r = (on ? ib : 0) * D.na + ia;
+        if (!(ASD_IN(r, nray(D)) && ASD_IN(ia, D.na))) continue;
+        const float4 Cs = __ldg(tabC + r);
+        const float4 p = sh.pts[on ? min(ka, kZcSlots - 1) : 0][t];
+        const float4 q = sh.z[on ? min(ka, kZcSlots - 1) : 0][t];
+        const ColFaces f{p.x, p.y, p.z, p.w, q.x, q.y, q.z, __float_as_uint(q.w)};
+        const float l = cA > kZcSlots || (f.bits & kCfMany)
+                            ? chord3_bf(__ldg(tabA + ia), Cs, 0.0f, col.rx, col.ry, rz, G.dz)
+                            : chord3_col(f, Cs, col.rx, col.ry, rz, hz);
+        const float y = __ldg(cor + r);
+        if (on) {
+          acc += l * y;
+          accl += l;
+        }
+        if (++ka == cA) {
+          ka = 0;
+          ib++;
+        }
+      }
+    }
+    if (in) m[idx] = sart_update(was, beta, acc, sart_norm(accl));
+  }
 }
 
 // Ray tables of one view for the standalone backward step (launcher path), in
@@ -2050,6 +2189,41 @@ bool zcol_fits(const Dims &d) {
   return d.nz > 1 && ((long long)d.na + kZcCols) * d.nb + kZcRows < (1LL << 31);
 }
 
+int seen_slices(const ViewGeo &g, const Dims &d) {
+  const float n = d.nb * g.dz_det * g.SO / (g.SD * g.dz) + 2.0f;
+  return n >= 2.0f && n < (float)d.nz ? (int)n : d.nz;
+}
+
+// The set-up of a voxel column is shared by its crossed slices, and a block of
+// columns waits for it, so the walk is the better form where a view crosses few
+// slices: in launches of more blocks than are resident at once (152 SMs, four
+// each) up to one for every 512 blocks with all slices crossed, and up to 23 with
+// a part of them, whose groups of lanes are not full; in smaller launches up to 5
+// with a part of them.  us a view of a plan, columns and walk, n^2 x nz:
+//   all crossed: 256 x 4 23 and 24, x 8 26 and 32, 512 x 4 67 and 47, x 8 80 and 69,
+//     x 12 117 and 97, x 16 119 and 120, x 32 200 and 235, 128 x 8 12 and 18;
+//   part of them (seen): 256 x 24 (9) 45 and 35, 256 x 64 (21) 64 and 65, 512 x 32
+//     (21) 188 and 173, 512 x 100 (32) 302 and 317, 128 x 32 (5) 18 and 14, 128 x 48
+//     (16) 21 and 26.
+ConeForm cone_form(const Dims &d, int batch, int seen) {
+  if (!zcol_fits(d)) return kConeVoxels;
+  const long long blocks = (long long)((d.nx + 31) / 32) * d.ny * batch;
+  const bool large = blocks > 152 * 4;
+  const bool few = seen < d.nz ? seen < (large ? 24 : 6) : large && 512LL * seen <= blocks;
+  return few ? kConeWalk : kConeColumns;
+}
+
+// One view by itself needs its ray tables first, two launches more.  us a view on
+// device buffers, columns and per voxel, n^2 x nz: 64 x 64 20 and 17, x 128 30 and
+// 33; 128 x 24 26 and 23, x 32 26 and 29, x 64 40 and 56; 256 x 8 28 and 28, x 16 38
+// and 52; 512 x 6 75 and 68, x 8 75 and 92; part of the slices (seen): 256 x 24 (9)
+// 45 and 34, 256 x 64 (8) 44 and 47, 512 x 24 (9) 115 and 126, x 16 (7) 88 and 78.
+bool atx_columns(const ViewGeo &g, const Dims &d) {
+  const int seen = seen_slices(g, d);
+  return zcol_fits(d) && seen >= (seen < d.nz ? 12 : 8) &&
+         (long long)d.nx * d.ny * seen >= 1 << 19;
+}
+
 size_t ray_table_pad(const Dims &d) { return zcol_fits(d) ? (size_t)zcol_pad(d) : 0; }
 
 size_t atx_zcol_scratch_bytes(const Dims &d) {
@@ -2073,7 +2247,7 @@ cudaError_t launch_atx_zcol(float *x, const float *y, float *sc, const ViewGeo &
   if (e == cudaSuccess)
     e = launch_iter(k_view_tab3, dim3((unsigned)((nr + 255) / 256)), dim3(256), st, y, tabA, tabC,
                     yt, flag, g, d);
-  const ZColShape s = zcol_shape(d, 1, 0);
+  const ZColShape s = zcol_shape(d, 1, 0, seen_slices(g, d));
   if (e == cudaSuccess)
     e = launch_iter(s.W == 32 ? k_atx_zcol<32> : k_atx_zcol<8>, zcol_grid(d, 1, s),
                     dim3(kZcThreads), st, x, sc, tabA, tabC, yt, flag, g, d, s.lsh(), s.seg);
@@ -2114,7 +2288,7 @@ cudaError_t launch_ax_siddon(const float *x, float *y, float *sr, const ViewGeo 
 }
 
 cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
-                            int view, cudaStream_t st, bool zcol, int zseg,
+                            int view, cudaStream_t st, ConeForm form, int zseg, int seen,
                             const int *zmap) {
   cudaError_t e;
   // fan beams: the fewest tiles a block (1, 2 or 4) that keep the launch within
@@ -2128,8 +2302,13 @@ cudaError_t launch_sart_atx(const Inst *insts, int batch, const Dims &d,
     tiles *= 2;
     grid = group_grid(d.nx, d.ny, d.nz, batch, tiles);
   }
-  if (d.nz > 1 && zcol) {
-    const ZColShape s = zcol_shape(d, batch, zseg);
+  if (d.nz > 1 && form == kConeWalk) {
+    const int seg = zseg > 0 ? zseg : zwalk_seg((long long)d.nx * d.ny * d.nz * batch);
+    const dim3 g((d.nx + kTileX - 1) / kTileX,
+                 (d.ny + kTileY - 1) / kTileY * ((d.nz + seg - 1) / seg), batch);
+    e = launch_iter(k_sart_atx_zwalk, g, dim3(kAtxThreads), st, insts, view, seg, zmap);
+  } else if (d.nz > 1 && form == kConeColumns) {
+    const ZColShape s = zcol_shape(d, batch, zseg, seen > 0 ? std::min(seen, d.nz) : d.nz);
     e = launch_iter(s.W == 32 ? k_sart_atx_zcol<32> : k_sart_atx_zcol<8>, zcol_grid(d, batch, s),
                     dim3(kZcThreads), st, insts, view, s.lsh(), s.seg, zmap);
   } else if (d.nz > 1 || d.nb > 1)

@@ -60,6 +60,9 @@ extern "C" long long dm_zcol_walk(float *x, const float *yv, float *sc, float c,
           q.rz = 0.0f - zc;
           q.cB = q.own && blo <= bhi ? bhi - blo + 1 : 0;
           q.cA = q.cB > 0 ? count : 0;
+          int s0, s1;  // a voxel with pairs lies in its column's range of slices
+          zcol_seen(G, D, q.col, s0, s1);
+          bad += q.cA > 0 && (iz < s0 || iz >= s1);
           q.r0 = zcol_first_ray(D, zcol_first(q.col, count), blo);
           mA = q.cA > mA ? q.cA : mA;
           mB = q.cA > 0 && q.cB > mB ? q.cB : mB;

@@ -442,7 +442,7 @@ def test_back_projection_waits_for_the_detector_rows(gpu, oracle_mod):
         assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("dims", [(32, 32, 1, 64, 1), (16, 16, 8, 32, 16), (64, 64, 64, 128, 128)])
+@pytest.mark.parametrize("dims", [(32, 32, 1, 64, 1), (16, 16, 8, 32, 16), (96, 96, 96, 160, 160)])
 def test_back_projection_leaves_the_callers_error(gpu, oracle_mod, dims):
     """An error of a call of the caller's own that it has not yet read (here a
     device number that does not exist) is still there after asdpocs_atx_device."""
@@ -489,7 +489,7 @@ def test_back_projection_beside_another_threads_capture(gpu, oracle_mod):
 
     from asd_pocs_mex_cuda_demo_gb300._lib import check, load
 
-    n, na = 64, 128
+    n, na = 96, 160
     N = n ** 3
     g = oracle_mod.gateway_geometry(-0.4, 541.0, 408.0, 541.0 / 949.0 * na / n, 1.0, na, na)
     y = torch.rand(na * na, device="cuda")

@@ -137,3 +137,78 @@ def test_plan_of_columns_beside_the_fan(gpu, case, monkeypatch):
     monkeypatch.setenv("ASDPOCS_CONE_ATX", "voxel")
     want = image()
     assert np.isfinite(want).all() and np.array_equal(got, want)
+
+
+# Sizes at which a plan's columns have 2, 4, 8 and 16 lanes, whole segments of
+# slices that no ray crosses, chunks that begin inside a segment, and the walk's
+# segments end early: nx, ny, nz, na, nb, part of the fan the image fills.
+FEW = [(64, 90, 2, 110, 6, 1.0), (70, 90, 3, 131, 2, 1.3), (64, 160, 7, 150, 15, 1.0),
+       (40, 160, 100, 161, 9, 1.2), (33, 95, 65, 100, 40, 1.0), (40, 100, 40, 80, 1, 1.0),
+       (96, 70, 20, 96, 60, 2.0)]
+
+
+@pytest.mark.parametrize("case", FEW, ids=[str(c[:5]) for c in FEW])
+@pytest.mark.parametrize("bad", [False, True])
+def test_forms_of_the_plan_step_agree(gpu, case, bad, monkeypatch):
+    """A plan's backward step per voxel, in columns and walked, over volumes of
+    which a view crosses few slices or few columns: the same bits, also with a
+    sinogram value that is not finite (whole windows) and for two instances of
+    different sizes in one launch."""
+    nx, ny, nz, na, nb, fill = case
+    phi = np.array([0.0, 33.0, 45.0, 118.0, 290.0])
+    vx = 400.0 / 700.0 * na / max(nx, ny) * fill
+    para = dict(SO=400.0, OD=300.0, vxlsize=vx, nx=nx, ny=ny, nz=nz, na=na, nb=nb, detsize=1.0,
+                phi_vec=phi, maxnumIter=2, numOfgradients=2, alpha=0.002)
+    ps = [para, dict(para, nx=nx - 9, nz=max(2, nz - 5), nb=nb + 2)]
+    rng = np.random.default_rng(nx + nz)
+    Ps = [rng.random(p["na"] * p["nb"] * len(phi)).astype(np.float32) for p in ps]
+    if bad:
+        Ps[0][na * nb + na // 2] = np.inf
+
+    def images(form):
+        monkeypatch.setenv("ASDPOCS_CONE_ATX", form)
+        with pkg.Plan(ps, [phi] * 2) as pl:
+            for k in range(2):
+                pl.set_sinogram(k, Ps[k])
+            pl.reset()
+            pl.run()
+            return [pl.image(k) for k in range(2)]
+
+    want = images("voxel")
+    assert bad or np.isfinite(want[0]).all()
+    assert np.abs(want[1]).max() > 0
+    for form in ("columns", "walk", ""):
+        for a, b in zip(images(form), want):
+            assert np.array_equal(a, b, equal_nan=True), form
+
+
+@pytest.mark.parametrize("dims", [(256, 256, 4, 400, 7), (256, 256, 8, 400, 14),
+                                  (256, 256, 24, 400, 13), (128, 128, 48, 220, 30)])
+def test_device_step_beside_a_few_crossed_slices(gpu, oracle_mod, dims):
+    """asdpocs_atx_device on both sides of its choice of form, against the form
+    it takes under capture."""
+    import torch
+
+    nx, ny, nz, na, nb = dims
+    f = np.float32
+    g = oracle_mod.gateway_geometry(-0.7, 541.0, 408.0, 541.0 / 949.0 * na / nx, 1.0, na, nb)
+    T = lambda a: torch.tensor(np.asarray(a, f), device=gpu)  # noqa: E731
+    y = T(np.random.default_rng(nz).standard_normal(na * nb))
+    yd, zd = T(g["y_det"]), T(g["z_det"])
+    out = [torch.full((nx * ny * nz,), np.nan, device=gpu) for _ in range(4)]
+
+    def call(x, sc):
+        check(load().asdpocs_atx_device(
+            C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr()), C.c_void_p(sc.data_ptr()),
+            g["cos_phi"], g["sin_phi"], C.c_void_p(yd.data_ptr()), C.c_void_p(zd.data_ptr()),
+            g["SO"], g["OD"], g["scale"], g["det"], g["det"], 1.0, nx, ny, nz, na, nb,
+            C.c_void_p(torch.cuda.current_stream().cuda_stream or None)))
+
+    call(out[0], out[1])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(out[2], out[3])
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], out[2]) and torch.equal(out[1], out[3])
+    assert float(out[1].max()) > 0

@@ -47,7 +47,8 @@ def walk(dm, g, y, nx, ny, nz, na, nb, lanes):
 # nx, ny, nz, na, nb, SO, OD, lanes of a column, part of the fan the image fills
 FULL = [(128, 128, 72, 257, 200, 541.0, 408.0, 8, 1.0), (160, 160, 48, 400, 120, 541.0, 408.0, 16, 1.0),
         (64, 64, 40, 48, 40, 100.0, 50.0, 8, 1.6), (48, 48, 9, 120, 30, 60.0, 60.0, 16, 1.7),
-        (24, 24, 40, 40, 120, 20.0, 10.0, 8, 1.0), (40, 40, 16, 30, 1, 541.0, 408.0, 8, 1.0)]
+        (24, 24, 40, 40, 120, 20.0, 10.0, 8, 1.0), (40, 40, 16, 30, 1, 541.0, 408.0, 8, 1.0),
+        (60, 50, 90, 100, 17, 400.0, 300.0, 16, 1.2), (50, 60, 3, 100, 3, 400.0, 300.0, 4, 1.0)]
 
 
 @pytest.mark.parametrize("case", FULL, ids=lambda c: str(c[:5]) + f"-{c[7]}")
