@@ -437,9 +437,11 @@ __device__ __forceinline__ void atx_block_sum(const ViewGeo &G, const Dims &D,
 // with one barrier and no atomics and agrees on the stored rays with another;
 // its fan-beam form is bound by latency, not by the units (1024 blocks of a
 // 512^2 image): 6 blocks per SM 0.70 ms, 5 0.75, 4 without the spills 0.76,
-// 7 0.88.
-template <bool kPlanar>
-__global__ void __launch_bounds__(kAtxThreads, kPlanar ? 6 : 3)
+// 7 0.88.  Detectors so fine that a tile sees more bins than the block stages go
+// per pair and are bound by the units, where the spills cost: 4 blocks (256^2 on
+// 8192 bins 115 us with 6, 90 with 4; 64^2 on 4096 174 and 162).
+template <bool kPlanar, int kBlocks>
+__global__ void __launch_bounds__(kAtxThreads, kBlocks)
     k_atx(float *__restrict__ x, const float *yv, float *__restrict__ sc, ViewGeo G, Dims D) {
   __shared__ AtxShared<kPlanar> sh;
   int ix, iy, iz;
@@ -2169,7 +2171,9 @@ cudaError_t launch_atx(float *x, const float *y, float *sc, const ViewGeo &g,
                        const Dims &d, cudaStream_t st) {
   const dim3 grid = tile_grid(d.nx, d.ny, d.nz, 1);
   const PdlScope scope(!capturing(st));
-  auto k = d.nz == 1 && d.nb == 1 ? k_atx<true> : k_atx<false>;
+  // bins that a tile sees, about: its diagonal at the axis' magnification
+  const bool fine = (kTileX + kTileY / 2) * g.SD > kTabA * g.SO * g.dy_det;
+  auto k = !(d.nz == 1 && d.nb == 1) ? k_atx<false, 3> : fine ? k_atx<true, 4> : k_atx<true, 6>;
   return launch_iter(k, grid, dim3(kAtxThreads), st, x, y, sc, g, d);
 }
 

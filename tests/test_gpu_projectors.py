@@ -525,3 +525,18 @@ def test_back_projection_beside_another_threads_capture(gpu, oracle_mod):
     assert not errors
     assert float(a[0]) == 3.0
     assert torch.equal(out[0], out[2]) and torch.equal(out[1], out[3])
+
+
+@pytest.mark.parametrize("na", [900, 1100, 4096])
+def test_back_projection_on_fine_detectors(gpu, oracle_mod, na):
+    """A 64^2 image on 14, 17 and 64 bins a voxel: blocks that stage their rays,
+    blocks that see more than they can stage, and both launch shapes."""
+    n = 64
+    y = np.random.default_rng(na).standard_normal(na).astype(np.float32)
+    for a in (0.3, 45.0, 200.0):
+        para = dict(SO=9000.0, OD=5000.0, vxlsize=9.0 / 14.0 * na / n, nx=n, ny=n, nz=1, na=na,
+                    nb=1, phi=-a / 180 * np.pi, detsize=1.0)
+        g = oracle_mod.gateway_geometry(para["phi"], 9000.0, 5000.0, para["vxlsize"], 1.0, na, 1)
+        bo, co = oracle_mod.atx(y, g, n, n, 1)
+        b, c = pkg.Atx_cone_gpu(y, para)
+        assert np.array_equal(b, bo) and np.array_equal(c, co), a
