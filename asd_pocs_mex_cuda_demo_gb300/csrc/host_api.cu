@@ -95,7 +95,10 @@ struct Workspace {
 };
 static Workspace g_ws[64];
 
-static int ws_acquire(Workspace *&w, size_t bytes, std::unique_lock<std::mutex> &lk) {
+// `least`, where given: what the caller can do with if the device has no room for
+// `bytes` (w->cap tells).
+static int ws_acquire(Workspace *&w, size_t bytes, std::unique_lock<std::mutex> &lk,
+                      size_t least = 0) {
   int dev = 0;
   ASD_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return set_error(ASDPOCS_ERR_NODEV, "device id");
@@ -106,7 +109,13 @@ static int ws_acquire(Workspace *&w, size_t bytes, std::unique_lock<std::mutex> 
     if (w->buf) cudaFree(w->buf);
     w->buf = nullptr;
     w->cap = 0;
-    ASD_CUDA(cudaMalloc(&w->buf, bytes));
+    cudaError_t e = cudaMalloc(&w->buf, bytes);
+    if (e == cudaErrorMemoryAllocation && least > 0 && least < bytes) {
+      cudaGetLastError();
+      bytes = least;
+      e = cudaMalloc(&w->buf, bytes);
+    }
+    ASD_CUDA(e);
     w->cap = bytes;
   }
   return 0;
@@ -184,10 +193,12 @@ class HostCall {
   bool staged = false;
 
  public:
-  char *dev = nullptr;  // the workspace: inputs, results, scratch
+  char *dev = nullptr;      // the workspace: inputs, results, scratch
+  bool has_scratch = true;  // else the device had no room for it
   // Byte sizes; the offsets of inputs and results are the caller's.
   int begin(size_t in, size_t out, size_t scratch) {
-    if (int e = ws_acquire(w, in + out + scratch, lk)) return e;
+    if (int e = ws_acquire(w, in + out + scratch, lk, in + out)) return e;
+    has_scratch = w->cap >= in + out + scratch;
     dev = (char *)w->buf;
     n_in = in;
     staged = in <= kStageIn && out <= kStageOut;
@@ -484,7 +495,7 @@ int asdpocs_adjoint_check(const float *X, const float *yv, float cos_phi, float 
   const Dims d{nx, ny, nz, na, nb};
   ViewGeo g = with_constants(
       ViewGeo{cos_phi, sin_phi, SO, OD, scale, dy_det, dz_det, dz, nullptr, nullptr});
-  const size_t zs = atx_columns(g, d) ? atx_zcol_scratch_bytes(d) : 0;
+  size_t zs = atx_columns(g, d) ? atx_zcol_scratch_bytes(d) : 0;
   const size_t oX = 0, oY = oX + align256(N * 4), oAx = oY + align256(M * 4),
                oSr = oAx + align256(M * 4), oAty = oSr + align256(M * 4),
                oSc = oAty + align256(N * 4), oA = oSc + align256(N * 4),
@@ -492,7 +503,8 @@ int asdpocs_adjoint_check(const float *X, const float *yv, float cos_phi, float 
                oD = oP + align256((size_t)kDotBlocks * 8), oT = oD + 256, tot = oT + zs;
   Workspace *w;
   std::unique_lock<std::mutex> lk;
-  if (int e = ws_acquire(w, tot, lk)) return e;
+  if (int e = ws_acquire(w, tot, lk, oT)) return e;
+  if (w->cap < tot) zs = 0;  // per voxel
   char *b = (char *)w->buf;
   ASD_CUDA(cudaMemcpyAsync(b + oX, X, N * 4, cudaMemcpyHostToDevice, w->st));
   ASD_CUDA(cudaMemcpyAsync(b + oY, yv, M * 4, cudaMemcpyHostToDevice, w->st));
@@ -549,7 +561,8 @@ static int atx_host(float *X, const float *yv, float *sc, float cos_phi,
                                            (const float *)(c.dev + oB)});
   float *x = (float *)c.out(oX), *sx = (float *)c.out(oS);
   const float *y = (const float *)(c.dev + oY);
-  ASD_CUDA(zs ? launch_atx_zcol(x, y, sx, g, d, c.dev + in + res, c.stream())
+  ASD_CUDA(zs && c.has_scratch
+               ? launch_atx_zcol(x, y, sx, g, d, c.dev + in + res, c.stream())
               : launch_atx(x, y, sx, g, d, c.stream()));
   ASD_CUDA(c.finish({{X, oX, N * 4}, {sc, oS, N * 4}}));
   return 0;
@@ -697,16 +710,18 @@ int asdpocs_tv_device(float *img_d, const float *img_old_d, int nx, int ny,
   if (!img_d) return set_error(ASDPOCS_ERR_ARG, "null pointer");
   if (int e = check_tv_dims(nx, ny, nz)) return e;
   const size_t N = (size_t)nx * ny * nz;
-  const size_t oA = 0, oB = align256(N * 4), oD = oB + align256(N * 4), oS = oD + align256(N * 4),
-               oP = oS + 256, tot = oP + align256(tv_partials_bytes());
+  // three work images, or one and two kernels a step where they do not fit
+  const size_t oS = 0, oP = 256, oA = oP + align256(tv_partials_bytes()),
+               oB = oA + align256(N * 4), oD = oB + align256(N * 4), tot = oD + align256(N * 4);
   Workspace *w;
   std::unique_lock<std::mutex> lk;
-  if (int e = ws_acquire(w, tot, lk)) return e;
+  if (int e = ws_acquire(w, tot, lk, oB)) return e;
   char *b = (char *)w->buf;
+  const bool three = w->cap >= tot;
   cudaStream_t st = (cudaStream_t)stream;
-  ASD_CUDA(tv_minimize_f32(img_d, img_old_d, (float *)(b + oA), (float *)(b + oB),
-                           (float *)(b + oD), (double *)(b + oS), (double *)(b + oP), nx, ny,
-                           nz, alpha, nTVIter, pos, st, true));
+  ASD_CUDA(tv_minimize_f32(img_d, img_old_d, (float *)(b + oA), three ? (float *)(b + oB) : nullptr,
+                           three ? (float *)(b + oD) : nullptr, (double *)(b + oS),
+                           (double *)(b + oP), nx, ny, nz, alpha, nTVIter, pos, st, true));
   // the workspace is reused by the next call: finish before releasing it
   ASD_CUDA(cudaStreamSynchronize(st));
   return 0;

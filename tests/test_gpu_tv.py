@@ -154,3 +154,30 @@ def test_tv3d_fp64_slab_lengths(gpu, oracle_mod, shape):
     img, old = rng.random(shape), rng.random(shape)
     out = pkg.imgTVGradMin3D(img, 0.1, 3, 1, old)
     assert rel_l2(out, oracle_mod.tv(img, 0.1, 3, 1, old)) < 1e-12
+
+
+def test_tv_device_with_room_for_one_work_image(gpu):
+    """A volume whose three work images do not fit what is left of the device's
+    memory: one is enough, as the result of a call with room shows.  An image of
+    1 GiB and 2.2 GiB left."""
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    dims, n = (1024, 1024, 256), 1 << 28
+    g = torch.Generator(gpu).manual_seed(5)
+    a = torch.rand(n, device=gpu, generator=g)
+    b = a.clone()
+    st = torch.cuda.current_stream().cuda_stream
+    torch.cuda.empty_cache()
+    # the workspace gives up what it has first, so leave room for that, too
+    left = (22 << 30) // 10
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device=gpu)
+    try:
+        check(load().asdpocs_tv_device(b.data_ptr(), None, *dims, 0.1, 3, 1, st))
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    check(load().asdpocs_tv_device(a.data_ptr(), None, *dims, 0.1, 3, 1, st))
+    a, b = a.double(), b.double()
+    assert float((a - b).norm() / a.norm()) < 1e-5
