@@ -66,8 +66,8 @@ __device__ __forceinline__ void ax_lane_partial(const RayMarch &R, bool planar, 
     ray_columns_fast<1>(R, lane, 32, ld, ys, ss);
 }
 
-// Cone beams: a warp takes kAxRows neighbouring rows of a detector column,
-// whose rays share their in-plane march.  One 256^3 view of a reconstruction,
+// Cone beams of many rays: a warp takes kAxRows neighbouring rows of a detector
+// column, whose rays share their in-plane march.  One 256^3 view of a reconstruction,
 // 512^2 detector: 283 us with one row a warp, 243 with two, 227 with four,
 // 243 with eight; four rows at 7 blocks per SM (72 registers instead of the
 // 95 it would take; issue 77 %) 206 us, 6 blocks 208, 8 blocks 213.
@@ -105,16 +105,16 @@ __device__ __forceinline__ void ax_rows_sum(const ViewGeo &G, const Dims &D, int
   }
 }
 
-template <bool kVol>
-__global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
+template <bool kByRows>
+__global__ void __launch_bounds__(kAxBlock, kByRows ? kAxRowBlocks : 1)
     k_ax(const float *x, float *__restrict__ y, float *__restrict__ sr, ViewGeo G, Dims D) {
   pdl_enter();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long w = (long long)blockIdx.x * kAxWarps + warp;
-  if (w >= (kVol ? ax_warps3(D) : nray(D))) return;  // the whole warp
+  if (w >= (kByRows ? ax_warps3(D) : nray(D))) return;  // the whole warp
   // plain loads: the previous kernel may write x while this one waits
   auto ld = [&](unsigned i) { return ASD_IN(i, nvox(D)) ? x[i] : 0.f; };
-  if constexpr (kVol) {
+  if constexpr (kByRows) {
     int ia, ib0;
     ax_rows(D, w, ia, ib0);
     float ys[kAxRows], ss[kAxRows];
@@ -535,16 +535,16 @@ __device__ __forceinline__ void ray_slopes(const Inst &I, const ViewGeo &G, cons
 
 // For 3D geometry also writes the view's ray slopes (Inst::tabc_mode: a
 // shared table's writer does so even after its own iterations have ended).
-// Volumes: a warp takes kAxRows rows of a detector column (lane k their k-th
-// ray's value, residual and slopes), else one ray.
-template <bool k3D, bool kVol>
-__global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
+// By rows (ax_by_rows): a warp takes kAxRows rows of a detector column (lane k
+// their k-th ray's value, residual and slopes), else one ray.
+template <bool k3D, bool kByRows>
+__global__ void __launch_bounds__(kAxBlock, kByRows ? kAxRowBlocks : 1)
     k_sart_ax(const Inst *__restrict__ insts, int view, const int *__restrict__ zmap) {
   const Inst &I = insts[zmap ? zmap[blockIdx.z] : blockIdx.z];
   const Dims D = I.d;
   const int lane = threadIdx.x & 31;
   const long long nr = nray(D), w = (long long)blockIdx.x * kAxWarps + (threadIdx.x >> 5);
-  const bool have = view < I.nv && w < (kVol ? ax_warps3(D) : nr);  // the whole warp
+  const bool have = view < I.nv && w < (kByRows ? ax_warps3(D) : nr);  // the whole warp
   ViewGeo G;
   int ia = 0, ib = 0;  // the warp's first ray
   RayMarch R;
@@ -557,36 +557,36 @@ __global__ void __launch_bounds__(kAxBlock, kVol ? kAxRowBlocks : 1)
   // sinogram too: whatever wrote that before the run (a kernel of the caller's
   // may, through asdpocs_plan_sinogram_ptr) is the kernel that view 0 waits for.
   if (have) {
-    if (!kVol) {
+    if (!kByRows) {
       m = I.m;
       // set, if at all, by the kernels between two sweeps
       if (view > 0) done = __ldcg(&I.s->done) != 0;
     }
     G = view_of(I, view);
-    if (kVol) {
+    if (kByRows) {
       ax_rows(D, w, ia, ib);
     } else {
       ia = (int)((unsigned)w % (unsigned)D.na);
       ib = (int)((unsigned)w / (unsigned)D.na);
       R = ax_ray(G, D, ia, ib, planar);
     }
-    own = lane < (kVol ? kAxRows : 1) && ib + lane < D.nb;
+    own = lane < (kByRows ? kAxRows : 1) && ib + lane < D.nb;
     r = (long long)(ib + lane) * D.na + ia;
     if (own && view > 0) p = ray_value(I, view, r, nr);
   }
   pdl_enter();
   if (!have) return;
   if (own && view == 0) p = ray_value(I, view, r, nr);
-  if (kVol || view == 0) done = ((volatile int *)&I.s->done)[0] != 0;
+  if (kByRows || view == 0) done = ((volatile int *)&I.s->done)[0] != 0;
   const bool tabc = k3D && (I.tabc_mode == kTabcShared || (!done && I.tabc_mode == kTabcOwn));
   const long long q = k3D && I.rays_t ? (long long)ia * D.nb + ib + lane : r;
   if (tabc && own) ray_slopes(I, G, D, view, ia, ib + lane, q);
   if (done) return;
   const double dd = own ? ray_squares(I, r, nr) : 0.0;
-  if (kVol) m = I.m;
+  if (kByRows) m = I.m;
   auto ld = [&](unsigned i) { return ASD_IN(i, nvox(D)) ? m[i] : 0.f; };
   float yv, sv;
-  if constexpr (kVol) {
+  if constexpr (kByRows) {
     float ys[kAxRows], ss[kAxRows];
     ax_rows_sum(G, D, ia, ib, ld, ys, ss);
     yv = ys[0];
@@ -2152,9 +2152,19 @@ static bool capturing(cudaStream_t st) {
   return cudaStreamIsCapturing(st, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone;
 }
 
+// Whether a launch of `batch` instances takes kAxRows rays a warp.  One ray each
+// where the warps of all rays are resident at once, or nearly (36 on each of 152
+// SMs): a warp of four is four times as long then and saves nothing.  us a view of
+// a plan, rows and rays: 64^3 on 128 x 16 4.5 and 3.4, x 40 5.3 and 4.4, x 48 5.5
+// and 6.3, 32^3 on 64 x 64 4.1 and 3.6, 128 x 128 x 64 on 256 x 20 7.1 and 5.6, x 24
+// 7.1 and 7.6, 256 x 256 x 64 on 512 x 8 9.5 and 7.8, x 16 11.0 and 11.9.
+static bool ax_by_rows(const Dims &d, int batch) {
+  return d.nz > 1 && d.nb > 2 && (long long)d.na * d.nb * batch > 152 * 36;
+}
+
 // Blocks of the forward kernels that take an instance at a time.
-static unsigned ax_blocks(const Dims &d) {
-  const long long warps = d.nz > 1 ? ax_warps3(d) : (long long)d.na * d.nb;
+static unsigned ax_blocks(const Dims &d, bool rows) {
+  const long long warps = rows ? ax_warps3(d) : (long long)d.na * d.nb;
   return (unsigned)((warps + kAxWarps - 1) / kAxWarps);
 }
 
@@ -2163,8 +2173,9 @@ cudaError_t launch_ax(const float *x, float *y, float *sr, const ViewGeo &g,
   const long long nr = (long long)d.na * d.nb;
   if (nr == 0) return cudaSuccess;
   const PdlScope scope(!capturing(st));
-  auto k = d.nz > 1 ? k_ax<true> : k_ax<false>;
-  return launch_iter(k, dim3(ax_blocks(d)), dim3(kAxBlock), st, x, y, sr, g, d);
+  const bool rows = ax_by_rows(d, 1);
+  auto k = rows ? k_ax<true> : k_ax<false>;
+  return launch_iter(k, dim3(ax_blocks(d, rows)), dim3(kAxBlock), st, x, y, sr, g, d);
 }
 
 cudaError_t launch_atx(float *x, const float *y, float *sc, const ViewGeo &g,
@@ -2262,7 +2273,8 @@ cudaError_t launch_sart_ax(const Inst *insts, int batch, const Dims &d,
                            int view, cudaStream_t st, bool exact, const int *zmap) {
   cudaError_t e;
   const long long nr = (long long)d.na * d.nb;
-  const dim3 grid(ax_blocks(d), 1, batch);
+  const bool rows = ax_by_rows(d, batch);
+  const dim3 grid(ax_blocks(d, rows), 1, batch);
   const int rpw = sid_rays(nr * batch, d);
   const dim3 grid_ex(sid_blocks(nr, rpw), 1, batch);
   const bool p3 = d.nz > 1 || d.nb > 1;
@@ -2272,7 +2284,7 @@ cudaError_t launch_sart_ax(const Inst *insts, int batch, const Dims &d,
     else
       e = launch_iter(k_sart_ax_exact<false>, grid_ex, dim3(kAxBlock), st, insts, view, zmap, rpw);
   } else {
-    if (d.nz > 1)
+    if (rows)
       e = launch_iter(k_sart_ax<true, true>, grid, dim3(kAxBlock), st, insts, view, zmap);
     else if (p3)
       e = launch_iter(k_sart_ax<true, false>, grid, dim3(kAxBlock), st, insts, view, zmap);

@@ -540,3 +540,33 @@ def test_back_projection_on_fine_detectors(gpu, oracle_mod, na):
         bo, co = oracle_mod.atx(y, g, n, n, 1)
         b, c = pkg.Atx_cone_gpu(y, para)
         assert np.array_equal(b, bo) and np.array_equal(c, co), a
+
+
+@pytest.mark.parametrize("dims", [(24, 20, 12, 137, 37), (40, 33, 17, 500, 9), (17, 40, 40, 64, 83)])
+def test_rays_by_rows_equal_rays_alone(gpu, oracle_mod, dims):
+    """A cone-beam Ax of few rays has a warp per ray, of many a warp for four rows
+    of a detector column: a detector's rows give the same bits when more rows lie
+    above them."""
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import check, load
+
+    nx, ny, nz, na, nb = dims
+    more = nb + 5500 // na + 2
+    assert na * nb < 5472 < na * more
+    x = torch.rand(nx * ny * nz, device="cuda", generator=torch.Generator("cuda").manual_seed(na))
+    g = oracle_mod.gateway_geometry(-0.7, 541.0, 408.0, 541.0 / 949.0 * na / max(nx, ny), 1.0, na,
+                                    more)
+    yd, zd = (torch.from_numpy(np.ascontiguousarray(g[k], np.float32)).cuda()
+              for k in ("y_det", "z_det"))
+    zd = zd.roll(-(more - nb) // 2).contiguous()  # the few rows near the middle
+    st = torch.cuda.current_stream().cuda_stream
+    out = []
+    for rows in (nb, more):
+        y, sr = torch.empty(na * rows, device="cuda"), torch.empty(na * rows, device="cuda")
+        check(load().asdpocs_ax_device(x.data_ptr(), y.data_ptr(), sr.data_ptr(), g["cos_phi"],
+                                       g["sin_phi"], yd.data_ptr(), zd.data_ptr(), g["SO"],
+                                       g["OD"], g["scale"], 1.0, nx, ny, nz, na, rows, st))
+        out.append((y[:na * nb], sr[:na * nb]))
+    assert float(out[0][1].max()) > 0
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
