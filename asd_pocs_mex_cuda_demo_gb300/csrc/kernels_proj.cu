@@ -2182,8 +2182,10 @@ cudaError_t launch_atx(float *x, const float *y, float *sc, const ViewGeo &g,
                        const Dims &d, cudaStream_t st) {
   const dim3 grid = tile_grid(d.nx, d.ny, d.nz, 1);
   const PdlScope scope(!capturing(st));
-  // bins that a tile sees, about: its diagonal at the axis' magnification
-  const bool fine = (kTileX + kTileY / 2) * g.SD > kTabA * g.SO * g.dy_det;
+  // bins that a tile sees, about: its diagonal at the magnification of the corner
+  // nearest the source
+  const float corner = 0.5f * sqrtf((float)d.nx * d.nx + (float)d.ny * d.ny);
+  const bool fine = (kTileX + kTileY / 2) * g.SD > kTabA * (g.SO - corner) * g.dy_det;
   auto k = !(d.nz == 1 && d.nb == 1) ? k_atx<false, 3> : fine ? k_atx<true, 4> : k_atx<true, 6>;
   return launch_iter(k, grid, dim3(kAtxThreads), st, x, y, sc, g, d);
 }
