@@ -2230,15 +2230,20 @@ ConeForm cone_form(const Dims &d, int batch, int seen) {
   return few ? kConeWalk : kConeColumns;
 }
 
-// One view by itself needs its ray tables first, two launches more.  us a view on
-// device buffers, columns and per voxel, n^2 x nz: 64 x 64 20 and 17, x 128 30 and
-// 33; 128 x 24 26 and 23, x 32 26 and 29, x 64 40 and 56; 256 x 8 28 and 28, x 16 38
-// and 52; 512 x 6 75 and 68, x 8 75 and 92; part of the slices (seen): 256 x 24 (9)
-// 45 and 34, 256 x 64 (8) 44 and 47, 512 x 24 (9) 115 and 126, x 16 (7) 88 and 78.
+// One view by itself needs its ray tables first, two launches more: about 1.4
+// million pairs of a voxel and a bin (the bins across a voxel at the axis, by the
+// rows).  us a view on device buffers, columns and per voxel, n^2 x nz (million
+// pairs): 64 x 64 (0.8) 20 and 17; 91 x 81 x 70 (1.2) 29 and 25; 98 x 88 x 59 (1.3)
+// 27 and 28; 93 x 83 x 52 (1.6) 28 and 28; 101 x 101 x 48 (1.9) 28 and 37; 128 x 64
+// (3.2) 40 and 56.  Few slices as for a plan: 256 x 8 28 and 28, x 16 38 and 52; 512 x
+// 6 75 and 68, x 8 75 and 92; part of the slices (seen): 256 x 24 (9) 45 and 34, 256
+// x 64 (8) 44 and 47, 512 x 24 (9) 115 and 126, x 16 (7) 88 and 78.
 bool atx_columns(const ViewGeo &g, const Dims &d) {
   const int seen = seen_slices(g, d);
-  return zcol_fits(d) && seen >= (seen < d.nz ? 12 : 8) &&
-         (long long)d.nx * d.ny * seen >= 1 << 19;
+  const float q = g.SD / g.SO;
+  const float pairs = (float)d.nx * d.ny * seen * fmaxf(q / g.dy_det, 1.0f) *
+                      fmaxf(q * g.dz / g.dz_det, 1.0f);
+  return zcol_fits(d) && seen >= (seen < d.nz ? 12 : 8) && pairs >= 1.4e6f;
 }
 
 size_t ray_table_pad(const Dims &d) { return zcol_fits(d) ? (size_t)zcol_pad(d) : 0; }
