@@ -326,12 +326,6 @@ __device__ __forceinline__ bool group_tile(int ny, int nz, int t, int &x0,
   return tyi < ty;
 }
 
-// Index of this block among the blocks of its instance, and their number.
-__device__ __forceinline__ int inst_block() {
-  return blockIdx.x + gridDim.x * blockIdx.y;
-}
-__device__ __forceinline__ int inst_blocks() { return gridDim.x * gridDim.y; }
-
 // Batched kernels run every instance of a plan in one grid sized for its
 // largest instance.  A block keeps the (x, y) position it would have in a
 // grid sized for its own instance alone -- so its tiles, its index among the

@@ -94,7 +94,6 @@ cudaError_t tv_minimize_f32(float *img, const float *img_old, float *work_a, flo
                             bool pdl);
 
 // Per-iteration ASD-POCS steps for a batch (ASD_POCS_cuda.m:137-170).
-cudaError_t launch_iter_begin(const Inst *insts, int batch, cudaStream_t st);
 // `zmap` (device, `batch` entries; null: 0 .. batch - 1): the instances of
 // `insts` a launch covers, as for launch_sart_ax.
 cudaError_t launch_after_sweep(const Inst *insts, int batch, const Dims &d,

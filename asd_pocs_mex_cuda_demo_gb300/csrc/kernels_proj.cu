@@ -15,7 +15,7 @@ namespace asd {
 
 namespace {
 
-constexpr int kAxWarps = 4;             // rays per Ax block
+constexpr int kAxWarps = 4;             // warps per Ax block
 constexpr int kAtxThreads = kTileThreads;
 constexpr int kTabA = 512;              // detector columns staged per block
 constexpr int kTabC = 1536;             // 3D rays staged per block
@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(kAxBlock, kByRows ? kAxRowBlocks : 1)
     ray_out_store(I, &I.s->cor_bad, view, r, q, nr, RayOut{p, dd}, yv * G.scale, sv * G.scale);
 }
 
-// k_sart_ax with the exact projection (siddon_warp_rays): a warp per 32 rays,
+// k_sart_ax with the exact projection (siddon_warp_rays): a warp per `rpw` rays,
 // lane j ray j's residual and normalisation.
 template <bool k3D>
 __global__ void __launch_bounds__(kAxBlock)
@@ -721,7 +721,7 @@ __device__ __forceinline__ ChordPre chord_load(const int *__restrict__ tab, size
 }
 __device__ __forceinline__ float chord_slot(const int *__restrict__ tab, size_t N, unsigned vi,
                                             int k) {
-  return __ldg((const float *)(tab + 2 * N) + (size_t)(k / 2) * 2 * N + 2 * vi + (k & 1));
+  return __ldg((const float *)tab + chord_word(N, vi, k));
 }
 
 // Asks for the chord table of the next view (the first after the last) in the
@@ -731,7 +731,8 @@ __device__ __forceinline__ float chord_slot(const int *__restrict__ tab, size_t 
 // iterations, 6 and 24 slices of 256^2 (9.4 and 38 MB) 2.38 -> 2.24 and 5.76 ->
 // 5.63 ms.  With 84 MB a view the L2 loses lines it still needs (8 slices of
 // 512^2 7.8 -> 9.1 ms), and with 94 MB in all there is nothing to fetch (1.62 ->
-// 1.64 ms).
+// 1.64 ms).  The instances of a launch are taken to be of this one's size: in an
+// uneven plan each decides for itself, and asks for its own table only.
 constexpr size_t kPrefetchMax = (size_t)40 << 20, kPrefetchAll = (size_t)96 << 20;
 __device__ __forceinline__ void prefetch_table(const Inst &I, const Dims &D, int view,
                                                unsigned part, unsigned parts) {
@@ -1722,13 +1723,12 @@ __device__ __forceinline__ void chords_voxel(const ViewGeo &G, const Dims &D,
   const float rx = G.cos_phi * (-G.SO) - w.xc;
   const float ry = G.sin_phi * (-G.SO) - w.yc;
   if (!ASD_IN(vi, N)) return;
-  float *ch = (float *)(tab + 2 * N) + 2 * vi;
   float accl = 0.f;
   for (int ka = 0; ka < cnt; ka++) {
     if (!(ASD_IN(lo + ka, D.na) && ASD_IN(ka, K))) continue;
     const float l = chord_sel<AX>(__ldg(tabA + lo + ka), rx, ry, G.dz);
     accl += l;
-    ch[(size_t)(ka / 2) * 2 * N + (ka & 1)] = l;
+    ((float *)tab)[chord_word(N, vi, ka)] = l;
   }
   ((int2 *)tab)[vi] =
       make_int2(cnt ? (int)(((unsigned)cnt << 24) | (unsigned)(w.b0 * D.na + lo)) : 0,

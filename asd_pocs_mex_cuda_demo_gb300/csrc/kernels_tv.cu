@@ -1582,10 +1582,6 @@ cudaError_t tv_minimize_f32(float *img, const float *img_old, float *wa, float *
                             pos, st, pdl);
 }
 
-cudaError_t launch_iter_begin(const Inst *, int, cudaStream_t) {
-  return cudaSuccess;
-}
-
 cudaError_t launch_after_sweep(const Inst *insts, int batch, const Dims &d,
                                cudaStream_t st, const int *zmap) {
   const dim3 grid = group_grid(d.nx, d.ny, d.nz, batch);
