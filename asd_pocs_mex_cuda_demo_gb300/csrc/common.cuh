@@ -251,7 +251,7 @@ __host__ __device__ inline size_t sino_elem_bytes(int fmt) {
   return fmt == ASDPOCS_STORE_F32 ? 4 : 2;
 }
 
-constexpr int kMaxPartials = 1 << 22;  // blocks per reduction (sanity bound)
+constexpr int kMaxTvTiles = 1 << 22;  // tiles of an image (the TV entry points)
 
 // Inst::tabc_mode.  kTabcOwn: the instance writes its own table while it
 // runs.  Instances sharing geometry share one table: its writer

@@ -249,6 +249,8 @@ static int check_tv_dims(int nx, int ny, int nz) {
                      "image of %d x %d x %d needs %lld tile rows (ceil(ny/8)*nz), over "
                      "the limit of %lld",
                      nx, ny, nz, tile_rows(ny, nz), kMaxGridRows);
+  if ((nx + kTileX - 1LL) / kTileX * tile_rows(ny, nz) > kMaxTvTiles)
+    return cuda_status(cudaErrorInvalidValue, "image of more than 2^22 tiles of 32 x 8");
   return 0;
 }
 

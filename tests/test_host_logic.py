@@ -47,6 +47,13 @@ def test_tv_rejects_images_beyond_one_launch(lib):
         pkg.imgTVGradMin3D(np.zeros((4, 1, 65536)), 0.1, 2, 1)
 
 
+def test_tv_rejects_images_of_more_than_2_22_tiles(lib):
+    """1025 x 4096 tiles of 32 x 8 voxels, refused before device work."""
+    one = np.zeros(1, np.float32)
+    assert lib.asdpocs_tv_device(one.ctypes.data, None, 32769, 32768, 1, 0.1, 0, 0, None) != 0
+    assert b"2^22 tiles" in lib.asdpocs_last_error()
+
+
 def test_bad_dimensions_are_rejected_before_device_work(lib):
     p = dict(PARA, nx=0)
     with pytest.raises(pkg.AsdpocsError, match="dimensions must be positive"):
