@@ -115,7 +115,9 @@ cudaError_t launch_iter(void (*k)(KArgs...), dim3 grid, dim3 block, cudaStream_t
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = pdl_now() ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by a later call too
+  return e;
 }
 
 // ---------------------------------------------------------------------------

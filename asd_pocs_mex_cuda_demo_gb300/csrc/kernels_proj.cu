@@ -2149,7 +2149,9 @@ __global__ void __launch_bounds__(256)
 // A caller's stream that is being captured gets ordinary launches.
 static bool capturing(cudaStream_t st) {
   cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(st, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+  cudaGetLastError();  // the launch that follows reports it
+  return true;
 }
 
 // Whether a launch of `batch` instances takes kAxRows rays a warp.  One ray each

@@ -570,3 +570,28 @@ def test_rays_by_rows_equal_rays_alone(gpu, oracle_mod, dims):
         out.append((y[:na * nb], sr[:na * nb]))
     assert float(out[0][1].max()) > 0
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+def test_refused_launches_leave_no_error_behind(gpu):
+    """A launch that CUDA refuses (an image of 65536 tile rows) is reported by its
+    own call; the next calls, which ask CUDA for its last error, work."""
+    import ctypes
+
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300 import phantoms
+    from asd_pocs_mex_cuda_demo_gb300._lib import AsdpocsError, check, load
+
+    rt = ctypes.CDLL("libcudart.so.13")
+    nx, ny, na = 8, 8 * 65536, 16
+    x, sc = torch.empty(nx * ny, device="cuda"), torch.empty(nx * ny, device="cuda")
+    y, yd, zd = (torch.rand(n, device="cuda") for n in (na, na, 1))
+    with pytest.raises(AsdpocsError, match="invalid"):
+        check(load().asdpocs_atx_device(x.data_ptr(), y.data_ptr(), sc.data_ptr(), 1.0, 0.0,
+                                        yd.data_ptr(), zd.data_ptr(), 4000.0, 2000.0, 1.0, 1.0,
+                                        1.0, 1.0, nx, ny, 1, na, 1,
+                                        torch.cuda.current_stream().cuda_stream))
+    assert rt.cudaPeekAtLastError() == 0
+    para = dict(SO=541.0, OD=408.0, vxlsize=1.0, nx=16, ny=16, nz=1, na=32, nb=1, detsize=1.0,
+                phi_vec=phantoms.views(3), maxnumIter=1, numOfgradients=1)
+    pkg.ASD_POCS_cuda(np.random.default_rng(0).random((32, 3)), para)
