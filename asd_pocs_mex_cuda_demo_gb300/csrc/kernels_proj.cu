@@ -2245,7 +2245,9 @@ bool atx_columns(const ViewGeo &g, const Dims &d) {
   const float q = g.SD / g.SO;
   const float pairs = (float)d.nx * d.ny * seen * fmaxf(q / g.dy_det, 1.0f) *
                       fmaxf(q * g.dz / g.dz_det, 1.0f);
-  return zcol_fits(d) && seen >= (seen < d.nz ? 12 : 8) && pairs >= 1.4e6f;
+  // volumes beyond a launch's rows are refused in either form (launch_atx)
+  return zcol_fits(d) && tile_rows(d.ny, d.nz) <= kMaxGridRows &&
+         seen >= (seen < d.nz ? 12 : 8) && pairs >= 1.4e6f;
 }
 
 size_t ray_table_pad(const Dims &d) { return zcol_fits(d) ? (size_t)zcol_pad(d) : 0; }

@@ -595,3 +595,27 @@ def test_refused_launches_leave_no_error_behind(gpu):
     para = dict(SO=541.0, OD=408.0, vxlsize=1.0, nx=16, ny=16, nz=1, na=32, nb=1, detsize=1.0,
                 phi_vec=phantoms.views(3), maxnumIter=1, numOfgradients=1)
     pkg.ASD_POCS_cuda(np.random.default_rng(0).random((32, 3)), para)
+
+
+def test_back_projection_refuses_volumes_beyond_a_launch(gpu):
+    """A volume of more than 65535 tile rows (ceil(ny / 8) * nz) is refused whichever
+    form its size would take, in a capture or not; one within them is not."""
+    import torch
+
+    from asd_pocs_mex_cuda_demo_gb300._lib import AsdpocsError, check, load
+
+    nx, ny, na, nb = 16, 2048, 64, 64
+    x, sc = torch.empty(nx * ny * 300, device="cuda"), torch.empty(nx * ny * 300, device="cuda")
+    y, yd = torch.rand(na * nb, device="cuda"), torch.arange(na, device="cuda") * 64.0 - 2016.0
+
+    def call(nz):
+        check(load().asdpocs_atx_device(x.data_ptr(), y.data_ptr(), sc.data_ptr(), 1.0, 0.0,
+                                        yd.data_ptr(), yd.data_ptr(), 4000.0, 2000.0, 1.0, 64.0,
+                                        64.0, 1.0, nx, ny, nz, na, nb,
+                                        torch.cuda.current_stream().cuda_stream))
+
+    call(255)
+    for nz in (256, 300):
+        with pytest.raises(AsdpocsError, match="invalid"):
+            call(nz)
+    torch.cuda.synchronize()
