@@ -721,7 +721,7 @@ __device__ __forceinline__ ChordPre chord_load(const int *__restrict__ tab, size
 }
 __device__ __forceinline__ float chord_slot(const int *__restrict__ tab, size_t N, unsigned vi,
                                             int k) {
-  return __ldg((const float *)tab + chord_word(N, vi, k));
+  return __ldg((const float *)(tab + 2 * N) + chord_word(N, vi, k));
 }
 
 // Asks for the chord table of the next view (the first after the last) in the
@@ -994,8 +994,10 @@ __global__ void __launch_bounds__(kAtxThreads) __maxnreg__(kRegs)
 // them: the footprint window's columns and magnification, the shadow's
 // columns and corner magnifications (zcol_setup) and, for each detector
 // column of the shadow, the in-plane part of the x and y face tests
-// (col_faces).  A block computes these once for its W columns, one thread per
-// (column, detector column), and keeps them in shared memory.  Each voxel then
+// (col_faces).  A block computes these once for its W columns, one lane of its
+// first warp per column, then one thread per (column, detector column), and keeps
+// them in shared memory.  It runs over the slices that may have pairs (zcol_seen);
+// the others' sums are 0.  Each voxel then
 // finds its rows (zcol_shadow, or zcol_rows where a window clips the shadow)
 // and evaluates the z parts of its pairs' face tests (col_hits).  Residuals
 // and slopes are stored with the rays of a detector column one after the
@@ -1006,17 +1008,18 @@ __global__ void __launch_bounds__(kAtxThreads) __maxnreg__(kRegs)
 // Most pairs hit the two in-plane faces; the others (about one pair in seven
 // crosses a z face) go to a list of the warp, whose items are then dealt to
 // the lanes, so that a warp runs the z faces about once per voxel and not for
-// every pair.  The chords go through shared memory and are accumulated in the reference's
-// order (rows outer).  Voxels with more pairs, columns with three or more
+// every pair.  The chords go through shared memory and are accumulated in the
+// reference's order (rows outer).  Voxels with more pairs, columns with three or more
 // in-plane hits and shadows wider than kZcSlots take a plain loop, views that
 // do not allow narrowing (an axis-parallel ray, a residual that is not
 // finite) the per-voxel form over the reference's window.
 // Sums pass through a tile of W columns by L voxels, so the image is read and
 // written W voxels at a time.
-// Instruction issue bounds it (80 % of cycles, 816 warp instructions per 32
-// voxels): 0.447 ms for one 256^3 view on a 512^2 detector (ncu), against
-// 0.618 with a thread per segment of a column, which computed the in-plane
-// part once per 8 voxels and the z faces for every pair, and 0.90 per voxel.
+// Instruction issue bounds it (81 % of cycles, 837 warp instructions per 32
+// voxels): 0.451 ms for one 256^3 view on a 512^2 detector (ncu), against
+// 0.618 with a thread per segment of a column (k_sart_atx_zwalk), which computes
+// the in-plane part once per 8 voxels and the z faces for every pair, and 0.90
+// per voxel.
 // Grid: x tiles of W x y x segments of `seg` slices, instances.
 // ---------------------------------------------------------------------------
 constexpr int kZcThreads = 256, kZcWarps = kZcThreads / 32;
@@ -1728,7 +1731,7 @@ __device__ __forceinline__ void chords_voxel(const ViewGeo &G, const Dims &D,
     if (!(ASD_IN(lo + ka, D.na) && ASD_IN(ka, K))) continue;
     const float l = chord_sel<AX>(__ldg(tabA + lo + ka), rx, ry, G.dz);
     accl += l;
-    ((float *)tab)[chord_word(N, vi, ka)] = l;
+    ((float *)(tab + 2 * N))[chord_word(N, (unsigned)vi, ka)] = l;
   }
   ((int2 *)tab)[vi] =
       make_int2(cnt ? (int)(((unsigned)cnt << 24) | (unsigned)(w.b0 * D.na + lo)) : 0,

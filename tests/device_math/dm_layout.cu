@@ -96,8 +96,8 @@ extern "C" int dm_atx_chords(float *x, const float *yv, float *sc, float c, floa
     float sum = 0.f;
     for (int k = 0; k < cnt; k++) {
       const float l = chord_planar_bf(tA[first % na + k], rx, ry, 1.0f);
-      if (chord_word(N, vi, k) >= tab.size()) return -2;
-      tab[chord_word(N, vi, k)] = l;
+      if (2 * N + chord_word(N, (unsigned)vi, k) >= tab.size()) return -2;
+      tab[2 * N + chord_word(N, (unsigned)vi, k)] = l;
       sum += l;
     }
     const int head = cnt << 24 | first;
@@ -109,7 +109,7 @@ extern "C" int dm_atx_chords(float *x, const float *yv, float *sc, float c, floa
     memcpy(&head, &tab[2 * vi], 4);
     float acc = 0.f;
     for (int k = 0; k < (int)((unsigned)head >> 24); k++)
-      acc += tab[chord_word(N, vi, k)] * yv[(head & 0xffffff) + k];
+      acc += tab[2 * N + chord_word(N, (unsigned)vi, k)] * yv[(head & 0xffffff) + k];
     x[vi] = acc * scale;
     sc[vi] = tab[2 * vi + 1] * scale;
   }
