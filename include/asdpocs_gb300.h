@@ -102,7 +102,11 @@ int asdpocs_ax_siddon_device(const float *x_d, float *y_d, float *sr_d, float co
                              int nz, int na, int nb, void *stream);
 
 /* Same computation as Atx_cone_mf_gpu_new on device buffers (x_d, sc_d
- * outputs, y_d input).  Asynchronous. */
+ * outputs, y_d input).  Asynchronous.  Large volumes go by voxel columns, with
+ * ray tables from a memory pool of the library's own that keeps up to 32 MB of
+ * each device mapped until the process ends; while `stream` is being captured,
+ * and where no memory is left, per voxel: the same bits, at less than half the
+ * speed for 256^3 voxels. */
 int asdpocs_atx_device(float *x_d, const float *y_d, float *sc_d,
                        float cos_phi, float sin_phi, const float *y_det_d,
                        const float *z_det_d, float SO, float OD, float scale,
@@ -159,7 +163,9 @@ int imgTVGradMin(const double *img, double *img_out, int rowN, int colN,
 int imgTVGradMin3D(const double *img, double *img_out, int Nx, int Ny, int Nz,
                    double alpha, int nTVIter, int pos, const double *img_old);
 
-/* FP32 device variants of the TV minimisation (in place on img_d). */
+/* FP32 device variant of the TV minimisation (in place on img_d; synchronous).
+ * The library keeps its scratch, the size of three images (of one where three do
+ * not fit, at about half the speed), for the next call on the device. */
 int asdpocs_tv_device(float *img_d, const float *img_old_d, int nx, int ny,
                       int nz, double alpha, int nTVIter, int pos, void *stream);
 
@@ -326,7 +332,8 @@ typedef struct {
   int tv_walk;         /* TV step: bands (2-D) or slabs (3-D) per walk */
   int ax_cols;         /* shared-geometry forward step: columns of loads per round, 1 or 2 */
   int ax_quads;        /* ... and quads of 4 instances per lane, 1 or 2 */
-  int zcol_segment;    /* cone-beam backward step: slices of a block, up to 256 */
+  int zcol_segment;    /* cone-beam backward step: slices of a block of voxel columns (or of
+                        * a thread's walk, in plans of few slices), up to 256 */
   int pdl;             /* programmatic dependent launches: -1 auto (plans on one stream),
                         * 0 off, 1 on */
   double iteration_ms; /* autotune: one iteration with the chosen shapes (device time) */
